@@ -38,14 +38,15 @@ enum Role { R_LAP, R_PA, R_PB, R_SG, R_SS, R_SB, R_COUNT };
 struct Shape {
     int depth = 16;  // slices per tile
     int bps = 0;     // blocks per SM (-1: one block per tile, scheduled by the hardware)
-    int variant = 0; // 0: staging by per-thread cp.async; 1: by TMA tensor copies (kernels that have both)
+    int variant = 0; // bit 0: staging by per-thread cp.async (0) or TMA tensor copies (1); bit 1: tall
+                     // tiles of the smoothing kernel
 };
 struct TileSet {
     Shape shape;
     std::vector<Tile> h;
     Tile* d = nullptr;  // device copy (capacity cap tiles)
     size_t cap = 0;
-    int occ[2] = {1, 1};  // resident blocks per SM of each variant at its registers and shared memory
+    int occ[4] = {1, 1, 1, 1};  // resident blocks per SM of each variant at its registers and shared memory
     int grid = 0;
 };
 // defaults (AUTOTUNE=0), the autotuner's usual choice on the 182x218x182 pair: slices per
@@ -244,9 +245,14 @@ bool has_tma_variant(int r) { return r != R_COUNT; }  // every solver kernel has
 
 // the staging variants kernel r may run with this handle's STAGING and cohort
 std::vector<int> allowed_variants(const fr_handle* h, int r) {
-    if (!has_tma_variant(r) || !h->tma_ok || h->P.staging == 1) return {0};
-    if (h->P.staging == 2) return {1};
-    return {0, 1};
+    std::vector<int> al = {0, 1};
+    if (!has_tma_variant(r) || !h->tma_ok || h->P.staging == 1)
+        al = {0};
+    else if (h->P.staging == 2)
+        al = {1};
+    if (r == R_SS && frg::sob_smooth_has_tall(h->P.smooth_width / 2))
+        for (size_t k = 0, n = al.size(); k < n; ++k) al.push_back(al[k] | 2);
+    return al;
 }
 
 const void* role_fn(const fr_handle* h, int r, int variant = 0) {
@@ -255,7 +261,7 @@ const void* role_fn(const fr_handle* h, int r, int variant = 0) {
         case R_PA: return variant ? (const void*)frg::ref_pass_a_tma_kernel : (const void*)frg::ref_pass_a_kernel;
         case R_PB: return variant ? (const void*)frg::ref_pass_b_staged_kernel : (const void*)frg::ref_pass_b_kernel;
         case R_SG: return variant ? (const void*)frg::sob_grad_tma_kernel : (const void*)frg::sob_grad_kernel;
-        case R_SS: return frg::sob_smooth3_fn(h->P.smooth_width / 2, variant);
+        case R_SS: return frg::sob_smooth3_fn(h->P.smooth_width / 2, variant & 1, variant & 2);
         default: return variant ? (const void*)frg::sob_pass_b_staged_kernel : (const void*)frg::sob_pass_b_kernel;
     }
 }
@@ -272,8 +278,14 @@ size_t role_smem(int r, int variant = 0) {
 }
 
 // threads per block and tile rows of kernel r's variant
-int role_threads(int r, int variant = 0) { return (r == R_PB && variant == 0) ? frg::kPassBThreads : 256; }
-int role_tile_y(int r, int variant = 0) { return (r == R_PB && variant == 0) ? frg::kPassBTileY : frg::kTileY; }
+int role_threads(int r, int variant = 0) {
+    if (r == R_SS) return frg::kSmoothThreads;
+    return (r == R_PB && variant == 0) ? frg::kPassBThreads : 256;
+}
+int role_tile_y(const fr_handle* h, int r, int variant = 0) {
+    if (r == R_SS) return frg::sob_smooth_tile_y(h->P.smooth_width / 2, variant & 2);
+    return (r == R_PB && variant == 0) ? frg::kPassBTileY : frg::kTileY;
+}
 
 typedef std::array<Shape, R_COUNT> Shapes;
 
@@ -281,7 +293,17 @@ Shapes default_shapes(const fr_handle* h) {
     Shapes sh{};
     for (int r = 0; r < R_COUNT; ++r) {
         const std::vector<int> al = allowed_variants(h, r);
-        const int v = al.size() == 1 ? al[0] : kDefaultVariant[r];
+        int want = kDefaultVariant[r];
+        if (r == R_SS) {  // tall smoothing tiles where they still give every SM one (sob_smooth_tile_y)
+            long long tiles = 0;
+            const int ty = frg::sob_smooth_tile_y(h->P.smooth_width / 2, true), d = kDefaultDepth[r];
+            for (const Pair& P : h->hpairs)
+                tiles += (long long)((P.X + frg::kTileX - 1) / frg::kTileX) * ((P.Y + ty - 1) / ty) * ((P.Z + d - 1) / d);
+            if (tiles >= h->num_sms) want |= 2;
+        }
+        int v = al[0];  // what is wanted where it is allowed, else the first that shares its tile height
+        for (int c : al)
+            if (c == want || ((c ^ want) & 2) < ((v ^ want) & 2)) v = c;
         sh[r] = Shape{kDefaultDepth[r], kDefaultPerTile[r] ? -1 : h->ts[r].occ[v], v};
     }
     return sh;
@@ -301,7 +323,7 @@ int build_role(fr_handle* h, int r, Shape sh, cudaStream_t s = 0) {
     for (int p = 0; p < h->npairs; ++p) {
         const Pair& P = h->hpairs[p];
         for (int z0 = 0; z0 < P.Z; z0 += sh.depth)
-            for (int y0 = 0; y0 < P.Y; y0 += role_tile_y(r, sh.variant))
+            for (int y0 = 0; y0 < P.Y; y0 += role_tile_y(h, r, sh.variant))
                 for (int x0 = 0; x0 < P.X; x0 += frg::kTileX) t.h.push_back(make_int4(p, x0, y0, z0));
     }
     if (t.h.size() > t.cap) return fail(h, FR_ERR_STATE, "tile table %d overflows (%zu > %zu)", r, t.h.size(), t.cap);
@@ -403,12 +425,15 @@ int encode_tmaps(fr_handle* h) {
             }
         }
         if (h->P.solver == FR_SOLVER_SOBOLEV) {
-            int wx = 0, rows = 0;
-            frg::sob_smooth_box(h->P.smooth_width / 2, &wx, &rows);
             const cuuint64_t dims[4] = {Xp, Y, Z, 3}, strides[3] = {4 * Xp, 4 * Xp * Y, fstride};
-            const cuuint32_t box[4] = {(cuuint32_t)wx, (cuuint32_t)rows, 1, 3};
-            int rc = encode_map(h, m + frg::TM_SOB_G, h->grad + P.off, 4, dims, strides, box);
-            if (rc != FR_OK) return rc;
+            for (int tall = 0; tall < 2; ++tall) {
+                int wx = 0, rows = 0;
+                frg::sob_smooth_box(h->P.smooth_width / 2, tall, &wx, &rows);
+                const cuuint32_t box[4] = {(cuuint32_t)wx, (cuuint32_t)rows, 1, 1};
+                int rc = encode_map(h, m + (tall ? frg::TM_SOB_G_TALL : frg::TM_SOB_G), h->grad + P.off, 4, dims,
+                                    strides, box);
+                if (rc != FR_OK) return rc;
+            }
         }
     }
     FR_CUDA(h, cudaMemcpy(h->tmaps, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice));
@@ -558,7 +583,7 @@ int setup_cohort(fr_handle* h, const fr_pair* pairs, int n) {
     }
     h->err.clear();  // a cohort whose maps cannot be encoded runs the cp.async variants
     for (int r : active_roles(h))
-        for (int v = 0; v < (has_tma_variant(r) ? 2 : 1); ++v) {
+        for (int v : allowed_variants(h, r)) {
             int occ = 0;
             if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, role_fn(h, r, v), role_threads(r, v),
                                                               role_smem(r, v)) !=
@@ -1613,7 +1638,7 @@ int fr_tile_shape(const fr_handle* h, int k, int* depth, int* blocks_per_sm) {
 int fr_tile_staging(const fr_handle* h, int k, int* tma) {
     if (!h || !tma || k < 0 || k > 2) return FR_ERR_INVALID_ARG;
     if (!h->block) return FR_ERR_STATE;
-    *tma = h->ts[active_roles(h)[k]].shape.variant;
+    *tma = h->ts[active_roles(h)[k]].shape.variant & 1;
     return FR_OK;
 }
 

@@ -16,8 +16,10 @@ enum TmapIndex {
     TM_LAP_PSI = 0,  // psi, 4-D (x, y, z, component), box 40 x 10 x 1 x 3 (Laplacian)
     TM_LAP_T,        // T, 3-D, box 32 x 8 x 1 (Laplacian; the sobolev gradient uses both,
                      // phi living where psi does)
-    TM_SOB_G,        // the sobolev gradient g, 4-D, box (32 + 2 HX) x (8 + 2 R) x 1 x 3 for the
-                     // smoothing radius R (HX = R rounded up to 4)
+    TM_SOB_G,        // the sobolev gradient g, 4-D, box (32 + 2 HX) x (TY + 2 R) x 1 x 1 for the
+                     // smoothing radius R (HX = R rounded up to 4, TY = sob_smooth_tile_y of
+                     // short and of tall tiles)
+    TM_SOB_G_TALL,
     TM_PA_V0,        // pass A: v (buffer 0, 1), 4-D, box 40 x 12 x 1 x 3 (2-voxel halo)
     TM_PA_V1,
     TM_PA_Q0,        // psi_inv (buffer 0, 1), 4-D, box 40 x 10 x 1 x 3

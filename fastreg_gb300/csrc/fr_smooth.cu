@@ -1,0 +1,272 @@
+// fr_smooth.cu -- the sobolev solver's separable Gaussian (x, y, z) fused with the momentum
+// update m = damping * m - step * gs, one launch over the cohort.
+//
+// A warp owns one component of a 32-column x TY-row tile and marches z; a block is the three
+// components of a tile, and its warps never wait on one another.  Per slice the warp stages
+// its own box of g (the rows plus an R halo, columns x0 - HX .. x0 + 31 + HX with HX = R
+// rounded up to 4) in a ring of shared-memory slots, by one TMA tensor copy or by 16-byte
+// cp.async per lane, and then keeps everything else in registers: each lane filters its own
+// column of every staged row along x, filters the results along y from a window of 2R + 2
+// rows, and feeds each row's value into the z filter of that row.
+//
+//   - The z filter is kept as 2R partial sums per row instead of the last 2R + 1 values: the
+//     chain of output slice z is fma(w_2R, y_z+R, ... fma(w_0, y_z-R, 0)), so slice k's value
+//     extends the 2R chains in flight by one tap each and starts a new one, and the shift to
+//     the next chain position is the destination register of the fma.  (A ring of values needs
+//     2R register moves per row and slice.)
+//   - Rows are taken in pairs, so that the taps of all three axes run as packed FP32 pairs
+//     (per lane the same fused multiply-adds as the scalar chain).
+//   - No block barrier and no second shared-memory array: exchanging the x pass through shared
+//     memory between two barriers per slice took 80 million warp instructions on the
+//     182x218x182 pair at radius 3, this takes 36 million: 67 us instead of 94 us (36 bytes per
+//     voxel, 39 us at the copy bandwidth), 274 instead of 403 us on eight pairs of 160x192x160,
+//     214 instead of 231 us at radius 7.
+//
+// What bounds it now: 12 warps per SM (164 registers: the chains of 16 rows) that wait on the
+// fixed latency of dependent multiply-adds (issue slots 50% used), with the shared-memory
+// loads of the x filter (one per tap and row, 36 us of LSU time) and HBM (39 us) close behind.
+//
+// The taps of every output are taken in the order -R..R for each axis, acc = fma(w, v, acc)
+// from 0, with the replicate boundary: slices outside the volume are the clamped slice, and
+// on tiles at an x or y edge the staged box is completed in shared memory (fix_edges).
+#include "fr_common.cuh"
+#include "fr_kernels.h"
+#include "fr_sob.h"
+#include "fr_tma.cuh"
+
+namespace frg {
+namespace {
+
+constexpr int kILP = 2;  // row pairs whose chains are interleaved: radius 2 takes 56 us instead of 62, others the same
+
+template <int R, int TY>
+struct SmoothGeom {
+    static constexpr int K = 2 * R + 1;
+    static constexpr int HX = (R + 3) / 4 * 4, WS = kTileX + 2 * HX, H = TY + 2 * R;
+    static constexpr int BOX = H * WS;                // floats of a staged slice
+    static constexpr int SLOT = (BOX + 31) / 32 * 32;  // slot stride: 128-byte multiple
+    // slots per warp: as many (up to 4) as keep the block's shared memory within 48 KB
+    static constexpr int NS = 3 * (4 * SLOT * 4 + 32) <= 48 * 1024 ? 4 : 3;
+    static_assert(TY % 2 == 0, "rows are taken in pairs");
+    static_assert(3 * (NS * SLOT * 4 + 8 * NS) <= 48 * 1024, "static shared memory");
+};
+
+// The replicate boundary of a staged slice (whole warp): the R columns beyond an x edge take
+// the edge column, then, where rows outside the volume were not staged from the clamped row
+// (TMA fills them with zeros), the R rows beyond a y edge take the edge row.  Only columns
+// and rows that outputs inside the volume read are written; what else the box holds reaches
+// outputs that are never stored.
+template <int R, bool TMA, int TY>
+__device__ __forceinline__ void fix_edges(float* box, int x0, int y0, int X, int Y) {
+    using G = SmoothGeom<R, TY>;
+    if constexpr (R > 0) {
+        const int lane = threadIdx.x & 31;
+        if (x0 == 0) {  // x0 is a multiple of 32, so only the first tile has x = 0 in its halo
+            for (int w = lane; w < G::H * R; w += 32) {
+                float* row = box + (w / R) * G::WS;
+                row[G::HX - R + w % R] = row[G::HX];
+            }
+        }
+        const int hi = X - 1 - x0 + G::HX;  // staged column of x = X - 1
+        if (hi + 1 < G::WS) {
+            for (int w = lane; w < G::H * R; w += 32) {
+                float* row = box + (w / R) * G::WS;
+                const int c = hi + 1 + w % R;
+                if (c < G::WS) row[c] = row[hi];
+            }
+        }
+        if constexpr (TMA) {
+            const int top = R - y0, bottom = Y - 1 - (y0 - R);  // staged rows of y = 0 and y = Y - 1
+            __syncwarp();
+            if (top > 0)
+                for (int w = lane; w < top * G::WS; w += 32) box[w] = box[top * G::WS + w % G::WS];
+            if (bottom + 1 < G::H) {
+                const int end = min(bottom + R, G::H - 1);
+                for (int w = lane; w < (end - bottom) * G::WS; w += 32)
+                    box[(bottom + 1) * G::WS + w] = box[bottom * G::WS + w % G::WS];
+            }
+            // these generic-proxy writes come before the tensor copy that refills the slot
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
+        __syncwarp();
+    }
+}
+
+template <int R, bool TMA, int TY>
+__global__ void __launch_bounds__(kSmoothThreads) sob_smooth3_kernel(SobIterArgs a) {
+    using G = SmoothGeom<R, TY>;
+    constexpr int K = G::K, WS = G::WS, NS = G::NS, NP = TY / 2;
+    __shared__ __align__(128) float rings[3][NS][G::SLOT];
+    __shared__ __align__(8) uint64_t bars[3][NS];
+    const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;  // this warp's component
+    float(*ring)[G::SLOT] = rings[c];
+    uint64_t* full = bars[c];
+    if (TMA) {
+        if (lane == 0) {
+            for (int k = 0; k < NS; ++k) mbar_init(full + k, 1);
+            mbar_fence_init();
+        }
+        __syncwarp();
+    }
+    unsigned phase = 0u;  // TMA: parity of each slot's next completion
+    int issue_slot = 0, slot = 0, pending = 0;  // slots filled and read in order; fills not yet read
+    bool failed = false;
+
+    for (int t = blockIdx.x; t < a.ntiles_s && !failed; t += gridDim.x) {
+        const Tile tl = a.tiles_s[t];
+        if (a.stop[tl.x]) continue;  // uniform over the block
+        const Pair P = a.pairs[tl.x];
+        const int X = P.X, Y = P.Y, Z = P.Z, Xp = P.Xp, XY = P.Xp * P.Y;
+        const int x0 = tl.y, y0 = tl.z, zt0 = tl.w, zt1 = min(tl.w + a.depth_s, Z);
+        const int nsl = (zt1 - zt0) + 2 * R;
+        const bool edge = x0 == 0 || x0 + kTileX - 1 + R > X - 1 || y0 == 0 || y0 + TY - 1 + R > Y - 1;
+        const float* __restrict__ gc = a.g + c * a.NT + P.off;
+        const CUtensorMap* mg = a.tmaps + (long long)tl.x * TM_COUNT + (TY == sob_smooth_tile_y(R, false) ? TM_SOB_G : TM_SOB_G_TALL);
+
+        // cp.async: chunk f = lane + 32 j of the box is (row f / (WS / 4), chunk f % (WS / 4));
+        // its offset inside a slice is fixed for the tile (-1: outside the padded row)
+        constexpr int NF = G::H * (WS / 4), NJ = TMA ? 1 : (NF + 31) / 32;
+        int goff[NJ];
+        if (!TMA) {
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) {
+                const int f = lane + 32 * j, r = f / (WS / 4), x = x0 - G::HX + 4 * (f % (WS / 4));
+                goff[j] = f < NF && x >= 0 && x < Xp ? Xp * min(max(y0 - R + r, 0), Y - 1) + x : -1;
+            }
+        }
+        auto issue = [&](int k) {  // slice k of the tile (z = zt0 - R + k, clamped) into the next slot
+            const int z = min(max(zt0 - R + k, 0), Z - 1);
+            if (TMA) {
+                if (lane == 0) {
+                    mbar_arrive_expect_tx(full + issue_slot, sizeof(float) * G::BOX);
+                    tma_load_4d(ring[issue_slot], mg, x0 - G::HX, y0 - R, z, c, full + issue_slot);
+                }
+            } else {
+                float* dst = ring[issue_slot] + 4 * lane;
+                const float* src = gc + (long long)XY * z;
+#pragma unroll
+                for (int j = 0; j < NJ; ++j)
+                    if (goff[j] >= 0) cp_async16(dst + 128 * j, src + goff[j]);
+            }
+            issue_slot = issue_slot + 1 == NS ? 0 : issue_slot + 1;
+            ++pending;
+        };
+        for (int k = 0; k < NS; ++k) {
+            if (k < nsl) issue(k);
+            if (!TMA) cp_async_commit();
+        }
+        float2 part[NP][R > 0 ? 2 * R : 1];  // the z chains in flight of each row pair
+#pragma unroll
+        for (int p = 0; p < NP; ++p)
+#pragma unroll
+            for (int j = 0; j < (R > 0 ? 2 * R : 1); ++j) part[p][j] = make_float2(0.f, 0.f);
+        const int x = x0 + lane, rows = x < X ? min(Y - y0, TY) : 0;  // rows that this lane stores
+        float* m = a.m + c * a.NT + P.off + (x + Xp * y0) + (long long)XY * (zt0 - 2 * R);
+        for (int k = 0; k < nsl; ++k, m += XY) {
+            const bool store = k >= 2 * R;  // slice zt0 + k - 2R is complete with this one
+            float mo[TY];
+            if (store)
+#pragma unroll
+                for (int r = 0; r < TY; ++r)
+                    if (r < rows) mo[r] = m[Xp * r];
+            if (TMA) {
+                const bool ok = mbar_wait_bounded(full + slot, (phase >> slot) & 1u);
+                if (!__all_sync(0xffffffffu, ok)) {
+                    failed = true;
+                    break;
+                }
+                phase ^= 1u << slot;
+                --pending;
+            } else {
+                cp_async_wait<NS - 1>();
+                __syncwarp();
+            }
+            float* box = ring[slot];
+            if (edge) fix_edges<R, TMA, TY>(box, x0, y0, X, Y);
+            const float* col = box + lane + G::HX - R;
+            float2 ev[G::H / 2], od[G::H / 2];  // x-filtered rows (2 r, 2 r + 1) and (2 r - 1, 2 r)
+            // row pairs in groups of kILP, whose chains are independent
+#pragma unroll
+            for (int r0 = 0; r0 < G::H / 2; r0 += kILP) {
+#pragma unroll
+                for (int q = 0; q < K; ++q)
+#pragma unroll
+                    for (int rp = r0; rp < r0 + kILP && rp < G::H / 2; ++rp)
+                        ev[rp] = __ffma2_rn(make_float2(a.taps[q], a.taps[q]),
+                                            make_float2(col[2 * rp * WS + q], col[(2 * rp + 1) * WS + q]),
+                                            q ? ev[rp] : make_float2(0.f, 0.f));
+#pragma unroll
+                for (int rp = r0; rp < r0 + kILP && rp < G::H / 2; ++rp)
+                    if (rp > 0) od[rp] = make_float2(ev[rp - 1].y, ev[rp].x);
+                // output rows 2 p, 2 p + 1 of p = rp - R: staged rows 2 p .. 2 p + 1 + 2 R
+                float2 v[kILP], o[kILP];
+#pragma unroll
+                for (int q = 0; q < K; ++q)
+#pragma unroll
+                    for (int rp = r0; rp < r0 + kILP && rp < G::H / 2; ++rp) {
+                        if (rp < R) continue;
+                        const int p = rp - R;
+                        v[rp - r0] = __ffma2_rn(make_float2(a.taps[q], a.taps[q]), q & 1 ? od[p + (q + 1) / 2] : ev[p + q / 2],
+                                                q ? v[rp - r0] : make_float2(0.f, 0.f));
+                    }
+#pragma unroll
+                for (int j = 2 * R; j >= 0; --j)
+#pragma unroll
+                    for (int rp = r0; rp < r0 + kILP && rp < G::H / 2; ++rp) {
+                        if (rp < R) continue;
+                        const int p = rp - R;
+                        const float2 n = __ffma2_rn(make_float2(a.taps[j], a.taps[j]), v[rp - r0],
+                                                    j > 0 ? part[p][j > 0 ? j - 1 : 0] : make_float2(0.f, 0.f));
+                        if (j == 2 * R)
+                            o[rp - r0] = n;
+                        else
+                            part[p][j] = n;
+                    }
+                if (store)
+#pragma unroll
+                    for (int rp = r0; rp < r0 + kILP && rp < G::H / 2; ++rp) {
+                        if (rp < R) continue;
+                        const int p = rp - R;
+                        if (2 * p < rows) m[Xp * (2 * p)] = a.damping * mo[2 * p] - a.step * o[rp - r0].x;
+                        if (2 * p + 1 < rows) m[Xp * (2 * p + 1)] = a.damping * mo[2 * p + 1] - a.step * o[rp - r0].y;
+                    }
+            }
+            __syncwarp();  // every lane has read the slot
+            if (k + NS < nsl) issue(k + NS);
+            if (!TMA) cp_async_commit();
+            slot = slot + 1 == NS ? 0 : slot + 1;
+        }
+    }
+    if (TMA && failed && lane == 0) {
+        // the copies that this warp has in flight end (bounded) before its shared memory goes
+        for (; pending > 0; --pending) {
+            mbar_wait_bounded(full + slot, (phase >> slot) & 1u);
+            slot = slot + 1 == NS ? 0 : slot + 1;
+        }
+        atomicOr(a.err, kErrTmaTimeout);
+    }
+}
+
+template <int R>
+const void* smooth_fn(int tma, bool tall) {
+    constexpr int kShort = sob_smooth_tile_y(R, false), kTall = sob_smooth_tile_y(R, true);
+    if (tall) return tma ? (const void*)sob_smooth3_kernel<R, true, kTall> : (const void*)sob_smooth3_kernel<R, false, kTall>;
+    return tma ? (const void*)sob_smooth3_kernel<R, true, kShort> : (const void*)sob_smooth3_kernel<R, false, kShort>;
+}
+
+}  // namespace
+
+const void* sob_smooth3_fn(int radius, int tma, bool tall) {
+    switch (radius) {
+        case 0: return smooth_fn<0>(tma, tall);
+        case 1: return smooth_fn<1>(tma, tall);
+        case 2: return smooth_fn<2>(tma, tall);
+        case 3: return smooth_fn<3>(tma, tall);
+        case 4: return smooth_fn<4>(tma, tall);
+        case 5: return smooth_fn<5>(tma, tall);
+        case 6: return smooth_fn<6>(tma, tall);
+        default: return smooth_fn<7>(tma, tall);
+    }
+}
+
+}  // namespace frg

@@ -1,8 +1,8 @@
 // fr_sob.cu -- kernels of the sobolev solver (see fr_sob.h for the iteration).
 //
 // Launches per iteration: sob_grad_kernel (W, residual, exact trilinear gradient,
-// FP64 data energy), sob_smooth3_kernel (separable Gaussian along x, y, z fused with
-// the momentum update), sob_pass_b_kernel (compositional update, max update norm,
+// FP64 data energy), sob_smooth3_kernel (fr_smooth.cu: separable Gaussian along x, y, z
+// fused with the momentum update), sob_pass_b_kernel (compositional update, max update norm,
 // on-device convergence test).
 #include <cmath>
 
@@ -307,418 +307,6 @@ __global__ void __launch_bounds__(256) sob_grad_tma_kernel(SobIterArgs a) {
     }
 }
 
-// The x pass of one staged slice: the K-tap filter along x of each of its 3 H staged rows
-// (WS columns; column s holds x = x0 - HX + s) into 32 outputs per row of Gx.  Task (row rr,
-// group gq) computes outputs 4 gq .. 4 gq + 3 of row rr from 1 + HX / 2 aligned 16-byte
-// shared-memory loads (one load per tap and output before).  Thread e of the 256 takes
-// tasks e + 256 j, whose group is e & 7 and whose offsets in a staged slice and in Gx do not
-// change within a tile, so they are computed once per tile (init) rather than per slice.
-// On a tile at an x edge the columns beyond the edges hold the edge column's value by the
-// time the x pass reads them (fix_edges: the replicate boundary).  Each output is the chain
-// acc = fma(w_q, g_q, acc), q = 0 .. K - 1.
-template <int R>
-struct SmoothXPass {
-    static constexpr int HX = (R + 3) / 4 * 4, WS = kTileX + 2 * HX, H = kSobTileY + 2 * R, K = 2 * R + 1;
-    static constexpr int NQ = 1 + HX / 2, NV = 4 * NQ;  // loads and values per task
-    static constexpr int NTASK = 3 * H * (kTileX / 4), NJ = (NTASK + 255) / 256;
-    static_assert(HX - R + 3 + K - 1 < NV, "a task's taps lie in its loads");
-    int src[NJ];  // offset of task j's first load in a staged slice (-1: no task j)
-    int dst[NJ];  // offset of its four outputs in Gx
-
-    // row_off(rr): offset in a staged slice of the row that Gx row rr filters
-    template <typename RowOff>
-    __device__ __forceinline__ void init(RowOff row_off) {
-        const int gq = threadIdx.x & 7;
-#pragma unroll
-        for (int j = 0; j < NJ; ++j) {
-            const int task = threadIdx.x + 256 * j, rr = task >> 3;
-            src[j] = task < NTASK ? row_off(rr) + 4 * gq : -1;
-            dst[j] = rr * kTileX + 4 * gq;
-        }
-    }
-
-    __device__ __forceinline__ void run(const SobIterArgs& a, const float* __restrict__ slice,
-                                        float* __restrict__ gx) const {
-#pragma unroll
-        for (int j = 0; j < NJ; ++j) {
-            if (src[j] < 0) continue;
-            const float* p = slice + src[j];
-            float v[NV];
-#pragma unroll
-            for (int u = 0; u < NQ; ++u) {
-                const float4 f = *reinterpret_cast<const float4*>(p + 4 * u);
-                v[4 * u] = f.x;
-                v[4 * u + 1] = f.y;
-                v[4 * u + 2] = f.z;
-                v[4 * u + 3] = f.w;
-            }
-            float out[4];
-#pragma unroll
-            for (int o = 0; o < 4; ++o) {
-                float acc = 0.f;
-#pragma unroll
-                for (int q = 0; q < K; ++q) acc = fmaf(a.taps[q], v[o + HX - R + q], acc);
-                out[o] = acc;
-            }
-            *reinterpret_cast<float4*>(gx + dst[j]) = make_float4(out[0], out[1], out[2], out[3]);
-        }
-    }
-
-    // The replicate boundary written into a staged slice of a tile at an x edge.  Outputs
-    // outside [0, X) are never stored, so only the R staged columns beyond each edge that
-    // outputs inside it read need the edge value: x = -R .. -1 take x = 0's, x = X .. X - 1 + R
-    // take x = X - 1's.  One (row, side, column) item per thread, 3 H * 2 R items (252 at
-    // R = 3); the other staged columns outside the volume keep whatever the copy left there
-    // and reach only outputs that are discarded.  The edge columns are only read, so the
-    // threads need no ordering among themselves; the block barrier that precedes the
-    // slice's x pass orders the writes before it.
-    __device__ __forceinline__ static void fix_edges(float* slice, int x0, int X) {
-        if constexpr (R > 0) {
-            constexpr int NW = 3 * H * 2 * R;
-            const bool left = x0 == 0;        // x0 is a multiple of 32 and HX <= 8
-            const int shi = X - 1 - x0 + HX;  // column of x = X - 1
-#pragma unroll
-            for (int w0 = 0; w0 < NW; w0 += 256) {
-                const int w = w0 + (int)threadIdx.x;
-                if (w < NW) {
-                    const int rr = w / (2 * R), k = w - rr * (2 * R);
-                    float* row = slice + rr * WS;
-                    if (k < R) {
-                        if (left) row[HX - R + k] = row[HX];
-                    } else {
-                        const int c = shi + 1 + (k - R);
-                        if (c < WS) row[c] = row[shi];
-                    }
-                }
-            }
-            // these generic-proxy writes come before the copy that next refills the buffer
-            // (a tensor copy writes through the async proxy)
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        }
-    }
-};
-
-// Separable Gaussian smoothing of g along x, y and z with the replicate boundary,
-// fused with the momentum update m = damping * m - step * gs.  A block owns a 32 x 8
-// column tile and marches z.  Each input slice (the tile's rows plus an R halo, clamped
-// into the volume; columns x0 - HX .. x0 + 31 + HX with HX = R rounded up to 4) is staged
-// in shared memory by 16-byte cp.async NB slices ahead (NB = 3 buffers, 2 for wide
-// kernels, so that the block stays within 48 KB of shared memory).  Per slice step one block
-// barrier separates two independent halves: the x pass of the next slice (shared memory
-// to a double-buffered Gx) and the y pass of this slice (Gx to a per-thread register ring
-// of 2R + 1 slices that the z pass reads).  On tiles at the x edges the R columns beyond
-// each edge are overwritten with the edge column in shared memory between two barriers
-// before the slice's x pass (the replicate boundary; SmoothXPass::fix_edges).  Each tap is
-// one fused multiply-add, acc = fma(w_k, g_k, acc), taken in the order k = -R..R for every
-// axis.  Resident blocks per SM the kernel is held to: as many as its (2R + 1)-slice ring
-// allows without spilling much (5 blocks are 48 registers a thread, 4 are 64, 3 are 85).
-template <int R>
-constexpr int kSmoothMinBlocksCp = R <= 4 ? 5 : 4;
-
-template <int R>
-__global__ void __launch_bounds__(256, kSmoothMinBlocksCp<R>) sob_smooth3_kernel(SobIterArgs a) {
-    constexpr int HX = (R + 3) / 4 * 4;                // staged x halo: whole 16-byte chunks
-    constexpr int WS = kTileX + 2 * HX, C = WS / 4;    // staged row: floats, chunks
-    constexpr int H = kSobTileY + 2 * R, K = 2 * R + 1;
-    constexpr int NB = 4 * (3 * 3 * H * WS + 2 * 3 * H * kTileX) <= 48 * 1024 ? 3 : 2;  // staging buffers
-    constexpr int NF = 3 * H * C;                      // chunks of one staged slice
-    constexpr int NJ = (NF + 255) / 256;               // chunks per thread
-    __shared__ __align__(16) float G[NB][3][H][WS];
-    __shared__ __align__(16) float Gx[2][3][H][kTileX];
-    const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
-
-    for (int t = blockIdx.x; t < a.ntiles_s; t += gridDim.x) {
-        const Tile tl = a.tiles_s[t];
-        if (a.stop[tl.x]) continue;  // uniform over the block
-        const Pair P = a.pairs[tl.x];
-        const int X = P.X, Y = P.Y, Z = P.Z, Xp = P.Xp, XY = P.Xp * P.Y;
-        const long long NT = a.NT;
-        const float* __restrict__ g0 = a.g + P.off;
-        float* m[3] = {a.m + P.off, a.m + NT + P.off, a.m + 2 * NT + P.off};
-        const int x0 = tl.y, y0 = tl.z, zt0 = tl.w, zt1 = min(tl.w + a.depth_s, Z);
-        const int nsl = (zt1 - zt0) + 2 * R;
-        const bool xedge = x0 - R < 0 || x0 + kTileX - 1 + R > X - 1;  // uniform over the block
-
-        // chunk f = tid + 256 j of a staged slice is (component c, row r, chunk k); its
-        // shared-memory offset is 4 f floats and its offset inside a slice of component c
-        // is fixed for the tile (-1: the chunk lies outside the padded row, never read)
-        int goff[NJ];
-#pragma unroll
-        for (int j = 0; j < NJ; ++j) {
-            const int f = tid + 256 * j;
-            goff[j] = -1;
-            if (f < NF) {
-                const int c = f / (H * C), rem = f - c * (H * C), r = rem / C, k = rem - r * C;
-                const int gy = min(max(y0 - R + r, 0), Y - 1), xs = x0 - HX + 4 * k;
-                if (xs >= 0 && xs < Xp) goff[j] = Xp * gy + xs;
-            }
-        }
-        auto stage = [&](int k) {  // staged slice k of the tile (z = zt0 - R + k, clamped)
-            if (k >= nsl) return;
-            const long long zoff = (long long)XY * min(max(zt0 - R + k, 0), Z - 1);
-            float* dst = &G[k % NB][0][0][0];
-#pragma unroll
-            for (int j = 0; j < NJ; ++j) {
-                const int f = tid + 256 * j;
-                if (goff[j] >= 0) cp_async16(dst + 4 * f, g0 + (f / (H * C)) * NT + zoff + goff[j]);
-            }
-        };
-        SmoothXPass<R> xp;  // staged rows are already the clamped rows
-        xp.init([](int rr) { return rr * WS; });
-        auto x_pass = [&](int k) {  // staged slice k -> Gx[k & 1]
-            xp.run(a, &G[k % NB][0][0][0], &Gx[k & 1][0][0][0]);
-        };
-        // on a tile at an x edge: slice k's edge columns, after the barrier that made every
-        // thread's copies of it visible, and a second barrier before its x pass (block-uniform)
-        auto fix_edges = [&](int k) {
-            if (!xedge) return;
-            SmoothXPass<R>::fix_edges(&G[k % NB][0][0][0], x0, X);
-            __syncthreads();
-        };
-
-        // this thread's column; its momentum is loaded one output slice ahead
-        const int x = x0 + tx, y = y0 + ty, col = x + Xp * y;
-        const bool inside = x < X && y < Y;
-        float mv[3] = {0.f, 0.f, 0.f};
-        if (inside)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) mv[c] = m[c][col + XY * zt0];
-
-        float2 ring01[K];  // the z ring of the y-pass results: components 0 and 1 packed, 2
-        float ring2[K];
-        // zeroed: the shift below copies every slot from the first step on, before the slots
-        // near the end are filled, and a copy of an indeterminate value is undefined behaviour
-        // (a build at 48 registers turned it into wrong results)
-#pragma unroll
-        for (int q = 0; q < K; ++q) {
-            ring01[q] = make_float2(0.f, 0.f);
-            ring2[q] = 0.f;
-        }
-        __syncthreads();  // the previous tile is done with G and Gx
-#pragma unroll
-        for (int k = 0; k < NB; ++k) {
-            stage(k);
-            cp_async_commit();
-        }
-        cp_async_wait<NB - 1>();  // slice 0 has landed
-        __syncthreads();
-        fix_edges(0);
-        x_pass(0);
-        for (int k = 0; k < nsl; ++k) {
-            cp_async_wait<NB - 2>();  // slice k + 1 has landed (the later ones may not)
-            __syncthreads();          // ... for every thread; Gx[k & 1] is complete; slice k's buffer
-                                      // and Gx[(k + 1) & 1] are no longer read
-            stage(k + NB);            // into slice k's buffer
-            cp_async_commit();
-            if (k + 1 < nsl) {
-                fix_edges(k + 1);
-                x_pass(k + 1);
-            }
-            // y pass of slice k for this thread's column, pushed into the z ring
-#pragma unroll
-            for (int q = 0; q < K - 1; ++q) {
-                ring01[q] = ring01[q + 1];
-                ring2[q] = ring2[q + 1];
-            }
-            {  // components 0 and 1 as one packed pair: per lane the same fused multiply-adds
-                float2 acc01 = make_float2(0.f, 0.f);
-                float acc2 = 0.f;
-#pragma unroll
-                for (int q = 0; q < K; ++q) {
-                    const float w = a.taps[q];
-                    acc01 = __ffma2_rn(make_float2(w, w),
-                                       make_float2(Gx[k & 1][0][ty + q][tx], Gx[k & 1][1][ty + q][tx]), acc01);
-                    acc2 = fmaf(w, Gx[k & 1][2][ty + q][tx], acc2);
-                }
-                ring01[K - 1] = acc01;
-                ring2[K - 1] = acc2;
-            }
-            // z pass and momentum for slice zt0 + k - 2R once the ring holds its 2R + 1 slices
-            const int zo = zt0 - 2 * R + k;
-            if (k >= 2 * R && inside) {
-                const int i = col + XY * zo;
-                float2 acc01 = make_float2(0.f, 0.f);
-                float acc2 = 0.f;
-#pragma unroll
-                for (int q = 0; q < K; ++q) {
-                    const float w = a.taps[q];
-                    acc01 = __ffma2_rn(make_float2(w, w), ring01[q], acc01);
-                    acc2 = fmaf(w, ring2[q], acc2);
-                }
-                const float accs[3] = {acc01.x, acc01.y, acc2};
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const float acc = accs[c];
-                    const float mo = mv[c];
-                    if (zo + 1 < zt1) mv[c] = m[c][i + XY];  // the next output slice's momentum
-                    m[c][i] = a.damping * mo - a.step * acc;
-                }
-            }
-        }
-        cp_async_wait<0>();
-    }
-}
-
-// The same smoothing with TMA staging: each input slice (3 components of the tile's rows
-// plus an R halo and columns x0 - HX .. x0 + 31 + HX) is one tensor copy, issued by one
-// thread NT - 1 slices ahead into a ring of NT buffers and completed on the buffer's
-// mbarrier.  Rows and slices outside the volume realise the replicate boundary: a slice
-// beyond an end is requested at the clamped z, and the x pass reads, for each staged row,
-// the row of the clamped y (inside the box whenever the tile is inside the volume); along x,
-// the R columns beyond each edge are overwritten with the edge column in shared memory
-// once the slice has landed (SmoothXPass::fix_edges), so the x pass runs without selects.
-// Waits are bounded as in ref_laplacian_tma_kernel.  Held to 5 resident blocks per SM up
-// to R = 4 and 4 above.
-template <int R>
-constexpr int kSmoothMinBlocks = R <= 4 ? 5 : 4;
-
-template <int R>
-__global__ void __launch_bounds__(256, kSmoothMinBlocks<R>) sob_smooth3_tma_kernel(SobIterArgs a) {
-    constexpr int HX = (R + 3) / 4 * 4;
-    constexpr int WS = kTileX + 2 * HX;
-    constexpr int H = kSobTileY + 2 * R, K = 2 * R + 1;
-    constexpr int BOX = 3 * H * WS;                    // floats copied per slice
-    constexpr int BSTRIDE = (BOX + 31) / 32 * 32;      // buffer stride: 128-byte multiple
-    // buffers: as many (up to 4) as keep the block's static shared memory within 48 KB
-    constexpr int NT = 4 * (4 * BSTRIDE + 2 * 3 * H * kTileX) + 32 <= 48 * 1024   ? 4
-                       : 4 * (3 * BSTRIDE + 2 * 3 * H * kTileX) + 24 <= 48 * 1024 ? 3
-                                                                                  : 2;
-    __shared__ __align__(128) float G[NT][BSTRIDE];
-    __shared__ __align__(16) float Gx[2][3][H][kTileX];
-    __shared__ __align__(8) uint64_t full[NT];
-    typedef SliceRing<NT> Ring;
-    const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
-    if (tid == 0) {
-        for (int k = 0; k < NT; ++k) mbar_init(full + k, 1);
-        mbar_fence_init();
-    }
-    __syncthreads();
-    unsigned nbase = 0, issued = 0;
-    bool failed = false;
-
-    for (int t = blockIdx.x; t < a.ntiles_s && !failed; t += gridDim.x) {
-        const Tile tl = a.tiles_s[t];
-        if (a.stop[tl.x]) continue;  // uniform over the block
-        const Pair P = a.pairs[tl.x];
-        const int X = P.X, Y = P.Y, Z = P.Z, Xp = P.Xp, XY = P.Xp * P.Y;
-        const long long NTv = a.NT;
-        float* m[3] = {a.m + P.off, a.m + NTv + P.off, a.m + 2 * NTv + P.off};
-        const CUtensorMap* mg = a.tmaps + (long long)tl.x * TM_COUNT + TM_SOB_G;
-        const int x0 = tl.y, y0 = tl.z, zt0 = tl.w, zt1 = min(tl.w + a.depth_s, Z);
-        const int nsl = (zt1 - zt0) + 2 * R;
-        const bool xedge = x0 - R < 0 || x0 + kTileX - 1 + R > X - 1;  // uniform over the block
-        auto issue = [&](int k) {  // staged slice k of the tile (z = zt0 - R + k, clamped)
-            const unsigned n = nbase + (unsigned)k;
-            uint64_t* bar = full + Ring::slot(n);
-            mbar_arrive_expect_tx(bar, sizeof(float) * BOX);
-            tma_load_4d(&G[Ring::slot(n)][0], mg, x0 - HX, y0 - R, min(max(zt0 - R + k, 0), Z - 1), 0, bar);
-            ++issued;
-        };
-        SmoothXPass<R> xp;  // staged row rr holds row r of component c; the filter reads the clamped row
-        xp.init([&](int rr) {
-            const int c = rr / H, r = rr - c * H;
-            const int rs = min(max(y0 - R + r, 0), Y - 1) - (y0 - R);
-            return (c * H + rs) * WS;
-        });
-        auto x_pass = [&](int k) {  // staged slice k -> Gx[k & 1] (its edge columns already fixed)
-            xp.run(a, &G[Ring::slot(nbase + (unsigned)k)][0], &Gx[k & 1][0][0][0]);
-        };
-        auto fix_edges = [&](int k) {  // after slice k has landed, before the barrier that precedes its x pass
-            if (xedge) SmoothXPass<R>::fix_edges(&G[Ring::slot(nbase + (unsigned)k)][0], x0, X);
-        };
-        auto wait = [&](int k) {
-            return mbar_wait_bounded(full + Ring::slot(nbase + (unsigned)k), Ring::parity(nbase + (unsigned)k));
-        };
-
-        const int x = x0 + tx, y = y0 + ty, col = x + Xp * y;
-        const bool inside = x < X && y < Y;
-        float mv[3] = {0.f, 0.f, 0.f};
-        if (inside)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) mv[c] = m[c][col + XY * zt0];
-
-        float2 ring01[K];  // the z ring of the y-pass results: components 0 and 1 packed, 2
-        float ring2[K];
-        // zeroed: the shift below copies every slot from the first step on, before the slots
-        // near the end are filled, and a copy of an indeterminate value is undefined behaviour
-        // (a build at 48 registers turned it into wrong results)
-#pragma unroll
-        for (int q = 0; q < K; ++q) {
-            ring01[q] = make_float2(0.f, 0.f);
-            ring2[q] = 0.f;
-        }
-        __syncthreads();  // the previous tile is done with G and Gx
-        if (tid == 0) {
-            tma_prefetch_map(mg);
-            for (int k = 0; k < min(NT, nsl); ++k) issue(k);
-        }
-        const bool ok0 = wait(0);  // slice 0 has landed
-        if (ok0) fix_edges(0);
-        if (__syncthreads_or(!ok0)) {
-            failed = true;
-            break;
-        }
-        x_pass(0);
-        for (int k = 0; k < nsl; ++k) {
-            const bool ok = k + 1 < nsl ? wait(k + 1) : true;  // slice k + 1 has landed
-            if (ok && k + 1 < nsl) fix_edges(k + 1);           // nobody reads its buffer before the barrier
-            // every thread is past step k - 1: Gx[k & 1] is complete, slice k's buffer and
-            // Gx[(k + 1) & 1] are no longer read, slice k + 1's edge columns are written; and
-            // the block agrees on the waits
-            if (__syncthreads_or(!ok)) {
-                failed = true;
-                break;
-            }
-            if (tid == 0 && k + NT < nsl) issue(k + NT);  // into slice k's buffer
-            if (k + 1 < nsl) x_pass(k + 1);
-#pragma unroll
-            for (int q = 0; q < K - 1; ++q) {
-                ring01[q] = ring01[q + 1];
-                ring2[q] = ring2[q + 1];
-            }
-            {  // components 0 and 1 as one packed pair: per lane the same fused multiply-adds
-                float2 acc01 = make_float2(0.f, 0.f);
-                float acc2 = 0.f;
-#pragma unroll
-                for (int q = 0; q < K; ++q) {
-                    const float w = a.taps[q];
-                    acc01 = __ffma2_rn(make_float2(w, w),
-                                       make_float2(Gx[k & 1][0][ty + q][tx], Gx[k & 1][1][ty + q][tx]), acc01);
-                    acc2 = fmaf(w, Gx[k & 1][2][ty + q][tx], acc2);
-                }
-                ring01[K - 1] = acc01;
-                ring2[K - 1] = acc2;
-            }
-            const int zo = zt0 - 2 * R + k;
-            if (k >= 2 * R && inside) {
-                const int i = col + XY * zo;
-                float2 acc01 = make_float2(0.f, 0.f);
-                float acc2 = 0.f;
-#pragma unroll
-                for (int q = 0; q < K; ++q) {
-                    const float w = a.taps[q];
-                    acc01 = __ffma2_rn(make_float2(w, w), ring01[q], acc01);
-                    acc2 = fmaf(w, ring2[q], acc2);
-                }
-                const float accs[3] = {acc01.x, acc01.y, acc2};
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const float acc = accs[c];
-                    const float mo = mv[c];
-                    if (zo + 1 < zt1) mv[c] = m[c][i + XY];
-                    m[c][i] = a.damping * mo - a.step * acc;
-                }
-            }
-        }
-        nbase += (unsigned)nsl;
-    }
-    if (failed && tid == 0) {
-        for (unsigned n = (issued > (unsigned)NT ? issued - NT : 0u); n < issued; ++n)
-            mbar_wait_bounded(full + Ring::slot(n), Ring::parity(n));
-        atomicOr(a.err, kErrTmaTimeout);
-    }
-}
-
 // phi += m o phi with the max update norm.  Held to 48 registers for 5 resident blocks
 // per SM (0.098 against 0.101 ms with 63 registers and 4 blocks): the kernel waits on its
 // corner loads, and more resident warps keep more of them in flight.
@@ -976,7 +564,7 @@ cudaError_t launch_sob_iter(const SobIterArgs& a, const int* grids, const int* v
     if (ev) cudaEventRecord(ev[1], s);
     {
         void* args[1] = {const_cast<SobIterArgs*>(&a)};
-        cudaLaunchKernel(sob_smooth3_fn(a.radius, variants[1]), dim3(grids[1]), dim3(256), args, 0, s);
+        cudaLaunchKernel(sob_smooth3_fn(a.radius, variants[1] & 1, variants[1] & 2), dim3(grids[1]), dim3(kSmoothThreads), args, 0, s);
     }
     if (ev) cudaEventRecord(ev[2], s);
     if (variants[2])
@@ -985,31 +573,6 @@ cudaError_t launch_sob_iter(const SobIterArgs& a, const int* grids, const int* v
         sob_pass_b_kernel<<<grids[2], 256, 0, s>>>(a);
     if (ev) cudaEventRecord(ev[3], s);
     return cudaGetLastError();
-}
-
-const void* sob_smooth3_fn(int radius, int variant) {
-    if (variant) {
-        switch (radius) {
-            case 0: return (const void*)sob_smooth3_tma_kernel<0>;
-            case 1: return (const void*)sob_smooth3_tma_kernel<1>;
-            case 2: return (const void*)sob_smooth3_tma_kernel<2>;
-            case 3: return (const void*)sob_smooth3_tma_kernel<3>;
-            case 4: return (const void*)sob_smooth3_tma_kernel<4>;
-            case 5: return (const void*)sob_smooth3_tma_kernel<5>;
-            case 6: return (const void*)sob_smooth3_tma_kernel<6>;
-            default: return (const void*)sob_smooth3_tma_kernel<7>;
-        }
-    }
-    switch (radius) {
-        case 0: return (const void*)sob_smooth3_kernel<0>;
-        case 1: return (const void*)sob_smooth3_kernel<1>;
-        case 2: return (const void*)sob_smooth3_kernel<2>;
-        case 3: return (const void*)sob_smooth3_kernel<3>;
-        case 4: return (const void*)sob_smooth3_kernel<4>;
-        case 5: return (const void*)sob_smooth3_kernel<5>;
-        case 6: return (const void*)sob_smooth3_kernel<6>;
-        default: return (const void*)sob_smooth3_kernel<7>;
-    }
 }
 
 }  // namespace frg

@@ -22,12 +22,20 @@
 namespace frg {
 
 constexpr int kMaxSmoothWidth = 15;
-constexpr int kSobTileY = 8;
-static_assert(kSobTileY == kTileY, "tile extents must agree");
+
+// The smoothing kernel (fr_smooth.cu): threads per block, and the rows of its 32-column
+// tiles.  Tall tiles filter fewer halo rows, short ones give small volumes more warps; the
+// autotuner times both.  On the 182x218x182 pair 16 rows take 67 us and 8 rows 77 us at
+// radius 3 (56 and 62 us at radius 2); 12 rows 87 us and 8 rows 94 us at radius 4.  On the 64^3
+// pair 16 rows take 15.8 us and 8 rows 13.9 us.  From radius 5 the chains of 8 rows fill the
+// registers (12 rows at radius 7: 227 us, 8 rows 214 us).
+constexpr int kSmoothThreads = 96;
+constexpr int sob_smooth_tile_y(int radius, bool tall) { return !tall || radius > 4 ? 8 : radius == 4 ? 12 : 16; }
+constexpr bool sob_smooth_has_tall(int radius) { return sob_smooth_tile_y(radius, true) != sob_smooth_tile_y(radius, false); }
 
 struct SobIterArgs {
     const Pair* pairs;
-    // each kernel's own table of 32 x 8 x depth tiles: gradient, smoothing, update
+    // each kernel's own table of 32 x 8 x depth tiles (smoothing: its own rows)
     const Tile* tiles_g;
     int ntiles_g, depth_g;
     const Tile* tiles_s;
@@ -64,17 +72,18 @@ size_t sob_grad_smem_bytes();  // dynamic shared memory of sob_grad_kernel
 __global__ void sob_grad_kernel(SobIterArgs a);
 size_t sob_grad_tma_smem_bytes();  // dynamic shared memory of sob_grad_tma_kernel
 __global__ void sob_grad_tma_kernel(SobIterArgs a);
-// the smoothing kernel instance for a radius and staging variant (1: TMA)
-const void* sob_smooth3_fn(int radius, int variant = 0);
-// box of the smoothing kernel's staged slice for radius R: x extent, rows
-inline void sob_smooth_box(int R, int* wx, int* rows) {
+// the smoothing kernel instance for a radius, staging variant (1: TMA) and tile height
+const void* sob_smooth3_fn(int radius, int tma, bool tall);
+// box of one component of the smoothing kernel's staged slice for radius R: x extent, rows
+inline void sob_smooth_box(int R, bool tall, int* wx, int* rows) {
     *wx = kTileX + 2 * ((R + 3) / 4 * 4);
-    *rows = kSobTileY + 2 * R;
+    *rows = sob_smooth_tile_y(R, tall) + 2 * R;
 }
 __global__ void sob_pass_b_kernel(SobIterArgs a);
 __global__ void sob_pass_b_staged_kernel(SobIterArgs a);
 
-// grids: {grad, smooth, pass_b}; variants: staging of {grad, smooth, pass_b} (1: TMA); with `ev`
+// grids: {grad, smooth, pass_b}; variants: of {grad, smooth, pass_b} (bit 0: TMA
+// staging, bit 1 of smooth: tall tiles); with `ev`
 // (4 events) each launch is bracketed
 cudaError_t launch_sob_iter(const SobIterArgs& a, const int* grids, const int* variants, cudaStream_t s,
                             cudaEvent_t* ev = nullptr);

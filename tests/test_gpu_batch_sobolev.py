@@ -203,3 +203,21 @@ def test_batched_convergence_and_keep_state(cuda, solver):
         assert fr.stats(pair=k).iterations == o2["iterations"]
         assert_bitexact(fr.get_field(N.FR_FIELD_PSI, pair=k).cpu().numpy(), o2["psi"], f"pair {k} psi, 2nd call")
         assert_bitexact(bufs[k][2].cpu().numpy(), o2["out_S"], f"pair {k} S o psi, 2nd call")
+
+
+@pytest.mark.parametrize("staging", [1, 2])
+@pytest.mark.parametrize("width", [1, 3, 5, 7, 9, 11])
+@pytest.mark.parametrize("dims", [(33, 17, 9), (101, 163, 161)])
+def test_smoothing_tile_heights(cuda, dims, width, staging):
+    """AUTOTUNE=0 smooths a small volume in short tiles and one with a tile for every SM in
+    tall ones (radius 4 and below); sizes one past a tile's columns and rows, and a
+    last tile that is nearly empty, with either staging, give the oracle's bits."""
+    d = images(dims, 1900 + width)
+    P = Params(volume_dims=dims, no_labels=4, max_iter=3, solver="sobolev", smooth_sigma=0.4 + 0.3 * width,
+               smooth_width=width, damping=0.9, step=0.5, staging=staging, autotune=0)
+    fr = FastReg(P)
+    fr(*(_to(cuda, d[k]) for k in ("T", "labT", "S", "labS")))
+    o = O.sob_register(P, d["T"], d["S"])
+    assert_bitexact(fr.get_field(N.FR_FIELD_PSI).cpu().numpy(), o["phi"], f"phi (width {width})")
+    assert_bitexact(fr.get_field(N.FR_FIELD_V).cpu().numpy(), o["m"], f"momentum (width {width})")
+    fr.close()
