@@ -102,8 +102,7 @@ struct fr_handle {
     int trace_cap = 0;  // iterations the trace array holds
 
     // sobolev-mode scratch
-    float* grad = nullptr;  // unsmoothed gradient / smoothing temporaries (3 planes x 2)
-    double* sob_energy = nullptr;
+    float* grad = nullptr;  // unsmoothed gradient (3 planes)
 
     // launch shape of the I/O kernels
     int grid_io = 0;
@@ -260,7 +259,7 @@ const void* role_fn(const fr_handle* h, int r, int variant = 0) {
         case R_LAP: return variant ? (const void*)frg::ref_laplacian_tma_kernel : (const void*)frg::ref_laplacian_kernel;
         case R_PA: return variant ? (const void*)frg::ref_pass_a_tma_kernel : (const void*)frg::ref_pass_a_kernel;
         case R_PB: return variant ? (const void*)frg::ref_pass_b_staged_kernel : (const void*)frg::ref_pass_b_kernel;
-        case R_SG: return variant ? (const void*)frg::sob_grad_tma_kernel : (const void*)frg::sob_grad_kernel;
+        case R_SG: return frg::sob_grad_fn(variant);
         case R_SS: return frg::sob_smooth3_fn(h->P.smooth_width / 2, variant & 1, variant & 2);
         default: return variant ? (const void*)frg::sob_pass_b_staged_kernel : (const void*)frg::sob_pass_b_kernel;
     }
@@ -270,7 +269,7 @@ size_t role_smem(int r, int variant = 0) {
     switch (r) {
         case R_LAP: return variant ? frg::ref_laplacian_tma_smem_bytes() : frg::ref_laplacian_smem_bytes();
         case R_PA: return variant ? frg::ref_pass_a_tma_smem_bytes() : frg::ref_pass_a_smem_bytes();
-        case R_SG: return variant ? frg::sob_grad_tma_smem_bytes() : frg::sob_grad_smem_bytes();
+        case R_SG: return frg::sob_grad_smem_bytes();
         case R_PB:
         case R_SB: return variant ? frg::gather_staged_smem_bytes() : 0;
         default: return 0;
@@ -279,6 +278,7 @@ size_t role_smem(int r, int variant = 0) {
 
 // threads per block and tile rows of kernel r's variant
 int role_threads(int r, int variant = 0) {
+    if (r == R_SG) return frg::sob_grad_threads(variant);
     if (r == R_SS) return frg::kSmoothThreads;
     return (r == R_PB && variant == 0) ? frg::kPassBThreads : 256;
 }
@@ -389,16 +389,12 @@ int encode_tmaps(fr_handle* h) {
         const Pair& P = h->hpairs[p];
         const cuuint64_t Xp = P.Xp, Y = P.Y, Z = P.Z;
         CUtensorMap* m = maps.data() + (size_t)p * frg::TM_COUNT;
-        {
-            const cuuint64_t dims[4] = {Xp, Y, Z, 3}, strides[3] = {4 * Xp, 4 * Xp * Y, fstride};
-            const cuuint32_t box[4] = {40, 10, 1, 3};
-            int rc = encode_map(h, m + frg::TM_LAP_PSI, h->psi + P.off, 4, dims, strides, box);
-            if (rc != FR_OK) return rc;
-        }
-        {
-            const cuuint64_t dims[3] = {Xp, Y, Z}, strides[2] = {4 * Xp, 4 * Xp * Y};
-            const cuuint32_t box[3] = {32, 8, 1};
-            int rc = encode_map(h, m + frg::TM_LAP_T, h->T + P.off, 3, dims, strides, box);
+        {  // psi and T: the Laplacian and the sobolev gradient
+            const cuuint64_t d4[4] = {Xp, Y, Z, 3}, s4[3] = {4 * Xp, 4 * Xp * Y, fstride};
+            const cuuint64_t d3[3] = {Xp, Y, Z}, s3[2] = {4 * Xp, 4 * Xp * Y};
+            const cuuint32_t b4[4] = {40, 10, 1, 3}, b3[3] = {32, 8, 1};
+            int rc = encode_map(h, m + frg::TM_LAP_PSI, h->psi + P.off, 4, d4, s4, b4);
+            if (rc == FR_OK) rc = encode_map(h, m + frg::TM_LAP_T, h->T + P.off, 3, d3, s3, b3);
             if (rc != FR_OK) return rc;
         }
         if (h->P.solver == FR_SOLVER_REFERENCE) {  // pass A's v, psi_inv, rho (both buffers) and S
@@ -521,7 +517,6 @@ int setup_cohort(fr_handle* h, const fr_pair* pairs, int n) {
         h->rho[0] = h->rho[1] = h->pinv[0] = h->pinv[1] = nullptr;
         h->LT = nullptr;
         add((void**)&h->grad, sizeof(float) * 3 * NT);
-        add((void**)&h->sob_energy, sizeof(double) * (size_t)n * want_trace);
     }
     add((void**)&h->stop, sizeof(int) * n);
     add((void**)&h->keys, sizeof(unsigned long long) * n);
@@ -700,7 +695,6 @@ frg::SobIterArgs sob_args(fr_handle* h, int iter) {
     a.stop = h->stop;
     a.keys = h->keys;
     a.trace = h->trace;
-    a.energy = h->sob_energy;
     a.counter = h->counter;
     a.tmaps = h->tmaps;
     a.err = h->dev_err;
@@ -1054,8 +1048,6 @@ int begin(fr_handle* h, const fr_pair* pairs, int n, cudaStream_t s) {
     FR_CUDA(h, cudaMemsetAsync(h->dev_err, 0, sizeof(unsigned int), s));
     FR_CUDA(h, cudaMemsetAsync(h->keys, 0, sizeof(unsigned long long) * n, s));
     FR_CUDA(h, cudaMemsetAsync(h->trace, 0, sizeof(unsigned long long) * n * (size_t)h->trace_cap, s));
-    if (h->sob_energy)
-        FR_CUDA(h, cudaMemsetAsync(h->sob_energy, 0, sizeof(double) * n * (size_t)h->trace_cap, s));
     frg::IoArgs a = io_args(h);
     frg::pack_init_kernel<<<h->grid_io, 256, 0, s>>>(a);
     FR_LAUNCHED(h);

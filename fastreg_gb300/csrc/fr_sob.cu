@@ -1,10 +1,11 @@
 // fr_sob.cu -- kernels of the sobolev solver (see fr_sob.h for the iteration).
 //
-// Launches per iteration: sob_grad_kernel (W, residual, exact trilinear gradient,
-// FP64 data energy), sob_smooth3_kernel (fr_smooth.cu: separable Gaussian along x, y, z
+// Launches per iteration: sob_grad_kernel (W, residual, exact trilinear gradient, graph
+// Laplacian), sob_smooth3_kernel (fr_smooth.cu: separable Gaussian along x, y, z
 // fused with the momentum update), sob_pass_b_kernel (compositional update, max update norm,
 // on-device convergence test).
 #include <cmath>
+#include <type_traits>
 
 #include "fr_common.cuh"
 #include "fr_kernels.h"
@@ -25,10 +26,10 @@ void gaussian_taps(float sigma, int width, float* taps) {
 }
 
 // Cell for the sobolev solver: clamp to [0, dim-1], floor clamped to dim-2 so that
-// both corners of every axis are inside the grid; clamped[axis] marks positions that
-// were outside [0, dim-1] (their derivative along that axis is 0).
+// both corners of every axis are inside the grid; in_x, in_y, in_z: the position was not
+// clamped (a clamped axis has derivative 0).
 struct SobCell {
-    long long base;
+    int base;
     int gx, gy, gz;
     float a, b, c;
     bool in_x, in_y, in_z;
@@ -39,246 +40,211 @@ __device__ __forceinline__ SobCell sob_locate(const Pair& P, float px, float py,
     const float cx = fminf(fmaxf(0.f, px), (float)(P.X - 1));
     const float cy = fminf(fmaxf(0.f, py), (float)(P.Y - 1));
     const float cz = fminf(fmaxf(0.f, pz), (float)(P.Z - 1));
-    const int gx = min((int)floorf(cx), P.X - 2);
-    const int gy = min((int)floorf(cy), P.Y - 2);
-    const int gz = min((int)floorf(cz), P.Z - 2);
-    s.a = cx - (float)gx;
-    s.b = cy - (float)gy;
-    s.c = cz - (float)gz;
-    s.in_x = px >= 0.f && px <= (float)(P.X - 1);
-    s.in_y = py >= 0.f && py <= (float)(P.Y - 1);
-    s.in_z = pz >= 0.f && pz <= (float)(P.Z - 1);
-    s.gx = gx;
-    s.gy = gy;
-    s.gz = gz;
-    s.base = lin(P, gx, gy, gz);
+    s.gx = min((int)floorf(cx), P.X - 2);
+    s.gy = min((int)floorf(cy), P.Y - 2);
+    s.gz = min((int)floorf(cz), P.Z - 2);
+    s.a = cx - (float)s.gx;
+    s.b = cy - (float)s.gy;
+    s.c = cz - (float)s.gz;
+    s.in_x = cx == px;  // false for a NaN
+    s.in_y = cy == py;
+    s.in_z = cz == pz;
+    s.base = s.gx + P.Xp * (s.gy + P.Y * s.gz);
     return s;
 }
 
-// W = S o phi, r = W - T, the exact trilinear gradient of the interpolant, the graph
-// Laplacian of u = phi - x and the FP64 data energy.  A block owns a 32 x 8 column tile
-// and marches z: phi's three components (tile rows plus a 1-voxel halo) and T are staged
-// slice by slice into a shared-memory ring by 16-byte cp.async kGAhead slices ahead of the
-// compute; the eight corners of S are gathered through L1.
+// W = S o phi, r = W - T, g = r * (exact trilinear gradient of the interpolant) + w_reg * (graph
+// Laplacian of u = phi - x).
+//
+// A block owns a 32 x 8 column tile and marches z, one voxel per thread and slice.  phi's three
+// components (the tile and a 1-voxel halo) and T are staged slice by slice in a ring of kGS
+// shared-memory slots; the eight corners of S are gathered through L1.  A thread keeps its own
+// column of phi in registers from slice to slice, and the Laplacian's term across a z face is
+// formed once and enters the next slice's sum negated: (p - q) + d and (q - p) - d differ in
+// sign only, and adding the zero of either sign to a sum that is not -0 gives the same bits
+// (a sum that starts from +0 is never -0).
+//
+// With TMA staging a ninth warp fills the ring, two tensor copies per slice, and warps do not
+// wait on one another: each waits for a slice's full barrier and arrives on its empty barrier
+// when it has read the slot, and the filling thread waits for the slot's eight arrivals.  The
+// cp.async variant stages one chunk per thread and component, with a block barrier per slice.
+//
+// Bound by issue slots (73% used, 59 million warp instructions on the 182x218x182 pair) and by
+// the corner loads' latency: 70.6 us there, where every thread waiting at a block barrier per
+// slice, seven shared-memory reads per component and an FP64 sum that nothing read took 82.5 us
+// (72.6 million instructions; 32 bytes per voxel are 34 us at the copy bandwidth).  Four blocks
+// (56 registers) with TMA: five need 40 registers, spill and take 100 us; six cp.async blocks
+// 75 us, five 79 us.  Four slots: three take 73 us, five 71 us.  Warps that own four rows
+// each, with the rows' values in registers, execute 42 million instructions but hold only 16
+// warps per SM and take 78 us.
 namespace {
-constexpr int kGAhead = 2;        // slices in flight ahead of the one computed
-constexpr int kGS = 3 + kGAhead;  // ring slots: slices z - 1, z, z + 1 and those in flight
-constexpr int kGW = kStageW, kGPlane = kGW * (kTileY + 2), kGTPlane = kTileX * kTileY;
+constexpr int kGS = 4;                               // ring slots: slices z and z + 1, the others in flight
+constexpr int kGW = kStageW, kGPlane = kGW * (kTileY + 2);  // box row and plane (floats)
+constexpr int kGTOff = (3 * kGPlane + 31) / 32 * 32;  // T's offset in a slot (128-byte aligned)
+constexpr int kGSlot = kGTOff + kTileX * kTileY;
+constexpr unsigned kGBytes = sizeof(float) * (3 * kGPlane + kTileX * kTileY);
+static_assert(kGSlot % 32 == 0, "slots on 128-byte boundaries");
 }  // namespace
 
-size_t sob_grad_smem_bytes() { return sizeof(float) * kGS * (3 * kGPlane + kGTPlane); }
+size_t sob_grad_smem_bytes() { return 128 + sizeof(float) * kGS * kGSlot + 2 * sizeof(uint64_t) * kGS; }
 
-__global__ void __launch_bounds__(256) sob_grad_kernel(SobIterArgs a) {
-    extern __shared__ __align__(16) float ring[];  // phi [3][kGS][10][kGW], then T [kGS][8][32]
-    float* tring = ring + 3 * kGS * kGPlane;
-    __shared__ double red[32];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int t = blockIdx.x; t < a.ntiles_g; t += gridDim.x) {
-        const Tile tl = a.tiles_g[t];
-        if (a.stop[tl.x]) continue;  // uniform over the block
-        const Pair P = a.pairs[tl.x];
-        const int Y = P.Y, Z = P.Z, Xp = P.Xp, XYp = P.Xp * P.Y;  // strides of the packed arrays
-        const long long NT = a.NT;
-        const float* __restrict__ S = a.S + P.off;
-        const float* __restrict__ Tg = a.T + P.off;
-        const float* __restrict__ Fg[3] = {a.phi + P.off, a.phi + NT + P.off, a.phi + 2 * NT + P.off};
-        float* G[3] = {a.g + P.off, a.g + NT + P.off, a.g + 2 * NT + P.off};
-        const int x = tl.y + tx, y = tl.z + ty;
-        const bool inside = x < P.X && y < Y;
-        const int z0 = tl.w, z1 = min(tl.w + a.depth_g, Z);
-        const int gq = stage_offset<1>(threadIdx.x, Y, Xp, tl.y, tl.z);
-        // T: thread e < 64 copies chunk e & 7 of tile row e >> 3 (x0 is a multiple of 32)
-        const int tr = (int)threadIdx.x >> 3, tk = (int)threadIdx.x & 7;
-        const int gt = (threadIdx.x < 64 && tl.z + tr < Y && tl.y + 4 * tk < Xp) ? Xp * (tl.z + tr) + tl.y + 4 * tk
-                                                                                 : -1;
-        auto stage = [&](int zs, int sl) {  // slice zs of phi (and T) into slot sl
-            if (zs < 0 || zs >= Z) return;
-            if (gq >= 0) {
-                float* dst = ring + sl * kGPlane + 4 * threadIdx.x;
-                const int off = gq + XYp * zs;
-#pragma unroll
-                for (int c = 0; c < 3; ++c) cp_async16(dst + c * kGS * kGPlane, Fg[c] + off);
-            }
-            if (gt >= 0) cp_async16(tring + sl * kGTPlane + 4 * threadIdx.x, Tg + gt + XYp * zs);
-        };
-        double e = 0.0;
-        __syncthreads();  // the previous tile is done with the ring
-        // prologue: slices z0 - 1 .. z0 + 1 (one group), then one group per slice ahead
-        stage(z0 - 1, 0);
-        stage(z0, 1);
-        stage(z0 + 1, 2);
-        cp_async_commit();
-#pragma unroll
-        for (int k = 1; k < kGAhead; ++k) {
-            if (z0 + 1 + k <= z1) stage(z0 + 1 + k, 2 + k);
-            cp_async_commit();
-        }
-        int sm = 0;  // slot of slice z - 1 (z, z + 1 follow it in the ring)
-        const int c0 = (ty + 1) * kGW + tx + kStageXO;
-        for (int z = z0; z < z1; ++z) {
-            cp_async_wait<kGAhead - 1>();  // slice z + 1 has landed ...
-            __syncthreads();               // ... for every thread, and slice z - 2's slot is free
-            {
-                int sl = sm + 2 + kGAhead;  // the slot of slice z - 2
-                sl = sl >= kGS ? sl - kGS : sl;
-                if (z + 1 + kGAhead <= z1) stage(z + 1 + kGAhead, sl);  // reads reach z1
-                cp_async_commit();
-            }
-            const int s0 = sm + 1 >= kGS ? sm + 1 - kGS : sm + 1;
-            const int sp = s0 + 1 >= kGS ? s0 + 1 - kGS : s0 + 1;
-            if (inside) {
-                const int i = x + Xp * y + XYp * z;
-                const float* q[3];
-#pragma unroll
-                for (int c = 0; c < 3; ++c) q[c] = ring + (c * kGS + s0) * kGPlane + c0;
-                const SobCell s = sob_locate(P, q[0][0], q[1][0], q[2][0]);
-                const int b = (int)s.base;
-                const float f000 = __ldg(S + b), f100 = __ldg(S + b + 1);
-                const float f010 = __ldg(S + b + Xp), f110 = __ldg(S + b + 1 + Xp);
-                const float f001 = __ldg(S + b + XYp), f101 = __ldg(S + b + 1 + XYp);
-                const float f011 = __ldg(S + b + Xp + XYp), f111 = __ldg(S + b + 1 + Xp + XYp);
-                // graph Laplacian of u = phi - x, neighbours inside the grid, order -x,+x,-y,+y,-z,+z
-                // (shared-memory work placed between the corner loads and their use)
-                const bool ok[6] = {x > 0, x < P.X - 1, y > 0, y < Y - 1, z > 0, z < Z - 1};
-                float lap[3];
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const float* qc = q[c];
-                    const float* qm = ring + (c * kGS + sm) * kGPlane + c0;
-                    const float* qp = ring + (c * kGS + sp) * kGPlane + c0;
-                    const float pc = qc[0];
-                    const float nb[6] = {qc[-1], qc[1], qc[-kGW], qc[kGW], qm[0], qp[0]};
-                    float acc = 0.f;
-#pragma unroll
-                    for (int k = 0; k < 6; ++k) {
-                        if (!ok[k]) continue;
-                        const float delta = (k / 2 == c) ? ((k & 1) ? 1.f : -1.f) : 0.f;
-                        acc = acc + ((pc - nb[k]) + delta);
-                    }
-                    lap[c] = acc;
-                }
-                const float e11 = lerpf_(f111, f110, s.c), e10 = lerpf_(f101, f100, s.c);
-                const float e01 = lerpf_(f011, f010, s.c), e00 = lerpf_(f001, f000, s.c);
-                const float A1 = lerpf_(e11, e10, s.b), A0 = lerpf_(e01, e00, s.b);
-                const float W = lerpf_(A1, A0, s.a);
-                const float dWa = s.in_x ? A1 - A0 : 0.f;
-                const float dWb = s.in_y ? lerpf_(e11 - e10, e01 - e00, s.a) : 0.f;
-                const float dWc = s.in_z ? lerpf_(lerpf_(f111 - f110, f101 - f100, s.b),
-                                                  lerpf_(f011 - f010, f001 - f000, s.b), s.a)
-                                         : 0.f;
-                const float r = W - tring[s0 * kGTPlane + ty * kTileX + tx];
-                G[0][i] = (r * dWa) + (P.w_reg * lap[0]);
-                G[1][i] = (r * dWb) + (P.w_reg * lap[1]);
-                G[2][i] = (r * dWc) + (P.w_reg * lap[2]);
-                e = fma((double)r, (double)r, e);  // r * r is exact in FP64: one DFMA, same bits
-            }
-            sm = s0;
-        }
-        cp_async_wait<0>();
-        e = block_sum_f64(e, red);
-        if (threadIdx.x == 0) atomicAdd(a.energy + (long long)(a.iter - 1) * a.npairs + tl.x, 0.5 * e);
-    }
-}
-
-// The same gradient with TMA staging: per slice one thread copies phi's box (40 columns
-// x 10 rows x 3 components: the tile and a 1-voxel halo; out-of-volume parts read as zero
-// and are masked by the grid-neighbour tests) and T's 32 x 8 box with two tensor copies
-// into a six-slot ring, completing on the slot's mbarrier; three slices are in flight
-// ahead of the one computed.  Waits are bounded as in ref_laplacian_tma_kernel.
-namespace {
-constexpr int kGBAhead = 3;
-constexpr int kGBS = 3 + kGBAhead;
-constexpr int kGBW = 40, kGBPlane = kGBW * 10;  // phi box row and plane (floats)
-constexpr int kGBTOff = 1216;                   // T box offset in a slot (floats, 128-byte aligned)
-constexpr int kGBSlot = kGBTOff + kTileX * kTileY;
-constexpr unsigned kGBBytes = sizeof(float) * (3 * kGBPlane + kTileX * kTileY);
-static_assert(3 * kGBPlane <= kGBTOff && (kGBSlot * 4) % 128 == 0, "slot layout");
-}  // namespace
-
-size_t sob_grad_tma_smem_bytes() { return 128 + sizeof(float) * kGBS * kGBSlot + sizeof(uint64_t) * kGBS; }
-
-__global__ void __launch_bounds__(256) sob_grad_tma_kernel(SobIterArgs a) {
+template <bool TMA>
+__global__ void __launch_bounds__(sob_grad_threads(TMA), TMA ? 4 : 6) sob_grad_kernel(SobIterArgs a) {
     extern __shared__ __align__(128) unsigned char grad_raw[];
     float* ring = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(grad_raw) + 127) & ~uintptr_t(127));
-    uint64_t* full = reinterpret_cast<uint64_t*>(ring + kGBS * kGBSlot);
-    __shared__ double red[32];
-    typedef SliceRing<kGBS> Ring;
+    uint64_t* full = reinterpret_cast<uint64_t*>(ring + kGS * kGSlot);
+    uint64_t* empty = full + kGS;
     const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
-    if (tid == 0) {
-        for (int k = 0; k < kGBS; ++k) mbar_init(full + k, 1);
-        mbar_fence_init();
+    if (TMA) {
+        if (tid == 0) {
+            for (int k = 0; k < kGS; ++k) {
+                mbar_init(full + k, 1);
+                mbar_init(empty + k, 8);
+            }
+            mbar_fence_init();
+        }
+        __syncthreads();
+        if (ty == 8) {  // the filling warp: one thread copies every slice of the block's tiles in order
+            if (tx != 0) return;
+            unsigned n = 0;  // fills: fill n goes to slot n % kGS, the (n / kGS)-th of that slot
+            bool ok = true;
+            for (int t = blockIdx.x; t < a.ntiles_g && ok; t += gridDim.x) {
+                const Tile tl = a.tiles_g[t];
+                if (a.stop[tl.x]) continue;
+                const CUtensorMap* maps = a.tmaps + (long long)tl.x * TM_COUNT;
+                const int z1 = min(tl.w + a.depth_g, a.pairs[tl.x].Z);
+                for (int z = tl.w - 1; z <= z1 && ok; ++z, ++n) {
+                    const int k = SliceRing<kGS>::slot(n);
+                    // the slot's previous reader has released it (an unused slot counts as released)
+                    ok = mbar_wait_bounded(empty + k, SliceRing<kGS>::parity(n) ^ 1u);
+                    if (!ok) break;
+                    mbar_arrive_expect_tx(full + k, kGBytes);
+                    tma_load_4d(ring + k * kGSlot, maps + TM_LAP_PSI, tl.y - 4, tl.z - 1, z, 0, full + k);
+                    tma_load_3d(ring + k * kGSlot + kGTOff, maps + TM_LAP_T, tl.y, tl.z, z, full + k);
+                }
+            }
+            if (!ok) {  // the copies in flight end (bounded) before the block's shared memory goes
+                for (unsigned m = n > (unsigned)kGS ? n - kGS : 0u; m < n; ++m)
+                    mbar_wait_bounded(full + SliceRing<kGS>::slot(m), SliceRing<kGS>::parity(m));
+                atomicOr(a.err, kErrTmaTimeout);
+            }
+            return;
+        }
     }
-    __syncthreads();
-    unsigned nbase = 0, issued = 0;
+    int slot = 0;           // slots are read in order
+    unsigned full_ph = 0u;  // bit k: parity of slot k's next fill
     bool failed = false;
+
     for (int t = blockIdx.x; t < a.ntiles_g && !failed; t += gridDim.x) {
         const Tile tl = a.tiles_g[t];
         if (a.stop[tl.x]) continue;  // uniform over the block
         const Pair P = a.pairs[tl.x];
-        const int Y = P.Y, Z = P.Z, Xp = P.Xp, XYp = P.Xp * P.Y;
+        const int X = P.X, Y = P.Y, Z = P.Z, Xp = P.Xp, XYp = P.Xp * P.Y;  // strides of the packed arrays
         const long long NT = a.NT;
         const float* __restrict__ S = a.S + P.off;
-        float* G[3] = {a.g + P.off, a.g + NT + P.off, a.g + 2 * NT + P.off};
-        const CUtensorMap* mphi = a.tmaps + (long long)tl.x * TM_COUNT + TM_LAP_PSI;
-        const CUtensorMap* mT = a.tmaps + (long long)tl.x * TM_COUNT + TM_LAP_T;
         const int x = tl.y + tx, y = tl.z + ty;
-        const bool inside = x < P.X && y < Y;
-        const int z0 = tl.w, z1 = min(tl.w + a.depth_g, Z);
-        const int nsl = z1 - z0 + 2;  // slices z0 - 1 .. z1 (outside the volume: zeros, unused)
-        auto issue = [&](int j) {
-            const unsigned n = nbase + (unsigned)j;
-            float* dst = ring + Ring::slot(n) * kGBSlot;
-            uint64_t* bar = full + Ring::slot(n);
-            mbar_arrive_expect_tx(bar, kGBBytes);
-            tma_load_4d(dst, mphi, tl.y - 4, tl.z - 1, z0 - 1 + j, 0, bar);
-            tma_load_3d(dst + kGBTOff, mT, tl.y, tl.z, z0 - 1 + j, bar);
-            ++issued;
-        };
-        double e = 0.0;
-        __syncthreads();  // the previous tile is done with the ring
-        if (tid == 0) {
-            tma_prefetch_map(mphi);
-            tma_prefetch_map(mT);
-            for (int j = 0; j < min(nsl, kGBS); ++j) issue(j);
-        }
-        const int c0 = (ty + 1) * kGBW + tx + 4;
-        for (int j0 = 0; j0 + 2 < nsl; ++j0) {
-            bool ok = true;
-            for (int j = (j0 == 0 ? 0 : j0 + 2); j <= j0 + 2; ++j)
-                ok = ok && mbar_wait_bounded(full + Ring::slot(nbase + j), Ring::parity(nbase + j));
-            if (__syncthreads_or(!ok)) {
-                failed = true;
-                break;
+        const bool inside = x < X && y < Y;
+        const int z0 = tl.w, z1 = min(tl.w + a.depth_g, Z);  // slices z0 - 1 .. z1 are staged
+        // cp.async: this thread's chunk of a slice of phi, and of T (threads below 64)
+        const int gq = TMA ? -1 : stage_offset<1>(tid, Y, Xp, tl.y, tl.z);
+        const int tr = tid >> 3, tk = tid & 7;
+        const int gt = !TMA && tid < 64 && tl.z + tr < Y && tl.y + 4 * tk < Xp ? Xp * (tl.z + tr) + tl.y + 4 * tk : -1;
+        auto stage = [&](int z, int k) {  // cp.async: slice z into slot k (one group)
+            if (TMA) return;
+            if (z >= 0 && z < Z && z <= z1) {
+                float* dst = ring + k * kGSlot;
+                if (gq >= 0)
+#pragma unroll
+                    for (int c = 0; c < 3; ++c)
+                        cp_async16(dst + c * kGPlane + 4 * tid, a.phi + c * NT + P.off + gq + XYp * z);
+                if (gt >= 0) cp_async16(dst + kGTOff + 4 * tid, a.T + P.off + gt + XYp * z);
             }
-            if (tid == 0 && j0 >= 1 && j0 - 1 + kGBS < nsl) issue(j0 - 1 + kGBS);
+            cp_async_commit();
+        };
+        auto next_slice = [&]() {  // the next slice in order has landed; its slot
+            const int k = slot;
+            if (TMA) {
+                const bool ok = mbar_wait_bounded(full + k, (full_ph >> k) & 1u);
+                if (!__all_sync(0xffffffffu, ok)) failed = true;
+                full_ph ^= 1u << k;
+            } else {
+                cp_async_wait<kGS - 3>();
+                __syncthreads();
+            }
+            slot = slot + 1 == kGS ? 0 : slot + 1;
+            return k;
+        };
+        auto release = [&](int k) {  // this warp has read slot k
+            if (TMA) {
+                __syncwarp();
+                if (tx == 0) mbar_arrive(empty + k);
+            }
+        };
+        if (!TMA) {
+            __syncthreads();  // the previous tile is done with the ring
+            slot = 0;
+#pragma unroll
+            for (int k = 0; k < kGS - 1; ++k) stage(z0 - 1 + k, k);
+        }
+        const bool xl = x > 0, xr = x < X - 1;
+        const bool y_edge = y == 0 || y >= Y - 1;  // uniform over the warp
+        const int c0 = (ty + 1) * kGW + tx + kStageXO;
+        // phi of this column at the slice computed, and the Laplacian's terms across the
+        // voxel's z face towards the slice above
+        float cur[3], up[3];
+        int at = next_slice();
+#pragma unroll
+        for (int c = 0; c < 3; ++c) up[c] = ring[at * kGSlot + c0 + c * kGPlane];
+        release(at);
+        stage(z0 - 1 + kGS - 1, kGS - 1);
+        at = next_slice();
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            cur[c] = ring[at * kGSlot + c0 + c * kGPlane];
+            up[c] = c == 2 ? (up[c] - cur[c]) + 1.f : up[c] - cur[c];
+        }
+        int i = x + Xp * y + XYp * z0;
+        float* const G[3] = {a.g + P.off, a.g + NT + P.off, a.g + 2 * NT + P.off};
+        for (int z = z0; z < z1; ++z, i += XYp) {
+            const float* q0 = ring + at * kGSlot;
+            const int above = next_slice();
+            if (TMA && failed) break;
+            stage(z - 1 + kGS, at == 0 ? kGS - 1 : at - 1);  // the slot of slice z - 1
             if (inside) {
-                const int z = z0 + j0;
-                const int i = x + Xp * y + XYp * z;
-                const float* qm = ring + Ring::slot(nbase + j0) * kGBSlot + c0;
-                const float* q0 = ring + Ring::slot(nbase + j0 + 1) * kGBSlot;
-                const float* qp = ring + Ring::slot(nbase + j0 + 2) * kGBSlot + c0;
-                const SobCell s = sob_locate(P, q0[c0], q0[c0 + kGBPlane], q0[c0 + 2 * kGBPlane]);
-                const int b = (int)s.base;
-                const float f000 = __ldg(S + b), f100 = __ldg(S + b + 1);
-                const float f010 = __ldg(S + b + Xp), f110 = __ldg(S + b + 1 + Xp);
-                const float f001 = __ldg(S + b + XYp), f101 = __ldg(S + b + 1 + XYp);
-                const float f011 = __ldg(S + b + Xp + XYp), f111 = __ldg(S + b + 1 + Xp + XYp);
-                const bool okn[6] = {x > 0, x < P.X - 1, y > 0, y < Y - 1, z > 0, z < Z - 1};
+                const float* qp = ring + above * kGSlot + c0;
+                const SobCell s = sob_locate(P, cur[0], cur[1], cur[2]);
+                const float* b = S + s.base;
+                const float f000 = __ldg(b), f100 = __ldg(b + 1);
+                const float f010 = __ldg(b + Xp), f110 = __ldg(b + 1 + Xp);
+                const float f001 = __ldg(b + XYp), f101 = __ldg(b + 1 + XYp);
+                const float f011 = __ldg(b + Xp + XYp), f111 = __ldg(b + 1 + Xp + XYp);
+                // neighbours inside the grid, in the order -x, +x, -y, +y, -z, +z
+                // (shared-memory work placed between the corner loads and their use)
                 float lap[3];
+                auto laplacian = [&](auto edge) {
+                    constexpr bool kEdge = decltype(edge)::value;
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const float* qc = q0 + c0 + c * kGBPlane;
-                    const float pc = qc[0];
-                    const float nb[6] = {qc[-1], qc[1], qc[-kGBW], qc[kGBW], qm[c * kGBPlane], qp[c * kGBPlane]};
-                    float acc = 0.f;
-#pragma unroll
-                    for (int k = 0; k < 6; ++k) {
-                        if (!okn[k]) continue;
-                        const float delta = (k / 2 == c) ? ((k & 1) ? 1.f : -1.f) : 0.f;
-                        acc = acc + ((pc - nb[k]) + delta);
+                    for (int c = 0; c < 3; ++c) {
+                        const float* q = q0 + c0 + c * kGPlane;
+                        const float p = cur[c], n = qp[c * kGPlane];
+                        const float dx = p - q[-1], ux = p - q[1], dy = p - q[-kGW], uy = p - q[kGW], uz = p - n;
+                        float acc = 0.f;
+                        if (xl) acc = acc + (c == 0 ? dx - 1.f : dx);
+                        if (xr) acc = acc + (c == 0 ? ux + 1.f : ux);
+                        if (!kEdge || y > 0) acc = acc + (c == 1 ? dy - 1.f : dy);
+                        if (!kEdge || y < Y - 1) acc = acc + (c == 1 ? uy + 1.f : uy);
+                        if (!kEdge || z > 0) acc = acc - up[c];
+                        up[c] = c == 2 ? uz + 1.f : uz;
+                        if (!kEdge || z < Z - 1) acc = acc + up[c];
+                        lap[c] = acc;
+                        cur[c] = n;
                     }
-                    lap[c] = acc;
-                }
+                };
+                if (y_edge || z == 0 || z == Z - 1)
+                    laplacian(std::true_type{});
+                else
+                    laplacian(std::false_type{});
+                const float tv = q0[kGTOff + ty * kTileX + tx];
                 const float e11 = lerpf_(f111, f110, s.c), e10 = lerpf_(f101, f100, s.c);
                 const float e01 = lerpf_(f011, f010, s.c), e00 = lerpf_(f001, f000, s.c);
                 const float A1 = lerpf_(e11, e10, s.b), A0 = lerpf_(e01, e00, s.b);
@@ -288,23 +254,22 @@ __global__ void __launch_bounds__(256) sob_grad_tma_kernel(SobIterArgs a) {
                 const float dWc = s.in_z ? lerpf_(lerpf_(f111 - f110, f101 - f100, s.b),
                                                   lerpf_(f011 - f010, f001 - f000, s.b), s.a)
                                          : 0.f;
-                const float r = W - q0[kGBTOff + ty * kTileX + tx];
+                const float r = W - tv;
                 G[0][i] = (r * dWa) + (P.w_reg * lap[0]);
                 G[1][i] = (r * dWb) + (P.w_reg * lap[1]);
                 G[2][i] = (r * dWc) + (P.w_reg * lap[2]);
-                e = fma((double)r, (double)r, e);  // r * r is exact in FP64: one DFMA, same bits
             }
+            release(at);
+            at = above;
         }
-        nbase += (unsigned)nsl;
-        if (failed) break;
-        e = block_sum_f64(e, red);
-        if (threadIdx.x == 0) atomicAdd(a.energy + (long long)(a.iter - 1) * a.npairs + tl.x, 0.5 * e);
+        if (!failed) release(at);
+        if (!TMA) cp_async_wait<0>();
     }
-    if (failed && tid == 0) {
-        for (unsigned n = (issued > (unsigned)kGBS ? issued - kGBS : 0u); n < issued; ++n)
-            mbar_wait_bounded(full + Ring::slot(n), Ring::parity(n));
-        atomicOr(a.err, kErrTmaTimeout);
-    }
+    if (TMA && failed && tx == 0) atomicOr(a.err, kErrTmaTimeout);
+}
+
+const void* sob_grad_fn(int tma) {
+    return tma ? (const void*)sob_grad_kernel<true> : (const void*)sob_grad_kernel<false>;
 }
 
 // phi += m o phi with the max update norm.  Held to 48 registers for 5 resident blocks
@@ -557,13 +522,10 @@ __global__ void __launch_bounds__(256, 4) sob_pass_b_staged_kernel(SobIterArgs a
 cudaError_t launch_sob_iter(const SobIterArgs& a, const int* grids, const int* variants, cudaStream_t s,
                             cudaEvent_t* ev) {
     if (ev) cudaEventRecord(ev[0], s);
-    if (variants[0])
-        sob_grad_tma_kernel<<<grids[0], 256, sob_grad_tma_smem_bytes(), s>>>(a);
-    else
-        sob_grad_kernel<<<grids[0], 256, sob_grad_smem_bytes(), s>>>(a);
+    void* args[1] = {const_cast<SobIterArgs*>(&a)};
+    cudaLaunchKernel(sob_grad_fn(variants[0]), dim3(grids[0]), dim3(sob_grad_threads(variants[0])), args, sob_grad_smem_bytes(), s);
     if (ev) cudaEventRecord(ev[1], s);
     {
-        void* args[1] = {const_cast<SobIterArgs*>(&a)};
         cudaLaunchKernel(sob_smooth3_fn(a.radius, variants[1] & 1, variants[1] & 2), dim3(grids[1]), dim3(kSmoothThreads), args, 0, s);
     }
     if (ev) cudaEventRecord(ev[2], s);

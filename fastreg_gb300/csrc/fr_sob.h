@@ -58,7 +58,6 @@ struct SobIterArgs {
     int* stop;
     unsigned long long* keys;
     unsigned long long* trace;
-    double* energy;  // [max_iter][npairs] 0.5 * sum (W - T)^2 before the update
     unsigned int* counter;
     const CUtensorMap* tmaps;  // [npairs][TM_COUNT] tensor maps (fr_kernels.h), TMA-staged variants
     unsigned int* err;         // device error word (kErrTmaTimeout: a staging wait gave up)
@@ -68,10 +67,9 @@ struct SobIterArgs {
 // and rounded to float.
 void gaussian_taps(float sigma, int width, float* taps);
 
-size_t sob_grad_smem_bytes();  // dynamic shared memory of sob_grad_kernel
-__global__ void sob_grad_kernel(SobIterArgs a);
-size_t sob_grad_tma_smem_bytes();  // dynamic shared memory of sob_grad_tma_kernel
-__global__ void sob_grad_tma_kernel(SobIterArgs a);
+constexpr int sob_grad_threads(int tma) { return tma ? 288 : 256; }  // with TMA a ninth warp stages
+size_t sob_grad_smem_bytes();         // dynamic shared memory of the gradient kernel
+const void* sob_grad_fn(int tma);     // the gradient kernel of a staging variant (1: TMA)
 // the smoothing kernel instance for a radius, staging variant (1: TMA) and tile height
 const void* sob_smooth3_fn(int radius, int tma, bool tall);
 // box of one component of the smoothing kernel's staged slice for radius R: x extent, rows

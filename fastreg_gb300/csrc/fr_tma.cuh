@@ -30,6 +30,11 @@ __device__ __forceinline__ void mbar_fence_init() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// this thread arrives
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
 // this thread arrives and the phase also waits for `bytes` of copies
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
