@@ -272,10 +272,16 @@ const void* sob_grad_fn(int tma) {
     return tma ? (const void*)sob_grad_kernel<true> : (const void*)sob_grad_kernel<false>;
 }
 
-// phi += m o phi with the max update norm.  Held to 48 registers for 5 resident blocks
-// per SM (0.098 against 0.101 ms with 63 registers and 4 blocks): the kernel waits on its
-// corner loads, and more resident warps keep more of them in flight.
-__global__ void __launch_bounds__(256, 5) sob_pass_b_kernel(SobIterArgs a) {
+// phi += m o phi with the max update norm.  phi is smooth, so the cell of slice z + 1 is often
+// the one above this slice's: its lower corners are then the upper ones already in registers,
+// and a lane loads 12 corners instead of 24.  The kernel is bound by the gathers' trips through
+// L1 (its data pipe 68% busy with 24 corners, several cache lines per load), then by their
+// latency: 80 us on the 182x218x182 pair, where 24 corners and an L2 prefetch of the next
+// cell's rows took 92 us (86 us with the reuse and the prefetch: it only adds to the L1
+// queue now).  Four blocks of 64 registers; five would spill the kept corners, three take 81 us.
+// The reference solver's pass B, whose psi stays near the grid, gains nothing from the
+// reuse (73 against 66 us): its loads mostly hit the same lines, and it needs the warps.
+__global__ void __launch_bounds__(256, 4) sob_pass_b_kernel(SobIterArgs a) {
     __shared__ unsigned long long red[32];
     __shared__ bool last;
     for (int t = blockIdx.x; t < a.ntiles_b; t += gridDim.x) {
@@ -293,6 +299,12 @@ __global__ void __launch_bounds__(256, 5) sob_pass_b_kernel(SobIterArgs a) {
             int i = x + X * y + XY * tl.w;
             // phi of the next slice is loaded while this slice's gathers are in flight
             float nx = phi[0][i], ny = phi[1][i], nz = phi[2][i];
+            float f[3][8];  // corners 111, 110, 101, 100, 011, 010, 001, 000 (x, y, z) of m's components
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+#pragma unroll
+                for (int q = 0; q < 8; ++q) f[c][q] = 0.f;
+            int above = -1;  // base of the cell whose lower corners are the upper ones in f (-1: none)
             for (int z = tl.w; z < z1; ++z, i += XY) {
                 const float px = nx, py = ny, pz = nz;
                 if (z + 1 < z1) {
@@ -301,37 +313,31 @@ __global__ void __launch_bounds__(256, 5) sob_pass_b_kernel(SobIterArgs a) {
                     nz = phi[2][i + XY];
                 }
                 const SobCell s = sob_locate(P, px, py, pz);
-                {  // L2 prefetch: the m rows the next slice's cell adds (phi is smooth, so that
-                   // cell is about this one plus a slice) and phi two slices on
-                    const int N = (int)P.N, o0 = min((int)s.base + 2 * XY, N - 1);
-                    const int o1 = min((int)s.base + 2 * XY + X, N - 1);
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        prefetch_l2(mc[c] + o0);
-                        prefetch_l2(mc[c] + o1);
-                    }
-                    if (z + 2 < P.Z)
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) prefetch_l2(phi[c] + i + 2 * XY);
-                }
                 float u[3];
-                {  // components 0 and 1 interpolated as one packed pair (trilerp3)
-                    const int b = (int)s.base;
-                    float f[3][8];
+                const int b = s.base;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    f[c][1] = f[c][0];
+                    f[c][3] = f[c][2];
+                    f[c][5] = f[c][4];
+                    f[c][7] = f[c][6];
+                    const float* __restrict__ F = mc[c];
+                    f[c][0] = __ldg(F + b + 1 + X + XY);
+                    f[c][2] = __ldg(F + b + 1 + XY);
+                    f[c][4] = __ldg(F + b + X + XY);
+                    f[c][6] = __ldg(F + b + XY);
+                }
+                if (b != above)
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
                         const float* __restrict__ F = mc[c];
-                        f[c][0] = __ldg(F + b + 1 + X + XY);
                         f[c][1] = __ldg(F + b + 1 + X);
-                        f[c][2] = __ldg(F + b + 1 + XY);
                         f[c][3] = __ldg(F + b + 1);
-                        f[c][4] = __ldg(F + b + X + XY);
                         f[c][5] = __ldg(F + b + X);
-                        f[c][6] = __ldg(F + b + XY);
                         f[c][7] = __ldg(F + b);
                     }
-                    trilerp3(f, s.a, s.b, s.c, u);
-                }
+                above = b + XY;
+                trilerp3(f, s.a, s.b, s.c, u);
                 phi[0][i] = px + u[0];
                 phi[1][i] = py + u[1];
                 phi[2][i] = pz + u[2];
