@@ -11,7 +11,14 @@
 // separable Gaussian (replicate boundary), the regulariser (the graph Laplacian is
 // symmetric) and the data gradient (the trilinear interpolant's gradient and Hessian).
 // Forward states are checkpointed every `checkpoint_every` iterations and each segment
-// is recomputed before it is reversed.  Layout: one pair, planes of N voxels.
+// is recomputed before it is reversed (the last one as part of the forward sweep).
+//
+// The workspace holds one pair in the packed layout of the cohort (fr_common.cuh), so the
+// forward iterations are the cohort's own three kernels (the same bits as a registration),
+// with a separate input and output state per iteration: a checkpoint or a segment's state is
+// written where it is kept and never copied.  The reverse iteration is four kernels: the
+// update's adjoint, the momentum's, the transposed smoothing (the smoothing kernel's
+// transposed form) and the gradient's.  fr_warp_adjoint works on the caller's unpadded planes.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -21,6 +28,7 @@
 
 #include "../../include/fastreg_gb300.h"
 #include "fr_common.cuh"
+#include "fr_kernels.h"
 #include "fr_limits.h"
 #include "fr_sob.h"
 
@@ -85,33 +93,6 @@ __device__ __forceinline__ void tri_eval(const AdjDims& D, const float* __restri
     t.H12 = (t.in[1] && t.in[2]) ? lerpf_(d11 - d10, d01 - d00, a) : 0.f;
 }
 
-__device__ __forceinline__ void coords(const AdjDims& D, int i, int& x, int& y, int& z) {
-    z = i / D.XY;
-    const int r = i - z * D.XY;
-    y = r / D.X;
-    x = r - y * D.X;
-}
-
-// graph Laplacian of u = phi - x (neighbours inside the grid; order -x,+x,-y,+y,-z,+z)
-__device__ __forceinline__ void lap_u(const AdjDims& D, const float* __restrict__ phi, int i, int x, int y, int z,
-                                      float out[3]) {
-    const bool ok[6] = {x > 0, x < D.X - 1, y > 0, y < D.Y - 1, z > 0, z < D.Z - 1};
-    const int off[6] = {-1, 1, -D.X, D.X, -D.XY, D.XY};
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const float* P = phi + (long long)c * D.N;
-        const float pc = __ldg(P + i);
-        float acc = 0.f;
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            if (!ok[k]) continue;
-            const float delta = (k / 2 == c) ? ((k & 1) ? 1.f : -1.f) : 0.f;
-            acc = acc + ((pc - __ldg(P + i + off[k])) + delta);
-        }
-        out[c] = acc;
-    }
-}
-
 #define GRID_STRIDE(i, n) for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += gridDim.x * blockDim.x)
 
 // Grid-stride loop over whole warps: every lane of a warp runs the same iterations (lane
@@ -147,239 +128,360 @@ __device__ __forceinline__ void scatter_cell_warp(float* F, int b, const float c
     }
 }
 
-// ---- forward (same arithmetic as the cohort kernels and the oracle) ----
-__global__ void adj_fwd_grad_kernel(AdjDims D, const float* __restrict__ S, const float* __restrict__ T,
-                                    const float* __restrict__ phi, float lambda, float* __restrict__ g) {
-    GRID_STRIDE(i, D.N) {
-        int x, y, z;
-        coords(D, i, x, y, z);
-        TriEval t;
-        tri_eval(D, S, __ldg(phi + i), __ldg(phi + D.N + i), __ldg(phi + 2 * D.N + i), t, false);
-        const float r = t.val - __ldg(T + i);
-        float lap[3];
-        lap_u(D, phi, i, x, y, z, lap);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) g[(long long)c * D.N + i] = (r * t.d[c]) + (lambda * lap[c]);
-    }
-}
+// One pair of the workspace.
+struct AdjPair {
+    int X, Y, Z, Xp, XYp;  // extents, row and slice pitch
+    int N;                 // XYp * Z
+    long long NT;          // plane stride of vector fields
+    int depth;             // slices per tile of the column kernels
+};
 
-// one separable pass of radius R (fma taps, replicate boundary); momentum: dst =
-// damping*dst - step*acc
-template <int R>
-__global__ void adj_fwd_smooth_kernel(AdjDims D, SobIterArgs a, int axis, const float* __restrict__ src, float* dst,
-                                      int momentum) {
-    const int dim = axis == 0 ? D.X : (axis == 1 ? D.Y : D.Z);
-    const int stride = axis == 0 ? 1 : (axis == 1 ? D.X : D.XY);
-    GRID_STRIDE(i, D.N) {
-        int x, y, z;
-        coords(D, i, x, y, z);
-        const int pos = axis == 0 ? x : (axis == 1 ? y : z);
+// The caller's fields into the packed workspace: S, T, phi = identity, m = v0; pad columns zero.
+__global__ void __launch_bounds__(256) adj_pack_kernel(AdjPair A, const float* __restrict__ S, const float* __restrict__ T,
+                                                       const float* __restrict__ v0, float* Sp, float* Tp, float* phi,
+                                                       float* m) {
+    const long long nu = (long long)A.X * A.Y * A.Z;
+    GRID_STRIDE(i, A.N) {
+        const int row = i / A.Xp, x = i - row * A.Xp, z = row / A.Y, y = row - z * A.Y;
+        const bool in = x < A.X;
+        const long long u = x + (long long)A.X * row;
+        Sp[i] = in ? __ldg(S + u) : 0.f;
+        Tp[i] = in ? __ldg(T + u) : 0.f;
+        const float pos[3] = {(float)x, (float)y, (float)z};
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const float* Sp = src + (long long)c * D.N;
-            float acc = 0.f;
-#pragma unroll
-            for (int k = -R; k <= R; ++k) {
-                const int q = min(max(pos + k, 0), dim - 1);
-                acc = fmaf(a.taps[k + R], __ldg(Sp + i + (q - pos) * stride), acc);
-            }
-            float* dp = dst + (long long)c * D.N + i;
-            *dp = momentum ? a.damping * *dp - a.step * acc : acc;
+            phi[c * A.NT + i] = pos[c];
+            m[c * A.NT + i] = in ? __ldg(v0 + c * nu + u) : 0.f;
         }
     }
 }
 
-__global__ void adj_fwd_update_kernel(AdjDims D, const float* __restrict__ m, float* phi) {
-    GRID_STRIDE(i, D.N) {
-        const float p[3] = {phi[i], phi[D.N + i], phi[2 * D.N + i]};
-        float u[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            TriEval t;
-            tri_eval(D, m + (long long)c * D.N, p[0], p[1], p[2], t, false);
-            u[c] = t.val;
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) phi[(long long)c * D.N + i] = p[c] + u[c];
+// The tables of the forward kernels and of the transposed smoothing: 32 x rows x depth tiles.
+struct AdjTables {
+    Tile* at[4];
+    int rows[4], depth[4], count[4];
+};
+__global__ void adj_tables_kernel(AdjPair A, AdjTables T) {
+    for (int k = 0; k < 4; ++k) {
+        const int nx = (A.X + kTileX - 1) / kTileX, ny = (A.Y + T.rows[k] - 1) / T.rows[k];
+        GRID_STRIDE(i, T.count[k])
+        T.at[k][i] = make_int4(0, (i % nx) * kTileX, (i / nx % ny) * T.rows[k], (i / (nx * ny)) * T.depth[k]);
     }
 }
 
-// ---- loss and the adjoint seeds ----
-__global__ void adj_loss_kernel(AdjDims D, const float* __restrict__ S, const float* __restrict__ T,
-                                const float* __restrict__ phi, const float* __restrict__ m, float* pbar, float* mbar,
-                                double* loss) {
+// The result: the adjoint of v0 out of the interleaved accumulator.
+__global__ void __launch_bounds__(256) adj_unpack_kernel(AdjPair A, const float4* __restrict__ mbar, float* out) {
+    const long long nu = (long long)A.X * A.Y * A.Z;
+    GRID_STRIDE(i, A.N) {
+        const int row = i / A.Xp, x = i - row * A.Xp;
+        if (x >= A.X) continue;
+        const float4 v = __ldg(mbar + i);
+        const long long u = x + (long long)A.X * row;
+        out[u] = v.x;
+        out[nu + u] = v.y;
+        out[2 * nu + u] = v.z;
+    }
+}
+
+// The trilinear interpolant at a cell: corners f in the order 111, 110, 101, 100, 011, 010, 001,
+// 000 (x, y, z), fractions a, b, c.
+__device__ __forceinline__ void tri_grad(const float f[8], const SobCell& s, float d[3], float* val, float H[3]) {
+    const float e11 = lerpf_(f[0], f[1], s.c), e10 = lerpf_(f[2], f[3], s.c);
+    const float e01 = lerpf_(f[4], f[5], s.c), e00 = lerpf_(f[6], f[7], s.c);
+    const float A1 = lerpf_(e11, e10, s.b), A0 = lerpf_(e01, e00, s.b);
+    const float d11 = f[0] - f[1], d10 = f[2] - f[3], d01 = f[4] - f[5], d00 = f[6] - f[7];
+    const float z1 = lerpf_(d11, d10, s.b), z0 = lerpf_(d01, d00, s.b);
+    d[0] = s.in_x ? A1 - A0 : 0.f;
+    d[1] = s.in_y ? lerpf_(e11 - e10, e01 - e00, s.a) : 0.f;
+    d[2] = s.in_z ? lerpf_(z1, z0, s.a) : 0.f;
+    if (val) *val = lerpf_(A1, A0, s.a);
+    if (H) {  // mixed second derivatives xy, xz, yz (the pure ones are 0)
+        H[0] = s.in_x && s.in_y ? (e11 - e10) - (e01 - e00) : 0.f;
+        H[1] = s.in_x && s.in_z ? z1 - z0 : 0.f;
+        H[2] = s.in_y && s.in_z ? lerpf_(d11 - d10, d01 - d00, s.a) : 0.f;
+    }
+}
+
+__device__ __forceinline__ void load_corners(const float* __restrict__ F, int b, int X, int XY, float f[8]) {
+    f[0] = __ldg(F + b + 1 + X + XY);
+    f[1] = __ldg(F + b + 1 + X);
+    f[2] = __ldg(F + b + 1 + XY);
+    f[3] = __ldg(F + b + 1);
+    f[4] = __ldg(F + b + X + XY);
+    f[5] = __ldg(F + b + X);
+    f[6] = __ldg(F + b + XY);
+    f[7] = __ldg(F + b);
+}
+
+__device__ __forceinline__ Pair as_pair(const AdjPair& A) {
+    Pair P{};
+    P.X = A.X;
+    P.Y = A.Y;
+    P.Z = A.Z;
+    P.Xp = A.Xp;
+    return P;
+}
+
+// J and the adjoint seeds: pbar = r dS(phi_K), mbar = 0.2 m_K (0 in the pad columns).  Every term
+// is a product of two FP32 values, exact in FP64, added by one fused multiply-add.
+__global__ void __launch_bounds__(256) adj_loss_kernel(AdjPair A, const float* __restrict__ S, const float* __restrict__ T,
+                                                       const float* __restrict__ phi, const float* __restrict__ m,
+                                                       float* pbar, float4* mbar, double* loss) {
     __shared__ double red[32];
-    double e = 0.0;
-    GRID_STRIDE(i, D.N) {
-        TriEval t;
-        tri_eval(D, S, __ldg(phi + i), __ldg(phi + D.N + i), __ldg(phi + 2 * D.N + i), t, false);
-        const float r = t.val - __ldg(T + i);
-        e = fma(0.5 * (double)r, (double)r, e);  // (r / 2) * r is exact in FP64: same bits
+    const Pair P = as_pair(A);
+    double er = 0.0, em = 0.0;
+    GRID_STRIDE(i, A.N) {
+        if (i % A.Xp >= A.X) {
+            mbar[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            continue;
+        }
+        const SobCell s = sob_locate(P, __ldg(phi + i), __ldg(phi + A.NT + i), __ldg(phi + 2 * A.NT + i));
+        float f[8], d[3], W;
+        load_corners(S, s.base, A.Xp, A.XYp, f);
+        tri_grad(f, s, d, &W, nullptr);
+        const float r = W - __ldg(T + i);
+        er = fma((double)r, (double)r, er);
+        float mc[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const float mc = __ldg(m + (long long)c * D.N + i);
-            e += 0.1 * (double)mc * (double)mc;
-            pbar[(long long)c * D.N + i] = r * t.d[c];
-            mbar[(long long)c * D.N + i] = 0.2f * mc;
+            mc[c] = __ldg(m + c * A.NT + i);
+            em = fma((double)mc[c], (double)mc[c], em);
+            pbar[c * A.NT + i] = r * d[c];
         }
+        mbar[i] = make_float4(0.2f * mc[0], 0.2f * mc[1], 0.2f * mc[2], 0.f);
     }
-    e = block_sum_f64(e, red);
+    const double e = block_sum_f64(0.5 * er + 0.1 * em, red);
     if (threadIdx.x == 0) atomicAdd(loss, e);
 }
 
-// phi' = phi + m'(phi): pbar_k = pbar + (dm'/dphi)^T pbar, mbar += scatter(w * pbar), the
-// scatter warp-aggregated (scatter_cell_warp)
-__global__ void adj_update_kernel(AdjDims D, const float* __restrict__ phi, const float* __restrict__ mn,
-                                  const float* __restrict__ pbar, float* pbar_k, float* mbar) {
-    WARP_STRIDE(i, act, D.N) {
-        const int k = act ? i : 0;
-        const float p[3] = {__ldg(phi + k), __ldg(phi + D.N + k), __ldg(phi + 2 * D.N + k)};
-        float acc[3] = {__ldg(pbar + k), __ldg(pbar + D.N + k), __ldg(pbar + 2 * D.N + k)};
+// Adds the contributions v[0..3] to the corners 00, 10, 01, 11 (x, y) of the face at `b` of the
+// interleaved field F: one 16-byte reduction per corner for the three components, and the x
+// corners that neighbouring lanes share added once: the lanes of a warp hold consecutive
+// voxels of a row, whose cells are usually consecutive along x, so lane k adds lane k - 1's x + 1
+// contribution to its own x one.  All 32 lanes must call it; inactive lanes pass act = false.
+__device__ __forceinline__ void red_add4(float4* p, float3 v) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(0.f)
+                 : "memory");
+}
+__device__ __forceinline__ void scatter_face_warp(float4* F, int b, const float3 v[4], bool act, int X) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int bprev = __shfl_up_sync(full, act ? b : -4, 1);
+    const bool merge = act && lane > 0 && bprev == b - 1;
+    const bool next_merges = __shfl_down_sync(full, (int)merge, 1) != 0 && lane < 31;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const float3 c1 = v[2 * j + 1];
+        float3 c0 = v[2 * j];
+        const float px = __shfl_up_sync(full, c1.x, 1), py = __shfl_up_sync(full, c1.y, 1),
+                    pz = __shfl_up_sync(full, c1.z, 1);
+        if (merge) c0 = make_float3(c0.x + px, c0.y + py, c0.z + pz);
+        if (act) {
+            red_add4(F + b + j * X, c0);
+            if (!next_merges) red_add4(F + b + 1 + j * X, c1);
+        }
+    }
+}
+
+// phi' = phi + m'(phi): pbar += (dm'/dphi)^T pbar (in place: a voxel reads only its own), mbar +=
+// scatter(w * pbar).
+//
+// A thread owns a column of a 32 x 8 x depth tile.  The reductions bound the kernel (about one lane's
+// reduction a cycle and SM whatever its width), so they are made few and wide: mbar is
+// interleaved, a 16-byte reduction per corner serves the three components; neighbouring lanes
+// share corners (scatter_face_warp); and the upper face of a voxel's cell, which is the lower
+// face of the next slice's cell where the cell moves up by exactly one slice, is held back and
+// added there.  The gathered corners are kept the same way, as in sob_pass_b_kernel.  On the
+// 128^3 pair 40 us; with one 4-byte reduction per corner and component, lanes merged, 144 us.
+__global__ void __launch_bounds__(256) adj_update_kernel(AdjPair A, const float* __restrict__ phi,
+                                                         const float* __restrict__ mn, float* pbar, float4* mbar) {
+    const Pair P = as_pair(A);
+    const int nx = (A.X + kTileX - 1) / kTileX, ny = (A.Y + kTileY - 1) / kTileY;
+    const int x = (blockIdx.x % nx) * kTileX + (threadIdx.x & 31), y = (blockIdx.x / nx % ny) * kTileY + (threadIdx.x >> 5);
+    const int z0 = (int)(blockIdx.x / (nx * ny)) * A.depth, z1 = min(z0 + A.depth, A.Z);
+    const bool act = x < A.X && y < A.Y;
+    const int Xp = A.Xp, XY = A.XYp;
+    int i = act ? x + Xp * y + XY * z0 : 0;
+    float f[3][8];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) f[c][q] = 0.f;
+    float3 held[4];  // the upper face's contributions of the previous slice's cell
+#pragma unroll
+    for (int q = 0; q < 4; ++q) held[q] = make_float3(0.f, 0.f, 0.f);
+    int above = -1;  // base of the cell above the previous slice's cell (-1: none)
+    float np[3], nb[3];  // phi and pbar of the next slice, loaded while this one's gathers are in flight
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        np[c] = __ldg(phi + c * A.NT + i);
+        nb[c] = pbar[c * A.NT + i];
+    }
+    for (int z = z0; z < z1; ++z, i += act ? XY : 0) {
+        const SobCell s = sob_locate(P, np[0], np[1], np[2]);
+        const int b = s.base;
+        const bool on = b == above;
+        float acc[3], pb[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            TriEval t;
-            tri_eval(D, mn + (long long)c * D.N, p[0], p[1], p[2], t, false);
-            const float pb = __ldg(pbar + (long long)c * D.N + k);
+            const float* __restrict__ F = mn + c * A.NT;
+            f[c][1] = f[c][0];
+            f[c][3] = f[c][2];
+            f[c][5] = f[c][4];
+            f[c][7] = f[c][6];
+            f[c][0] = __ldg(F + b + 1 + Xp + XY);
+            f[c][2] = __ldg(F + b + 1 + XY);
+            f[c][4] = __ldg(F + b + Xp + XY);
+            f[c][6] = __ldg(F + b + XY);
+            if (!on) {
+                f[c][1] = __ldg(F + b + 1 + Xp);
+                f[c][3] = __ldg(F + b + 1);
+                f[c][5] = __ldg(F + b + Xp);
+                f[c][7] = __ldg(F + b);
+            }
+            acc[c] = pb[c] = nb[c];
+        }
+        if (act && z + 1 < z1)
 #pragma unroll
-            for (int j = 0; j < 3; ++j) acc[j] += pb * t.d[j];
-            float cw[8];
+            for (int c = 0; c < 3; ++c) {
+                np[c] = __ldg(phi + c * A.NT + i + XY);
+                nb[c] = pbar[c * A.NT + i + XY];
+            }
 #pragma unroll
-            for (int q = 0; q < 8; ++q) cw[q] = t.w[q] * pb;
-            scatter_cell_warp(mbar + (long long)c * D.N, t.off[0], cw, act, D.X, D.XY);
+        for (int c = 0; c < 3; ++c) {
+            float d[3];
+            tri_grad(f[c], s, d, nullptr, nullptr);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) acc[k] += pb[c] * d[k];
         }
         if (act)
 #pragma unroll
-            for (int j = 0; j < 3; ++j) pbar_k[(long long)j * D.N + i] = acc[j];
+            for (int c = 0; c < 3; ++c) pbar[c * A.NT + i] = acc[c];
+        // what the cell does not take over from the slice below is added where it belongs
+        const bool flush = act && !on && above >= 0;
+        if (__any_sync(0xffffffffu, flush)) scatter_face_warp(mbar, above, held, flush, Xp);
+        float3 low[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float w = ((q & 1) ? s.a : 1.f - s.a) * ((q & 2) ? s.b : 1.f - s.b);
+            const float w0 = w * (1.f - s.c), w1 = w * s.c;
+            low[q] = make_float3(w0 * pb[0], w0 * pb[1], w0 * pb[2]);
+            if (on) low[q] = make_float3(low[q].x + held[q].x, low[q].y + held[q].y, low[q].z + held[q].z);
+            held[q] = make_float3(w1 * pb[0], w1 * pb[1], w1 * pb[2]);
+        }
+        scatter_face_warp(mbar, b, low, act, Xp);
+        above = b + XY;
+    }
+    scatter_face_warp(mbar, above, held, act && above >= 0, Xp);
+}
+
+// m' = damping * m - step * gs: gs = -step * mbar (planes), mbar = damping * mbar; zero pad columns stay zero
+__global__ void __launch_bounds__(256) adj_momentum_kernel(AdjPair A, float damping, float step, float4* mbar, float* gs) {
+    GRID_STRIDE(i, A.N) {
+        const float4 v = mbar[i];
+        gs[i] = -step * v.x;
+        gs[A.NT + i] = -step * v.y;
+        gs[2 * A.NT + i] = -step * v.z;
+        mbar[i] = make_float4(damping * v.x, damping * v.y, damping * v.z, 0.f);
     }
 }
 
-// m' = damping * m - step * gs: gsbar = -step * mbar, mbar_k = damping * mbar
-__global__ void adj_momentum_kernel(AdjDims D, float damping, float step, float* mbar, float* gsbar) {
-    GRID_STRIDE(i, 3 * D.N) {
-        const float mb = mbar[i];
-        gsbar[i] = -step * mb;
-        mbar[i] = damping * mb;
-    }
+// s + c += a * b with the product and the sum exact to about twice the FP32 precision (the
+// compensated dot product Dot2 of Ogita, Rump and Oishi, 2005)
+__device__ __forceinline__ void dot2(float a, float b, float& s, float& c) {
+    const float p = a * b, e = fmaf(a, b, -p);
+    const float t = s + p, u = t - s;
+    c += e + ((s - (t - u)) + (p - u));
+    s = t;
 }
 
-// transpose of one replicate-boundary pass of radius R, gather form: dst(y) = sum over x
-// of src(x) * sum_k w_k [clamp(x + k) == y]
-template <int R>
-__global__ void adj_smooth_t_kernel(AdjDims D, SobIterArgs a, int axis, const float* __restrict__ src, float* dst) {
-    const int dim = axis == 0 ? D.X : (axis == 1 ? D.Y : D.Z);
-    const int stride = axis == 0 ? 1 : (axis == 1 ? D.X : D.XY);
-    GRID_STRIDE(i, D.N) {
-        int x, y, z;
-        coords(D, i, x, y, z);
-        const int pos = axis == 0 ? x : (axis == 1 ? y : z);
-        float acc[3] = {0.f, 0.f, 0.f};
-        if (pos >= R && pos <= dim - 1 - R) {
-            // clamped taps land only on the first and last position: inside, the weight of
-            // s = pos + j is the single tap at -j (the sum below with one nonzero term)
+// g = (S(phi) - T) dS(phi) + lambda lap(phi - x): pbar += lambda lap^T(gbar) + (gbar . dS) dS + r H
+// gbar; lambda_bar += gbar . lap.  A thread owns a column of a 32 x 8 x depth tile; its own
+// column of phi and gbar stays in registers from slice to slice, the neighbours along x and y
+// come through L1, and the Laplacians' terms across a z face are formed once (sob_grad_kernel).
+// The kernel waits on its loads, so all of a voxel's are issued before the arithmetic (64 us on
+// the 128^3 pair when each neighbour was loaded where it was used, 46 us now); lambda_bar is
+// summed in compensated FP32 per thread and in FP64 beyond, as the FP64 pipe of this GPU takes
+// 16 cycles per warp and operation (78 us with six FP64 operations and six conversions a voxel).
+__global__ void __launch_bounds__(256) adj_grad_kernel(AdjPair A, const float* __restrict__ S, const float* __restrict__ T,
+                                                       const float* __restrict__ phi, float lambda,
+                                                       const float* __restrict__ gbar, float* pbar, double* lbar) {
+    __shared__ double red[32];
+    const Pair P = as_pair(A);
+    const int nx = (A.X + kTileX - 1) / kTileX, ny = (A.Y + kTileY - 1) / kTileY;
+    const int x = (blockIdx.x % nx) * kTileX + (threadIdx.x & 31), y = (blockIdx.x / nx % ny) * kTileY + (threadIdx.x >> 5);
+    const int z0 = (int)(blockIdx.x / (nx * ny)) * A.depth, z1 = min(z0 + A.depth, A.Z);
+    const int Xp = A.Xp, XY = A.XYp;
+    float ls = 0.f, lc = 0.f;
+    if (x < A.X && y < A.Y) {
+        const bool xl = x > 0, xr = x < A.X - 1, yl = y > 0, yr = y < A.Y - 1;
+        int i = x + Xp * y + XY * z0;
+        float p[3], g[3], pz[3], gz[3];  // phi and gbar here, and their terms across the face below
 #pragma unroll
-            for (int j = -R; j <= R; ++j) {
-                const float w = a.taps[R - j];
-#pragma unroll
-                for (int c = 0; c < 3; ++c) acc[c] += w * __ldg(src + (long long)c * D.N + i + j * stride);
-            }
-        } else if (pos >= 1 && pos <= dim - 2) {
-            for (int s = max(pos - R, 0); s <= min(pos + R, dim - 1); ++s) {
-                const float w = a.taps[pos - s + R];
-#pragma unroll
-                for (int c = 0; c < 3; ++c) acc[c] += w * __ldg(src + (long long)c * D.N + i + (s - pos) * stride);
-            }
-        } else {
-            for (int s = max(pos - R, 0); s <= min(pos + R, dim - 1); ++s) {
-                float w = 0.f;
-                for (int k = -R; k <= R; ++k)
-                    if (min(max(s + k, 0), dim - 1) == pos) w += a.taps[k + R];
-                if (w == 0.f) continue;
-#pragma unroll
-                for (int c = 0; c < 3; ++c) acc[c] += w * __ldg(src + (long long)c * D.N + i + (s - pos) * stride);
+        for (int c = 0; c < 3; ++c) {
+            p[c] = __ldg(phi + c * A.NT + i);
+            g[c] = __ldg(gbar + c * A.NT + i);
+            pz[c] = gz[c] = 0.f;
+            if (z0 > 0) {
+                pz[c] = __ldg(phi + c * A.NT + i - XY) - p[c];
+                if (c == 2) pz[c] += 1.f;
+                gz[c] = __ldg(gbar + c * A.NT + i - XY) - g[c];
             }
         }
+        for (int z = z0; z < z1; ++z, i += XY) {
+            const bool zr = z < A.Z - 1;
+            const SobCell s = sob_locate(P, p[0], p[1], p[2]);
+            float f[8], add[3], gb[3], pn[3][5], gn[3][5], old[3];
+            // every load of the voxel before the arithmetic: neighbours -x, +x, -y, +y, +z (its own
+            // value where there is none), corners, T and pbar
+            load_corners(S, s.base, Xp, XY, f);
+            const float tv = __ldg(T + i);
+            const int off[5] = {xl ? -1 : 0, xr ? 1 : 0, yl ? -Xp : 0, yr ? Xp : 0, zr ? XY : 0};
 #pragma unroll
-        for (int c = 0; c < 3; ++c) dst[(long long)c * D.N + i] = acc[c];
+            for (int c = 0; c < 3; ++c) {
+#pragma unroll
+                for (int k = 0; k < 5; ++k) {
+                    pn[c][k] = __ldg(phi + c * A.NT + i + off[k]);
+                    gn[c][k] = __ldg(gbar + c * A.NT + i + off[k]);
+                }
+                old[c] = pbar[c * A.NT + i];
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const float pc = p[c], gc = g[c];
+                gb[c] = gc;
+                float l = 0.f;
+                if (xl) l += c == 0 ? (pc - pn[c][0]) - 1.f : pc - pn[c][0];
+                if (xr) l += c == 0 ? (pc - pn[c][1]) + 1.f : pc - pn[c][1];
+                if (yl) l += c == 1 ? (pc - pn[c][2]) - 1.f : pc - pn[c][2];
+                if (yr) l += c == 1 ? (pc - pn[c][3]) + 1.f : pc - pn[c][3];
+                l -= pz[c];
+                pz[c] = !zr ? 0.f : c == 2 ? (pc - pn[c][4]) + 1.f : pc - pn[c][4];
+                l += pz[c];
+                const float t = (((gc - gn[c][0]) + (gc - gn[c][1])) + (gc - gn[c][2])) + (gc - gn[c][3]);
+                const float up = gc - gn[c][4];
+                add[c] = lambda * ((t - gz[c]) + up);
+                gz[c] = up;
+                p[c] = pn[c][4];
+                g[c] = gn[c][4];
+                dot2(gc, l, ls, lc);
+            }
+            float d[3], W, H[3];
+            tri_grad(f, s, d, &W, H);
+            const float r = W - tv;
+            const float gd = (gb[0] * d[0] + gb[1] * d[1]) + gb[2] * d[2];
+            const float h[3] = {gb[1] * H[0] + gb[2] * H[1], gb[0] * H[0] + gb[2] * H[2], gb[0] * H[1] + gb[1] * H[2]};
+#pragma unroll
+            for (int k = 0; k < 3; ++k) pbar[k * A.NT + i] = old[k] + (add[k] + (gd * d[k] + r * h[k]));
+        }
     }
-}
-
-// g = (S(phi) - T) dS(phi) + lambda lap(phi - x): pbar_k += lambda lap^T(gbar)
-// + (gbar . dS) dS + r H gbar; lambda_bar += gbar . lap
-__global__ void adj_grad_kernel(AdjDims D, const float* __restrict__ S, const float* __restrict__ T,
-                                const float* __restrict__ phi, float lambda, const float* __restrict__ gbar,
-                                float* pbar_k, double* lbar) {
-    __shared__ double red[32];
-    double lb = 0.0;
-    GRID_STRIDE(i, D.N) {
-        int x, y, z;
-        coords(D, i, x, y, z);
-        float lap[3];
-        lap_u(D, phi, i, x, y, z, lap);
-        const float gb[3] = {__ldg(gbar + i), __ldg(gbar + D.N + i), __ldg(gbar + 2 * D.N + i)};
-#pragma unroll
-        for (int c = 0; c < 3; ++c) lb += (double)gb[c] * (double)lap[c];
-        const bool ok[6] = {x > 0, x < D.X - 1, y > 0, y < D.Y - 1, z > 0, z < D.Z - 1};
-        const int off[6] = {-1, 1, -D.X, D.X, -D.XY, D.XY};
-        float add[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-            for (int k = 0; k < 6; ++k)
-                if (ok[k]) add[c] += lambda * (gb[c] - __ldg(gbar + (long long)c * D.N + i + off[k]));
-        TriEval t;
-        tri_eval(D, S, __ldg(phi + i), __ldg(phi + D.N + i), __ldg(phi + 2 * D.N + i), t, true);
-        const float r = t.val - __ldg(T + i);
-        const float gd = (gb[0] * t.d[0] + gb[1] * t.d[1]) + gb[2] * t.d[2];
-        const float h[3] = {gb[1] * t.H01 + gb[2] * t.H02, gb[0] * t.H01 + gb[2] * t.H12, gb[0] * t.H02 + gb[1] * t.H12};
-#pragma unroll
-        for (int j = 0; j < 3; ++j) pbar_k[(long long)j * D.N + i] += add[j] + (gd * t.d[j] + r * h[j]);
-    }
-    lb = block_sum_f64(lb, red);
+    const double lb = block_sum_f64((double)ls + (double)lc, red);
     if (threadIdx.x == 0) atomicAdd(lbar, lb);
-}
-
-__global__ void adj_identity_kernel(AdjDims D, float* phi) {
-    GRID_STRIDE(i, D.N) {
-        int x, y, z;
-        coords(D, i, x, y, z);
-        phi[i] = (float)x;
-        phi[D.N + i] = (float)y;
-        phi[2 * D.N + i] = (float)z;
-    }
-}
-
-// one separable pass (transposed: the adjoint's) with the radius as a template argument
-template <int R>
-void launch_smooth_r(bool transposed, int grid, cudaStream_t s, const AdjDims& D, const SobIterArgs& a, int axis,
-                     const float* src, float* dst, int momentum) {
-    if (transposed)
-        adj_smooth_t_kernel<R><<<grid, 256, 0, s>>>(D, a, axis, src, dst);
-    else
-        adj_fwd_smooth_kernel<R><<<grid, 256, 0, s>>>(D, a, axis, src, dst, momentum);
-}
-
-void launch_smooth(int radius, bool transposed, int grid, cudaStream_t s, const AdjDims& D, const SobIterArgs& a,
-                   int axis, const float* src, float* dst, int momentum) {
-    switch (radius) {
-        case 0: launch_smooth_r<0>(transposed, grid, s, D, a, axis, src, dst, momentum); break;
-        case 1: launch_smooth_r<1>(transposed, grid, s, D, a, axis, src, dst, momentum); break;
-        case 2: launch_smooth_r<2>(transposed, grid, s, D, a, axis, src, dst, momentum); break;
-        case 3: launch_smooth_r<3>(transposed, grid, s, D, a, axis, src, dst, momentum); break;
-        case 4: launch_smooth_r<4>(transposed, grid, s, D, a, axis, src, dst, momentum); break;
-        case 5: launch_smooth_r<5>(transposed, grid, s, D, a, axis, src, dst, momentum); break;
-        case 6: launch_smooth_r<6>(transposed, grid, s, D, a, axis, src, dst, momentum); break;
-        default: launch_smooth_r<7>(transposed, grid, s, D, a, axis, src, dst, momentum); break;
-    }
 }
 
 }  // namespace frg
 
 namespace {
-
-struct AdjBuffers {
-    float* block = nullptr;
-    size_t floats = 0;
-};
 
 // The device workspace of fr_sobolev_loss_grad (checkpoints, segment states and adjoint
 // fields, about 40 fields of 3 N floats for 50 iterations), kept per device and reused by
@@ -473,91 +575,191 @@ extern "C" int fr_sobolev_loss_grad(const float* d_T, const float* d_S, const in
         set_global_error("fr_sobolev_loss_grad: volume too large (limit 2^30 voxels)");
         return FR_ERR_INVALID_ARG;
     }
-    AdjDims D{dims[0], dims[1], dims[2], dims[0] * dims[1], (int)N64};
-    const size_t N = (size_t)N64, N3 = 3 * N;
-    const int K = iters, ck = std::min(checkpoint_every, iters);
-    const int nck = (K + ck - 1) / ck + 1;
+    AdjPair A{};
+    A.X = dims[0];
+    A.Y = dims[1];
+    A.Z = dims[2];
+    A.Xp = (A.X + 3) / 4 * 4;
+    A.XYp = A.Xp * A.Y;
+    A.N = A.XYp * A.Z;
+    A.NT = ((long long)A.N + 31) / 32 * 32;
+    const size_t N3 = 3 * (size_t)A.NT;
+    const int K = iters, ck = std::min(checkpoint_every, iters), nseg = (K + ck - 1) / ck;
     cudaStream_t s = (cudaStream_t)stream;
-    SobIterArgs a{};
-    gaussian_taps(smooth_sigma, smooth_width, a.taps);
-    a.radius = smooth_width / 2;
-    a.damping = damping;
-    a.step = step;
-    // buffers: checkpoints (phi, m) x nck, segment states (phi_k, m_{k+1}) x ck, working phi, m,
-    // g, tmp, adjoint pbar, pbar_k, mbar, gbar (+ 2 doubles)
-    const size_t floats = N3 * (2 * nck + 2 * ck + 8) + 64;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
         cudaGetLastError();
         set_global_error("fr_sobolev_loss_grad: no current CUDA device");
         return FR_ERR_CUDA;
     }
+    const int R = smooth_width / 2;
+    // Tiles of the gradient, the smoothing, the update and the transposed smoothing (the update's
+    // also give the reverse kernels' columns).  A tile of d slices takes d + extra steps; blocks
+    // beyond `per_sm` per SM slow one another down instead of filling idle issue slots.  With the
+    // blocks per SM below the depth chosen is within 4% of the best one measured at 45x54x45,
+    // 64^3, 96^3 and 128^3 (20 iterations); the column kernels gain from many small tiles (128^3:
+    // 6.15 ms at 6 slices, 6.48 at 13), so theirs are held to 6 slices.
+    struct Cut {
+        int rows, depth, count;
+    };
+    auto cut = [&](int per_sm, int rows, int extra, int most, double* cost) {
+        const long long cols = (long long)((A.X + kTileX - 1) / kTileX) * ((A.Y + rows - 1) / rows);
+        Cut best{rows, 1, 0};
+        *cost = 1e300;
+        for (int d = 1; d <= std::min(A.Z, most); ++d) {
+            const long long tiles = cols * ((A.Z + d - 1) / d);
+            const double c = std::max(1.0, (double)tiles / ((double)sms * per_sm)) * (d + extra) * (rows + extra);
+            if (c < *cost) {
+                *cost = c;
+                best = Cut{rows, d, (int)tiles};
+            }
+        }
+        return best;
+    };
+    double cost = 0.0, cost_tall = 0.0;
+    Cut cuts[4];
+    cuts[0] = cut(6, kTileY, 2, 128, &cost);
+    cuts[2] = cut(4, kTileY, 1, 6, &cost);
+    const Cut low = cut(3, sob_smooth_tile_y(R, false), 2 * R + 1, 128, &cost);
+    const Cut high = cut(3, sob_smooth_tile_y(R, true), 2 * R + 1, 128, &cost_tall);
+    const bool tall = cost_tall < cost;
+    cuts[1] = cuts[3] = tall ? high : low;
+    A.depth = cuts[2].depth;
+
+    // the workspace: checkpoints (phi, m) x nseg, the states of a segment (phi, m) x ck, two
+    // working states, g, gbar, pbar, the interleaved mbar, S and T; and a small head
+    auto round_up = [](size_t b) { return (b + 255) / 256 * 256; };
+    size_t head = round_up(sizeof(Pair)) + round_up(64);
+    for (const Cut& c : cuts) head += round_up(sizeof(Tile) * (size_t)c.count);
+    const size_t plane = round_up(N3 * sizeof(float)), scalar = round_up((size_t)A.NT * sizeof(float));
+    const size_t bytes = head + plane * (2 * nseg + 2 * ck + 4 + 3) + round_up((size_t)A.NT * sizeof(float4)) + 2 * scalar;
     bool cached = false;
-    float* blk = acquire_workspace(dev, floats, &cached);
+    char* blk = reinterpret_cast<char*>(acquire_workspace(dev, (bytes + 3) / 4, &cached));
     if (!blk) {
         set_global_error("fr_sobolev_loss_grad: device allocation failed");
         return FR_ERR_ALLOC;
     }
-    float* ckpt = blk;                          // [nck][2][3N]
-    float* seg = ckpt + N3 * 2 * nck;          // [ck][2][3N]
-    float* phi = seg + N3 * 2 * ck;
-    float* m = phi + N3;
-    float* g = m + N3;
-    float* tmp = g + N3;
-    float* pbar = tmp + N3;
-    float* pbar_k = pbar + N3;
-    float* mbar = pbar_k + N3;
-    float* gbar = mbar + N3;
-    double* dd = (double*)(((uintptr_t)(gbar + N3) + 15) & ~(uintptr_t)15);  // loss, lambda_bar
-    const int grid = grid_for(N64);
-    int rc = FR_OK;
-    auto fwd_step = [&]() {
-        adj_fwd_grad_kernel<<<grid, 256, 0, s>>>(D, d_S, d_T, phi, lambda, g);
-        launch_smooth(a.radius, false, grid, s, D, a, 0, g, tmp, 0);
-        launch_smooth(a.radius, false, grid, s, D, a, 1, tmp, g, 0);
-        launch_smooth(a.radius, false, grid, s, D, a, 2, g, m, 1);
-        adj_fwd_update_kernel<<<grid, 256, 0, s>>>(D, m, phi);
+    char* at = blk;
+    auto take = [&](size_t b) {
+        char* p = at;
+        at += round_up(b);
+        return p;
     };
-    auto copy = [&](float* dst, const float* src) {
-        return cudaMemcpyAsync(dst, src, N3 * sizeof(float), cudaMemcpyDeviceToDevice, s);
+    Pair* pair = (Pair*)take(sizeof(Pair));
+    char* small = take(64);  // loss and lambda_bar; the pair's stop word
+    double* dd = (double*)small;
+    AdjTables tables{};
+    for (int k = 0; k < 4; ++k) {
+        tables.at[k] = (Tile*)take(sizeof(Tile) * (size_t)cuts[k].count);
+        tables.rows[k] = cuts[k].rows;
+        tables.depth[k] = cuts[k].depth;
+        tables.count[k] = cuts[k].count;
+    }
+    auto field = [&]() { return (float*)take(N3 * sizeof(float)); };
+    struct State {
+        float *phi, *m;
+    };
+    std::vector<State> ckpt(nseg), seg(ck);  // seg[j]: the state after iteration j of a segment
+    for (State& c : ckpt) c = State{field(), field()};
+    for (State& c : seg) c = State{field(), field()};
+    State work[2] = {{field(), field()}, {field(), field()}};
+    float *g = field(), *gbar = field(), *pbar = field();
+    float4* mbar = (float4*)take((size_t)A.NT * sizeof(float4));
+    float *Sp = (float*)take((size_t)A.NT * sizeof(float)), *Tp = (float*)take((size_t)A.NT * sizeof(float));
+
+    SobIterArgs a{};
+    a.pairs = pair;
+    a.tiles_g = tables.at[0];
+    a.ntiles_g = cuts[0].count;
+    a.depth_g = cuts[0].depth;
+    a.tiles_b = tables.at[2];
+    a.ntiles_b = cuts[2].count;
+    a.depth_b = cuts[2].depth;
+    a.npairs = 1;
+    a.NT = A.NT;
+    a.S = Sp;
+    a.T = Tp;
+    a.g = g;
+    a.damping = damping;
+    a.step = step;
+    a.lambda = lambda;
+    gaussian_taps(smooth_sigma, smooth_width, a.taps);
+    a.radius = R;
+    fold_weights(a.taps, R, a.fold);
+    a.stop = (int*)(small + 16);  // 0: no convergence test ends the unrolled iterations
+    const int grid = grid_for(A.N), columns = cuts[2].count;
+    int rc = FR_OK;
+    auto ok = [&](cudaError_t e) {
+        if (e != cudaSuccess) rc = FR_ERR_CUDA;
+        return rc == FR_OK;
+    };
+    // iteration k (0-based) from one state to another; a segment's last phi is needed only
+    // where the next segment or the loss starts from it
+    auto forward = [&](int k, const State& from, const State& to, bool update) {
+        a.iter = k + 1;
+        a.phi = from.phi;
+        a.m = from.m;
+        a.phi_n = to.phi;
+        a.m_n = to.m;
+        a.tiles_s = tables.at[1];
+        a.ntiles_s = cuts[1].count;
+        a.depth_s = cuts[1].depth;
+        ok(launch_sob_kernel(0, a, cuts[0].count, 0, s));
+        ok(launch_sob_kernel(1, a, cuts[1].count, kUnrolled | (tall ? 2 : 0), s));
+        if (update) ok(launch_sob_kernel(2, a, cuts[2].count, kUnrolled, s));
+    };
+    auto smooth_adjoint = [&]() {  // gbar = G^T g
+        SobIterArgs t = a;
+        t.m_n = gbar;
+        t.tiles_s = tables.at[3];
+        t.ntiles_s = cuts[3].count;
+        t.depth_s = cuts[3].depth;
+        void* args[1] = {&t};
+        ok(cudaLaunchKernel(sob_smooth3_unrolled_fn(R, true, tall), dim3(cuts[3].count), dim3(kSmoothThreads), args, 0, s));
     };
     do {
-        if (cudaMemsetAsync(dd, 0, 2 * sizeof(double), s) != cudaSuccess) { rc = FR_ERR_CUDA; break; }
-        adj_identity_kernel<<<grid, 256, 0, s>>>(D, phi);
-        if (copy(m, d_v0) != cudaSuccess) { rc = FR_ERR_CUDA; break; }
-        // forward with checkpoints every ck iterations
-        for (int k = 0; k < K; ++k) {
-            if (k % ck == 0) {
-                copy(ckpt + N3 * 2 * (k / ck), phi);
-                copy(ckpt + N3 * (2 * (k / ck) + 1), m);
-            }
-            fwd_step();
+        Pair hp{};
+        hp.X = A.X;
+        hp.Y = A.Y;
+        hp.Z = A.Z;
+        hp.Xp = A.Xp;
+        hp.N = A.N;
+        hp.w_reg = lambda;
+        if (!ok(cudaMemcpyAsync(pair, &hp, sizeof hp, cudaMemcpyHostToDevice, s))) break;
+        if (!ok(cudaMemsetAsync(small, 0, 64, s))) break;
+        adj_tables_kernel<<<sms, 256, 0, s>>>(A, tables);
+        adj_pack_kernel<<<grid, 256, 0, s>>>(A, d_S, d_T, d_v0, Sp, Tp, ckpt[0].phi, ckpt[0].m);
+        // forward: a segment's first state is its checkpoint, and the last segment's states stay
+        State st = ckpt[0];
+        for (int k = 0; k < K && rc == FR_OK; ++k) {
+            const int j = k % ck;
+            const bool last_segment = k / ck == nseg - 1;
+            const State to = last_segment ? seg[j] : j == ck - 1 ? ckpt[k / ck + 1] : work[k & 1];
+            forward(k, st, to, true);
+            st = to;
         }
-        adj_loss_kernel<<<grid, 256, 0, s>>>(D, d_S, d_T, phi, m, pbar, mbar, dd);
+        adj_loss_kernel<<<grid, 256, 0, s>>>(A, Sp, Tp, st.phi, st.m, pbar, mbar, dd);
         if (!d_grad_v0) break;
         // reverse, one segment at a time
-        for (int s0 = ((K - 1) / ck) * ck; s0 >= 0; s0 -= ck) {
-            const int s1 = std::min(s0 + ck, K);
-            copy(phi, ckpt + N3 * 2 * (s0 / ck));
-            copy(m, ckpt + N3 * (2 * (s0 / ck) + 1));
-            for (int k = s0; k < s1; ++k) {
-                copy(seg + N3 * 2 * (k - s0), phi);  // phi_k
-                fwd_step();
-                copy(seg + N3 * (2 * (k - s0) + 1), m);  // m_{k+1}
+        for (int q = nseg - 1; q >= 0 && rc == FR_OK; --q) {
+            const int s0 = q * ck, s1 = std::min(s0 + ck, K);
+            if (q < nseg - 1) {
+                st = ckpt[q];
+                for (int k = s0; k < s1; ++k) {
+                    forward(k, st, seg[k - s0], k + 1 < s1);
+                    st = seg[k - s0];
+                }
             }
             for (int k = s1 - 1; k >= s0; --k) {
-                const float* phik = seg + N3 * 2 * (k - s0);
-                const float* mn = seg + N3 * (2 * (k - s0) + 1);
-                adj_update_kernel<<<grid, 256, 0, s>>>(D, phik, mn, pbar, pbar_k, mbar);
-                adj_momentum_kernel<<<grid, 256, 0, s>>>(D, damping, step, mbar, g);
-                launch_smooth(a.radius, true, grid, s, D, a, 2, g, tmp, 0);
-                launch_smooth(a.radius, true, grid, s, D, a, 1, tmp, g, 0);
-                launch_smooth(a.radius, true, grid, s, D, a, 0, g, gbar, 0);
-                adj_grad_kernel<<<grid, 256, 0, s>>>(D, d_S, d_T, phik, lambda, gbar, pbar_k, dd + 1);
-                std::swap(pbar, pbar_k);
+                const float* phik = k == s0 ? ckpt[q].phi : seg[k - s0 - 1].phi;
+                adj_update_kernel<<<columns, 256, 0, s>>>(A, phik, seg[k - s0].m, pbar, mbar);
+                adj_momentum_kernel<<<grid, 256, 0, s>>>(A, damping, step, mbar, g);
+                smooth_adjoint();
+                adj_grad_kernel<<<columns, 256, 0, s>>>(A, Sp, Tp, phik, lambda, gbar, pbar, dd + 1);
             }
         }
-        if (copy(d_grad_v0, mbar) != cudaSuccess) { rc = FR_ERR_CUDA; break; }
+        adj_unpack_kernel<<<grid, 256, 0, s>>>(A, mbar, d_grad_v0);
     } while (0);
     double host[2] = {0.0, 0.0};
     if (rc == FR_OK) {
@@ -567,7 +769,7 @@ extern "C" int fr_sobolev_loss_grad(const float* d_T, const float* d_S, const in
             rc = FR_ERR_CUDA;
     }
     if (rc != FR_OK) cudaStreamSynchronize(s);  // nothing may still use the workspace
-    release_workspace(dev, blk, cached);
+    release_workspace(dev, reinterpret_cast<float*>(blk), cached);
     if (rc != FR_OK) {
         cudaGetLastError();
         set_global_error("fr_sobolev_loss_grad: a CUDA call failed");

@@ -240,7 +240,7 @@ std::vector<int> active_roles(const fr_handle* h) {
 }
 
 // kernels with a TMA-staged variant
-bool has_tma_variant(int r) { return r != R_COUNT; }  // every solver kernel has one
+bool has_tma_variant(int r) { return r != R_PB && r != R_SB; }  // the update kernels gather through L1
 
 // the staging variants kernel r may run with this handle's STAGING and cohort
 std::vector<int> allowed_variants(const fr_handle* h, int r) {
@@ -258,10 +258,10 @@ const void* role_fn(const fr_handle* h, int r, int variant = 0) {
     switch (r) {
         case R_LAP: return variant ? (const void*)frg::ref_laplacian_tma_kernel : (const void*)frg::ref_laplacian_kernel;
         case R_PA: return variant ? (const void*)frg::ref_pass_a_tma_kernel : (const void*)frg::ref_pass_a_kernel;
-        case R_PB: return variant ? (const void*)frg::ref_pass_b_staged_kernel : (const void*)frg::ref_pass_b_kernel;
+        case R_PB: return (const void*)frg::ref_pass_b_kernel;
         case R_SG: return frg::sob_grad_fn(variant);
         case R_SS: return frg::sob_smooth3_fn(h->P.smooth_width / 2, variant & 1, variant & 2);
-        default: return variant ? (const void*)frg::sob_pass_b_staged_kernel : (const void*)frg::sob_pass_b_kernel;
+        default: return frg::sob_pass_b_fn(false);
     }
 }
 
@@ -270,8 +270,6 @@ size_t role_smem(int r, int variant = 0) {
         case R_LAP: return variant ? frg::ref_laplacian_tma_smem_bytes() : frg::ref_laplacian_smem_bytes();
         case R_PA: return variant ? frg::ref_pass_a_tma_smem_bytes() : frg::ref_pass_a_smem_bytes();
         case R_SG: return frg::sob_grad_smem_bytes();
-        case R_PB:
-        case R_SB: return variant ? frg::gather_staged_smem_bytes() : 0;
         default: return 0;
     }
 }
@@ -280,11 +278,11 @@ size_t role_smem(int r, int variant = 0) {
 int role_threads(int r, int variant = 0) {
     if (r == R_SG) return frg::sob_grad_threads(variant);
     if (r == R_SS) return frg::kSmoothThreads;
-    return (r == R_PB && variant == 0) ? frg::kPassBThreads : 256;
+    return r == R_PB ? frg::kPassBThreads : 256;
 }
 int role_tile_y(const fr_handle* h, int r, int variant = 0) {
     if (r == R_SS) return frg::sob_smooth_tile_y(h->P.smooth_width / 2, variant & 2);
-    return (r == R_PB && variant == 0) ? frg::kPassBTileY : frg::kTileY;
+    return r == R_PB ? frg::kPassBTileY : frg::kTileY;
 }
 
 typedef std::array<Shape, R_COUNT> Shapes;
@@ -409,16 +407,6 @@ int encode_tmaps(fr_handle* h) {
             }
             int rc = encode_map(h, m + frg::TM_PA_S, h->S + P.off, 3, d3, s3, b3);
             if (rc != FR_OK) return rc;
-        }
-        {  // the gathered field of the update kernel: v (both buffers) or the momentum
-            const cuuint64_t d4[4] = {Xp, Y, Z, 3}, s4[3] = {4 * Xp, 4 * Xp * Y, fstride};
-            const cuuint32_t bg[4] = {frg::kGBX, frg::kGBY, frg::kGBZ, 3};
-            const int nb = h->P.solver == FR_SOLVER_REFERENCE ? 2 : 1;
-            for (int k = 0; k < nb; ++k) {
-                int rc = encode_map(h, m + (nb == 2 ? frg::TM_PB_V0 + k : frg::TM_SB_M), h->v[k] + P.off, 4, d4, s4,
-                                    bg);
-                if (rc != FR_OK) return rc;
-            }
         }
         if (h->P.solver == FR_SOLVER_SOBOLEV) {
             const cuuint64_t dims[4] = {Xp, Y, Z, 3}, strides[3] = {4 * Xp, 4 * Xp * Y, fstride};
@@ -566,9 +554,6 @@ int setup_cohort(fr_handle* h, const fr_pair* pairs, int n) {
                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)frg::ref_pass_a_tma_smem_bytes()));
     }
-    FR_CUDA(h, cudaFuncSetAttribute(role_fn(h, h->P.solver == FR_SOLVER_REFERENCE ? R_PB : R_SB, 1),
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)frg::gather_staged_smem_bytes()));
     h->tma_ok = encode_tmaps(h) == FR_OK;
     if (!h->tma_ok && h->P.staging == 2) {
         const std::string why = h->err;
@@ -654,10 +639,7 @@ int launch_ref_iter(fr_handle* h, int iter, float t, cudaStream_t s, cudaEvent_t
     else
         frg::ref_pass_a_kernel<<<h->ts[R_PA].grid, 256, frg::ref_pass_a_smem_bytes(), s>>>(a);
     if (ev) cudaEventRecord(ev[2], s);
-    if (h->ts[R_PB].shape.variant)
-        frg::ref_pass_b_staged_kernel<<<h->ts[R_PB].grid, 256, frg::gather_staged_smem_bytes(), s>>>(a);
-    else
-        frg::ref_pass_b_kernel<<<h->ts[R_PB].grid, frg::kPassBThreads, 0, s>>>(a);
+    frg::ref_pass_b_kernel<<<h->ts[R_PB].grid, frg::kPassBThreads, 0, s>>>(a);
     if (ev) cudaEventRecord(ev[3], s);
     FR_LAUNCHED(h);
     return FR_OK;
@@ -682,8 +664,8 @@ frg::SobIterArgs sob_args(fr_handle* h, int iter) {
     a.NT = h->NT;
     a.S = h->S;
     a.T = h->T;
-    a.phi = h->psi;
-    a.m = h->v[0];
+    a.phi = a.phi_n = h->psi;
+    a.m = a.m_n = h->v[0];
     a.g = h->grad;
     a.damping = h->P.damping;
     a.step = h->P.step;

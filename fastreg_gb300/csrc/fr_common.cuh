@@ -290,6 +290,11 @@ __device__ __forceinline__ void cp_async16(float* smem, const float* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
+// the same, or 16 bytes of zeros (nothing is read then)
+__device__ __forceinline__ void cp_async16_or_zero(float* smem, const float* gmem, bool copy) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(copy ? 16 : 0) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int Pending>
 __device__ __forceinline__ void cp_async_wait() {

@@ -92,9 +92,20 @@ __device__ __forceinline__ void fix_edges(float* box, int x0, int y0, int X, int
     }
 }
 
-template <int R, bool TMA, int TY>
+// The transpose, with cp.async staging.  Inside the volume it is the same filter
+// (the taps are symmetric) of g continued by zeros, since a tap that the forward pass clamps
+// lands on the first or last position of its axis; those positions take, from the position s
+// beside them, all taps up to tap R - s instead of that tap alone: fold[s] more.
+// MODE: what the filter feeds.
+enum SmoothMode {
+    kInPlace,    // the momentum, updated in place (m_n is m; a second pointer costs the TMA kernel 4%)
+    kOutOfPlace, // the momentum, read from m and written to m_n
+    kTranspose   // m_n = G^T g
+};
+template <int R, bool TMA, int TY, SmoothMode MODE>
 __global__ void __launch_bounds__(kSmoothThreads) sob_smooth3_kernel(SobIterArgs a) {
     using G = SmoothGeom<R, TY>;
+    constexpr bool ADJ = MODE == kTranspose;
     constexpr int K = G::K, WS = G::WS, NS = G::NS, NP = TY / 2;
     __shared__ __align__(128) float rings[3][NS][G::SLOT];
     __shared__ __align__(8) uint64_t bars[3][NS];
@@ -131,7 +142,9 @@ __global__ void __launch_bounds__(kSmoothThreads) sob_smooth3_kernel(SobIterArgs
 #pragma unroll
             for (int j = 0; j < NJ; ++j) {
                 const int f = lane + 32 * j, r = f / (WS / 4), x = x0 - G::HX + 4 * (f % (WS / 4));
-                goff[j] = f < NF && x >= 0 && x < Xp ? Xp * min(max(y0 - R + r, 0), Y - 1) + x : -1;
+                const int yr = y0 - R + r;
+                const bool in = f < NF && x >= 0 && x < Xp && (!ADJ || (yr >= 0 && yr < Y));
+                goff[j] = in ? Xp * min(max(yr, 0), Y - 1) + x : -1;
             }
         }
         auto issue = [&](int k) {  // slice k of the tile (z = zt0 - R + k, clamped) into the next slot
@@ -146,7 +159,12 @@ __global__ void __launch_bounds__(kSmoothThreads) sob_smooth3_kernel(SobIterArgs
                 const float* src = gc + (long long)XY * z;
 #pragma unroll
                 for (int j = 0; j < NJ; ++j)
-                    if (goff[j] >= 0) cp_async16(dst + 128 * j, src + goff[j]);
+                    if (ADJ) {  // zeros outside the volume
+                        const bool in = goff[j] >= 0 && zt0 - R + k >= 0 && zt0 - R + k < Z;
+                        if (lane + 32 * j < NF) cp_async16_or_zero(dst + 128 * j, in ? src + goff[j] : src, in);
+                    } else if (goff[j] >= 0) {
+                        cp_async16(dst + 128 * j, src + goff[j]);
+                    }
             }
             issue_slot = issue_slot + 1 == NS ? 0 : issue_slot + 1;
             ++pending;
@@ -161,11 +179,14 @@ __global__ void __launch_bounds__(kSmoothThreads) sob_smooth3_kernel(SobIterArgs
 #pragma unroll
             for (int j = 0; j < (R > 0 ? 2 * R : 1); ++j) part[p][j] = make_float2(0.f, 0.f);
         const int x = x0 + lane, rows = x < X ? min(Y - y0, TY) : 0;  // rows that this lane stores
-        float* m = a.m + c * a.NT + P.off + (x + Xp * y0) + (long long)XY * (zt0 - 2 * R);
-        for (int k = 0; k < nsl; ++k, m += XY) {
+        const long long m0 = c * a.NT + P.off + (x + Xp * y0) + (long long)XY * (zt0 - 2 * R);
+        float* mn = a.m_n + m0;
+        const float* ms = MODE == kOutOfPlace ? a.m + m0 : nullptr;
+        for (int k = 0; k < nsl; ++k, mn += XY, ms += MODE == kOutOfPlace ? XY : 0) {
+            const float* m = MODE == kOutOfPlace ? ms : mn;
             const bool store = k >= 2 * R;  // slice zt0 + k - 2R is complete with this one
             float mo[TY];
-            if (store)
+            if (store && !ADJ)
 #pragma unroll
                 for (int r = 0; r < TY; ++r)
                     if (r < rows) mo[r] = m[Xp * r];
@@ -182,7 +203,7 @@ __global__ void __launch_bounds__(kSmoothThreads) sob_smooth3_kernel(SobIterArgs
                 __syncwarp();
             }
             float* box = ring[slot];
-            if (edge) fix_edges<R, TMA, TY>(box, x0, y0, X, Y);
+            if (edge && !ADJ) fix_edges<R, TMA, TY>(box, x0, y0, X, Y);
             const float* col = box + lane + G::HX - R;
             float2 ev[G::H / 2], od[G::H / 2];  // x-filtered rows (2 r, 2 r + 1) and (2 r - 1, 2 r)
             // row pairs in groups of kILP, whose chains are independent
@@ -195,6 +216,16 @@ __global__ void __launch_bounds__(kSmoothThreads) sob_smooth3_kernel(SobIterArgs
                         ev[rp] = __ffma2_rn(make_float2(a.taps[q], a.taps[q]),
                                             make_float2(col[2 * rp * WS + q], col[(2 * rp + 1) * WS + q]),
                                             q ? ev[rp] : make_float2(0.f, 0.f));
+                if (ADJ && edge && (x == 0 || x == X - 1)) {  // the ends of the x axis
+                    const int step = x == 0 ? 1 : -1;
+#pragma unroll
+                    for (int rp = r0; rp < r0 + kILP && rp < G::H / 2; ++rp)
+#pragma unroll
+                        for (int d = 0; d < R; ++d) {
+                            ev[rp].x = fmaf(a.fold[d], col[2 * rp * WS + R + step * d], ev[rp].x);
+                            ev[rp].y = fmaf(a.fold[d], col[(2 * rp + 1) * WS + R + step * d], ev[rp].y);
+                        }
+                }
 #pragma unroll
                 for (int rp = r0; rp < r0 + kILP && rp < G::H / 2; ++rp)
                     if (rp > 0) od[rp] = make_float2(ev[rp - 1].y, ev[rp].x);
@@ -209,6 +240,19 @@ __global__ void __launch_bounds__(kSmoothThreads) sob_smooth3_kernel(SobIterArgs
                         v[rp - r0] = __ffma2_rn(make_float2(a.taps[q], a.taps[q]), q & 1 ? od[p + (q + 1) / 2] : ev[p + q / 2],
                                                 q ? v[rp - r0] : make_float2(0.f, 0.f));
                     }
+                if (ADJ && edge)  // the ends of the y axis
+#pragma unroll
+                    for (int rp = r0; rp < r0 + kILP && rp < G::H / 2; ++rp) {
+                        if (rp < R) continue;
+                        auto row = [&](int i) { return i & 1 ? ev[i / 2].y : ev[i / 2].x; };
+                        const int i0 = 2 * (rp - R), i1 = i0 + 1;  // output rows; their own staged rows are i + R
+#pragma unroll
+                        for (int d = 0; d < R; ++d) {
+                            if (y0 + i0 == 0) v[rp - r0].x = fmaf(a.fold[d], row(i0 + R + d), v[rp - r0].x);
+                            if (y0 + i0 == Y - 1) v[rp - r0].x = fmaf(a.fold[d], row(i0 + R - d), v[rp - r0].x);
+                            if (y0 + i1 == Y - 1) v[rp - r0].y = fmaf(a.fold[d], row(i1 + R - d), v[rp - r0].y);
+                        }
+                    }
 #pragma unroll
                 for (int j = 2 * R; j >= 0; --j)
 #pragma unroll
@@ -222,13 +266,28 @@ __global__ void __launch_bounds__(kSmoothThreads) sob_smooth3_kernel(SobIterArgs
                         else
                             part[p][j] = n;
                     }
+                if (ADJ) {  // the ends of the z axis: this slice's extra share of output slices 0 and Z - 1
+                    const int zc = zt0 - R + k;
+#pragma unroll
+                    for (int d = 0; d < R; ++d)
+#pragma unroll
+                        for (int rp = r0; rp < r0 + kILP && rp < G::H / 2; ++rp) {
+                            if (rp < R) continue;
+                            const float2 w = make_float2(a.fold[d], a.fold[d]);
+                            if (zc == d) part[rp - R][R + d] = __ffma2_rn(w, v[rp - r0], part[rp - R][R + d]);
+                            if (zc == Z - 1 - d) part[rp - R][R - d] = __ffma2_rn(w, v[rp - r0], part[rp - R][R - d]);
+                        }
+                }
                 if (store)
 #pragma unroll
                     for (int rp = r0; rp < r0 + kILP && rp < G::H / 2; ++rp) {
                         if (rp < R) continue;
                         const int p = rp - R;
-                        if (2 * p < rows) m[Xp * (2 * p)] = a.damping * mo[2 * p] - a.step * o[rp - r0].x;
-                        if (2 * p + 1 < rows) m[Xp * (2 * p + 1)] = a.damping * mo[2 * p + 1] - a.step * o[rp - r0].y;
+                        if (2 * p < rows)
+                            mn[Xp * (2 * p)] = ADJ ? o[rp - r0].x : a.damping * mo[2 * p] - a.step * o[rp - r0].x;
+                        if (2 * p + 1 < rows)
+                            mn[Xp * (2 * p + 1)] =
+                                ADJ ? o[rp - r0].y : a.damping * mo[2 * p + 1] - a.step * o[rp - r0].y;
                     }
             }
             __syncwarp();  // every lane has read the slot
@@ -250,8 +309,21 @@ __global__ void __launch_bounds__(kSmoothThreads) sob_smooth3_kernel(SobIterArgs
 template <int R>
 const void* smooth_fn(int tma, bool tall) {
     constexpr int kShort = sob_smooth_tile_y(R, false), kTall = sob_smooth_tile_y(R, true);
-    if (tall) return tma ? (const void*)sob_smooth3_kernel<R, true, kTall> : (const void*)sob_smooth3_kernel<R, false, kTall>;
-    return tma ? (const void*)sob_smooth3_kernel<R, true, kShort> : (const void*)sob_smooth3_kernel<R, false, kShort>;
+    if (tall)
+        return tma ? (const void*)sob_smooth3_kernel<R, true, kTall, kInPlace>
+                   : (const void*)sob_smooth3_kernel<R, false, kTall, kInPlace>;
+    return tma ? (const void*)sob_smooth3_kernel<R, true, kShort, kInPlace>
+               : (const void*)sob_smooth3_kernel<R, false, kShort, kInPlace>;
+}
+
+template <int R>
+const void* smooth_unrolled_fn(bool transposed, bool tall) {
+    constexpr int kShort = sob_smooth_tile_y(R, false), kTall = sob_smooth_tile_y(R, true);
+    if (transposed)
+        return tall ? (const void*)sob_smooth3_kernel<R, false, kTall, kTranspose>
+                    : (const void*)sob_smooth3_kernel<R, false, kShort, kTranspose>;
+    return tall ? (const void*)sob_smooth3_kernel<R, false, kTall, kOutOfPlace>
+                : (const void*)sob_smooth3_kernel<R, false, kShort, kOutOfPlace>;
 }
 
 }  // namespace
@@ -266,6 +338,19 @@ const void* sob_smooth3_fn(int radius, int tma, bool tall) {
         case 5: return smooth_fn<5>(tma, tall);
         case 6: return smooth_fn<6>(tma, tall);
         default: return smooth_fn<7>(tma, tall);
+    }
+}
+
+const void* sob_smooth3_unrolled_fn(int radius, bool transposed, bool tall) {
+    switch (radius) {
+        case 0: return smooth_unrolled_fn<0>(transposed, tall);
+        case 1: return smooth_unrolled_fn<1>(transposed, tall);
+        case 2: return smooth_unrolled_fn<2>(transposed, tall);
+        case 3: return smooth_unrolled_fn<3>(transposed, tall);
+        case 4: return smooth_unrolled_fn<4>(transposed, tall);
+        case 5: return smooth_unrolled_fn<5>(transposed, tall);
+        case 6: return smooth_unrolled_fn<6>(transposed, tall);
+        default: return smooth_unrolled_fn<7>(transposed, tall);
     }
 }
 

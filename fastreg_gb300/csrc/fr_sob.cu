@@ -25,32 +25,12 @@ void gaussian_taps(float sigma, int width, float* taps) {
     for (int k = 0; k < width; ++k) taps[k] = (float)(w[k] / sum);
 }
 
-// Cell for the sobolev solver: clamp to [0, dim-1], floor clamped to dim-2 so that
-// both corners of every axis are inside the grid; in_x, in_y, in_z: the position was not
-// clamped (a clamped axis has derivative 0).
-struct SobCell {
-    int base;
-    int gx, gy, gz;
-    float a, b, c;
-    bool in_x, in_y, in_z;
-};
-
-__device__ __forceinline__ SobCell sob_locate(const Pair& P, float px, float py, float pz) {
-    SobCell s;
-    const float cx = fminf(fmaxf(0.f, px), (float)(P.X - 1));
-    const float cy = fminf(fmaxf(0.f, py), (float)(P.Y - 1));
-    const float cz = fminf(fmaxf(0.f, pz), (float)(P.Z - 1));
-    s.gx = min((int)floorf(cx), P.X - 2);
-    s.gy = min((int)floorf(cy), P.Y - 2);
-    s.gz = min((int)floorf(cz), P.Z - 2);
-    s.a = cx - (float)s.gx;
-    s.b = cy - (float)s.gy;
-    s.c = cz - (float)s.gz;
-    s.in_x = cx == px;  // false for a NaN
-    s.in_y = cy == py;
-    s.in_z = cz == pz;
-    s.base = s.gx + P.Xp * (s.gy + P.Y * s.gz);
-    return s;
+void fold_weights(const float* taps, int radius, float* fold) {
+    for (int k = 0; k <= radius; ++k) {
+        double sum = 0.0;
+        for (int q = 0; q < radius - k; ++q) sum += (double)taps[q];
+        fold[k] = (float)sum;
+    }
 }
 
 // W = S o phi, r = W - T, g = r * (exact trilinear gradient of the interpolant) + w_reg * (graph
@@ -281,7 +261,10 @@ const void* sob_grad_fn(int tma) {
 // queue now).  Four blocks of 64 registers; five would spill the kept corners, three take 81 us.
 // The reference solver's pass B, whose psi stays near the grid, gains nothing from the
 // reuse (73 against 66 us): its loads mostly hit the same lines, and it needs the warps.
+// UNROLLED: from phi to phi_n, without the update norm and the convergence test; else in place.
+template <bool UNROLLED>
 __global__ void __launch_bounds__(256, 4) sob_pass_b_kernel(SobIterArgs a) {
+    constexpr bool NORM = !UNROLLED;
     __shared__ unsigned long long red[32];
     __shared__ bool last;
     for (int t = blockIdx.x; t < a.ntiles_b; t += gridDim.x) {
@@ -293,8 +276,11 @@ __global__ void __launch_bounds__(256, 4) sob_pass_b_kernel(SobIterArgs a) {
         if (x < P.X && y < P.Y) {
             const long long NT = a.NT;
             const int X = P.Xp, XY = P.Xp * P.Y;  // strides of the packed arrays
-            float* phi[3] = {a.phi + P.off, a.phi + NT + P.off, a.phi + 2 * NT + P.off};
-            const float* __restrict__ mc[3] = {a.m + P.off, a.m + NT + P.off, a.m + 2 * NT + P.off};
+            float* phi_n[3] = {a.phi_n + P.off, a.phi_n + NT + P.off, a.phi_n + 2 * NT + P.off};
+            const float* phi[3] = {phi_n[0], phi_n[1], phi_n[2]};
+            if (UNROLLED)
+                for (int c = 0; c < 3; ++c) phi[c] = a.phi + c * NT + P.off;
+            const float* __restrict__ mc[3] = {a.m_n + P.off, a.m_n + NT + P.off, a.m_n + 2 * NT + P.off};
             const int z1 = min(tl.w + a.depth_b, P.Z);
             int i = x + X * y + XY * tl.w;
             // phi of the next slice is loaded while this slice's gathers are in flight
@@ -338,19 +324,21 @@ __global__ void __launch_bounds__(256, 4) sob_pass_b_kernel(SobIterArgs a) {
                     }
                 above = b + XY;
                 trilerp3(f, s.a, s.b, s.c, u);
-                phi[0][i] = px + u[0];
-                phi[1][i] = py + u[1];
-                phi[2][i] = pz + u[2];
-                const float nrm = norm3_rd(u[0], u[1], u[2]);
-                if (nrm == nrm) {
+                phi_n[0][i] = px + u[0];
+                phi_n[1][i] = py + u[1];
+                phi_n[2][i] = pz + u[2];
+                const float nrm = NORM ? norm3_rd(u[0], u[1], u[2]) : 0.f;
+                if (NORM && nrm == nrm) {
                     const unsigned long long k = norm_key(nrm, i);
                     best = k > best ? k : best;
                 }
             }
         }
+        if (!NORM) continue;
         const unsigned long long bm = block_max_u64(best, red);
         if (threadIdx.x == 0 && bm) atomicMax(a.keys + tl.x, bm);
     }
+    if (!NORM) return;
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) last = (atomicAdd(a.counter, 1u) == gridDim.x - 1);
@@ -367,180 +355,31 @@ __global__ void __launch_bounds__(256, 4) sob_pass_b_kernel(SobIterArgs a) {
     if (threadIdx.x == 0) *a.counter = 0u;
 }
 
-// The compositional update with the gathered neighbourhood of m staged in shared memory,
-// as ref_pass_b_staged_kernel does for v: per slice the block reduces its cells' bounding
-// box and, when it fits kGBX x kGBY x kGBZ, one tensor copy brings that box of m's three
-// components into one of two buffers while the previous slice is gathered.  The sobolev
-// cell's floor is clamped to dim - 2, so every corner is inside the grid; slices whose
-// cells do not fit gather from global memory as sob_pass_b_kernel does, with the same
-// arithmetic.  Waits are bounded as in ref_pass_b_staged_kernel.
-__global__ void __launch_bounds__(256, 4) sob_pass_b_staged_kernel(SobIterArgs a) {
-    constexpr int kPlane = kGBX * kGBY * kGBZ;
-    constexpr unsigned kBytes = sizeof(float) * 3 * kPlane;
-    extern __shared__ __align__(128) unsigned char sb_raw[];
-    float* box = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(sb_raw) + 127) & ~uintptr_t(127));
-    uint64_t* full = reinterpret_cast<uint64_t*>(box + 2 * 3 * kPlane);
-    __shared__ unsigned long long red[32];
-    __shared__ bool last;
-    __shared__ CellBoxSets cb;
-    const int tid = threadIdx.x;
-    if (tid == 0) {
-        mbar_init(full, 1);
-        mbar_init(full + 1, 1);
-        mbar_fence_init();
-        for (int k = 0; k < 3; ++k) cellbox_clear(cb, k);
-    }
-    __syncthreads();
-    unsigned g = 0, nbox = 0;
-    bool failed = false, wait_failed = false;
-    for (int t = blockIdx.x; t < a.ntiles_b && !failed; t += gridDim.x) {
-        const Tile tl = a.tiles_b[t];
-        if (a.stop[tl.x]) continue;
-        const Pair P = a.pairs[tl.x];
-        const int x = tl.y + (int)(tid & 31), y = tl.z + (int)(tid >> 5);
-        const bool col = x < P.X && y < P.Y;
-        const long long NT = a.NT;
-        const int X = P.Xp, XY = P.Xp * P.Y;  // strides of the packed arrays
-        float* phi[3] = {a.phi + P.off, a.phi + NT + P.off, a.phi + 2 * NT + P.off};
-        const float* __restrict__ mc[3] = {a.m + P.off, a.m + NT + P.off, a.m + 2 * NT + P.off};
-        const CUtensorMap* mm = a.tmaps + (long long)tl.x * TM_COUNT + TM_SB_M;
-        const int z0 = tl.w, z1 = min(tl.w + a.depth_b, P.Z);
-        unsigned long long best = 0ull;
-        int i = x + X * y + XY * z0;
-        float px = 0.f, py = 0.f, pz = 0.f;
-        SobCell cl{};
-        if (col) {
-            px = phi[0][i];
-            py = phi[1][i];
-            pz = phi[2][i];
-            cl = sob_locate(P, px, py, pz);
-        }
-        auto plan = [&](unsigned set, int o[3]) -> bool {
-            int lo[3], hi[3];
-            if (!cellbox_read(cb, (int)set, lo, hi)) return false;
-            o[0] = lo[0] & ~3;
-            o[1] = lo[1];
-            o[2] = lo[2];
-            const bool fits = hi[0] + 1 - o[0] < kGBX && hi[1] + 1 - o[1] < kGBY && hi[2] + 1 - o[2] < kGBZ;
-            if (fits && tid == 0) {
-                uint64_t* bar = full + (nbox & 1);
-                mbar_arrive_expect_tx(bar, kBytes);
-                tma_load_4d(box + (nbox & 1) * 3 * kPlane, mm, o[0], o[1], o[2], 0, bar);
-            }
-            return fits;
-        };
-        ++g;
-        cellbox_add(cb, (int)(g % 3), col, cl.gx, cl.gy, cl.gz);
-        if (__syncthreads_or(wait_failed)) {
-            failed = true;
-            break;
-        }
-        if (tid == 0) cellbox_clear(cb, (int)((g - 1) % 3));
-        int org[3] = {0, 0, 0};
-        bool staged = plan(g % 3, org);
-        unsigned mybox = nbox;
-        if (staged) ++nbox;
-        for (int z = z0; z < z1; ++z, i += XY) {
-            const float cx = px, cy = py, cz = pz;
-            const SobCell c = cl;
-            const bool cur_staged = staged;
-            const unsigned cur_box = mybox;
-            const int o0 = org[0], o1 = org[1], o2 = org[2];
-            const bool nact = col && z + 1 < z1;
-            if (nact) {
-                px = phi[0][i + XY];
-                py = phi[1][i + XY];
-                pz = phi[2][i + XY];
-                cl = sob_locate(P, px, py, pz);
-            }
-            ++g;
-            cellbox_add(cb, (int)(g % 3), nact, cl.gx, cl.gy, cl.gz);
-            if (__syncthreads_or(wait_failed)) {
-                failed = true;
-                break;
-            }
-            if (tid == 0) cellbox_clear(cb, (int)((g - 1) % 3));
-            staged = plan(g % 3, org);
-            mybox = nbox;
-            if (staged) ++nbox;
-            if (!col) continue;
-            float u[3];
-            if (cur_staged) {
-                if (!mbar_wait_bounded(full + (cur_box & 1), (cur_box >> 1) & 1)) wait_failed = true;
-                const float* b0 =
-                    box + (cur_box & 1) * 3 * kPlane + ((c.gz - o2) * kGBY + (c.gy - o1)) * kGBX + (c.gx - o0);
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    const float* f = b0 + k * kPlane;
-                    constexpr int SX = 1, SY = kGBX, SZ = kGBX * kGBY;
-                    u[k] = lerpf_(lerpf_(lerpf_(f[SX + SY + SZ], f[SX + SY], c.c), lerpf_(f[SX + SZ], f[SX], c.c), c.b),
-                                  lerpf_(lerpf_(f[SY + SZ], f[SY], c.c), lerpf_(f[SZ], f[0], c.c), c.b), c.a);
-                }
-            } else {
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    const float* __restrict__ F = mc[k];
-                    const int b = (int)c.base;
-                    u[k] = lerpf_(lerpf_(lerpf_(__ldg(F + b + 1 + X + XY), __ldg(F + b + 1 + X), c.c),
-                                         lerpf_(__ldg(F + b + 1 + XY), __ldg(F + b + 1), c.c), c.b),
-                                  lerpf_(lerpf_(__ldg(F + b + X + XY), __ldg(F + b + X), c.c),
-                                         lerpf_(__ldg(F + b + XY), __ldg(F + b), c.c), c.b),
-                                  c.a);
-                }
-            }
-            phi[0][i] = cx + u[0];
-            phi[1][i] = cy + u[1];
-            phi[2][i] = cz + u[2];
-            const float nrm = norm3_rd(u[0], u[1], u[2]);
-            if (nrm == nrm) {
-                const unsigned long long k = norm_key(nrm, i);
-                best = k > best ? k : best;
-            }
-        }
-        if (failed) break;
-        const unsigned long long bm = block_max_u64(best, red);
-        if (tid == 0 && bm) atomicMax(a.keys + tl.x, bm);
-    }
-    if (failed) {
-        if (tid == 0) {
-            for (unsigned n = (nbox > 2u ? nbox - 2u : 0u); n < nbox; ++n)
-                mbar_wait_bounded(full + (n & 1), (n >> 1) & 1);
-            atomicOr(a.err, kErrTmaTimeout);
-        }
-        return;
-    }
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) last = (atomicAdd(a.counter, 1u) == gridDim.x - 1);
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    for (int p = tid; p < a.npairs; p += blockDim.x) {
-        if (a.stop[p]) continue;
-        const unsigned long long k = atomicExch(a.keys + p, 0ull);
-        a.trace[(long long)(a.iter - 1) * a.npairs + p] = k;
-        const float mx = __uint_as_float((unsigned)(k >> 32));
-        if (mx <= a.max_update_norm) a.stop[p] = a.iter;
-    }
-    if (tid == 0) *a.counter = 0u;
+const void* sob_pass_b_fn(bool unrolled) {
+    return unrolled ? (const void*)sob_pass_b_kernel<true> : (const void*)sob_pass_b_kernel<false>;
+}
+
+cudaError_t launch_sob_kernel(int k, const SobIterArgs& a, int grid, int variant, cudaStream_t s) {
+    void* args[1] = {const_cast<SobIterArgs*>(&a)};
+    if (k == 0)
+        return cudaLaunchKernel(sob_grad_fn(variant), dim3(grid), dim3(sob_grad_threads(variant)), args,
+                                sob_grad_smem_bytes(), s);
+    if (k == 1)
+        return cudaLaunchKernel(variant & kUnrolled ? sob_smooth3_unrolled_fn(a.radius, false, variant & 2)
+                                                    : sob_smooth3_fn(a.radius, variant & 1, variant & 2),
+                                dim3(grid), dim3(kSmoothThreads), args, 0, s);
+    return cudaLaunchKernel(sob_pass_b_fn(variant & kUnrolled), dim3(grid), dim3(256), args, 0, s);
 }
 
 cudaError_t launch_sob_iter(const SobIterArgs& a, const int* grids, const int* variants, cudaStream_t s,
                             cudaEvent_t* ev) {
-    if (ev) cudaEventRecord(ev[0], s);
-    void* args[1] = {const_cast<SobIterArgs*>(&a)};
-    cudaLaunchKernel(sob_grad_fn(variants[0]), dim3(grids[0]), dim3(sob_grad_threads(variants[0])), args, sob_grad_smem_bytes(), s);
-    if (ev) cudaEventRecord(ev[1], s);
-    {
-        cudaLaunchKernel(sob_smooth3_fn(a.radius, variants[1] & 1, variants[1] & 2), dim3(grids[1]), dim3(kSmoothThreads), args, 0, s);
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < 3 && e == cudaSuccess; ++k) {
+        if (ev) cudaEventRecord(ev[k], s);
+        e = launch_sob_kernel(k, a, grids[k], variants[k], s);
     }
-    if (ev) cudaEventRecord(ev[2], s);
-    if (variants[2])
-        sob_pass_b_staged_kernel<<<grids[2], 256, gather_staged_smem_bytes(), s>>>(a);
-    else
-        sob_pass_b_kernel<<<grids[2], 256, 0, s>>>(a);
     if (ev) cudaEventRecord(ev[3], s);
-    return cudaGetLastError();
+    return e;
 }
 
 }  // namespace frg

@@ -46,12 +46,15 @@ struct SobIterArgs {
     long long NT;
     const float* S;
     const float* T;
-    float* phi;   // positions (3 planes)
-    float* m;     // momentum (3 planes)
-    float* g;     // gradient (3 planes)
+    const float* phi;  // positions (3 planes), read
+    const float* m;    // momentum (3 planes), read (unrolled iterations)
+    float* phi_n;      // positions, written: phi itself except in unrolled iterations
+    float* m_n;        // momentum, written and gathered: m itself except in unrolled iterations
+    float* g;          // gradient (3 planes)
     float damping, step;
     float lambda;  // W_REG; the kernels take each pair's weight from Pair::w_reg
     float taps[kMaxSmoothWidth];
+    float fold[kMaxSmoothWidth / 2 + 1];  // transposed smoothing: sum of the taps before tap R - s
     int radius;
     float max_update_norm;
     int iter;
@@ -63,6 +66,10 @@ struct SobIterArgs {
     unsigned int* err;         // device error word (kErrTmaTimeout: a staging wait gave up)
 };
 
+// fold[s] = sum of taps[0 .. R - s - 1]: what the transposed replicate boundary adds to the tap
+// that an end position takes from position s beside it
+void fold_weights(const float* taps, int radius, float* fold);
+
 // Gaussian taps exp(-k^2 / (2 sigma^2)), k = -R..R, normalised; computed in double
 // and rounded to float.
 void gaussian_taps(float sigma, int width, float* taps);
@@ -72,18 +79,52 @@ size_t sob_grad_smem_bytes();         // dynamic shared memory of the gradient k
 const void* sob_grad_fn(int tma);     // the gradient kernel of a staging variant (1: TMA)
 // the smoothing kernel instance for a radius, staging variant (1: TMA) and tile height
 const void* sob_smooth3_fn(int radius, int tma, bool tall);
+// the unrolled registration's (cp.async staging): the momentum from m to m_n, or transposed,
+// m_n = G^T g, which needs `fold` and zeros in the pad columns of g
+const void* sob_smooth3_unrolled_fn(int radius, bool transposed, bool tall);
 // box of one component of the smoothing kernel's staged slice for radius R: x extent, rows
 inline void sob_smooth_box(int R, bool tall, int* wx, int* rows) {
     *wx = kTileX + 2 * ((R + 3) / 4 * 4);
     *rows = sob_smooth_tile_y(R, tall) + 2 * R;
 }
-__global__ void sob_pass_b_kernel(SobIterArgs a);
-__global__ void sob_pass_b_staged_kernel(SobIterArgs a);
+const void* sob_pass_b_fn(bool unrolled);  // the update kernel
+constexpr int kUnrolled = 4;  // variant bit: the unrolled registration's kernel (separate in and out states)
+
+// one of them: k = 0 gradient, 1 smoothing, 2 update
+cudaError_t launch_sob_kernel(int k, const SobIterArgs& a, int grid, int variant, cudaStream_t s);
 
 // grids: {grad, smooth, pass_b}; variants: of {grad, smooth, pass_b} (bit 0: TMA
 // staging, bit 1 of smooth: tall tiles); with `ev`
 // (4 events) each launch is bracketed
 cudaError_t launch_sob_iter(const SobIterArgs& a, const int* grids, const int* variants, cudaStream_t s,
                             cudaEvent_t* ev = nullptr);
+
+// Cell for the sobolev solver: clamp to [0, dim-1], floor clamped to dim-2 so that
+// both corners of every axis are inside the grid; in_x, in_y, in_z: the position was not
+// clamped (a clamped axis has derivative 0).
+struct SobCell {
+    int base;
+    int gx, gy, gz;
+    float a, b, c;
+    bool in_x, in_y, in_z;
+};
+
+__device__ __forceinline__ SobCell sob_locate(const Pair& P, float px, float py, float pz) {
+    SobCell s;
+    const float cx = fminf(fmaxf(0.f, px), (float)(P.X - 1));
+    const float cy = fminf(fmaxf(0.f, py), (float)(P.Y - 1));
+    const float cz = fminf(fmaxf(0.f, pz), (float)(P.Z - 1));
+    s.gx = min((int)floorf(cx), P.X - 2);
+    s.gy = min((int)floorf(cy), P.Y - 2);
+    s.gz = min((int)floorf(cz), P.Z - 2);
+    s.a = cx - (float)s.gx;
+    s.b = cy - (float)s.gy;
+    s.c = cz - (float)s.gz;
+    s.in_x = cx == px;  // false for a NaN
+    s.in_y = cy == py;
+    s.in_z = cz == pz;
+    s.base = s.gx + P.Xp * (s.gy + P.Y * s.gz);
+    return s;
+}
 
 }  // namespace frg

@@ -167,6 +167,31 @@ def test_hypergradient_tuned_cohort(cuda):
     fr.close()
 
 
+@pytest.mark.parametrize("dims,width,K,ck", [((37, 19, 23), w, 4, 3) for w in (1, 3, 5, 7, 9, 11, 13, 15)] +
+                         [((4, 5, 4), 7, 3, 1), ((33, 8, 9), 15, 3, 2), ((5, 34, 6), 9, 3, 3), ((64, 17, 4), 5, 2, 5)] +
+                         [((161, 163, 101), 7, 2, 1), ((161, 163, 101), 9, 2, 2)])
+def test_loss_gradient_over_sizes_and_widths(cuda, dims, width, K, ck):
+    """Every radius of the transposed smoothing, short and tall tiles (the largest volume), ends
+    of an axis closer together than the filter, a last tile of one row or column, and segments
+    of one iteration, a remainder and all: against the FP32 oracle, whose forward has the same
+    arithmetic (J), and whose reverse sweep adds the same terms in another order.  A voxel sums
+    about 8 scattered and 3 (2 R + 1) filtered terms per iteration in FP32, K iterations deep:
+    within 100 roundings of 6e-8 of the field's norm, 1e-5 with the margin of the test above;
+    dJ/dlambda, a sum that may cancel, within 1e-4 relative plus 1e-6 of J."""
+    import torch
+    d = images(dims, 40 + width)
+    P = Params(volume_dims=dims, solver="sobolev", smooth_sigma=0.4 + 0.3 * width, smooth_width=width, damping=0.9,
+               step=0.5)
+    v0 = smooth_noise(rng(width), (3,) + dims[::-1], 0.3)
+    T, S = (torch.from_numpy(d[k]).to(cuda) for k in ("T", "S"))
+    J, gv, gl = _loss_grad(T, S, torch.from_numpy(v0).to(cuda), 0.2, K, ck, P)
+    J32, gv32, gl32 = O.sob_loss_grad(P, d["T"], d["S"], v0, 0.2, K, True, prec=32)
+    gv = gv.cpu().numpy().astype(np.float64)
+    assert abs(J - J32) <= 1e-9 * abs(J32)
+    assert np.linalg.norm(gv - gv32) <= 1e-5 * np.linalg.norm(gv32.astype(np.float64))
+    assert abs(gl - gl32) <= 1e-4 * abs(gl32) + 1e-6 * abs(J32), (gl, gl32)
+
+
 @pytest.mark.slow
 def test_adjoint_at_128cube_50_iterations(cuda):
     """The differentiated workload at its stated size: the 128^3 pair (blobs, max
