@@ -24,6 +24,7 @@
 #include "fr_tma.cuh"
 #include "fr_sob.h"
 
+#include <atomic>
 #include <chrono>
 #include <map>
 #include <mutex>
@@ -1513,6 +1514,22 @@ int fr_time_kernels(fr_handle* h, int iters, float* ms, int* n_kernels, void* st
     return FR_OK;
 }
 
+// Blocks of a standalone kernel that are resident on the current device at once.
+// The device queries cost a small call about as much as its launch, so the answer is kept per
+// device in the kernel's own `slots` (a device's answer does not change; 0: not asked yet).
+static int resident_blocks(const void* fn, std::atomic<int>* slots, int threads = 256) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) dev = -1;
+    if (dev >= 0 && dev < 64)
+        if (const int known = slots[dev].load(std::memory_order_relaxed)) return known;
+    int sms = 0, per_sm = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, 0);
+    if (sms < 1 || per_sm < 1) return std::max(sms, 1) * std::max(per_sm, 1);
+    if (dev >= 0 && dev < 64) slots[dev].store(sms * per_sm, std::memory_order_relaxed);
+    return sms * per_sm;
+}
+
 int fr_warp(const float* d_pos, const float* d_img, const int16_t* d_lab, const int dims[3], float* d_out,
             int16_t* d_out_lab, void* stream) {
     g_parse_error.clear();
@@ -1535,20 +1552,20 @@ int fr_warp(const float* d_pos, const float* d_img, const int16_t* d_lab, const 
     P.Xp = P.X;  // the caller's unpadded layout
     P.N = (long long)P.X * P.Y * P.Z;
     P.off = 0;
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    static std::atomic<int> slots2[64], slots32[64], slots64[64];
     auto aligned = [](const void* p, uintptr_t a) { return ((uintptr_t)p & (a - 1)) == 0; };
-    const bool vec2 = P.N % 2 == 0 && frg::fits_index32(P.X, P.Y, P.Z) && aligned(d_pos, 8) && aligned(d_out, 8) &&
-                      (!d_out_lab || aligned(d_out_lab, 4));
-    const void* fn = vec2 ? (const void*)frg::warp2_kernel : (const void*)frg::warp_kernel;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, 0);
-    const long long want = ((vec2 ? P.N / 2 : P.N) + 255) / 256;
-    int grid = (int)std::max(1LL, std::min<long long>(want, (long long)std::max(per_sm, 1) * std::max(sms, 1)));
-    if (vec2)
+    const bool small = frg::fits_index32(P.X, P.Y, P.Z);
+    if (small && P.N % 2 == 0 && aligned(d_pos, 8) && aligned(d_out, 8) && (!d_out_lab || aligned(d_out_lab, 4))) {
+        const int grid = (int)std::min<long long>((P.N / 2 + 255) / 256, resident_blocks((const void*)frg::warp2_kernel, slots2));
         frg::warp2_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(d_pos, d_img, d_lab, d_out, d_out_lab, P.X, P.Y, P.Z);
-    else
+    } else if (small) {
+        const long long items = (P.N + 256 * frg::kWarpVox - 1) / (256 * frg::kWarpVox);
+        const int grid = (int)std::min<long long>(items, resident_blocks((const void*)frg::warp32_kernel, slots32));
+        frg::warp32_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(d_pos, d_img, d_lab, d_out, d_out_lab, P.X, P.Y, P.Z);
+    } else {
+        const int grid = (int)std::min<long long>((P.N + 255) / 256, resident_blocks((const void*)frg::warp_kernel, slots64));
         frg::warp_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(d_pos, d_img, d_lab, d_out, d_out_lab, P);
+    }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         g_parse_error = std::string("fr_warp: ") + cudaGetErrorString(e);
@@ -1566,23 +1583,6 @@ static int field_op_check(const void* a, const void* b, const void* c, const int
     if (!frg::fits_index32(dims[0], dims[1], dims[2])) {
         g_parse_error = std::string(who) + ": dims must be >= 1 with N + 2 X Y + 2 X + 2 <= 2^31-1";
         return FR_ERR_INVALID_ARG;
-    }
-    return FR_OK;
-}
-
-static int field_op_launch(const void* fn, long long work, const char* who, void (*launch)(int grid, void* ctx),
-                           void* ctx) {
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, 0);
-    const int grid =
-        (int)std::max(1LL, std::min<long long>((work + 255) / 256, (long long)std::max(per_sm, 1) * std::max(sms, 1)));
-    launch(grid, ctx);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) {
-        g_parse_error = std::string(who) + ": " + cudaGetErrorString(e);
-        return FR_ERR_CUDA;
     }
     return FR_OK;
 }
@@ -1623,39 +1623,38 @@ int fr_estimate_inverse(const float* d_psi, float* d_psi_inv, const int dims[3],
         g_parse_error = "fr_estimate_inverse: sweeps must be >= 0";
         return FR_ERR_INVALID_ARG;
     }
-    struct Ctx {
-        const float* psi;
-        float* pinv;
-        const int* d;
-        int sweeps;
-        cudaStream_t s;
-    } c{d_psi, d_psi_inv, dims, sweeps, (cudaStream_t)stream};
-    return field_op_launch(
-        (const void*)frg::estimate_inverse_kernel, (long long)dims[0] * dims[1] * dims[2], "fr_estimate_inverse",
-        [](int grid, void* p) {
-            Ctx* c = (Ctx*)p;
-            frg::estimate_inverse_kernel<<<grid, 256, 0, c->s>>>(c->psi, c->pinv, c->d[0], c->d[1], c->d[2], c->sweeps);
-        },
-        &c);
+    static std::atomic<int> slots[64];
+    const long long blocks = ((long long)dims[0] * dims[1] * dims[2] + 255) / 256;
+    const int grid = (int)std::min<long long>(blocks, resident_blocks((const void*)frg::estimate_inverse_kernel, slots));
+    frg::estimate_inverse_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(d_psi, d_psi_inv, dims[0], dims[1], dims[2],
+                                                                        sweeps);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) {
+        g_parse_error = std::string("fr_estimate_inverse: ") + cudaGetErrorString(e);
+        return FR_ERR_CUDA;
+    }
+    return FR_OK;
 }
 
 int fr_interpolate_field(const float* d_field, const float* d_pos, const int dims[3], float* d_out, void* stream) {
     int rc = field_op_check(d_field, d_pos, d_out, dims, "fr_interpolate_field");
     if (rc != FR_OK) return rc;
-    struct Ctx {
-        const float* f;
-        const float* pos;
-        float* out;
-        const int* d;
-        cudaStream_t s;
-    } c{d_field, d_pos, d_out, dims, (cudaStream_t)stream};
-    return field_op_launch(
-        (const void*)frg::interpolate_field_kernel, (long long)dims[0] * dims[1] * dims[2], "fr_interpolate_field",
-        [](int grid, void* p) {
-            Ctx* c = (Ctx*)p;
-            frg::interpolate_field_kernel<<<grid, 256, 0, c->s>>>(c->f, c->pos, c->out, c->d[0], c->d[1], c->d[2]);
-        },
-        &c);
+    static std::atomic<int> slots[64];
+    const int X = dims[0], Y = dims[1], Z = dims[2];
+    const long long cols = ((long long)X * Y + frg::kFieldThreads - 1) / frg::kFieldThreads;
+    // columns of up to 16 slices (64.7 us on 182x218x182; 8 take 67.2 us, 24 67.6 us), shorter
+    // where that leaves blocks of the GPU without work; the grid's second extent is 16 bits
+    const long long want = cols * Z / std::max(resident_blocks((const void*)frg::interpolate_field_kernel, slots,
+                                                               frg::kFieldThreads), 1);
+    const int depth = (int)std::max(std::max(1LL, std::min(16LL, want)), (Z + 65534LL) / 65535);
+    frg::interpolate_field_kernel<<<dim3((unsigned)cols, (unsigned)((Z + depth - 1) / depth)), frg::kFieldThreads, 0,
+                                    (cudaStream_t)stream>>>(d_field, d_pos, d_out, X, Y, Z, depth);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) {
+        g_parse_error = std::string("fr_interpolate_field: ") + cudaGetErrorString(e);
+        return FR_ERR_CUDA;
+    }
+    return FR_OK;
 }
 
 }  // extern "C"

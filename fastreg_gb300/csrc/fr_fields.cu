@@ -29,14 +29,61 @@ __global__ void __launch_bounds__(256) estimate_inverse_kernel(const float* __re
     }
 }
 
-__global__ void __launch_bounds__(256) interpolate_field_kernel(const float* __restrict__ field,
-                                                                const float* __restrict__ pos, float* __restrict__ out,
-                                                                int X, int Y, int Z) {
-    const int N = X * Y * Z, XY = X * Y;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-        const Cell32 cl = locate32(X, Y, Z, X, __ldg(pos + i), __ldg(pos + N + i), __ldg(pos + 2 * N + i));
+// A thread owns a column of `depth` slices, a block kFieldThreads consecutive voxels of a
+// slice (rows run on, so every warp but the last is full and its rows start where its lanes do).
+// The kernel is bound by the gathers' trips through L1, several cache lines per load.  Positions
+// are mostly those of a smooth map, so the cell of the next slice is often the one above this
+// slice's: its lower four corners are the upper ones already in registers, and a lane loads
+// 12 corners instead of 24; all are issued before the arithmetic.  64.7 us on 182x218x182 (36
+// bytes per voxel, 39 us at the copy bandwidth); 84 us with three component samples one after
+// the other, 80 us with 24 corners loaded together, 70 us on 32 x 8 tiles with the reuse.
+__global__ void __launch_bounds__(kFieldThreads, 2) interpolate_field_kernel(const float* __restrict__ field,
+                                                                             const float* __restrict__ pos,
+                                                                             float* __restrict__ out, int X, int Y,
+                                                                             int Z, int depth) {
+    const int N = X * Y * Z, XY = X * Y, last = N - 1;
+    const int col = blockIdx.x * kFieldThreads + threadIdx.x;
+    if (col >= XY) return;
+    const int z0 = blockIdx.y * depth, z1 = min(z0 + depth, Z);
+    const float* __restrict__ p[3] = {pos, pos + N, pos + 2 * (long long)N};
+    const float* __restrict__ F[3] = {field, field + N, field + 2 * (long long)N};
+    float* const O[3] = {out, out + N, out + 2 * (long long)N};
+    int i = col + XY * z0;
+    float n[3], f[3][8];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) out[(long long)c * N + i] = tri_unchecked32(field + (long long)c * N, X, XY, N, cl);
+    for (int c = 0; c < 3; ++c) {
+        n[c] = __ldcs(p[c] + i);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) f[c][q] = 0.f;
+    }
+    int above = -1;  // base of the cell whose lower corners are the upper ones in f (-1: none)
+    for (int z = z0; z < z1; ++z, i += XY) {
+        const Cell32 cl = locate32(X, Y, Z, X, n[0], n[1], n[2]);
+        const int b = cl.base;
+        if (z + 1 < z1)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) n[c] = __ldcs(p[c] + i + XY);
+        // corners past the last voxel (of weight 0) are clamped, as in tri_unchecked32
+        const int o[8] = {min(b + 1 + X + XY, last), min(b + 1 + X, last), min(b + 1 + XY, last), min(b + 1, last),
+                          min(b + X + XY, last),     min(b + X, last),     min(b + XY, last),     b};
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+#pragma unroll
+            for (int q = 0; q < 8; q += 2) {
+                f[c][q + 1] = f[c][q];
+                f[c][q] = __ldg(F[c] + o[q]);
+            }
+        }
+        if (b != above)
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+#pragma unroll
+                for (int q = 1; q < 8; q += 2) f[c][q] = __ldg(F[c] + o[q]);
+        above = b + XY;
+        float v[3];
+        trilerp3(f, cl.a, cl.b, cl.c, v);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) __stcs(O[c] + i, v[c]);
     }
 }
 

@@ -68,3 +68,58 @@ def test_empty_and_undersized_cohorts_are_refused(cuda):
     _check_pair("reference", Params(volume_dims=(12, 10, 9), **kw), p, buf,
                 fr.get_field(N.FR_FIELD_PSI).cpu().numpy(), "after the refusals")
     fr.close()
+
+
+@pytest.mark.parametrize("dims", [(1, 1, 1), (31, 1, 1), (1, 63, 1), (4, 4, 4), (5, 13, 1), (3, 1, 43), (43, 3, 1), (9, 7, 61)])
+def test_field_operations_at_remainders(cuda, dims):
+    """fr_warp and fr_interpolate_field where the last item of a warp's 64 voxels is partly or
+    nearly empty, on buffers that are only element-aligned: the oracle's bits."""
+    import torch
+    from fastreg_gb300 import interpolate_field, warp
+    X, Y, Z = dims
+    r = np.random.Generator(np.random.PCG64(17))
+    img, lab = r.normal(0, 1, (Z, Y, X)).astype(np.float32), r.integers(0, 9, (Z, Y, X)).astype(np.int16)
+    field = r.normal(0, 1, (3, Z, Y, X)).astype(np.float32)
+    pos = np.stack([r.uniform(-1, n, (Z, Y, X)) for n in dims]).astype(np.float32)
+
+    def shifted(a):  # one element past an allocation's start
+        t = torch.empty(a.size + 1, dtype=torch.from_numpy(a).dtype, device=cuda)[1:].view(a.shape)
+        t.copy_(torch.from_numpy(a))
+        return t
+
+    for to in (lambda a: _to(cuda, a), shifted):
+        out, out_lab = to(np.zeros_like(img)), to(np.zeros_like(lab))
+        warp(to(pos), to(img), to(lab), out=out, out_lab=out_lab)
+        o_img, o_lab = O.warp(pos, img, lab)
+        assert_bitexact(out.cpu().numpy(), o_img, f"warp {dims}")
+        assert_bitexact(out_lab.cpu().numpy(), o_lab, f"warp labels {dims}")
+        assert_bitexact(warp(to(pos), to(img)).cpu().numpy(), o_img, f"warp without labels {dims}")
+        assert_bitexact(interpolate_field(to(field), to(pos), out=to(np.zeros_like(field))).cpu().numpy(),
+                        O.interpolate_field(field, pos), f"field {dims}")
+
+
+@pytest.mark.parametrize("dims", [(2, 2, 2), (33, 9, 2), (31, 8, 40), (70, 17, 33)])
+def test_warp_adjoint_over_sizes(cuda, dims):
+    """fr_warp_adjoint at tile edges, single-slice columns and columns longer than a tile, maps that
+    keep cells stacked (a uniform shift) and that do not (noise), outside positions and a NaN;
+    both outputs, and each alone.  A voxel of img_bar sums a few dozen FP32 terms in any
+    order, a component of pos_bar about ten: 1e-5 of the largest value, as in the test of one size."""
+    import ctypes as C
+    import torch
+    lib = N.load()
+    X, Y, Z = dims
+    r = np.random.Generator(np.random.PCG64(23))
+    img, wbar = (r.normal(0, 1, (Z, Y, X)).astype(np.float32) for _ in range(2))
+    grid = np.stack(np.meshgrid(np.arange(Z), np.arange(Y), np.arange(X), indexing="ij")[::-1]).astype(np.float32)
+    for pos in (grid + np.float32(0.3), grid + r.uniform(-2.5, 2.5, grid.shape).astype(np.float32)):
+        pos[:, 0, 0, 0] = np.nan
+        pb64, ib64 = O.warp_adjoint(pos, img, wbar)
+        a = [_to(cuda, v) for v in (pos, img, wbar)]
+        for want_pos, want_img in ((1, 1), (1, 0), (0, 1)):
+            pb, ib = torch.empty_like(a[0]), torch.empty_like(a[1])
+            assert lib.fr_warp_adjoint(*(v.data_ptr() for v in a), (C.c_int * 3)(*dims), pb.data_ptr() if want_pos else None,
+                                       ib.data_ptr() if want_img else None, None) == N.FR_OK
+            if want_pos:
+                assert np.abs(pb.cpu().numpy() - pb64).max() <= 1e-5 * max(1.0, np.abs(pb64).max())
+            if want_img:
+                assert np.abs(ib.cpu().numpy() - ib64).max() <= 1e-5 * max(1.0, np.abs(ib64).max())
