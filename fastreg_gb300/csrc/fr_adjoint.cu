@@ -34,99 +34,7 @@
 
 namespace frg {
 
-struct AdjDims {
-    int X, Y, Z, XY, N;
-};
-
-struct TriEval {
-    int off[8];
-    float w[8];
-    float val, d[3], H01, H02, H12;
-    bool in[3];
-};
-
-__device__ __forceinline__ void sob_cell(const AdjDims& D, float px, float py, float pz, int& base, float& a,
-                                         float& b, float& c, bool* in) {
-    const float cx = fminf(fmaxf(0.f, px), (float)(D.X - 1));
-    const float cy = fminf(fmaxf(0.f, py), (float)(D.Y - 1));
-    const float cz = fminf(fmaxf(0.f, pz), (float)(D.Z - 1));
-    const int gx = min((int)floorf(cx), D.X - 2), gy = min((int)floorf(cy), D.Y - 2), gz = min((int)floorf(cz), D.Z - 2);
-    a = cx - (float)gx;
-    b = cy - (float)gy;
-    c = cz - (float)gz;
-    in[0] = px >= 0.f && px <= (float)(D.X - 1);
-    in[1] = py >= 0.f && py <= (float)(D.Y - 1);
-    in[2] = pz >= 0.f && pz <= (float)(D.Z - 1);
-    base = gx + D.X * (gy + D.Y * gz);
-}
-
-// value, masked gradient and (optionally) Hessian of the trilinear interpolant of F
-__device__ __forceinline__ void tri_eval(const AdjDims& D, const float* __restrict__ F, float px, float py, float pz,
-                                         TriEval& t, bool hessian) {
-    int b;
-    float a, bb, c;
-    sob_cell(D, px, py, pz, b, a, bb, c, t.in);
-    const int X = D.X, XY = D.XY;
-    const int off[8] = {0, 1, X, 1 + X, XY, 1 + XY, X + XY, 1 + X + XY};
-    float f[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        t.off[q] = b + off[q];
-        f[q] = F ? __ldg(F + b + off[q]) : 0.f;
-        const float wx = (q & 1) ? a : 1.f - a, wy = (q & 2) ? bb : 1.f - bb, wz = (q & 4) ? c : 1.f - c;
-        t.w[q] = wx * wy * wz;
-    }
-    if (!F) return;
-    const float f000 = f[0], f100 = f[1], f010 = f[2], f110 = f[3], f001 = f[4], f101 = f[5], f011 = f[6],
-                f111 = f[7];
-    const float e11 = lerpf_(f111, f110, c), e10 = lerpf_(f101, f100, c);
-    const float e01 = lerpf_(f011, f010, c), e00 = lerpf_(f001, f000, c);
-    const float A1 = lerpf_(e11, e10, bb), A0 = lerpf_(e01, e00, bb);
-    t.val = lerpf_(A1, A0, a);
-    const float d11 = f111 - f110, d10 = f101 - f100, d01 = f011 - f010, d00 = f001 - f000;
-    t.d[0] = t.in[0] ? A1 - A0 : 0.f;
-    t.d[1] = t.in[1] ? lerpf_(e11 - e10, e01 - e00, a) : 0.f;
-    t.d[2] = t.in[2] ? lerpf_(lerpf_(d11, d10, bb), lerpf_(d01, d00, bb), a) : 0.f;
-    if (!hessian) return;
-    t.H01 = (t.in[0] && t.in[1]) ? (e11 - e10) - (e01 - e00) : 0.f;
-    t.H02 = (t.in[0] && t.in[2]) ? lerpf_(d11, d10, bb) - lerpf_(d01, d00, bb) : 0.f;
-    t.H12 = (t.in[1] && t.in[2]) ? lerpf_(d11 - d10, d01 - d00, a) : 0.f;
-}
-
 #define GRID_STRIDE(i, n) for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += gridDim.x * blockDim.x)
-
-// Grid-stride loop over whole warps: every lane of a warp runs the same iterations (lane
-// i of a warp holds voxel base + i; `act` is false past the end), so the body may use
-// warp shuffles.
-#define WARP_STRIDE(i, act, n)                                                                  \
-    for (int i##_w = blockIdx.x * blockDim.x + (threadIdx.x & ~31); i##_w < (n);                  \
-         i##_w += gridDim.x * blockDim.x)                                                        \
-        for (int i = i##_w + (threadIdx.x & 31), act = i < (n), i##_once = 1; i##_once; i##_once = 0)
-
-// Scatter-add of one cell's eight corner contributions cw[q] (q: bit 0 x, bit 1 y, bit 2 z;
-// the corners of tri_eval) into F, with the corners that neighbouring lanes share added
-// once: the lanes of a warp hold consecutive voxels of a row, whose cells are usually
-// consecutive along x (a smooth map), so lane k's x + 1 corners are lane k + 1's x corners.
-// Lane k then adds lane k - 1's x + 1 contribution to its own x one (one atomic for both),
-// halving the atomics of such runs.  All 32 lanes must call it; inactive lanes pass
-// act = false.
-__device__ __forceinline__ void scatter_cell_warp(float* F, int b, const float cw[8], bool act, int X, int XY) {
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int bprev = __shfl_up_sync(full, act ? b : -4, 1);
-    const bool merge = act && lane > 0 && bprev == b - 1;
-    const bool next_merges = __shfl_down_sync(full, (int)merge, 1) != 0 && lane < 31;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int o = ((j & 1) ? X : 0) + ((j & 2) ? XY : 0);
-        const float c0 = cw[2 * j], c1 = cw[2 * j + 1];
-        const float c1prev = __shfl_up_sync(full, c1, 1);
-        if (act) {
-            atomicAdd(F + b + o, merge ? c0 + c1prev : c0);
-            if (!next_merges) atomicAdd(F + b + 1 + o, c1);
-        }
-    }
-}
 
 // One pair of the workspace.
 struct AdjPair {
@@ -780,27 +688,94 @@ extern "C" int fr_sobolev_loss_grad(const float* d_T, const float* d_S, const in
     return FR_OK;
 }
 
-extern "C" int fr_warp_adjoint(const float* d_pos, const float* d_img, const float* d_wbar, const int dims[3],
-                               float* d_pos_bar, float* d_img_bar, void* stream);
-
 namespace frg {
-__global__ void warp_adjoint_kernel(AdjDims D, const float* __restrict__ pos, const float* __restrict__ img,
-                                    const float* __restrict__ wbar, float* pos_bar, float* img_bar) {
-    WARP_STRIDE(i, act, D.N) {
-        const int k = act ? i : 0;
-        TriEval t;
-        tri_eval(D, img, __ldg(pos + k), __ldg(pos + D.N + k), __ldg(pos + 2 * D.N + k), t, false);
-        const float wb = __ldg(wbar + k);
-        if (pos_bar && act)
+// scatter_face_warp of one channel
+__device__ __forceinline__ void scatter_face_warp(float* F, int b, const float v[4], bool act, int X) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int bprev = __shfl_up_sync(full, act ? b : -4, 1);
+    const bool merge = act && lane > 0 && bprev == b - 1;
+    const bool next_merges = __shfl_down_sync(full, (int)merge, 1) != 0 && lane < 31;
 #pragma unroll
-            for (int j = 0; j < 3; ++j) pos_bar[(long long)j * D.N + i] = wb * t.d[j];
-        if (img_bar) {  // uniform: every lane calls the warp scatter
-            float cw[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) cw[q] = t.w[q] * wb;
-            scatter_cell_warp(img_bar, t.off[0], cw, act, D.X, D.XY);
+    for (int j = 0; j < 2; ++j) {
+        const float c1 = v[2 * j + 1], c1prev = __shfl_up_sync(full, c1, 1);
+        if (act) {
+            atomicAdd(F + b + j * X, merge ? v[2 * j] + c1prev : v[2 * j]);
+            if (!next_merges) atomicAdd(F + b + 1 + j * X, c1);
         }
     }
+}
+
+// pos_bar = wbar * d img/d pos, img_bar += the trilinear weights times wbar, on the caller's
+// unpadded planes.  A thread owns a column of a 32 x 8 x depth tile: the corners and the upper
+// face of a cell that the next slice's cell stands on are kept and held back as in
+// adj_update_kernel, as the reductions bound the kernel: 57 us on 160x192x160, where eight
+// corners per voxel, lanes merged, took 83 us.
+__global__ void __launch_bounds__(256) warp_adjoint_kernel(Pair P, int depth, const float* __restrict__ pos,
+                                                           const float* __restrict__ img,
+                                                           const float* __restrict__ wbar, float* pos_bar,
+                                                           float* img_bar) {
+    const int X = P.X, XY = P.X * P.Y;
+    const long long N = P.N;
+    const int nx = (P.X + kTileX - 1) / kTileX, ny = (P.Y + kTileY - 1) / kTileY;
+    const int x = (blockIdx.x % nx) * kTileX + (threadIdx.x & 31), y = (blockIdx.x / nx % ny) * kTileY + (threadIdx.x >> 5);
+    const int z0 = (int)(blockIdx.x / (nx * ny)) * depth, z1 = min(z0 + depth, P.Z);
+    const bool act = x < P.X && y < P.Y;
+    int i = act ? x + X * y + XY * z0 : 0;
+    float f[8] = {}, held[4] = {};
+    int above = -1;  // base of the cell above the previous slice's cell (-1: none)
+    float np[3], nw = __ldg(wbar + i);  // the next slice's position and wbar
+#pragma unroll
+    for (int c = 0; c < 3; ++c) np[c] = __ldg(pos + c * N + i);
+    for (int z = z0; z < z1; ++z, i += act ? XY : 0) {
+        const SobCell s = sob_locate(P, np[0], np[1], np[2]);
+        const float w = nw;
+        const int b = s.base;
+        const bool on = b == above;
+        if (pos_bar) {
+            f[1] = f[0];
+            f[3] = f[2];
+            f[5] = f[4];
+            f[7] = f[6];
+            f[0] = __ldg(img + b + 1 + X + XY);
+            f[2] = __ldg(img + b + 1 + XY);
+            f[4] = __ldg(img + b + X + XY);
+            f[6] = __ldg(img + b + XY);
+            if (!on) {
+                f[1] = __ldg(img + b + 1 + X);
+                f[3] = __ldg(img + b + 1);
+                f[5] = __ldg(img + b + X);
+                f[7] = __ldg(img + b);
+            }
+        }
+        if (act && z + 1 < z1) {
+            nw = __ldg(wbar + i + XY);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) np[c] = __ldg(pos + c * N + i + XY);
+        }
+        if (pos_bar) {
+            float d[3];
+            tri_grad(f, s, d, nullptr, nullptr);
+            if (act)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) __stcs(pos_bar + c * N + i, w * d[c]);
+        }
+        if (img_bar) {  // uniform: every lane calls the warp scatter
+            const bool flush = act && !on && above >= 0;
+            if (__any_sync(0xffffffffu, flush)) scatter_face_warp(img_bar, above, held, flush, X);
+            float low[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float k = ((q & 1) ? s.a : 1.f - s.a) * ((q & 2) ? s.b : 1.f - s.b);
+                low[q] = (k * (1.f - s.c)) * w;
+                if (on) low[q] += held[q];
+                held[q] = (k * s.c) * w;
+            }
+            scatter_face_warp(img_bar, b, low, act, X);
+        }
+        above = b + XY;
+    }
+    if (img_bar) scatter_face_warp(img_bar, above, held, act && above >= 0, X);
 }
 }  // namespace frg
 
@@ -816,14 +791,26 @@ extern "C" int fr_warp_adjoint(const float* d_pos, const float* d_img, const flo
         set_global_error("fr_warp_adjoint: invalid dims (each >= 2, N + 2 X Y + 2 X + 2 <= 2^31-1)");
         return FR_ERR_INVALID_ARG;
     }
-    AdjDims D{dims[0], dims[1], dims[2], dims[0] * dims[1], dims[0] * dims[1] * dims[2]};
+    Pair P{};
+    P.X = P.Xp = dims[0];
+    P.Y = dims[1];
+    P.Z = dims[2];
+    P.N = (long long)dims[0] * dims[1] * dims[2];
     cudaStream_t s = (cudaStream_t)stream;
-    if (d_img_bar && cudaMemsetAsync(d_img_bar, 0, sizeof(float) * (size_t)D.N, s) != cudaSuccess) {
+    if (d_img_bar && cudaMemsetAsync(d_img_bar, 0, sizeof(float) * (size_t)P.N, s) != cudaSuccess) {
         cudaGetLastError();
         set_global_error("fr_warp_adjoint: memset failed");
         return FR_ERR_CUDA;
     }
-    warp_adjoint_kernel<<<grid_for(D.N), 256, 0, s>>>(D, d_pos, d_img, d_wbar, d_pos_bar, d_img_bar);
+    // long columns hold more faces back, short ones fill the GPU: up to 16 slices while there are
+    // eight blocks per SM
+    const long long cols = (long long)((P.X + kTileX - 1) / kTileX) * ((P.Y + kTileY - 1) / kTileY);
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int depth = (int)std::max(1LL, std::min(16LL, cols * P.Z / (8LL * std::max(sms, 1))));
+    const long long blocks = cols * ((P.Z + depth - 1) / depth);
+    warp_adjoint_kernel<<<(unsigned)blocks, 256, 0, s>>>(P, depth, d_pos, d_img, d_wbar, d_pos_bar, d_img_bar);
     if (cudaGetLastError() != cudaSuccess) {
         set_global_error("fr_warp_adjoint: launch failed");
         return FR_ERR_CUDA;
