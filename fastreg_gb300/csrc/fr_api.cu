@@ -217,6 +217,8 @@ int check_device_error(fr_handle* h) {
     if (!h->dev_err) return FR_OK;
     unsigned int e = 0;
     FR_CUDA(h, cudaMemcpy(&e, h->dev_err, sizeof e, cudaMemcpyDeviceToHost));
+    if (e & frg::kErrSmemAlign)
+        return fail(h, FR_ERR_CUDA, "a TMA staging ring is not on a 128-byte boundary (device error word %u)", e);
     if (e & frg::kErrTmaTimeout)
         return fail(h, FR_ERR_CUDA, "a TMA staging wait gave up after its time limit (device error word %u)", e);
     return FR_OK;

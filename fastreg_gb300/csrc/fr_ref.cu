@@ -27,10 +27,11 @@ __device__ __forceinline__ float det_ref(const float m[3][3]) {
     return first - second;
 }
 
-// entropy flux of the (Dv)v diagonal term (vector_fields.cu:376-378)
+// entropy flux of the (Dv)v diagonal term (vector_fields.cu:376-378): max(c,0)^2 - min(c,0)^2
+// + min(n,0)^2 - max(n,0)^2.  The first difference is c |c|: one square is zero, a zero of
+// either sign vanishes in the sum, and where c is a NaN the row's other terms are NaN too.
 __device__ __forceinline__ float entropy_flux(float c, float n) {
-    return ((fmaxf(c, 0.f) * fmaxf(c, 0.f) - fminf(c, 0.f) * fminf(c, 0.f)) + fminf(n, 0.f) * fminf(n, 0.f)) -
-           fmaxf(n, 0.f) * fmaxf(n, 0.f);
+    return (c * fabsf(c) + fminf(n, 0.f) * fminf(n, 0.f)) - fmaxf(n, 0.f) * fmaxf(n, 0.f);
 }
 
 // ----------------------------------------------------------------------------------
@@ -42,8 +43,7 @@ __device__ __forceinline__ float entropy_flux(float c, float n) {
 // 3-slice window (one ring of five components), so the stencil reads are shared-memory
 // loads and the global traffic is one coalesced pass per field.  T o psi_inv and
 // L o psi_inv are gathered from the interleaved LT field (eight 16-byte loads per voxel).
-// The LT rows of the next slice's cell and the rho/S slice three steps ahead are
-// prefetched into L2 (the kernel is latency-bound).
+// The LT rows of the next slice's cell are prefetched into L2 (the kernel is latency-bound).
 // ----------------------------------------------------------------------------------
 namespace {
 // prefetch distance: slices in flight ahead of the one being computed
@@ -188,11 +188,12 @@ constexpr unsigned kTLBytes = sizeof(float) * (3 * kTQPlane + kTileX * kTileY); 
 static_assert(3 * kTQPlane <= kTTOff && (kTTOff * 4) % 128 == 0 && (kTSlot * 4) % 128 == 0, "slot layout");
 }  // namespace
 
-size_t ref_laplacian_tma_smem_bytes() { return 128 + sizeof(float) * kTLS * kTSlot + sizeof(uint64_t) * kTLS; }
+size_t ref_laplacian_tma_smem_bytes() { return sizeof(float) * kTLS * kTSlot + sizeof(uint64_t) * kTLS; }
 
 __global__ void __launch_bounds__(256) ref_laplacian_tma_kernel(RefIterArgs a) {
     extern __shared__ __align__(128) unsigned char lap_raw[];
-    float* ring = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(lap_raw) + 127) & ~uintptr_t(127));
+    float* ring = reinterpret_cast<float*>(lap_raw);
+    if (!ring_aligned(ring, a.err)) return;
     uint64_t* full = reinterpret_cast<uint64_t*>(ring + kTLS * kTSlot);
     typedef SliceRing<kTLS> Ring;
     const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
@@ -309,8 +310,7 @@ template <int VC, int QC, int QR, int QS, int RW>
 __device__ __forceinline__ void pass_a_voxel(const RefIterArgs& a, const Pair& P, int X, int Y, int Z, int N, int Xp,
                                              int XYp, int y, int z, int i, bool dv_xy, const float* const vb[5],
                                              const float* const qb[3], const float4* __restrict__ LT,
-                                             const float* __restrict__ Tg, const float* __restrict__ Sg,
-                                             const float* __restrict__ Rg, const float* __restrict__ const* Vg,
+                                             const float* __restrict__ Tg, const float* __restrict__ const* Vg,
                                              float* rho_n,
                                              float* const* Vn, float* const* Qn) {
     auto V = [&](int k, int c) { return vb[k] + c * VC; };
@@ -335,12 +335,7 @@ __device__ __forceinline__ void pass_a_voxel(const RefIterArgs& a, const Pair& P
     const float det = det_ref(M);
 
     // central-difference gradient of S and the potential gradient
-    // rho and S are read through L1 (their 7-point stencils stay in cache)
     const float Si = Q(1, 4)[0];
-    if (z + 3 < Z) {  // the S and rho slice this column reads three steps on
-        prefetch_l2(Sg + i + 3 * XYp);
-        prefetch_l2(Rg + i + 3 * XYp);
-    }
     const float gs[3] = {(Q(1, 4)[1] - Q(1, 4)[-1]) * 0.5f,
                          (Q(1, 4)[RW] - Q(1, 4)[-RW]) * 0.5f,
                          (Q(2, 4)[0] - Q(0, 4)[0]) * 0.5f};
@@ -523,7 +518,7 @@ __global__ void __launch_bounds__(256, 3) ref_pass_a_kernel(RefIterArgs a) {
             if (active) {
                 const int i = x + Xp * y + XYp * z;
                 pass_a_voxel<kVS * kVPlane, kQS * kQPlane, 3 * kQS * kQPlane, 4 * kQS * kQPlane, kVW>(
-                    a, P, X, Y, Z, N, Xp, XYp, y, z, i, dv_xy, vb, qb, LT, Tg, Sg, Rg, Vg, rho_n, Vn, Qn);
+                    a, P, X, Y, Z, N, Xp, XYp, y, z, i, dv_xy, vb, qb, LT, Tg, Vg, rho_n, Vn, Qn);
             }
 #pragma unroll
             for (int k = 0; k < 4; ++k) vb[k] = vb[k + 1];
@@ -539,16 +534,24 @@ __global__ void __launch_bounds__(256, 3) ref_pass_a_kernel(RefIterArgs a) {
 }
 
 // ----------------------------------------------------------------------------------
-// Pass A with TMA staging.  Per slice, one thread issues four tensor copies: v's box of 40
-// columns x 12 rows x 3 components (2-voxel halo) into the v ring, and psi_inv's 40 x 10 x
-// 3 box, rho's and S's 40 x 10 boxes into one slot of the psi_inv ring; each ring slot
-// completes on its own mbarrier.  The v ring holds the 5 slices z - 2 .. z + 2 and the
-// psi_inv ring the 3 slices z - 1 .. z + 1 that slice z reads, each with one more slice in
-// flight; one block barrier per slice frees the slots of slices z - 3 / z - 2 for the next
-// copies.  Out-of-volume parts of a box read as zero and are never used (the stencils
+// Pass A with TMA staging.  Fill n of a tile holds v's slice zs0 - 2 + n (a box of 40 columns x 12
+// rows x 3 components, 2-voxel halo) in a slot of the v ring and, from n = 2 on, slice zs0 - 3 + n
+// of psi_inv (40 x 10 x 3), rho and S (40 x 10) in a slot of the q ring, all copied by one thread
+// and completing on one barrier.  Slice zs0 + j reads v's fills j .. j + 4 and the q ring's
+// j + 2 .. j + 4; one block barrier per slice frees the slots of slices z - 3 / z - 2 for the next
+// fill.  Out-of-volume parts of a box read as zero and are never used (the stencils
 // that reach them are masked, as in the cp.async kernel).  Waits are bounded as in
 // ref_laplacian_tma_kernel.  The voxel arithmetic is pass_a_voxel, shared with
 // ref_pass_a_kernel.
+//
+// Bound by issue slots (three blocks of 80 registers, 600 instructions per voxel of which 250 are
+// the reference's arithmetic) and by the LT gather's latency.  163 us on the 182x218x182 pair
+// (76 bytes per voxel, 82 us at the copy bandwidth) and 384 us on four 160x192x160 pairs, 180 and
+// 431 us with cp.async staging, whose threads each form eight staging addresses per slice.
+// With a barrier per field, ring slots by division and generic addressing this kernel took
+// 193 us; per-slot empty barriers in place of the block barrier 220 us (the extra state
+// spills); the LT rows prefetched by one tensor copy instead of per thread 165 us, not
+// prefetched 170 us; rho and S three slices ahead prefetched as well 167 us.
 // ----------------------------------------------------------------------------------
 namespace {
 constexpr int kPVS = 6, kPQS = 4;                 // ring slots: v (5 + 1), psi_inv/rho/S (3 + 1)
@@ -564,26 +567,26 @@ static_assert((kPVSlot * 4) % 128 == 0 && (kPQR * 4) % 128 == 0 && (kPQSo * 4) %
 }  // namespace
 
 size_t ref_pass_a_tma_smem_bytes() {
-    return 128 + sizeof(float) * (kPVS * kPVSlot + kPQS * kPQSlot) + sizeof(uint64_t) * (kPVS + kPQS);
+    return sizeof(float) * (kPVS * kPVSlot + kPQS * kPQSlot) + sizeof(uint64_t) * kPVS;
 }
 
 __global__ void __launch_bounds__(256, 3) ref_pass_a_tma_kernel(RefIterArgs a) {
     extern __shared__ __align__(128) unsigned char pa_raw[];
-    float* vring = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(pa_raw) + 127) & ~uintptr_t(127));
+    float* vring = reinterpret_cast<float*>(pa_raw);
+    if (!ring_aligned(vring, a.err)) return;
     float* qring = vring + kPVS * kPVSlot;
-    uint64_t* fullv = reinterpret_cast<uint64_t*>(qring + kPQS * kPQSlot);
-    uint64_t* fullq = fullv + kPVS;
-    typedef SliceRing<kPVS> VRing;
-    typedef SliceRing<kPQS> QRing;
+    uint64_t* full = reinterpret_cast<uint64_t*>(qring + kPQS * kPQSlot);
     const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
     if (tid == 0) {
-        for (int k = 0; k < kPVS; ++k) mbar_init(fullv + k, 1);
-        for (int k = 0; k < kPQS; ++k) mbar_init(fullq + k, 1);
+        for (int k = 0; k < kPVS; ++k) mbar_init(full + k, 1);
         mbar_fence_init();
     }
     __syncthreads();
-    const int src = (a.iter - 1) & 1;  // the buffers this iteration reads
-    unsigned nbv = 0, nbq = 0, iv = 0, iq = 0;  // fills before this tile; fills issued (thread 0)
+    // fills go through the rings in order, across the block's tiles: the next slots to fill
+    // (thread 0) and to read, and per slot the parity of its next completion
+    int fv = 0, fq = 0, rv = 0, rq = 0;
+    unsigned phase = 0u;
+    int flying = 0;  // fills issued and not waited for (thread 0)
     bool failed = false;
     for (int t = blockIdx.x; t < a.ntiles_a && !failed; t += gridDim.x) {
         const Tile tl = a.tiles_a[t];
@@ -595,86 +598,87 @@ __global__ void __launch_bounds__(256, 3) ref_pass_a_tma_kernel(RefIterArgs a) {
         if (zs0 >= zs1 || tl.y + kTileX <= 1 || tl.z + kTileY <= 1 || tl.y >= X - 1 || tl.z >= Y - 1) continue;
         const long long NT = a.NT;
         const float* __restrict__ Vg[3] = {a.v + P.off, a.v + NT + P.off, a.v + 2 * NT + P.off};
-        const float* __restrict__ Rg = a.rho + P.off;
-        const float* __restrict__ Sg = a.S + P.off;
         const float* __restrict__ Tg = a.T + P.off;
         const float4* __restrict__ LT = a.LT + P.off;
         float* rho_n = a.rho_n + P.off;
         float* Vn[3] = {a.v_n + P.off, a.v_n + NT + P.off, a.v_n + 2 * NT + P.off};
         float* Qn[3] = {a.pinv_n + P.off, a.pinv_n + NT + P.off, a.pinv_n + 2 * NT + P.off};
-        const int pair = tl.x;
-        const int x0 = tl.y, y0 = tl.z;
-        const int x = x0 + tx, y = y0 + ty;
+        const int x = tl.y + tx, y = tl.z + ty;
         const bool active = x >= 1 && x <= X - 2 && y >= 1 && y <= Y - 2;
         const bool dv_xy = x >= 2 && x <= X - 3 && y >= 2 && y <= Y - 2;
-        const int nsteps = zs1 - zs0;
-        const int nv = nsteps + 4, nq = nsteps + 2;  // v slices zs0 - 2 .. zs1 + 1; psi_inv zs0 - 1 .. zs1
-        // the copies (thread 0 only); the maps' addresses are formed where they are used
-        auto issue_v = [&](int f) {
-            const unsigned n = nbv + (unsigned)f;
-            uint64_t* bar = fullv + VRing::slot(n);
-            const CUtensorMap* mv = a.tmaps + (long long)pair * TM_COUNT + TM_PA_V0 + src;
-            mbar_arrive_expect_tx(bar, kPVBytes);
-            tma_load_4d(vring + VRing::slot(n) * kPVSlot, mv, x0 - 4, y0 - 2, zs0 - 2 + f, 0, bar);
-            ++iv;
-        };
-        auto issue_q = [&](int f) {
-            const unsigned n = nbq + (unsigned)f;
-            uint64_t* bar = fullq + QRing::slot(n);
-            float* dst = qring + QRing::slot(n) * kPQSlot;
-            const CUtensorMap* maps = a.tmaps + (long long)pair * TM_COUNT;
-            const int z = zs0 - 1 + f;
-            mbar_arrive_expect_tx(bar, kPQBytes);
-            tma_load_4d(dst, maps + TM_PA_Q0 + src, x0 - 4, y0 - 1, z, 0, bar);
-            tma_load_3d(dst + kPQR, maps + TM_PA_R0 + src, x0 - 4, y0 - 1, z, bar);
-            tma_load_3d(dst + kPQSo, maps + TM_PA_S, x0 - 4, y0 - 1, z, bar);
-            ++iq;
+        const int nfill = zs1 - zs0 + 4;
+        auto issue = [&](int n) {  // thread 0
+            const CUtensorMap* maps = a.tmaps + (long long)tl.x * TM_COUNT;
+            const int src = (a.iter - 1) & 1, zv = zs0 - 2 + n;  // src: the buffers this iteration reads
+            uint64_t* bar = full + fv;
+            mbar_arrive_expect_tx(bar, n >= 2 ? kPVBytes + kPQBytes : kPVBytes);
+            tma_load_4d(vring + fv * kPVSlot, maps + TM_PA_V0 + src, tl.y - 4, tl.z - 2, zv, 0, bar);
+            if (n >= 2) {
+                float* dst = qring + fq * kPQSlot;
+                tma_load_4d(dst, maps + TM_PA_Q0 + src, tl.y - 4, tl.z - 1, zv - 1, 0, bar);
+                tma_load_3d(dst + kPQR, maps + TM_PA_R0 + src, tl.y - 4, tl.z - 1, zv - 1, bar);
+                tma_load_3d(dst + kPQSo, maps + TM_PA_S, tl.y - 4, tl.z - 1, zv - 1, bar);
+                fq = fq + 1 == kPQS ? 0 : fq + 1;
+            }
+            fv = fv + 1 == kPVS ? 0 : fv + 1;
+            ++flying;
         };
         __syncthreads();  // the previous tile is done with the rings
-        if (tid == 0) {
-            for (int f = 0; f < min(nv, kPVS); ++f) issue_v(f);
-            for (int f = 0; f < min(nq, kPQS); ++f) issue_q(f);
+        if (tid == 0)
+            for (int n = 0; n < min(nfill, kPVS); ++n) issue(n);
+
+        const int vc0 = (ty + 2) * kPW + tx + 4, qc0 = (ty + 1) * kPW + tx + 4;
+        const float* vb[5];  // this thread's column in the slices read, rotated by one per step
+        const float* qb[3];
+        bool ok = true;
+        auto land = [&]() {  // waits for the next fill
+            ok = mbar_wait_bounded(full + rv, (phase >> rv) & 1u) && ok;
+            phase ^= 1u << rv;
+            --flying;
+        };
+        auto next_v = [&](int k) {
+            vb[k] = vring + rv * kPVSlot + vc0;
+            rv = rv + 1 == kPVS ? 0 : rv + 1;
+        };
+        auto next_q = [&](int k) {
+            qb[k] = qring + rq * kPQSlot + qc0;
+            rq = (rq + 1) & (kPQS - 1);
+        };
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            land();
+            next_v(k + 1);
+            if (k >= 2) next_q(k - 1);
         }
-        const int vc0 = (ty + 2) * kPW + tx + 4;
-        const int qc0 = (ty + 1) * kPW + tx + 4;
-        for (int j0 = 0; j0 < nsteps; ++j0) {
-            // slice z = zs0 + j0 reads v fills j0 .. j0 + 4 and psi_inv fills j0 .. j0 + 2
-            bool ok = true;
-            for (int f = (j0 == 0 ? 0 : j0 + 4); f <= j0 + 4; ++f)
-                ok = ok && mbar_wait_bounded(fullv + VRing::slot(nbv + f), VRing::parity(nbv + f));
-            for (int f = (j0 == 0 ? 0 : j0 + 2); f <= j0 + 2; ++f)
-                ok = ok && mbar_wait_bounded(fullq + QRing::slot(nbq + f), QRing::parity(nbq + f));
-            // every thread is past slice z - 1: the slots of v fill j0 - 1 and psi_inv fill
-            // j0 - 1 are free; the block agrees on whether any wait gave up
+        for (int z = zs0; z < zs1; ++z) {
+            land();
+            // every thread is past slice z - 1, whose oldest fill is free, and the block agrees on
+            // whether any wait gave up
             if (__syncthreads_or(!ok)) {
                 failed = true;
                 break;
             }
-            if (tid == 0 && j0 >= 1) {
-                if (j0 - 1 + kPVS < nv) issue_v(j0 - 1 + kPVS);
-                if (j0 - 1 + kPQS < nq) issue_q(j0 - 1 + kPQS);
-            }
+            if (tid == 0 && z > zs0 && z - zs0 - 1 + kPVS < nfill) issue(z - zs0 - 1 + kPVS);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) vb[k] = vb[k + 1];
+            qb[0] = qb[1];
+            qb[1] = qb[2];
+            next_v(4);
+            next_q(2);
             if (active) {
-                const int z = zs0 + j0;
                 const int i = x + Xp * y + XYp * z;
-                const float* vb[5];
-#pragma unroll
-                for (int k = 0; k < 5; ++k) vb[k] = vring + VRing::slot(nbv + j0 + k) * kPVSlot + vc0;
-                const float* qb[3];
-#pragma unroll
-                for (int k = 0; k < 3; ++k) qb[k] = qring + QRing::slot(nbq + j0 + k) * kPQSlot + qc0;
                 pass_a_voxel<kPVPlane, kPQPlane, kPQR, kPQSo, kPW>(a, P, X, Y, Z, N, Xp, XYp, y, z, i, dv_xy, vb, qb,
-                                                                   LT, Tg, Sg, Rg, Vg, rho_n, Vn, Qn);
+                                                                   LT, Tg, Vg, rho_n, Vn, Qn);
             }
         }
-        nbv += (unsigned)nv;  // every fill of the tile has been waited for
-        nbq += (unsigned)nq;
     }
     if (failed && tid == 0) {
-        for (unsigned n = (iv > (unsigned)kPVS ? iv - kPVS : 0u); n < iv; ++n)
-            mbar_wait_bounded(fullv + VRing::slot(n), VRing::parity(n));
-        for (unsigned n = (iq > (unsigned)kPQS ? iq - kPQS : 0u); n < iq; ++n)
-            mbar_wait_bounded(fullq + QRing::slot(n), QRing::parity(n));
+        // the copies in flight end (bounded) before the block's shared memory goes
+        for (; flying > 0; --flying) {
+            mbar_wait_bounded(full + rv, (phase >> rv) & 1u);
+            phase ^= 1u << rv;
+            rv = rv + 1 == kPVS ? 0 : rv + 1;
+        }
         atomicOr(a.err, kErrTmaTimeout);
     }
 }

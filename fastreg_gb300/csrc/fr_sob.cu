@@ -66,12 +66,13 @@ constexpr unsigned kGBytes = sizeof(float) * (3 * kGPlane + kTileX * kTileY);
 static_assert(kGSlot % 32 == 0, "slots on 128-byte boundaries");
 }  // namespace
 
-size_t sob_grad_smem_bytes() { return 128 + sizeof(float) * kGS * kGSlot + 2 * sizeof(uint64_t) * kGS; }
+size_t sob_grad_smem_bytes() { return sizeof(float) * kGS * kGSlot + 2 * sizeof(uint64_t) * kGS; }
 
 template <bool TMA>
 __global__ void __launch_bounds__(sob_grad_threads(TMA), TMA ? 4 : 6) sob_grad_kernel(SobIterArgs a) {
     extern __shared__ __align__(128) unsigned char grad_raw[];
-    float* ring = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(grad_raw) + 127) & ~uintptr_t(127));
+    float* ring = reinterpret_cast<float*>(grad_raw);
+    if (TMA && !ring_aligned(ring, a.err)) return;
     uint64_t* full = reinterpret_cast<uint64_t*>(ring + kGS * kGSlot);
     uint64_t* empty = full + kGS;
     const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;

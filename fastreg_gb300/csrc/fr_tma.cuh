@@ -100,5 +100,16 @@ struct SliceRing {
 
 // Codes of the device error word (RefIterArgs::err, SobIterArgs::err).
 constexpr unsigned kErrTmaTimeout = 1u;
+constexpr unsigned kErrSmemAlign = 2u;
+
+// A staging ring at the start of dynamic shared memory.  The array's alignment attribute puts
+// it on the 128-byte boundary that tensor copies need; a pointer rounded up by hand would lose
+// its address space and turn every read of the ring into a generic load.  False (and the error
+// word set) if the boundary is missed: no copy is issued then.
+__device__ __forceinline__ bool ring_aligned(const void* ring, unsigned* err) {
+    if ((smem_u32(ring) & 127u) == 0u) return true;
+    if (threadIdx.x == 0) atomicOr(err, kErrSmemAlign);
+    return false;
+}
 
 }  // namespace frg
