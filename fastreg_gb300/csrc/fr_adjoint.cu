@@ -64,19 +64,6 @@ __global__ void __launch_bounds__(256) adj_pack_kernel(AdjPair A, const float* _
     }
 }
 
-// The tables of the forward kernels and of the transposed smoothing: 32 x rows x depth tiles.
-struct AdjTables {
-    Tile* at[4];
-    int rows[4], depth[4], count[4];
-};
-__global__ void adj_tables_kernel(AdjPair A, AdjTables T) {
-    for (int k = 0; k < 4; ++k) {
-        const int nx = (A.X + kTileX - 1) / kTileX, ny = (A.Y + T.rows[k] - 1) / T.rows[k];
-        GRID_STRIDE(i, T.count[k])
-        T.at[k][i] = make_int4(0, (i % nx) * kTileX, (i / nx % ny) * T.rows[k], (i / (nx * ny)) * T.depth[k]);
-    }
-}
-
 // The result: the adjoint of v0 out of the interleaved accumulator.
 __global__ void __launch_bounds__(256) adj_unpack_kernel(AdjPair A, const float4* __restrict__ mbar, float* out) {
     const long long nu = (long long)A.X * A.Y * A.Z;
@@ -538,8 +525,7 @@ extern "C" int fr_sobolev_loss_grad(const float* d_T, const float* d_S, const in
     // the workspace: checkpoints (phi, m) x nseg, the states of a segment (phi, m) x ck, two
     // working states, g, gbar, pbar, the interleaved mbar, S and T; and a small head
     auto round_up = [](size_t b) { return (b + 255) / 256 * 256; };
-    size_t head = round_up(sizeof(Pair)) + round_up(64);
-    for (const Cut& c : cuts) head += round_up(sizeof(Tile) * (size_t)c.count);
+    const size_t head = round_up(sizeof(Pair)) + round_up(64);
     const size_t plane = round_up(N3 * sizeof(float)), scalar = round_up((size_t)A.NT * sizeof(float));
     const size_t bytes = head + plane * (2 * nseg + 2 * ck + 4 + 3) + round_up((size_t)A.NT * sizeof(float4)) + 2 * scalar;
     bool cached = false;
@@ -555,15 +541,7 @@ extern "C" int fr_sobolev_loss_grad(const float* d_T, const float* d_S, const in
         return p;
     };
     Pair* pair = (Pair*)take(sizeof(Pair));
-    char* small = take(64);  // loss and lambda_bar; the pair's stop word
-    double* dd = (double*)small;
-    AdjTables tables{};
-    for (int k = 0; k < 4; ++k) {
-        tables.at[k] = (Tile*)take(sizeof(Tile) * (size_t)cuts[k].count);
-        tables.rows[k] = cuts[k].rows;
-        tables.depth[k] = cuts[k].depth;
-        tables.count[k] = cuts[k].count;
-    }
+    double* dd = (double*)take(64);  // loss and lambda_bar
     auto field = [&]() { return (float*)take(N3 * sizeof(float)); };
     struct State {
         float *phi, *m;
@@ -578,10 +556,15 @@ extern "C" int fr_sobolev_loss_grad(const float* d_T, const float* d_S, const in
 
     SobIterArgs a{};
     a.pairs = pair;
-    a.tiles_g = tables.at[0];
+    a.single = 1;  // tiles and pair from the arguments, no convergence test
+    a.pair0.X = A.X;
+    a.pair0.Y = A.Y;
+    a.pair0.Z = A.Z;
+    a.pair0.Xp = A.Xp;
+    a.pair0.N = A.N;
+    a.pair0.w_reg = lambda;
     a.ntiles_g = cuts[0].count;
     a.depth_g = cuts[0].depth;
-    a.tiles_b = tables.at[2];
     a.ntiles_b = cuts[2].count;
     a.depth_b = cuts[2].depth;
     a.npairs = 1;
@@ -595,7 +578,6 @@ extern "C" int fr_sobolev_loss_grad(const float* d_T, const float* d_S, const in
     gaussian_taps(smooth_sigma, smooth_width, a.taps);
     a.radius = R;
     fold_weights(a.taps, R, a.fold);
-    a.stop = (int*)(small + 16);  // 0: no convergence test ends the unrolled iterations
     const int grid = grid_for(A.N), columns = cuts[2].count;
     int rc = FR_OK;
     auto ok = [&](cudaError_t e) {
@@ -610,33 +592,23 @@ extern "C" int fr_sobolev_loss_grad(const float* d_T, const float* d_S, const in
         a.m = from.m;
         a.phi_n = to.phi;
         a.m_n = to.m;
-        a.tiles_s = tables.at[1];
         a.ntiles_s = cuts[1].count;
         a.depth_s = cuts[1].depth;
-        ok(launch_sob_kernel(0, a, cuts[0].count, 0, s));
-        ok(launch_sob_kernel(1, a, cuts[1].count, kUnrolled | (tall ? 2 : 0), s));
-        if (update) ok(launch_sob_kernel(2, a, cuts[2].count, kUnrolled, s));
+        ok(launch_sob_kernel(0, a, cuts[0].count, 0, s, true));
+        ok(launch_sob_kernel(1, a, cuts[1].count, kUnrolled | (tall ? 2 : 0), s, true));
+        if (update) ok(launch_sob_kernel(2, a, cuts[2].count, kUnrolled, s, true));
     };
     auto smooth_adjoint = [&]() {  // gbar = G^T g
         SobIterArgs t = a;
         t.m_n = gbar;
-        t.tiles_s = tables.at[3];
         t.ntiles_s = cuts[3].count;
         t.depth_s = cuts[3].depth;
         void* args[1] = {&t};
-        ok(cudaLaunchKernel(sob_smooth3_unrolled_fn(R, true, tall), dim3(cuts[3].count), dim3(kSmoothThreads), args, 0, s));
+        ok(launch_kernel(sob_smooth3_unrolled_fn(R, true, tall), cuts[3].count, kSmoothThreads, 0, args, s, true));
     };
     do {
-        Pair hp{};
-        hp.X = A.X;
-        hp.Y = A.Y;
-        hp.Z = A.Z;
-        hp.Xp = A.Xp;
-        hp.N = A.N;
-        hp.w_reg = lambda;
-        if (!ok(cudaMemcpyAsync(pair, &hp, sizeof hp, cudaMemcpyHostToDevice, s))) break;
-        if (!ok(cudaMemsetAsync(small, 0, 64, s))) break;
-        adj_tables_kernel<<<sms, 256, 0, s>>>(A, tables);
+        if (!ok(cudaMemcpyAsync(pair, &a.pair0, sizeof(Pair), cudaMemcpyHostToDevice, s))) break;
+        if (!ok(cudaMemsetAsync(dd, 0, 64, s))) break;
         adj_pack_kernel<<<grid, 256, 0, s>>>(A, d_S, d_T, d_v0, Sp, Tp, ckpt[0].phi, ckpt[0].m);
         // forward: a segment's first state is its checkpoint, and the last segment's states stay
         State st = ckpt[0];

@@ -587,6 +587,9 @@ int setup_cohort(fr_handle* h, const fr_pair* pairs, int n) {
 frg::RefIterArgs ref_args(fr_handle* h, int iter, float t) {
     frg::RefIterArgs a{};
     a.pairs = h->d_pairs;
+    a.pair0 = h->hpairs[0];
+    a.single = h->npairs == 1;
+    a.check_stop = h->P.max_update_norm >= 0.f;  // an update norm is never below 0
     a.tiles_l = h->ts[R_LAP].d;
     a.ntiles_l = (int)h->ts[R_LAP].h.size();
     a.depth_l = h->ts[R_LAP].shape.depth;
@@ -631,18 +634,14 @@ frg::RefIterArgs ref_args(fr_handle* h, int iter, float t) {
 
 int launch_ref_iter(fr_handle* h, int iter, float t, cudaStream_t s, cudaEvent_t* ev) {
     frg::RefIterArgs a = ref_args(h, iter, t);
-    if (ev) cudaEventRecord(ev[0], s);
-    if (h->ts[R_LAP].shape.variant)
-        frg::ref_laplacian_tma_kernel<<<h->ts[R_LAP].grid, 256, frg::ref_laplacian_tma_smem_bytes(), s>>>(a);
-    else
-        frg::ref_laplacian_kernel<<<h->ts[R_LAP].grid, 256, frg::ref_laplacian_smem_bytes(), s>>>(a);
-    if (ev) cudaEventRecord(ev[1], s);
-    if (h->ts[R_PA].shape.variant)
-        frg::ref_pass_a_tma_kernel<<<h->ts[R_PA].grid, 256, frg::ref_pass_a_tma_smem_bytes(), s>>>(a);
-    else
-        frg::ref_pass_a_kernel<<<h->ts[R_PA].grid, 256, frg::ref_pass_a_smem_bytes(), s>>>(a);
-    if (ev) cudaEventRecord(ev[2], s);
-    frg::ref_pass_b_kernel<<<h->ts[R_PB].grid, frg::kPassBThreads, 0, s>>>(a);
+    void* args[1] = {&a};
+    const int roles[3] = {R_LAP, R_PA, R_PB};
+    for (int k = 0; k < 3; ++k) {
+        const int r = roles[k], v = h->ts[r].shape.variant;
+        if (ev) cudaEventRecord(ev[k], s);
+        FR_CUDA(h, frg::launch_kernel(role_fn(h, r, v), h->ts[r].grid, role_threads(r, v), role_smem(r, v), args, s,
+                                      !ev));
+    }
     if (ev) cudaEventRecord(ev[3], s);
     FR_LAUNCHED(h);
     return FR_OK;
@@ -654,6 +653,9 @@ int kernels_per_iter(const fr_handle*) { return 3; }
 frg::SobIterArgs sob_args(fr_handle* h, int iter) {
     frg::SobIterArgs a{};
     a.pairs = h->d_pairs;
+    a.pair0 = h->hpairs[0];
+    a.single = h->npairs == 1;
+    a.check_stop = h->P.max_update_norm >= 0.f;  // an update norm is never below 0
     a.tiles_g = h->ts[R_SG].d;
     a.ntiles_g = (int)h->ts[R_SG].h.size();
     a.depth_g = h->ts[R_SG].shape.depth;
@@ -691,8 +693,15 @@ int launch_iter(fr_handle* h, int iter, float t, cudaStream_t s, cudaEvent_t* ev
     const frg::SobIterArgs a = sob_args(h, iter);
     const int grids[3] = {h->ts[R_SG].grid, h->ts[R_SS].grid, h->ts[R_SB].grid};
     const int variants[3] = {h->ts[R_SG].shape.variant, h->ts[R_SS].shape.variant, h->ts[R_SB].shape.variant};
-    cudaError_t e = frg::launch_sob_iter(a, grids, variants, s, ev);
+    cudaError_t e = frg::launch_sob_iter(a, grids, variants, s, !ev, ev);
     if (e != cudaSuccess) return fail(h, FR_ERR_CUDA, "sobolev launch failed: %s", cudaGetErrorString(e));
+    return FR_OK;
+}
+
+// An iteration that the caller steps may have been run before: its record starts from 0 again
+// (a registration's are cleared when it begins).
+int clear_trace(fr_handle* h, int iter, cudaStream_t s) {
+    FR_CUDA(h, cudaMemsetAsync(h->trace + (size_t)(iter - 1) * h->npairs, 0, sizeof(unsigned long long) * h->npairs, s));
     return FR_OK;
 }
 
@@ -877,11 +886,11 @@ int launch_role(fr_handle* h, int r, int iter, float t, cudaStream_t s) {
     // no pair converges while shapes are timed (a stopped pair's tiles would be skipped)
     if (r == R_LAP || r == R_PA || r == R_PB) {
         ra = ref_args(h, iter, t);
-        ra.max_update_norm = -INFINITY;
+        ra.check_stop = 0;
         args[0] = &ra;
     } else {
         sa = sob_args(h, iter);
-        sa.max_update_norm = -INFINITY;
+        sa.check_stop = 0;
         args[0] = &sa;
     }
     const int v = h->ts[r].shape.variant;
@@ -1320,7 +1329,8 @@ int fr_step(fr_handle* h, int iter, float t, void* stream) {
     if (!h->have_state) return fail(h, FR_ERR_STATE, "fr_step before fr_begin");
     if (iter < 1 || iter > h->trace_cap) return fail(h, FR_ERR_INVALID_ARG, "iter %d outside [1, %d]", iter, h->trace_cap);
     if (!(t > 0.f)) return fail(h, FR_ERR_INVALID_ARG, "t must be > 0");
-    int rc = launch_iter(h, iter, t, (cudaStream_t)stream);
+    int rc = clear_trace(h, iter, (cudaStream_t)stream);
+    if (rc == FR_OK) rc = launch_iter(h, iter, t, (cudaStream_t)stream);
     if (rc == FR_OK) {
         h->last_iter = iter;
         h->stats_ready = false;
@@ -1494,7 +1504,8 @@ int fr_time_kernels(fr_handle* h, int iters, float* ms, int* n_kernels, void* st
         // iterations cycle through the schedule; every kernel reads what it would read
         const int slot = 1 + (it - 1) % std::max(h->trace_cap, 1);
         const float t = ts.empty() ? h->P.alpha : ts[(slot - 1) % ts.size()];
-        rc = launch_iter(h, slot, t, s, ev);
+        rc = clear_trace(h, slot, s);
+        if (rc == FR_OK) rc = launch_iter(h, slot, t, s, ev);
         if (rc != FR_OK) break;
         cudaError_t e = cudaEventSynchronize(ev[nk]);
         for (int k = 0; k < nk && e == cudaSuccess; ++k) {

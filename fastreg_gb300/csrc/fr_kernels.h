@@ -33,6 +33,9 @@ enum TmapIndex {
 // Arguments of one reference-mode iteration (all three launches take the same block).
 struct RefIterArgs {
     const Pair* pairs;
+    Pair pair0;      // the pair of a single-pair cohort
+    int single;      // npairs == 1: the kernels take tiles and pair from the arguments (take_tile)
+    int check_stop;  // max_update_norm can be reached: test for convergence, skip converged pairs
     const Tile* tiles_l;  // 32 x 8 x depth_l tiles (Laplacian)
     int ntiles_l, depth_l;
     const Tile* tiles_a;  // 32 x 8 x depth_a tiles (pass A)

@@ -87,13 +87,14 @@ constexpr int kTPlane = kTileX * kTileY;
 size_t ref_laplacian_smem_bytes() { return sizeof(float) * kLS * (3 * kQPlane + (kLStageT ? kTPlane : 0)); }
 
 __global__ void __launch_bounds__(256) ref_laplacian_kernel(RefIterArgs a) {
+    pdl_wait();
     extern __shared__ __align__(16) float ring[];  // psi [3][kLS][kQR][kQW], then T [kLS][8][32]
     float* tring = ring + 3 * kLS * kQPlane;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     for (int t = blockIdx.x; t < a.ntiles_l; t += gridDim.x) {
-        const Tile tl = a.tiles_l[t];
-        if (a.stop[tl.x]) continue;  // uniform over the block
-        const Pair P = a.pairs[tl.x];
+        Tile tl;
+        Pair P;
+        if (!take_tile(a, a.tiles_l, t, kTileY, a.depth_l, tl, P)) continue;  // uniform over the block
         const int X = P.X, Y = P.Y, Z = P.Z, Xp = P.Xp, XYp = P.Xp * P.Y;  // strides of the packed arrays
         const int zs0 = max(tl.w, 1), zs1 = min(tl.w + a.depth_l, Z - 1);
         if (zs0 >= zs1 || tl.y + kTileX <= 1 || tl.z + kTileY <= 1 || tl.y >= X - 1 || tl.z >= Y - 1) continue;
@@ -191,6 +192,7 @@ static_assert(3 * kTQPlane <= kTTOff && (kTTOff * 4) % 128 == 0 && (kTSlot * 4) 
 size_t ref_laplacian_tma_smem_bytes() { return sizeof(float) * kTLS * kTSlot + sizeof(uint64_t) * kTLS; }
 
 __global__ void __launch_bounds__(256) ref_laplacian_tma_kernel(RefIterArgs a) {
+    pdl_wait();
     extern __shared__ __align__(128) unsigned char lap_raw[];
     float* ring = reinterpret_cast<float*>(lap_raw);
     if (!ring_aligned(ring, a.err)) return;
@@ -212,9 +214,9 @@ __global__ void __launch_bounds__(256) ref_laplacian_tma_kernel(RefIterArgs a) {
     unsigned wph = 0u;
     bool failed = false;
     for (int t = blockIdx.x; t < a.ntiles_l && !failed; t += gridDim.x) {
-        const Tile tl = a.tiles_l[t];
-        if (a.stop[tl.x]) continue;  // uniform over the block
-        const Pair P = a.pairs[tl.x];
+        Tile tl;
+        Pair P;
+        if (!take_tile(a, a.tiles_l, t, kTileY, a.depth_l, tl, P)) continue;  // uniform over the block
         const int X = P.X, Y = P.Y, Z = P.Z, Xp = P.Xp, XYp = P.Xp * P.Y;
         const int zs0 = max(tl.w, 1), zs1 = min(tl.w + a.depth_l, Z - 1);
         if (zs0 >= zs1 || tl.y + kTileX <= 1 || tl.z + kTileY <= 1 || tl.y >= X - 1 || tl.z >= Y - 1) continue;
@@ -429,6 +431,7 @@ __device__ __forceinline__ void pass_a_voxel(const RefIterArgs& a, const Pair& P
 }
 
 __global__ void __launch_bounds__(256, 3) ref_pass_a_kernel(RefIterArgs a) {
+    pdl_wait();
     extern __shared__ __align__(16) float smem[];
     PassASmem sm;
     sm.v = smem;
@@ -436,9 +439,9 @@ __global__ void __launch_bounds__(256, 3) ref_pass_a_kernel(RefIterArgs a) {
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
 
     for (int t = blockIdx.x; t < a.ntiles_a; t += gridDim.x) {
-        const Tile tl = a.tiles_a[t];
-        if (a.stop[tl.x]) continue;  // uniform over the block
-        const Pair P = a.pairs[tl.x];
+        Tile tl;
+        Pair P;
+        if (!take_tile(a, a.tiles_a, t, kTileY, a.depth_a, tl, P)) continue;  // uniform over the block
         const int X = P.X, Y = P.Y, Z = P.Z, N = (int)P.N;
         const int Xp = P.Xp, XYp = P.Xp * P.Y;  // strides of the packed arrays
         const int zs0 = max(tl.w, 1), zs1 = min(tl.w + a.depth_a, Z - 1);
@@ -571,6 +574,7 @@ size_t ref_pass_a_tma_smem_bytes() {
 }
 
 __global__ void __launch_bounds__(256, 3) ref_pass_a_tma_kernel(RefIterArgs a) {
+    pdl_wait();
     extern __shared__ __align__(128) unsigned char pa_raw[];
     float* vring = reinterpret_cast<float*>(pa_raw);
     if (!ring_aligned(vring, a.err)) return;
@@ -589,9 +593,9 @@ __global__ void __launch_bounds__(256, 3) ref_pass_a_tma_kernel(RefIterArgs a) {
     int flying = 0;  // fills issued and not waited for (thread 0)
     bool failed = false;
     for (int t = blockIdx.x; t < a.ntiles_a && !failed; t += gridDim.x) {
-        const Tile tl = a.tiles_a[t];
-        if (a.stop[tl.x]) continue;  // uniform over the block
-        const Pair P = a.pairs[tl.x];
+        Tile tl;
+        Pair P;
+        if (!take_tile(a, a.tiles_a, t, kTileY, a.depth_a, tl, P)) continue;  // uniform over the block
         const int X = P.X, Y = P.Y, Z = P.Z, N = (int)P.N;
         const int Xp = P.Xp, XYp = P.Xp * P.Y;
         const int zs0 = max(tl.w, 1), zs1 = min(tl.w + a.depth_a, Z - 1);
@@ -691,13 +695,13 @@ __global__ void __launch_bounds__(256, 3) ref_pass_a_tma_kernel(RefIterArgs a) {
 // blocks held 32 (at 64 registers; at 48, for 5 blocks of 256, it spills).
 // ----------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kPassBThreads, 9) ref_pass_b_kernel(RefIterArgs a) {
+    pdl_wait();
     __shared__ unsigned long long red[32];
-    __shared__ bool last;
     const int tid = threadIdx.x;
     for (int t = blockIdx.x; t < a.ntiles_b; t += gridDim.x) {
-        const Tile tl = a.tiles_b[t];
-        if (a.stop[tl.x]) continue;  // uniform over the block
-        const Pair P = a.pairs[tl.x];
+        Tile tl;
+        Pair P;
+        if (!take_tile(a, a.tiles_b, t, kPassBTileY, a.depth_b, tl, P)) continue;  // uniform over the block
         const int x = tl.y + (int)(threadIdx.x & 31), y = tl.z + (int)(threadIdx.x >> 5);
         unsigned long long best = 0ull;
         if (x >= 1 && x <= P.X - 2 && y >= 1 && y <= P.Y - 2) {
@@ -739,24 +743,10 @@ __global__ void __launch_bounds__(kPassBThreads, 9) ref_pass_b_kernel(RefIterArg
             }
         }
         const unsigned long long bm = block_max_u64(best, red);
-        if (tid == 0 && bm) atomicMax(a.keys + tl.x, bm);
+        if (tid == 0) note_max(a, tl.x, bm);
     }
 
-    // the last block to finish records this iteration and decides convergence
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) last = (atomicAdd(a.counter, 1u) == gridDim.x - 1);
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    for (int p = tid; p < a.npairs; p += blockDim.x) {
-        if (a.stop[p]) continue;
-        const unsigned long long k = atomicExch(a.keys + p, 0ull);
-        a.trace[(long long)(a.iter - 1) * a.npairs + p] = k;
-        const float mx = __uint_as_float((unsigned)(k >> 32));
-        if (mx <= a.max_update_norm) a.stop[p] = a.iter;
-    }
-    if (tid == 0) *a.counter = 0u;
+    record_and_test(a);
 }
 
 }  // namespace frg

@@ -70,6 +70,7 @@ size_t sob_grad_smem_bytes() { return sizeof(float) * kGS * kGSlot + 2 * sizeof(
 
 template <bool TMA>
 __global__ void __launch_bounds__(sob_grad_threads(TMA), TMA ? 4 : 6) sob_grad_kernel(SobIterArgs a) {
+    pdl_wait();
     extern __shared__ __align__(128) unsigned char grad_raw[];
     float* ring = reinterpret_cast<float*>(grad_raw);
     if (TMA && !ring_aligned(ring, a.err)) return;
@@ -90,10 +91,11 @@ __global__ void __launch_bounds__(sob_grad_threads(TMA), TMA ? 4 : 6) sob_grad_k
             unsigned n = 0;  // fills: fill n goes to slot n % kGS, the (n / kGS)-th of that slot
             bool ok = true;
             for (int t = blockIdx.x; t < a.ntiles_g && ok; t += gridDim.x) {
-                const Tile tl = a.tiles_g[t];
-                if (a.stop[tl.x]) continue;
+                Tile tl;
+                Pair P;
+                if (!take_tile(a, a.tiles_g, t, kTileY, a.depth_g, tl, P)) continue;
                 const CUtensorMap* maps = a.tmaps + (long long)tl.x * TM_COUNT;
-                const int z1 = min(tl.w + a.depth_g, a.pairs[tl.x].Z);
+                const int z1 = min(tl.w + a.depth_g, P.Z);
                 for (int z = tl.w - 1; z <= z1 && ok; ++z, ++n) {
                     const int k = SliceRing<kGS>::slot(n);
                     // the slot's previous reader has released it (an unused slot counts as released)
@@ -117,9 +119,9 @@ __global__ void __launch_bounds__(sob_grad_threads(TMA), TMA ? 4 : 6) sob_grad_k
     bool failed = false;
 
     for (int t = blockIdx.x; t < a.ntiles_g && !failed; t += gridDim.x) {
-        const Tile tl = a.tiles_g[t];
-        if (a.stop[tl.x]) continue;  // uniform over the block
-        const Pair P = a.pairs[tl.x];
+        Tile tl;
+        Pair P;
+        if (!take_tile(a, a.tiles_g, t, kTileY, a.depth_g, tl, P)) continue;  // uniform over the block
         const int X = P.X, Y = P.Y, Z = P.Z, Xp = P.Xp, XYp = P.Xp * P.Y;  // strides of the packed arrays
         const long long NT = a.NT;
         const float* __restrict__ S = a.S + P.off;
@@ -265,13 +267,13 @@ const void* sob_grad_fn(int tma) {
 // UNROLLED: from phi to phi_n, without the update norm and the convergence test; else in place.
 template <bool UNROLLED>
 __global__ void __launch_bounds__(256, 4) sob_pass_b_kernel(SobIterArgs a) {
+    pdl_wait();
     constexpr bool NORM = !UNROLLED;
     __shared__ unsigned long long red[32];
-    __shared__ bool last;
     for (int t = blockIdx.x; t < a.ntiles_b; t += gridDim.x) {
-        const Tile tl = a.tiles_b[t];
-        if (a.stop[tl.x]) continue;
-        const Pair P = a.pairs[tl.x];
+        Tile tl;
+        Pair P;
+        if (!take_tile(a, a.tiles_b, t, kTileY, a.depth_b, tl, P)) continue;  // uniform over the block
         const int x = tl.y + (int)(threadIdx.x & 31), y = tl.z + (int)(threadIdx.x >> 5);
         unsigned long long best = 0ull;
         if (x < P.X && y < P.Y) {
@@ -337,47 +339,31 @@ __global__ void __launch_bounds__(256, 4) sob_pass_b_kernel(SobIterArgs a) {
         }
         if (!NORM) continue;
         const unsigned long long bm = block_max_u64(best, red);
-        if (threadIdx.x == 0 && bm) atomicMax(a.keys + tl.x, bm);
+        if (threadIdx.x == 0) note_max(a, tl.x, bm);
     }
-    if (!NORM) return;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = (atomicAdd(a.counter, 1u) == gridDim.x - 1);
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    for (int p = threadIdx.x; p < a.npairs; p += blockDim.x) {
-        if (a.stop[p]) continue;
-        const unsigned long long k = atomicExch(a.keys + p, 0ull);
-        a.trace[(long long)(a.iter - 1) * a.npairs + p] = k;
-        const float mx = __uint_as_float((unsigned)(k >> 32));
-        if (mx <= a.max_update_norm) a.stop[p] = a.iter;
-    }
-    if (threadIdx.x == 0) *a.counter = 0u;
+    if (NORM) record_and_test(a);
 }
 
 const void* sob_pass_b_fn(bool unrolled) {
     return unrolled ? (const void*)sob_pass_b_kernel<true> : (const void*)sob_pass_b_kernel<false>;
 }
 
-cudaError_t launch_sob_kernel(int k, const SobIterArgs& a, int grid, int variant, cudaStream_t s) {
+cudaError_t launch_sob_kernel(int k, const SobIterArgs& a, int grid, int variant, cudaStream_t s, bool behind) {
     void* args[1] = {const_cast<SobIterArgs*>(&a)};
-    if (k == 0)
-        return cudaLaunchKernel(sob_grad_fn(variant), dim3(grid), dim3(sob_grad_threads(variant)), args,
-                                sob_grad_smem_bytes(), s);
+    if (k == 0) return launch_kernel(sob_grad_fn(variant), grid, sob_grad_threads(variant), sob_grad_smem_bytes(), args, s, behind);
     if (k == 1)
-        return cudaLaunchKernel(variant & kUnrolled ? sob_smooth3_unrolled_fn(a.radius, false, variant & 2)
-                                                    : sob_smooth3_fn(a.radius, variant & 1, variant & 2),
-                                dim3(grid), dim3(kSmoothThreads), args, 0, s);
-    return cudaLaunchKernel(sob_pass_b_fn(variant & kUnrolled), dim3(grid), dim3(256), args, 0, s);
+        return launch_kernel(variant & kUnrolled ? sob_smooth3_unrolled_fn(a.radius, false, variant & 2)
+                                                 : sob_smooth3_fn(a.radius, variant & 1, variant & 2),
+                             grid, kSmoothThreads, 0, args, s, behind);
+    return launch_kernel(sob_pass_b_fn(variant & kUnrolled), grid, 256, 0, args, s, behind);
 }
 
 cudaError_t launch_sob_iter(const SobIterArgs& a, const int* grids, const int* variants, cudaStream_t s,
-                            cudaEvent_t* ev) {
+                            bool behind, cudaEvent_t* ev) {
     cudaError_t e = cudaSuccess;
     for (int k = 0; k < 3 && e == cudaSuccess; ++k) {
         if (ev) cudaEventRecord(ev[k], s);
-        e = launch_sob_kernel(k, a, grids[k], variants[k], s);
+        e = launch_sob_kernel(k, a, grids[k], variants[k], s, behind);
     }
     if (ev) cudaEventRecord(ev[3], s);
     return e;

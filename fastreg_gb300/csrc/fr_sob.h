@@ -35,6 +35,9 @@ constexpr bool sob_smooth_has_tall(int radius) { return sob_smooth_tile_y(radius
 
 struct SobIterArgs {
     const Pair* pairs;
+    Pair pair0;      // the pair of a single-pair cohort
+    int single;      // npairs == 1: the kernels take tiles and pair from the arguments (take_tile)
+    int check_stop;  // max_update_norm can be reached: test for convergence, skip converged pairs
     // each kernel's own table of 32 x 8 x depth tiles (smoothing: its own rows)
     const Tile* tiles_g;
     int ntiles_g, depth_g;
@@ -91,13 +94,13 @@ const void* sob_pass_b_fn(bool unrolled);  // the update kernel
 constexpr int kUnrolled = 4;  // variant bit: the unrolled registration's kernel (separate in and out states)
 
 // one of them: k = 0 gradient, 1 smoothing, 2 update
-cudaError_t launch_sob_kernel(int k, const SobIterArgs& a, int grid, int variant, cudaStream_t s);
+cudaError_t launch_sob_kernel(int k, const SobIterArgs& a, int grid, int variant, cudaStream_t s, bool behind);
 
 // grids: {grad, smooth, pass_b}; variants: of {grad, smooth, pass_b} (bit 0: TMA
 // staging, bit 1 of smooth: tall tiles); with `ev`
 // (4 events) each launch is bracketed
 cudaError_t launch_sob_iter(const SobIterArgs& a, const int* grids, const int* variants, cudaStream_t s,
-                            cudaEvent_t* ev = nullptr);
+                            bool behind, cudaEvent_t* ev = nullptr);
 
 // Cell for the sobolev solver: clamp to [0, dim-1], floor clamped to dim-2 so that
 // both corners of every axis are inside the grid; in_x, in_y, in_z: the position was not

@@ -150,6 +150,29 @@ def test_convergence_stops_on_device(cuda):
     assert_bitexact(iT.cpu().numpy(), o["out_T"], "T o psi_inv")
 
 
+@pytest.mark.parametrize("max_update_norm", [-1e-10, 0.0])
+def test_an_iteration_run_again_is_recorded_again(cuda, max_update_norm):
+    """fr_step of an iteration that was run before records its own largest update norm, not the
+    larger one of the first run, with and without a convergence test."""
+    dims = (37, 21, 18)
+    st = random_state(dims, 5)
+    d = images(dims, 6)
+    P = _params(dims, max_iter=3, alpha=0.02, max_update_norm=max_update_norm)
+    seen = []
+    for scales in ((1.0,), (8.0, 1.0)):
+        fr = FastReg(P)
+        fr.begin([tuple(_to(cuda, d[k]) for k in ("T", "labT", "S", "labS"))])
+        for s in scales:
+            for which, key in ((N.FR_FIELD_RHO, "rho"), (N.FR_FIELD_PSI, "psi"), (N.FR_FIELD_PSI_INV, "psi_inv")):
+                fr.set_field(which, _to(cuda, st[key]))
+            fr.set_field(N.FR_FIELD_V, _to(cuda, (st["v"] * np.float32(s)).astype(np.float32)))
+            fr.step(1, 0.02)
+        norms, vox = fr.trace()
+        seen.append((norms[0], vox[0]))
+        fr.close()
+    assert seen[0] == seen[1] and seen[0][0] > 0
+
+
 def test_reset_iter_schedule(cuda):
     """RESET_ITER restarts t (solver.cu:428-432)."""
     dims = (16, 14, 12)
