@@ -70,7 +70,8 @@ struct fr_handle {
     int npairs = 0;
     long long NT = 0;
     std::vector<Pair> hpairs;
-    std::vector<Tile> htiles;  // 32 x 8 x 16 tiles of the I/O kernels
+    std::vector<Tile> htiles;  // 32 x 8 x io_depth tiles of finalize_kernel
+    int io_depth = 16;
     TileSet ts[R_COUNT];       // the solver kernels' own tables
     bool tuned = false;        // the shapes of this cohort are settled
     std::vector<fr_pair> io;  // caller buffers of the current registration
@@ -105,8 +106,7 @@ struct fr_handle {
     // sobolev-mode scratch
     float* grad = nullptr;  // unsmoothed gradient (3 planes)
 
-    // launch shape of the I/O kernels
-    int grid_io = 0;
+    int grid_io = 0;  // blocks of finalize_kernel
 
     // graph of all iterations of a registration
     cudaStream_t cap_stream = nullptr;
@@ -213,15 +213,19 @@ int occupancy_grid(fr_handle* h, const void* fn, int ntiles, size_t smem = 0) {
 
 // The staged kernels' error word (set when a bounded wait gave up); the caller has
 // synchronised the work that could set it.
-int check_device_error(fr_handle* h) {
-    if (!h->dev_err) return FR_OK;
-    unsigned int e = 0;
-    FR_CUDA(h, cudaMemcpy(&e, h->dev_err, sizeof e, cudaMemcpyDeviceToHost));
+int report_device_error(fr_handle* h, unsigned int e) {
     if (e & frg::kErrSmemAlign)
         return fail(h, FR_ERR_CUDA, "a TMA staging ring is not on a 128-byte boundary (device error word %u)", e);
     if (e & frg::kErrTmaTimeout)
         return fail(h, FR_ERR_CUDA, "a TMA staging wait gave up after its time limit (device error word %u)", e);
     return FR_OK;
+}
+
+int check_device_error(fr_handle* h) {
+    if (!h->dev_err) return FR_OK;
+    unsigned int e = 0;
+    FR_CUDA(h, cudaMemcpy(&e, h->dev_err, sizeof e, cudaMemcpyDeviceToHost));
+    return report_device_error(h, e);
 }
 
 void release(fr_handle* h) {
@@ -344,6 +348,9 @@ int apply_shapes(fr_handle* h, const Shapes& sh, cudaStream_t s = 0) {
     return FR_OK;
 }
 
+// the records of a registration: stop words .. trace (setup_cohort's order)
+size_t results_bytes(const fr_handle* h) { return (size_t)((const char*)(h->trace + (size_t)h->npairs * h->trace_cap) - (const char*)h->stop); }
+
 // ---- tensor maps of the TMA-staged kernels ----
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -462,12 +469,24 @@ int setup_cohort(fr_handle* h, const fr_pair* pairs, int n) {
         P.off = off;
         P.w_reg = h->P.w_reg;
         off += (long long)align_up((size_t)P.N, 32);
-        for (int z0 = 0; z0 < P.Z; z0 += frg::kTileZ)  // the I/O kernels' table
-            for (int y0 = 0; y0 < P.Y; y0 += frg::kTileY)
-                for (int x0 = 0; x0 < P.X; x0 += frg::kTileX) h->htiles.push_back(make_int4(p, x0, y0, z0));
     }
     h->NT = std::max(off, 32LL);
     const long long NT = h->NT;
+    // finalize_kernel's table: tiles as deep as leaves four for every SM, up to 16 slices
+    auto columns = [](const Pair& P) {
+        return (long long)((P.X + frg::kTileX - 1) / frg::kTileX) * ((P.Y + frg::kTileY - 1) / frg::kTileY);
+    };
+    for (h->io_depth = 16; h->io_depth > 2; h->io_depth /= 2) {
+        long long tiles = 0;
+        for (const Pair& P : h->hpairs) tiles += columns(P) * ((P.Z + h->io_depth - 1) / h->io_depth);
+        if (tiles >= 4LL * h->num_sms) break;
+    }
+    for (int p = 0; p < n; ++p) {
+        const Pair& P = h->hpairs[p];
+        for (int z0 = 0; z0 < P.Z; z0 += h->io_depth)
+            for (int y0 = 0; y0 < P.Y; y0 += frg::kTileY)
+                for (int x0 = 0; x0 < P.X; x0 += frg::kTileX) h->htiles.push_back(make_int4(p, x0, y0, z0));
+    }
     const int ntiles = (int)h->htiles.size();
     h->trace_cap = want_trace;
 
@@ -509,18 +528,20 @@ int setup_cohort(fr_handle* h, const fr_pair* pairs, int n) {
         h->LT = nullptr;
         add((void**)&h->grad, sizeof(float) * 3 * NT);
     }
+    // what begins a registration as zeros and is read back after it, side by side: one clearing,
+    // one copy to the host
     add((void**)&h->stop, sizeof(int) * n);
+    add((void**)&h->dev_err, sizeof(unsigned int));
     add((void**)&h->keys, sizeof(unsigned long long) * n);
+    add((void**)&h->dice, sizeof(unsigned long long) * (size_t)n * (2 * 256 + 1));
+    add((void**)&h->pair_energy, sizeof(double) * 2 * n);
+    add((void**)&h->pair_folds, sizeof(long long) * n);
     add((void**)&h->trace, sizeof(unsigned long long) * (size_t)n * want_trace);
     add((void**)&h->counter, sizeof(unsigned int) * 4);
-    add((void**)&h->dev_err, sizeof(unsigned int));
     add((void**)&h->tmaps, sizeof(CUtensorMap) * (size_t)n * frg::TM_COUNT);
     add((void**)&h->tile_partials, sizeof(double) * 2 * ntiles);
     add((void**)&h->pair_tiles, sizeof(int) * (n + 1));
     add((void**)&h->tile_folds, sizeof(long long) * ntiles);
-    add((void**)&h->dice, sizeof(unsigned long long) * (size_t)n * (2 * 256 + 1));
-    add((void**)&h->pair_energy, sizeof(double) * 2 * n);
-    add((void**)&h->pair_folds, sizeof(long long) * n);
     size_t total = 0;
     for (auto& s : slots) total = align_up(total, 256) + s.bytes;
     total = align_up(total, 256);
@@ -710,6 +731,7 @@ frg::IoArgs io_args(fr_handle* h) {
     a.pairs = h->d_pairs;
     a.tiles = h->d_tiles;
     a.ntiles = (int)h->htiles.size();
+    a.io_depth = h->io_depth;
     a.npairs = h->npairs;
     a.NT = h->NT;
     a.io = h->d_io;
@@ -740,6 +762,14 @@ frg::IoArgs io_args(fr_handle* h) {
     a.counter = h->counter + 1;
     a.write_outputs = 1;
     return a;
+}
+
+// blocks of pack_init_kernel: per pair, enough for the largest, at most a few per SM in all
+dim3 pack_grid(const fr_handle* h) {
+    long long most = 1;
+    for (const Pair& P : h->hpairs) most = std::max(most, (P.N / 4 + 255) / 256);
+    const long long cap = std::max(8LL * h->num_sms / h->npairs, 16LL);
+    return dim3((unsigned)std::min(most, cap), (unsigned)std::min(h->npairs, 65535));
 }
 
 // Move each pair's final state into buffer 0 so that a KEEP_STATE call starts from it.
@@ -918,7 +948,7 @@ int autotune(fr_handle* h, cudaStream_t s) {
     FR_CUDA(h, cudaMemsetAsync(h->stop, 0, sizeof(int) * h->npairs, s));
     frg::IoArgs io = io_args(h);
     io.keep_state = 0;
-    frg::pack_init_kernel<<<h->grid_io, 256, 0, s>>>(io);
+    frg::pack_init_kernel<<<pack_grid(h), 256, 0, s>>>(io);
     FR_LAUNCHED(h);
     const std::vector<float> ts = t_schedule(h->P);
     const int warm = std::min(kTuneWarmIters, (h->trace_cap - 1) / 2 * 2);  // the trace holds iteration warm + 1
@@ -1038,12 +1068,9 @@ int begin(fr_handle* h, const fr_pair* pairs, int n, cudaStream_t s) {
         rc = autotune(h, s);  // leaves the state to the initialisation below
         if (rc != FR_OK) return rc;
     }
-    FR_CUDA(h, cudaMemsetAsync(h->stop, 0, sizeof(int) * n, s));
-    FR_CUDA(h, cudaMemsetAsync(h->dev_err, 0, sizeof(unsigned int), s));
-    FR_CUDA(h, cudaMemsetAsync(h->keys, 0, sizeof(unsigned long long) * n, s));
-    FR_CUDA(h, cudaMemsetAsync(h->trace, 0, sizeof(unsigned long long) * n * (size_t)h->trace_cap, s));
+    FR_CUDA(h, cudaMemsetAsync(h->stop, 0, results_bytes(h), s));
     frg::IoArgs a = io_args(h);
-    frg::pack_init_kernel<<<h->grid_io, 256, 0, s>>>(a);
+    frg::pack_init_kernel<<<pack_grid(h), 256, 0, s>>>(a);
     FR_LAUNCHED(h);
     h->have_state = true;
     h->finished = false;
@@ -1067,20 +1094,18 @@ int host_stats(fr_handle* h) {
     if (h->stats_ready) return FR_OK;
     const int n = h->npairs;
     FR_CUDA(h, cudaStreamSynchronize(h->last_stream));
-    std::vector<int> stop(n);
-    std::vector<double> energy(2 * n);
-    std::vector<long long> folds(n);
-    std::vector<unsigned long long> dice((size_t)n * (2 * 256 + 1));
-    std::vector<unsigned long long> trace((size_t)n * h->trace_cap);
+    std::vector<unsigned long long> records(results_bytes(h) / sizeof(unsigned long long));
+    FR_CUDA(h, cudaMemcpy(records.data(), h->stop, results_bytes(h), cudaMemcpyDeviceToHost));
+    auto at = [&](const void* d) { return (const char*)records.data() + ((const char*)d - (const char*)h->stop); };
+    const int* stop = (const int*)at(h->stop);
+    const double* energy = (const double*)at(h->pair_energy);
+    const long long* folds = (const long long*)at(h->pair_folds);
+    const unsigned long long *dice = (const unsigned long long*)at(h->dice),
+                             *trace = (const unsigned long long*)at(h->trace);
     {
-        int rc = check_device_error(h);
+        int rc = report_device_error(h, *(const unsigned int*)at(h->dev_err));
         if (rc != FR_OK) return rc;
     }
-    FR_CUDA(h, cudaMemcpy(stop.data(), h->stop, sizeof(int) * n, cudaMemcpyDeviceToHost));
-    FR_CUDA(h, cudaMemcpy(energy.data(), h->pair_energy, sizeof(double) * 2 * n, cudaMemcpyDeviceToHost));
-    FR_CUDA(h, cudaMemcpy(folds.data(), h->pair_folds, sizeof(long long) * n, cudaMemcpyDeviceToHost));
-    FR_CUDA(h, cudaMemcpy(dice.data(), h->dice, sizeof(unsigned long long) * dice.size(), cudaMemcpyDeviceToHost));
-    FR_CUDA(h, cudaMemcpy(trace.data(), h->trace, sizeof(unsigned long long) * trace.size(), cudaMemcpyDeviceToHost));
     h->stats.assign(n, fr_stats{});
     for (int p = 0; p < n; ++p) {
         fr_stats& st = h->stats[p];
@@ -1096,7 +1121,7 @@ int host_stats(fr_handle* h) {
         st.energy = st.e_data + (double)h->hpairs[p].w_reg * st.e_reg;
         st.folds = folds[p];
         st.no_labels = h->P.no_labels;
-        const unsigned long long* dp = dice.data() + (size_t)p * (2 * 256 + 1);
+        const unsigned long long* dp = dice + (size_t)p * (2 * 256 + 1);
         double num = 0.0, den = 0.0;
         for (int l = 0; l < FR_MAX_LABELS; ++l) {
             st.dice_inter[l] = (int64_t)dp[l];

@@ -50,7 +50,6 @@ typedef int4 Tile;
 
 constexpr int kTileX = 32;  // threads along x (one warp per row)
 constexpr int kTileY = 8;   // rows per block
-constexpr int kTileZ = 16;  // slices marched by each thread
 // The solver kernels walk their own tile tables of 32 x 8 x depth tiles; the depth of
 // each table and the kernel's blocks per SM are chosen on the host (fr_api.cu: defaults,
 // or the autotuner's choice for the cohort's size class).

@@ -17,51 +17,66 @@
 
 namespace frg {
 
+// Four voxels of a padded row per thread (rows start on 16-byte boundaries), pairs along blockIdx.y:
+// 16-byte stores, and no loads but the caller's (and the kept state's) once each.  Pad columns
+// are written as zeros.  108 bytes per voxel in the reference solver, 116 us at the copy
+// bandwidth on 182x218x182; one voxel per thread on columns of 16 slices, two blocks per SM,
+// took 277 us there and 35 us on the 64^3 pair's 64 tiles.
 __global__ void __launch_bounds__(256) pack_init_kernel(IoArgs a) {
-    for (int t = blockIdx.x; t < a.ntiles; t += gridDim.x) {
-        const Tile tl = a.tiles[t];
-        const Pair P = a.pairs[tl.x];
-        const PairIO io = a.io[tl.x];
-        const int x = tl.y + (int)(threadIdx.x & 31), y = tl.z + (int)(threadIdx.x >> 5);
-        if (x >= P.X || y >= P.Y) continue;
+    for (int p = blockIdx.y; p < a.npairs; p += gridDim.y) {
+        const Pair P = a.pairs[p];
+        const PairIO io = a.io[p];
         const long long NT = a.NT;
-        const int z1 = min(tl.w + kTileZ, P.Z);
-        for (int z = tl.w; z < z1; ++z) {
-            const long long u = user_lin(P, x, y, z);  // caller's layout
-            const long long g = P.off + lin(P, x, y, z);
-            a.S[g] = io.img_S[u];
-            a.T[g] = io.img_T[u];
-            a.labS[g] = io.lab_S[u];
-            a.labT[g] = io.lab_T[u];
-            if (a.sobolev) {
-                if (!a.keep_state) {
-                    const float pos[3] = {(float)x, (float)y, (float)z};
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        a.v0[c * NT + g] = 0.f;
-                        a.psi[c * NT + g] = pos[c];
-                    }
-                }
-                continue;
+        const int groups = (int)(P.N / 4), row4 = P.Xp / 4;
+        auto put = [&](float* f, int g, const float v[4]) {
+            *reinterpret_cast<float4*>(f + P.off + 4LL * g) = make_float4(v[0], v[1], v[2], v[3]);
+        };
+        for (int g = blockIdx.x * 256 + threadIdx.x; g < groups; g += gridDim.x * 256) {
+            const int row = g / row4, x0 = 4 * (g - row * row4), z = row / P.Y, y = row - z * P.Y;
+            const long long u = x0 + (long long)P.X * row;  // caller's layout
+            float S[4], T[4], zero[4], rho[4], pos[3][4];
+            short4 lS, lT;
+            int16_t* const ls[4] = {&lS.x, &lS.y, &lS.z, &lS.w};
+            int16_t* const lt[4] = {&lT.x, &lT.y, &lT.z, &lT.w};
+    #pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const bool in = x0 + k < P.X;
+                S[k] = in ? io.img_S[u + k] : 0.f;
+                T[k] = in ? io.img_T[u + k] : 0.f;
+                *ls[k] = in ? io.lab_S[u + k] : (int16_t)0;
+                *lt[k] = in ? io.lab_T[u + k] : (int16_t)0;
+                zero[k] = 0.f;
+                rho[k] = in ? a.rho_init : 0.f;
+                pos[0][k] = in ? (float)(x0 + k) : 0.f;
+                pos[1][k] = in ? (float)y : 0.f;
+                pos[2][k] = in ? (float)z : 0.f;
             }
-            a.rho0[g] = a.rho_init;
-            a.rho1[g] = a.rho_init;
-            a.LT[g] = make_float4(0.f, 0.f, 0.f, io.img_T[u]);  // the Laplacian is 0 on the boundary
-            if (!a.keep_state) {
-                const float pos[3] = {(float)x, (float)y, (float)z};
-#pragma unroll
+            put(a.S, g, S);
+            put(a.T, g, T);
+            *reinterpret_cast<short4*>(a.labS + P.off + 4LL * g) = lS;
+            *reinterpret_cast<short4*>(a.labT + P.off + 4LL * g) = lT;
+            if (!a.keep_state)
+    #pragma unroll
                 for (int c = 0; c < 3; ++c) {
-                    a.v0[c * NT + g] = 0.f;
-                    a.v1[c * NT + g] = 0.f;
-                    a.psi[c * NT + g] = pos[c];
-                    a.pinv0[c * NT + g] = pos[c];
-                    a.pinv1[c * NT + g] = pos[c];
+                    put(a.v0 + c * NT, g, zero);
+                    put(a.psi + c * NT, g, pos[c]);
                 }
-            } else {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    a.v1[c * NT + g] = a.v0[c * NT + g];
-                    a.pinv1[c * NT + g] = a.pinv0[c * NT + g];
+            if (a.sobolev) continue;
+            put(a.rho0, g, rho);
+            put(a.rho1, g, rho);
+    #pragma unroll
+            for (int k = 0; k < 4; ++k)  // the Laplacian is 0 on the boundary
+                a.LT[P.off + 4LL * g + k] = make_float4(0.f, 0.f, 0.f, T[k]);
+    #pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                if (!a.keep_state) {
+                    put(a.v1 + c * NT, g, zero);
+                    put(a.pinv0 + c * NT, g, pos[c]);
+                    put(a.pinv1 + c * NT, g, pos[c]);
+                } else {
+                    const long long at = c * NT + P.off + 4LL * g;
+                    *reinterpret_cast<float4*>(a.v1 + at) = *reinterpret_cast<const float4*>(a.v0 + at);
+                    *reinterpret_cast<float4*>(a.pinv1 + at) = *reinterpret_cast<const float4*>(a.pinv0 + at);
                 }
             }
         }
@@ -89,7 +104,12 @@ __device__ __forceinline__ float det_true(const float J[3][3]) {
     return (f00 * c0 - f01 * c1) + f02 * c2;
 }
 
-__global__ void __launch_bounds__(256) finalize_kernel(IoArgs a) {
+// A thread marches a column of a 32 x 8 x io_depth tile, psi of the slice below, this one and the one
+// above in registers.  It waits on its loads and gathers, so it is held to five blocks per SM (48
+// registers): 197 us on the 182x218x182 pair with the reference solver, 237 us with four; 326 us
+// with 64-bit indices, every neighbour loaded and two blocks of 128 registers.  On the 64^3 pair
+// 21 us with tiles of two slices, 51 us with 16 (64 blocks).
+__global__ void __launch_bounds__(256, 5) finalize_kernel(IoArgs a) {
     __shared__ double red[32];
     __shared__ unsigned int hist[2 * 256 + 1];
     __shared__ bool last;
@@ -105,35 +125,45 @@ __global__ void __launch_bounds__(256) finalize_kernel(IoArgs a) {
         __syncthreads();
         const int x = tl.y + (int)(threadIdx.x & 31), y = tl.z + (int)(threadIdx.x >> 5);
         double ed = 0.0, er = 0.0;
-        long long folds = 0;
+        int folds = 0;
         if (x < P.X && y < P.Y) {
             const long long NT = a.NT;
+            const int X = P.X, Y = P.Y, Z = P.Z, Xp = P.Xp, XY = P.Xp * P.Y, N = (int)P.N;
             const float* __restrict__ S = a.S + P.off;
             const float* __restrict__ T = a.T + P.off;
             const int16_t* __restrict__ labS = a.labS + P.off;
             const int16_t* __restrict__ labT = a.labT + P.off;
-            const float* __restrict__ psi = a.psi + P.off;
+            const float* __restrict__ psi[3] = {a.psi + P.off, a.psi + NT + P.off, a.psi + 2 * NT + P.off};
             const float* __restrict__ pi = pinv + P.off;
-            const int z1 = min(tl.w + kTileZ, P.Z);
-            for (int z = tl.w; z < z1; ++z) {
-                const long long i = lin(P, x, y, z);
+            const int z1 = min(tl.w + a.io_depth, Z);
+            int i = x + Xp * (y + Y * tl.w);
+            // deformation Jacobian with the mirrored one-sided boundary: the neighbours on either side
+            const int x1 = x == X - 1 ? x - 1 : x + 1, x2 = x == 0 ? x + 1 : x - 1;
+            const int y1 = y == Y - 1 ? y - 1 : y + 1, y2 = y == 0 ? y + 1 : y - 1;
+            const int ox1 = x1 - x, ox2 = x2 - x, oy1 = Xp * (y1 - y), oy2 = Xp * (y2 - y);
+            float pm[3], pc[3], pn[3];  // psi at z - 1, z, z + 1
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                pc[r] = __ldg(psi[r] + i);
+                pm[r] = tl.w > 0 ? __ldg(psi[r] + i - XY) : 0.f;
+            }
+            for (int z = tl.w; z < z1; ++z, i += XY) {
+#pragma unroll
+                for (int r = 0; r < 3; ++r) pn[r] = z + 1 < Z ? __ldg(psi[r] + i + XY) : 0.f;
                 // S o psi
-                const Cell cs = locate(P, __ldg(psi + i), __ldg(psi + NT + i), __ldg(psi + 2 * NT + i));
-                const float ws = tri_unchecked(S, P, cs);
+                const Cell32 cs = locate32(X, Y, Z, Xp, pc[0], pc[1], pc[2]);
+                const float ws = tri_unchecked32(S, Xp, XY, N, cs);
                 // floor-corner label (reference, cuda_utils.hpp:81) or the nearest
                 // voxel (sobolev solver)
-                const int16_t wl = a.sobolev ? __ldg(labS + nearest_index(P, __ldg(psi + i), __ldg(psi + NT + i),
-                                                                          __ldg(psi + 2 * NT + i)))
-                                             : __ldg(labS + cs.base);
+                const int16_t wl = a.sobolev ? __ldg(labS + nearest_index(P, pc[0], pc[1], pc[2])) : __ldg(labS + cs.base);
                 // T o psi_inv
-                float wt;
-                int16_t wtl;
-                if (done == 0 || a.sobolev) {
-                    wt = __ldg(T + i);
-                    wtl = __ldg(labT + i);
-                } else {
-                    const Cell ct = locate(P, __ldg(pi + i), __ldg(pi + NT + i), __ldg(pi + 2 * NT + i));
-                    wt = tri_unchecked(T, P, ct);
+                const float tv = __ldg(T + i);
+                const int16_t lb = __ldg(labT + i);
+                float wt = tv;
+                int16_t wtl = lb;
+                if (!(done == 0 || a.sobolev)) {
+                    const Cell32 ct = locate32(X, Y, Z, Xp, __ldg(pi + i), __ldg(pi + NT + i), __ldg(pi + 2 * NT + i));
+                    wt = tri_unchecked32(T, Xp, XY, N, ct);
                     wtl = __ldg(labT + ct.base);
                 }
                 if (a.write_outputs) {
@@ -145,27 +175,23 @@ __global__ void __launch_bounds__(256) finalize_kernel(IoArgs a) {
                 }
 
                 // data energy
-                const float df = __ldg(T + i) - ws;
+                const float df = tv - ws;
                 ed = fma((double)df, (double)df, ed);  // df * df is exact in FP64: same bits
 
-                // deformation Jacobian with the mirrored one-sided boundary
-                int x1 = x + 1, x2 = x - 1, y1 = y + 1, y2 = y - 1, z1_ = z + 1, z2_ = z - 1;
-                if (x == 0) x2 = x + 1; else if (x == P.X - 1) x1 = x - 1;
-                if (y == 0) y2 = y + 1; else if (y == P.Y - 1) y1 = y - 1;
-                if (z == 0) z2_ = z + 1; else if (z == P.Z - 1) z1_ = z - 1;
-                const long long ix1 = lin(P, x1, y, z), ix2 = lin(P, x2, y, z);
-                const long long iy1 = lin(P, x, y1, z), iy2 = lin(P, x, y2, z);
-                const long long iz1 = lin(P, x, y, z1_), iz2 = lin(P, x, y, z2_);
+                const int z1_ = z == Z - 1 ? z - 1 : z + 1, z2_ = z == 0 ? z + 1 : z - 1;
                 const float cx1[3] = {(float)x1, (float)y, (float)z}, cx2[3] = {(float)x2, (float)y, (float)z};
                 const float cy1[3] = {(float)x, (float)y1, (float)z}, cy2[3] = {(float)x, (float)y2, (float)z};
                 const float cz1[3] = {(float)x, (float)y, (float)z1_}, cz2[3] = {(float)x, (float)y, (float)z2_};
                 float J[3][3];
 #pragma unroll
                 for (int r = 0; r < 3; ++r) {
-                    const float* __restrict__ Q = psi + r * NT;
-                    J[r][0] = ((__ldg(Q + ix1) - cx1[r]) - (__ldg(Q + ix2) - cx2[r])) * 0.5f;
-                    J[r][1] = ((__ldg(Q + iy1) - cy1[r]) - (__ldg(Q + iy2) - cy2[r])) * 0.5f;
-                    J[r][2] = ((__ldg(Q + iz1) - cz1[r]) - (__ldg(Q + iz2) - cz2[r])) * 0.5f;
+                    const float* __restrict__ Q = psi[r] + i;
+                    const float zu = z == Z - 1 ? pm[r] : pn[r], zd = z == 0 ? pn[r] : pm[r];
+                    J[r][0] = ((__ldg(Q + ox1) - cx1[r]) - (__ldg(Q + ox2) - cx2[r])) * 0.5f;
+                    J[r][1] = ((__ldg(Q + oy1) - cy1[r]) - (__ldg(Q + oy2) - cy2[r])) * 0.5f;
+                    J[r][2] = ((zu - cz1[r]) - (zd - cz2[r])) * 0.5f;
+                    pm[r] = pc[r];
+                    pc[r] = pn[r];
                 }
                 const float r0 = (J[0][0] * J[0][0] + J[0][1] * J[0][1]) + J[0][2] * J[0][2];
                 const float r1 = (J[1][0] * J[1][0] + J[1][1] * J[1][1]) + J[1][2] * J[1][2];
@@ -174,8 +200,8 @@ __global__ void __launch_bounds__(256) finalize_kernel(IoArgs a) {
                 if (det_true(J) <= 0.f) folds++;
 
                 // Dice counts on [0, X-1) x [0, Y-1) x [0, Z-1)
-                if (x < P.X - 1 && y < P.Y - 1 && z < P.Z - 1) {
-                    const int la = wl, lb = __ldg(labT + i);
+                if (x < X - 1 && y < Y - 1 && z < Z - 1) {
+                    const int la = wl;
                     const bool ok = la >= 0 && la < a.no_labels && lb >= 0 && lb < a.no_labels;
                     if (!ok) {
                         atomicAdd(&hist[2 * 256], 1u);
@@ -190,7 +216,7 @@ __global__ void __launch_bounds__(256) finalize_kernel(IoArgs a) {
         // per-tile partials (summed per pair in tile order by the last block)
         ed = block_sum_f64(ed, red);
         er = block_sum_f64(er, red);
-        double fd = block_sum_f64((double)folds, red);
+        const double fd = block_sum_f64((double)folds, red);
         if (tid == 0) {
             a.tile_partials[2 * (long long)t] = ed;
             a.tile_partials[2 * (long long)t + 1] = er;

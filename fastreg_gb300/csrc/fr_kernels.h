@@ -93,8 +93,8 @@ struct PairIO {
 // Arguments of the start-of-registration and end-of-registration kernels.
 struct IoArgs {
     const Pair* pairs;
-    const Tile* tiles;
-    int ntiles;
+    const Tile* tiles;  // 32 x 8 x io_depth tiles (finalize_kernel)
+    int ntiles, io_depth;
     int npairs;
     long long NT;
     const PairIO* io;
