@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(256) adj_pack_kernel(AdjPair A, const float* _
 
 // The result: the adjoint of v0 out of the interleaved accumulator.
 __global__ void __launch_bounds__(256) adj_unpack_kernel(AdjPair A, const float4* __restrict__ mbar, float* out) {
+    pdl_wait();
     const long long nu = (long long)A.X * A.Y * A.Z;
     GRID_STRIDE(i, A.N) {
         const int row = i / A.Xp, x = i - row * A.Xp;
@@ -122,6 +123,7 @@ __device__ __forceinline__ Pair as_pair(const AdjPair& A) {
 __global__ void __launch_bounds__(256) adj_loss_kernel(AdjPair A, const float* __restrict__ S, const float* __restrict__ T,
                                                        const float* __restrict__ phi, const float* __restrict__ m,
                                                        float* pbar, float4* mbar, double* loss) {
+    pdl_wait();
     __shared__ double red[32];
     const Pair P = as_pair(A);
     double er = 0.0, em = 0.0;
@@ -190,6 +192,7 @@ __device__ __forceinline__ void scatter_face_warp(float4* F, int b, const float3
 // 128^3 pair 40 us; with one 4-byte reduction per corner and component, lanes merged, 144 us.
 __global__ void __launch_bounds__(256) adj_update_kernel(AdjPair A, const float* __restrict__ phi,
                                                          const float* __restrict__ mn, float* pbar, float4* mbar) {
+    pdl_wait();
     const Pair P = as_pair(A);
     const int nx = (A.X + kTileX - 1) / kTileX, ny = (A.Y + kTileY - 1) / kTileY;
     const int x = (blockIdx.x % nx) * kTileX + (threadIdx.x & 31), y = (blockIdx.x / nx % ny) * kTileY + (threadIdx.x >> 5);
@@ -272,6 +275,7 @@ __global__ void __launch_bounds__(256) adj_update_kernel(AdjPair A, const float*
 
 // m' = damping * m - step * gs: gs = -step * mbar (planes), mbar = damping * mbar; zero pad columns stay zero
 __global__ void __launch_bounds__(256) adj_momentum_kernel(AdjPair A, float damping, float step, float4* mbar, float* gs) {
+    pdl_wait();
     GRID_STRIDE(i, A.N) {
         const float4 v = mbar[i];
         gs[i] = -step * v.x;
@@ -301,6 +305,7 @@ __device__ __forceinline__ void dot2(float a, float b, float& s, float& c) {
 __global__ void __launch_bounds__(256) adj_grad_kernel(AdjPair A, const float* __restrict__ S, const float* __restrict__ T,
                                                        const float* __restrict__ phi, float lambda,
                                                        const float* __restrict__ gbar, float* pbar, double* lbar) {
+    pdl_wait();
     __shared__ double red[32];
     const Pair P = as_pair(A);
     const int nx = (A.X + kTileX - 1) / kTileX, ny = (A.Y + kTileY - 1) / kTileY;
@@ -584,9 +589,8 @@ extern "C" int fr_sobolev_loss_grad(const float* d_T, const float* d_S, const in
         if (e != cudaSuccess) rc = FR_ERR_CUDA;
         return rc == FR_OK;
     };
-    // iteration k (0-based) from one state to another; a segment's last phi is needed only
-    // where the next segment or the loss starts from it
-    auto forward = [&](int k, const State& from, const State& to, bool update) {
+    // iteration k (0-based) from one state to another
+    auto forward = [&](int k, const State& from, const State& to) {
         a.iter = k + 1;
         a.phi = from.phi;
         a.m = from.m;
@@ -596,7 +600,14 @@ extern "C" int fr_sobolev_loss_grad(const float* d_T, const float* d_S, const in
         a.depth_s = cuts[1].depth;
         ok(launch_sob_kernel(0, a, cuts[0].count, 0, s, true));
         ok(launch_sob_kernel(1, a, cuts[1].count, kUnrolled | (tall ? 2 : 0), s, true));
-        if (update) ok(launch_sob_kernel(2, a, cuts[2].count, kUnrolled, s, true));
+        ok(launch_sob_kernel(2, a, cuts[2].count, kUnrolled, s, true));
+    };
+    // the reverse kernels' blocks are placed while the kernel ahead drains, as the forward ones' are: short
+    // kernels gain most (45x54x45, 20 iterations: 1.93 -> 1.69 ms; 128^3, 50 iterations: 13.3 -> 12.7 ms, of
+    // which 0.25 ms is a segment's last state taken from the checkpoint)
+    auto reverse = [&](const void* fn, int blocks, auto... v) {
+        void* args[] = {&v...};
+        ok(launch_kernel(fn, blocks, 256, 0, args, s, true));
     };
     auto smooth_adjoint = [&]() {  // gbar = G^T g
         SobIterArgs t = a;
@@ -616,30 +627,32 @@ extern "C" int fr_sobolev_loss_grad(const float* d_T, const float* d_S, const in
             const int j = k % ck;
             const bool last_segment = k / ck == nseg - 1;
             const State to = last_segment ? seg[j] : j == ck - 1 ? ckpt[k / ck + 1] : work[k & 1];
-            forward(k, st, to, true);
+            forward(k, st, to);
             st = to;
         }
-        adj_loss_kernel<<<grid, 256, 0, s>>>(A, Sp, Tp, st.phi, st.m, pbar, mbar, dd);
+        reverse((const void*)adj_loss_kernel, grid, A, Sp, Tp, st.phi, st.m, pbar, mbar, dd);
         if (!d_grad_v0) break;
         // reverse, one segment at a time
         for (int q = nseg - 1; q >= 0 && rc == FR_OK; --q) {
             const int s0 = q * ck, s1 = std::min(s0 + ck, K);
             if (q < nseg - 1) {
                 st = ckpt[q];
-                for (int k = s0; k < s1; ++k) {
-                    forward(k, st, seg[k - s0], k + 1 < s1);
+                for (int k = s0; k < s1 - 1; ++k) {
+                    forward(k, st, seg[k - s0]);
                     st = seg[k - s0];
                 }
             }
             for (int k = s1 - 1; k >= s0; --k) {
                 const float* phik = k == s0 ? ckpt[q].phi : seg[k - s0 - 1].phi;
-                adj_update_kernel<<<columns, 256, 0, s>>>(A, phik, seg[k - s0].m, pbar, mbar);
-                adj_momentum_kernel<<<grid, 256, 0, s>>>(A, damping, step, mbar, g);
+                // a segment's last state is the next one's checkpoint
+                const float* mn = k == s1 - 1 && q < nseg - 1 ? ckpt[q + 1].m : seg[k - s0].m;
+                reverse((const void*)adj_update_kernel, columns, A, phik, mn, pbar, mbar);
+                reverse((const void*)adj_momentum_kernel, grid, A, damping, step, mbar, g);
                 smooth_adjoint();
-                adj_grad_kernel<<<columns, 256, 0, s>>>(A, Sp, Tp, phik, lambda, gbar, pbar, dd + 1);
+                reverse((const void*)adj_grad_kernel, columns, A, Sp, Tp, phik, lambda, gbar, pbar, dd + 1);
             }
         }
-        adj_unpack_kernel<<<grid, 256, 0, s>>>(A, mbar, d_grad_v0);
+        reverse((const void*)adj_unpack_kernel, grid, A, mbar, d_grad_v0);
     } while (0);
     double host[2] = {0.0, 0.0};
     if (rc == FR_OK) {
