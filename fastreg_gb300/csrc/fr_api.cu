@@ -50,7 +50,7 @@ struct TileSet {
     int occ[4] = {1, 1, 1, 1};  // resident blocks per SM of each variant at its registers and shared memory
     int grid = 0;
 };
-// defaults (AUTOTUNE=0), the autotuner's usual choice on the 182x218x182 pair: slices per
+// defaults (AUTOTUNE=0), near the autotuner's choices on the 182x218x182 pair: slices per
 // tile, and whether each tile is its own block (scheduled by the hardware) instead of a
 // persistent grid at the occupancy limit
 static const int kDefaultDepth[R_COUNT] = {16, 24, 24, 12, 32, 8};
