@@ -523,8 +523,15 @@ extern "C" int fr_sobolev_loss_grad(const float* d_T, const float* d_S, const in
     cuts[2] = cut(4, kTileY, 1, 6, &cost);
     const Cut low = cut(3, sob_smooth_tile_y(R, false), 2 * R + 1, 128, &cost);
     const Cut high = cut(3, sob_smooth_tile_y(R, true), 2 * R + 1, 128, &cost_tall);
-    const bool tall = cost_tall < cost;
-    cuts[1] = cuts[3] = tall ? high : low;
+    const long long columns8 = (long long)((A.X + kTileX - 1) / kTileX) * ((A.Y + kTileY - 1) / kTileY);
+    // smoothing in two launches where it is the faster (sob_smooth_z_kernel)
+    const bool split = sob_smooth_split(R, A.N, true);
+    auto slices = [&](bool tall) {  // tiles of one slice each
+        const int rows = sob_smooth_tile_y(R, tall);
+        return Cut{rows, 1, (A.X + kTileX - 1) / kTileX * ((A.Y + rows - 1) / rows) * A.Z};
+    };
+    const bool tall = split ? slices(true).count >= 2 * sms : cost_tall < cost;
+    cuts[1] = cuts[3] = split ? slices(tall) : tall ? high : low;
     A.depth = cuts[2].depth;
 
     // the workspace: checkpoints (phi, m) x nseg, the states of a segment (phi, m) x ck, two
@@ -570,6 +577,8 @@ extern "C" int fr_sobolev_loss_grad(const float* d_T, const float* d_S, const in
     a.pair0.w_reg = lambda;
     a.ntiles_g = cuts[0].count;
     a.depth_g = cuts[0].depth;
+    a.depth_z = sob_smooth_z_depth(columns8, A.Z, sms);
+    a.ntiles_z = (int)(columns8 * ((A.Z + a.depth_z - 1) / a.depth_z));
     a.ntiles_b = cuts[2].count;
     a.depth_b = cuts[2].depth;
     a.npairs = 1;
@@ -599,7 +608,8 @@ extern "C" int fr_sobolev_loss_grad(const float* d_T, const float* d_S, const in
         a.ntiles_s = cuts[1].count;
         a.depth_s = cuts[1].depth;
         ok(launch_sob_kernel(0, a, cuts[0].count, 0, s, true));
-        ok(launch_sob_kernel(1, a, cuts[1].count, kUnrolled | (tall ? 2 : 0), s, true));
+        a.mid = gbar;  // free until the reverse iteration's smoothing
+        ok(launch_sob_kernel(1, a, cuts[1].count, kUnrolled | (tall ? 2 : 0) | (split ? kSplit : 0), s, true));
         ok(launch_sob_kernel(2, a, cuts[2].count, kUnrolled, s, true));
     };
     // the reverse kernels' blocks are placed while the kernel ahead drains, as the forward ones' are: short
@@ -614,6 +624,11 @@ extern "C" int fr_sobolev_loss_grad(const float* d_T, const float* d_S, const in
         t.m_n = gbar;
         t.ntiles_s = cuts[3].count;
         t.depth_s = cuts[3].depth;
+        t.mid = work[0].phi;  // the forward sweep is done with it
+        if (split) {
+            ok(launch_smooth_split(t, kSmoothTransposed, tall, cuts[3].count, s, true));
+            return;
+        }
         void* args[1] = {&t};
         ok(launch_kernel(sob_smooth3_unrolled_fn(R, true, tall), cuts[3].count, kSmoothThreads, 0, args, s, true));
     };

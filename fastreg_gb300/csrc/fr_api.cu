@@ -47,7 +47,7 @@ struct TileSet {
     std::vector<Tile> h;
     Tile* d = nullptr;  // device copy (capacity cap tiles)
     size_t cap = 0;
-    int occ[4] = {1, 1, 1, 1};  // resident blocks per SM of each variant at its registers and shared memory
+    int occ[frg::kSplit + 4] = {};  // resident blocks per SM of each variant at its registers and shared memory
     int grid = 0;
 };
 // defaults (AUTOTUNE=0), near the autotuner's choices on the 182x218x182 pair: slices per
@@ -72,6 +72,8 @@ struct fr_handle {
     std::vector<Pair> hpairs;
     std::vector<Tile> htiles;  // 32 x 8 x io_depth tiles of finalize_kernel
     int io_depth = 16;
+    std::vector<Tile> planes;  // tiles of the smoothing's plane filter, where it is a launch of its own
+    int planes_rows = 0;       // their rows (0: not made for this cohort)
     TileSet ts[R_COUNT];       // the solver kernels' own tables
     bool tuned = false;        // the shapes of this cohort are settled
     std::vector<fr_pair> io;  // caller buffers of the current registration
@@ -82,6 +84,7 @@ struct fr_handle {
     size_t block_bytes = 0;
     Pair* d_pairs = nullptr;
     Tile* d_tiles = nullptr;
+    Tile* d_planes = nullptr;
     frg::PairIO* d_io = nullptr;
     float *S = nullptr, *T = nullptr;
     int16_t *labS = nullptr, *labT = nullptr;
@@ -258,6 +261,11 @@ std::vector<int> allowed_variants(const fr_handle* h, int r) {
         al = {1};
     if (r == R_SS && frg::sob_smooth_has_tall(h->P.smooth_width / 2))
         for (size_t k = 0, n = al.size(); k < n; ++k) al.push_back(al[k] | 2);
+    // in two launches, staged by cp.async: by rule, as timed alone it looks faster on volumes whose fields
+    // only just fit L2 than it is between the other kernels (128^3 at radius 3: 14.8 against 13.2 ms)
+    if (r == R_SS && al[0] == 0 && frg::sob_smooth_split(h->P.smooth_width / 2, h->NT, false))
+        for (size_t k = 0, n = al.size(); k < n; ++k)
+            if (!(al[k] & 1)) al.push_back(al[k] | frg::kSplit);
     return al;
 }
 
@@ -267,7 +275,13 @@ const void* role_fn(const fr_handle* h, int r, int variant = 0) {
         case R_PA: return variant ? (const void*)frg::ref_pass_a_tma_kernel : (const void*)frg::ref_pass_a_kernel;
         case R_PB: return (const void*)frg::ref_pass_b_kernel;
         case R_SG: return frg::sob_grad_fn(variant);
-        case R_SS: return frg::sob_smooth3_fn(h->P.smooth_width / 2, variant & 1, variant & 2);
+        case R_SS:
+            if (variant & frg::kSplit) {
+                const void *planes, *z;
+                frg::sob_smooth_split_fns(h->P.smooth_width / 2, frg::kSmoothInPlace, variant & 2, &planes, &z);
+                return planes;
+            }
+            return frg::sob_smooth3_fn(h->P.smooth_width / 2, variant & 1, variant & 2);
         default: return frg::sob_pass_b_fn(false);
     }
 }
@@ -288,7 +302,7 @@ int role_threads(int r, int variant = 0) {
     return r == R_PB ? frg::kPassBThreads : 256;
 }
 int role_tile_y(const fr_handle* h, int r, int variant = 0) {
-    if (r == R_SS) return frg::sob_smooth_tile_y(h->P.smooth_width / 2, variant & 2);
+    if (r == R_SS && !(variant & frg::kSplit)) return frg::sob_smooth_tile_y(h->P.smooth_width / 2, variant & 2);
     return r == R_PB ? frg::kPassBTileY : frg::kTileY;
 }
 
@@ -300,15 +314,18 @@ Shapes default_shapes(const fr_handle* h) {
         const std::vector<int> al = allowed_variants(h, r);
         int want = kDefaultVariant[r];
         if (r == R_SS) {  // tall smoothing tiles where they still give every SM one (sob_smooth_tile_y)
+            const int R = h->P.smooth_width / 2, ty = frg::sob_smooth_tile_y(R, true);
+            const bool split = al[0] == 0 && frg::sob_smooth_split(R, h->NT, false);
             long long tiles = 0;
-            const int ty = frg::sob_smooth_tile_y(h->P.smooth_width / 2, true), d = kDefaultDepth[r];
+            const int d = split ? 1 : kDefaultDepth[r];
             for (const Pair& P : h->hpairs)
                 tiles += (long long)((P.X + frg::kTileX - 1) / frg::kTileX) * ((P.Y + ty - 1) / ty) * ((P.Z + d - 1) / d);
-            if (tiles >= h->num_sms) want |= 2;
+            if (frg::sob_smooth_has_tall(R) && tiles >= (split ? 2 : 1) * h->num_sms) want |= 2;
+            if (split) want |= frg::kSplit;
         }
         int v = al[0];  // what is wanted where it is allowed, else the first that shares its tile height
         for (int c : al)
-            if (c == want || ((c ^ want) & 2) < ((v ^ want) & 2)) v = c;
+            if (c == want || (v != want && ((c ^ want) & 2) < ((v ^ want) & 2))) v = c;
         sh[r] = Shape{kDefaultDepth[r], kDefaultPerTile[r] ? -1 : h->ts[r].occ[v], v};
     }
     return sh;
@@ -322,6 +339,8 @@ int build_role(fr_handle* h, int r, Shape sh, cudaStream_t s = 0) {
         const std::vector<int> al = allowed_variants(h, r);
         if (std::find(al.begin(), al.end(), sh.variant) == al.end()) sh.variant = al[0];
     }
+    const bool split = r == R_SS && (sh.variant & frg::kSplit);
+    if (split) sh.bps = -1;  // the shape is the z filter's
     if (sh.bps != -1) sh.bps = std::min(std::max(sh.bps, 1), t.occ[sh.variant]);
     t.shape = sh;
     t.h.clear();
@@ -334,6 +353,26 @@ int build_role(fr_handle* h, int r, Shape sh, cudaStream_t s = 0) {
     if (t.h.size() > t.cap) return fail(h, FR_ERR_STATE, "tile table %d overflows (%zu > %zu)", r, t.h.size(), t.cap);
     FR_CUDA(h, cudaMemcpyAsync(t.d, t.h.data(), sizeof(Tile) * t.h.size(), cudaMemcpyHostToDevice, s));
     FR_CUDA(h, cudaStreamSynchronize(s));  // t.h is rewritten by the next build
+    if (split) {  // the plane filter takes a slice per tile
+        const int rows = frg::sob_smooth_tile_y(h->P.smooth_width / 2, sh.variant & 2);
+        if (h->planes_rows != rows) {
+            h->planes_rows = 0;
+            h->planes.clear();
+            for (int p = 0; p < h->npairs; ++p) {
+                const Pair& P = h->hpairs[p];
+                for (int z0 = 0; z0 < P.Z; ++z0)
+                    for (int y0 = 0; y0 < P.Y; y0 += rows)
+                        for (int x0 = 0; x0 < P.X; x0 += frg::kTileX) h->planes.push_back(make_int4(p, x0, y0, z0));
+            }
+            if (h->planes.size() > t.cap) return fail(h, FR_ERR_STATE, "the table of the smoothing's planes overflows");
+            FR_CUDA(h, cudaMemcpyAsync(h->d_planes, h->planes.data(), sizeof(Tile) * h->planes.size(),
+                                       cudaMemcpyHostToDevice, s));
+            FR_CUDA(h, cudaStreamSynchronize(s));
+            h->planes_rows = rows;
+        }
+        t.grid = (int)h->planes.size();
+        return FR_OK;
+    }
     t.grid = sh.bps == -1 ? (int)t.h.size()
                           : (int)std::max(1LL, std::min<long long>((long long)sh.bps * h->num_sms, (long long)t.h.size()));
     return FR_OK;
@@ -458,6 +497,7 @@ int setup_cohort(fr_handle* h, const fr_pair* pairs, int n) {
     h->npairs = n;
     h->hpairs.assign(n, Pair{});
     h->htiles.clear();
+    h->planes_rows = 0;
     long long off = 0;
     for (int p = 0; p < n; ++p) {
         Pair& P = h->hpairs[p];
@@ -509,6 +549,7 @@ int setup_cohort(fr_handle* h, const fr_pair* pairs, int n) {
         h->ts[r].cap = cap;
         add((void**)&h->ts[r].d, sizeof(Tile) * cap);
     }
+    if (h->P.solver == FR_SOLVER_SOBOLEV) add((void**)&h->d_planes, sizeof(Tile) * cap);
     add((void**)&h->d_io, sizeof(frg::PairIO) * n);
     add((void**)&h->S, sizeof(float) * NT);
     add((void**)&h->T, sizeof(float) * NT);
@@ -683,6 +724,15 @@ frg::SobIterArgs sob_args(fr_handle* h, int iter) {
     a.tiles_s = h->ts[R_SS].d;
     a.ntiles_s = (int)h->ts[R_SS].h.size();
     a.depth_s = h->ts[R_SS].shape.depth;
+    if (h->ts[R_SS].shape.variant & frg::kSplit) {
+        a.tiles_z = a.tiles_s;
+        a.ntiles_z = a.ntiles_s;
+        a.depth_z = a.depth_s;
+        a.tiles_s = h->d_planes;
+        a.ntiles_s = (int)h->planes.size();
+        a.depth_s = 1;
+        a.mid = h->v[1];  // the reference solver's second velocity buffer
+    }
     a.tiles_b = h->ts[R_SB].d;
     a.ntiles_b = (int)h->ts[R_SB].h.size();
     a.depth_b = h->ts[R_SB].shape.depth;
@@ -910,22 +960,18 @@ std::mutex g_tune_mu;
 std::map<std::string, Shapes> g_tuned;
 
 int launch_role(fr_handle* h, int r, int iter, float t, cudaStream_t s) {
-    frg::RefIterArgs ra{};
-    frg::SobIterArgs sa{};
-    void* args[1];
+    const int v = h->ts[r].shape.variant;
     // no pair converges while shapes are timed (a stopped pair's tiles would be skipped)
     if (r == R_LAP || r == R_PA || r == R_PB) {
-        ra = ref_args(h, iter, t);
+        frg::RefIterArgs ra = ref_args(h, iter, t);
         ra.check_stop = 0;
-        args[0] = &ra;
+        void* args[1] = {&ra};
+        FR_CUDA(h, frg::launch_kernel(role_fn(h, r, v), h->ts[r].grid, role_threads(r, v), role_smem(r, v), args, s, true));
     } else {
-        sa = sob_args(h, iter);
+        frg::SobIterArgs sa = sob_args(h, iter);
         sa.check_stop = 0;
-        args[0] = &sa;
+        FR_CUDA(h, frg::launch_sob_kernel(r - R_SG, sa, h->ts[r].grid, v, s, true));
     }
-    const int v = h->ts[r].shape.variant;
-    FR_CUDA(h, cudaLaunchKernel(role_fn(h, r, v), dim3(h->ts[r].grid), dim3(role_threads(r, v)), args,
-                                role_smem(r, v), s));
     return FR_OK;
 }
 
@@ -985,7 +1031,10 @@ int autotune(fr_handle* h, cudaStream_t s) {
             if (occ / 2 >= 1 && occ / 2 < occ - 1) bps.push_back(occ / 2);
             bps.push_back(-1);  // one block per tile
             for (int depth : depths)
-                for (int b : bps) cand.push_back(Shape{depth, b, v});
+                for (int b : bps) {
+                    if (r == R_SS && (v & frg::kSplit) && b != -1) continue;
+                    cand.push_back(Shape{depth, b, v});
+                }
         }
         // two passes over the candidates, each candidate's faster time kept (less noise)
         std::vector<float> best_of(cand.size(), 1e30f);

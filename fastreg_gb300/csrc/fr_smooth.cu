@@ -100,14 +100,19 @@ __device__ __forceinline__ void fix_edges(float* box, int x0, int y0, int X, int
 enum SmoothMode {
     kInPlace,    // the momentum, updated in place (m_n is m; a second pointer costs the TMA kernel 4%)
     kOutOfPlace, // the momentum, read from m and written to m_n
-    kTranspose   // m_n = G^T g
+    kTranspose,  // m_n = G^T g
+    kPlanes,     // mid = g filtered along x and y only (sob_smooth_z_kernel does the rest)
+    kPlanesTranspose
 };
+constexpr int kPlaneSlots = 1;  // the plane forms take one slice per tile
 template <int R, bool TMA, int TY, SmoothMode MODE>
 __global__ void __launch_bounds__(kSmoothThreads) sob_smooth3_kernel(SobIterArgs a) {
     pdl_wait();
     using G = SmoothGeom<R, TY>;
-    constexpr bool ADJ = MODE == kTranspose;
-    constexpr int K = G::K, WS = G::WS, NS = G::NS, NP = TY / 2;
+    constexpr bool ADJ = MODE == kTranspose || MODE == kPlanesTranspose;
+    constexpr bool kPlane = MODE == kPlanes || MODE == kPlanesTranspose, kMomentum = !ADJ && !kPlane;
+    constexpr int RZ = kPlane ? 0 : R;  // slices read beyond a tile's ends
+    constexpr int K = G::K, WS = G::WS, NS = kPlane ? kPlaneSlots : G::NS, NP = TY / 2;
     __shared__ __align__(128) float rings[3][NS][G::SLOT];
     __shared__ __align__(8) uint64_t bars[3][NS];
     const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;  // this warp's component
@@ -139,7 +144,7 @@ __global__ void __launch_bounds__(kSmoothThreads) sob_smooth3_kernel(SobIterArgs
         }
         const int X = P.X, Y = P.Y, Z = P.Z, Xp = P.Xp, XY = P.Xp * P.Y;
         const int x0 = tl.y, y0 = tl.z, zt0 = tl.w, zt1 = min(tl.w + a.depth_s, Z);
-        const int nsl = (zt1 - zt0) + 2 * R;
+        const int nsl = (zt1 - zt0) + 2 * RZ;
         const bool edge = x0 == 0 || x0 + kTileX - 1 + R > X - 1 || y0 == 0 || y0 + TY - 1 + R > Y - 1;
         const float* __restrict__ gc = a.g + c * a.NT + P.off;
         const CUtensorMap* mg = a.tmaps + (long long)tl.x * TM_COUNT + (TY == sob_smooth_tile_y(R, false) ? TM_SOB_G : TM_SOB_G_TALL);
@@ -157,8 +162,8 @@ __global__ void __launch_bounds__(kSmoothThreads) sob_smooth3_kernel(SobIterArgs
                 goff[j] = in ? Xp * min(max(yr, 0), Y - 1) + x : -1;
             }
         }
-        auto issue = [&](int k) {  // slice k of the tile (z = zt0 - R + k, clamped) into the next slot
-            const int z = min(max(zt0 - R + k, 0), Z - 1);
+        auto issue = [&](int k) {  // slice k of the tile (z = zt0 - RZ + k, clamped) into the next slot
+            const int z = min(max(zt0 - RZ + k, 0), Z - 1);
             if (TMA) {
                 if (lane == 0) {
                     mbar_arrive_expect_tx(full + issue_slot, sizeof(float) * G::BOX);
@@ -170,7 +175,7 @@ __global__ void __launch_bounds__(kSmoothThreads) sob_smooth3_kernel(SobIterArgs
 #pragma unroll
                 for (int j = 0; j < NJ; ++j)
                     if (ADJ) {  // zeros outside the volume
-                        const bool in = goff[j] >= 0 && zt0 - R + k >= 0 && zt0 - R + k < Z;
+                        const bool in = goff[j] >= 0 && zt0 - RZ + k >= 0 && zt0 - RZ + k < Z;
                         if (lane + 32 * j < NF) cp_async16_or_zero(dst + 128 * j, in ? src + goff[j] : src, in);
                     } else if (goff[j] >= 0) {
                         cp_async16(dst + 128 * j, src + goff[j]);
@@ -183,20 +188,20 @@ __global__ void __launch_bounds__(kSmoothThreads) sob_smooth3_kernel(SobIterArgs
             if (k < nsl) issue(k);
             if (!TMA) cp_async_commit();
         }
-        float2 part[NP][R > 0 ? 2 * R : 1];  // the z chains in flight of each row pair
+        float2 part[NP][RZ > 0 ? 2 * RZ : 1];  // the z chains in flight of each row pair
 #pragma unroll
         for (int p = 0; p < NP; ++p)
 #pragma unroll
-            for (int j = 0; j < (R > 0 ? 2 * R : 1); ++j) part[p][j] = make_float2(0.f, 0.f);
+            for (int j = 0; j < (RZ > 0 ? 2 * RZ : 1); ++j) part[p][j] = make_float2(0.f, 0.f);
         const int x = x0 + lane, rows = x < X ? min(Y - y0, TY) : 0;  // rows that this lane stores
-        const long long m0 = c * a.NT + P.off + (x + Xp * y0) + (long long)XY * (zt0 - 2 * R);
-        float* mn = a.m_n + m0;
+        const long long m0 = c * a.NT + P.off + (x + Xp * y0) + (long long)XY * (zt0 - 2 * RZ);
+        float* mn = (kPlane ? a.mid : a.m_n) + m0;
         const float* ms = MODE == kOutOfPlace ? a.m + m0 : nullptr;
         for (int k = 0; k < nsl; ++k, mn += XY, ms += MODE == kOutOfPlace ? XY : 0) {
             const float* m = MODE == kOutOfPlace ? ms : mn;
-            const bool store = k >= 2 * R;  // slice zt0 + k - 2R is complete with this one
+            const bool store = k >= 2 * RZ;  // slice zt0 + k - 2RZ is complete with this one
             float mo[TY];
-            if (store && !ADJ)
+            if (store && kMomentum)
 #pragma unroll
                 for (int r = 0; r < TY; ++r)
                     if (r < rows) mo[r] = m[Xp * r];
@@ -264,19 +269,23 @@ __global__ void __launch_bounds__(kSmoothThreads) sob_smooth3_kernel(SobIterArgs
                         }
                     }
 #pragma unroll
-                for (int j = 2 * R; j >= 0; --j)
+                for (int j = 2 * RZ; j >= 0; --j)
 #pragma unroll
                     for (int rp = r0; rp < r0 + kILP && rp < G::H / 2; ++rp) {
                         if (rp < R) continue;
                         const int p = rp - R;
+                        if (kPlane) {
+                            o[rp - r0] = v[rp - r0];
+                            continue;
+                        }
                         const float2 n = __ffma2_rn(make_float2(a.taps[j], a.taps[j]), v[rp - r0],
                                                     j > 0 ? part[p][j > 0 ? j - 1 : 0] : make_float2(0.f, 0.f));
-                        if (j == 2 * R)
+                        if (j == 2 * RZ)
                             o[rp - r0] = n;
                         else
                             part[p][j] = n;
                     }
-                if (ADJ) {  // the ends of the z axis: this slice's extra share of output slices 0 and Z - 1
+                if (ADJ && !kPlane) {  // the ends of the z axis: this slice's extra share of output slices 0 and Z - 1
                     const int zc = zt0 - R + k;
 #pragma unroll
                     for (int d = 0; d < R; ++d)
@@ -294,10 +303,10 @@ __global__ void __launch_bounds__(kSmoothThreads) sob_smooth3_kernel(SobIterArgs
                         if (rp < R) continue;
                         const int p = rp - R;
                         if (2 * p < rows)
-                            mn[Xp * (2 * p)] = ADJ ? o[rp - r0].x : a.damping * mo[2 * p] - a.step * o[rp - r0].x;
+                            mn[Xp * (2 * p)] = !kMomentum ? o[rp - r0].x : a.damping * mo[2 * p] - a.step * o[rp - r0].x;
                         if (2 * p + 1 < rows)
                             mn[Xp * (2 * p + 1)] =
-                                ADJ ? o[rp - r0].y : a.damping * mo[2 * p + 1] - a.step * o[rp - r0].y;
+                                !kMomentum ? o[rp - r0].y : a.damping * mo[2 * p + 1] - a.step * o[rp - r0].y;
                     }
             }
             __syncwarp();  // every lane has read the slot
@@ -313,6 +322,70 @@ __global__ void __launch_bounds__(kSmoothThreads) sob_smooth3_kernel(SobIterArgs
             slot = slot + 1 == NS ? 0 : slot + 1;
         }
         atomicOr(a.err, kErrTmaTimeout);
+    }
+}
+
+// The smoothing in two launches: the plane forms above filter every slice along x and y into
+// `mid`, this kernel filters mid along z and feeds the momentum (or, transposed, m_n), tap for
+// tap in the same order, so the bits are those of the one launch.  No slice is filtered along x
+// and y twice (a march of d slices filters d + 2 R), no z chains are held across a slice (the plane
+// kernel's 16 rows take 64 registers instead of 168), and every slice is a tile of its own, which
+// is what small volumes and wide filters lack; large volumes at small radii pay 24 bytes per voxel
+// more of traffic instead.  20 unrolled iterations: radius 3, 64^3 1.33 -> 1.14 ms, 96^3 2.46 -> 2.36,
+// 128^3 4.83 -> 4.82; radius 5, 91x109x91 3.76 -> 2.98; radius 7, 128^3 9.04 -> 6.30; radius 1, 64^3
+// 0.95 -> 1.03.  A thread takes kZBatch slices' loads together; bound by their latency.
+constexpr int kZBatch = 4;
+template <int R, SmoothMode MODE>
+__global__ void __launch_bounds__(256) sob_smooth_z_kernel(SobIterArgs a) {
+    pdl_wait();
+    constexpr bool ADJ = MODE == kTranspose;
+    constexpr int U = kZBatch;
+    for (int t = blockIdx.x; t < 3 * a.ntiles_z; t += gridDim.x) {
+        const int c = t % 3;
+        Tile tl;
+        Pair P;
+        if (!take_tile(a, a.tiles_z, t / 3, kTileY, a.depth_z, tl, P)) continue;
+        const int X = P.X, Y = P.Y, Z = P.Z, XY = P.Xp * P.Y;
+        const int x = tl.y + (threadIdx.x & 31), y = tl.z + (threadIdx.x >> 5);
+        if (x >= X || y >= Y) continue;
+        const int zt0 = tl.w, zt1 = min(zt0 + a.depth_z, Z), nsl = zt1 - zt0 + 2 * R;
+        const long long at = c * a.NT + P.off + x + P.Xp * y;
+        const float* __restrict__ g = a.mid + at;
+        const float* m = (MODE == kOutOfPlace ? a.m : a.m_n) + at;
+        float* mn = a.m_n + at;
+        float part[R > 0 ? 2 * R : 1];
+#pragma unroll
+        for (int j = 0; j < (R > 0 ? 2 * R : 1); ++j) part[j] = 0.f;
+        for (int k0 = 0; k0 < nsl; k0 += U) {
+            float v[U], mo[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int k = k0 + u, z = zt0 - R + k;
+                const bool in = k < nsl && (!ADJ || (z >= 0 && z < Z));
+                v[u] = in ? __ldg(g + XY * min(max(z, 0), Z - 1)) : 0.f;
+                mo[u] = !ADJ && k >= 2 * R && k < nsl ? m[XY * (z - R)] : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int k = k0 + u, z = zt0 - R + k;
+                float o = 0.f;
+#pragma unroll
+                for (int j = 2 * R; j >= 0; --j) {
+                    const float n = fmaf(a.taps[j], v[u], j > 0 ? part[j > 0 ? j - 1 : 0] : 0.f);
+                    if (j == 2 * R)
+                        o = n;
+                    else
+                        part[j] = n;
+                }
+                if (ADJ)
+#pragma unroll
+                    for (int d = 0; d < R; ++d) {
+                        if (z == d) part[R + d] = fmaf(a.fold[d], v[u], part[R + d]);
+                        if (z == Z - 1 - d) part[R - d] = fmaf(a.fold[d], v[u], part[R - d]);
+                    }
+                if (k >= 2 * R && k < nsl) mn[XY * (z - R)] = ADJ ? o : a.damping * mo[u] - a.step * o;
+            }
+        }
     }
 }
 
@@ -336,7 +409,42 @@ const void* smooth_unrolled_fn(bool transposed, bool tall) {
                 : (const void*)sob_smooth3_kernel<R, false, kShort, kOutOfPlace>;
 }
 
+template <int R>
+void smooth_split_fns(SmoothForm form, bool tall, const void** planes, const void** z) {
+    constexpr int kShort = sob_smooth_tile_y(R, false), kTall = sob_smooth_tile_y(R, true);
+    if (form == kSmoothTransposed)
+        *planes = tall ? (const void*)sob_smooth3_kernel<R, false, kTall, kPlanesTranspose>
+                       : (const void*)sob_smooth3_kernel<R, false, kShort, kPlanesTranspose>;
+    else
+        *planes = tall ? (const void*)sob_smooth3_kernel<R, false, kTall, kPlanes>
+                       : (const void*)sob_smooth3_kernel<R, false, kShort, kPlanes>;
+    *z = form == kSmoothTransposed ? (const void*)sob_smooth_z_kernel<R, kTranspose>
+         : form == kSmoothUnrolled ? (const void*)sob_smooth_z_kernel<R, kOutOfPlace>
+                                   : (const void*)sob_smooth_z_kernel<R, kInPlace>;
+}
+
 }  // namespace
+
+void sob_smooth_split_fns(int radius, SmoothForm form, bool tall, const void** planes, const void** z) {
+    switch (radius) {
+        case 0: return smooth_split_fns<0>(form, tall, planes, z);
+        case 1: return smooth_split_fns<1>(form, tall, planes, z);
+        case 2: return smooth_split_fns<2>(form, tall, planes, z);
+        case 3: return smooth_split_fns<3>(form, tall, planes, z);
+        case 4: return smooth_split_fns<4>(form, tall, planes, z);
+        case 5: return smooth_split_fns<5>(form, tall, planes, z);
+        case 6: return smooth_split_fns<6>(form, tall, planes, z);
+        default: return smooth_split_fns<7>(form, tall, planes, z);
+    }
+}
+
+cudaError_t launch_smooth_split(const SobIterArgs& a, SmoothForm form, bool tall, int grid, cudaStream_t s, bool behind) {
+    const void *planes, *z;
+    sob_smooth_split_fns(a.radius, form, tall, &planes, &z);
+    void* args[1] = {const_cast<SobIterArgs*>(&a)};
+    const cudaError_t e = launch_kernel(planes, grid, kSmoothThreads, 0, args, s, behind);
+    return e != cudaSuccess ? e : launch_kernel(z, 3 * a.ntiles_z, 256, 0, args, s, behind);
+}
 
 const void* sob_smooth3_fn(int radius, int tma, bool tall) {
     switch (radius) {

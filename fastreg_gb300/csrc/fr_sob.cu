@@ -351,6 +351,8 @@ const void* sob_pass_b_fn(bool unrolled) {
 cudaError_t launch_sob_kernel(int k, const SobIterArgs& a, int grid, int variant, cudaStream_t s, bool behind) {
     void* args[1] = {const_cast<SobIterArgs*>(&a)};
     if (k == 0) return launch_kernel(sob_grad_fn(variant), grid, sob_grad_threads(variant), sob_grad_smem_bytes(), args, s, behind);
+    if (k == 1 && (variant & kSplit))
+        return launch_smooth_split(a, variant & kUnrolled ? kSmoothUnrolled : kSmoothInPlace, variant & 2, grid, s, behind);
     if (k == 1)
         return launch_kernel(variant & kUnrolled ? sob_smooth3_unrolled_fn(a.radius, false, variant & 2)
                                                  : sob_smooth3_fn(a.radius, variant & 1, variant & 2),

@@ -45,6 +45,8 @@ struct SobIterArgs {
     int ntiles_s, depth_s;
     const Tile* tiles_b;
     int ntiles_b, depth_b;
+    const Tile* tiles_z;  // 32 x 8 x depth tiles of the z filter where it is a launch of its own
+    int ntiles_z, depth_z;
     int npairs;
     long long NT;
     const float* S;
@@ -54,6 +56,7 @@ struct SobIterArgs {
     float* phi_n;      // positions, written: phi itself except in unrolled iterations
     float* m_n;        // momentum, written and gathered: m itself except in unrolled iterations
     float* g;          // gradient (3 planes)
+    float* mid;        // g filtered along x and y (3 planes), smoothing in two launches
     float damping, step;
     float lambda;  // W_REG; the kernels take each pair's weight from Pair::w_reg
     float taps[kMaxSmoothWidth];
@@ -85,6 +88,26 @@ const void* sob_smooth3_fn(int radius, int tma, bool tall);
 // the unrolled registration's (cp.async staging): the momentum from m to m_n, or transposed,
 // m_n = G^T g, which needs `fold` and zeros in the pad columns of g
 const void* sob_smooth3_unrolled_fn(int radius, bool transposed, bool tall);
+// the smoothing in two launches (fr_smooth.cu): every slice along x and y into `mid`, then along z;
+// grid: the tiles of the first, 32 columns by the tile height by one slice
+enum SmoothForm { kSmoothInPlace, kSmoothUnrolled, kSmoothTransposed };
+void sob_smooth_split_fns(int radius, SmoothForm form, bool tall, const void** planes, const void** z);
+cudaError_t launch_smooth_split(const SobIterArgs& a, SmoothForm form, bool tall, int grid, cudaStream_t s, bool behind);
+// Where the two launches are the faster for N packed voxels, one launch -> two.  Unrolled (20
+// iterations), radius 2: 64^3 0.97 -> 0.93 ms, 96^3 1.96 -> 1.99; radius 3: 64^3 1.33 -> 1.10, 112^3 3.74 ->
+// 3.67, 128^3 4.83 -> 4.85; radius 4: 64^3 1.46 -> 1.07, 182x218x182 14.5 -> 14.2; radius 5: 128^3 5.99 ->
+// 5.47, 182x218x182 the same; radius 7: 128^3 9.04 -> 6.30, 182x218x182 20.6 -> 17.6.  Registrations (200
+// iterations), whose other kernels take more of L2, radius 2: 60x64x60 3.3 -> 3.0 ms; radius 3: 64^3 4.1 ->
+// 3.3, 112^3 the same, 128^3 13.2 -> 14.8; radius 4: 96^3 7.9 -> 6.8, 128^3 14.8 -> 15.4; radius 5: 91x109x91
+// 5.2 -> 4.6, 128^3 19.0 -> 16.5, from 160^3 on one launch (the autotuner times both).
+inline bool sob_smooth_split(int radius, long long N, bool unrolled) {
+    return radius >= (unrolled ? 4 : 5) || (radius >= 3 && N <= 3 << 19) || (radius == 2 && N <= 1 << 18);
+}
+// slices per tile of the z filter: as many, up to 32, as leave two blocks for every SM
+inline int sob_smooth_z_depth(long long columns, int Z, int sms) {  // columns: 32 x 8, of all pairs
+    const long long d = 3 * columns * Z / (2LL * (sms > 0 ? sms : 1));
+    return d < 2 ? 2 : d > 32 ? 32 : (int)d;
+}
 // box of one component of the smoothing kernel's staged slice for radius R: x extent, rows
 inline void sob_smooth_box(int R, bool tall, int* wx, int* rows) {
     *wx = kTileX + 2 * ((R + 3) / 4 * 4);
@@ -92,6 +115,7 @@ inline void sob_smooth_box(int R, bool tall, int* wx, int* rows) {
 }
 const void* sob_pass_b_fn(bool unrolled);  // the update kernel
 constexpr int kUnrolled = 4;  // variant bit: the unrolled registration's kernel (separate in and out states)
+constexpr int kSplit = 8;     // variant bit of the smoothing: in two launches
 
 // one of them: k = 0 gradient, 1 smoothing, 2 update
 cudaError_t launch_sob_kernel(int k, const SobIterArgs& a, int grid, int variant, cudaStream_t s, bool behind);

@@ -221,3 +221,22 @@ def test_smoothing_tile_heights(cuda, dims, width, staging):
     assert_bitexact(fr.get_field(N.FR_FIELD_PSI).cpu().numpy(), o["phi"], f"phi (width {width})")
     assert_bitexact(fr.get_field(N.FR_FIELD_V).cpu().numpy(), o["m"], f"momentum (width {width})")
     fr.close()
+
+
+@pytest.mark.parametrize("width", [5, 7, 9, 11, 13, 15])
+@pytest.mark.parametrize("dims_list", [[(33, 17, 9)], [(4, 4, 5)], [(64, 33, 40)],
+                                       [(31, 8, 5), (4, 34, 33), (65, 9, 66), (5, 4, 4)]])
+def test_smoothing_in_two_launches(cuda, dims_list, width):
+    """Small volumes and wide filters are smoothed in two launches (AUTOTUNE=0, cp.async): axes
+    shorter than the filter, sizes one past a tile's columns, rows and slices, and an uneven
+    cohort, against the oracle's bits."""
+    pairs_np = [images(d, 2100 + 10 * width + k) for k, d in enumerate(dims_list)]
+    kw = dict(no_labels=4, max_iter=3, solver="sobolev", smooth_sigma=0.4 + 0.3 * width, smooth_width=width,
+              damping=0.9, step=0.5, staging=1, autotune=0)
+    fr = FastReg(Params(volume_dims=dims_list[0], **kw))
+    fr.register_batch([tuple(_to(cuda, p[k]) for k in ("T", "labT", "S", "labS")) for p in pairs_np])
+    for k, (d, p) in enumerate(zip(dims_list, pairs_np)):
+        o = O.sob_register(Params(volume_dims=d, **kw), p["T"], p["S"])
+        assert_bitexact(fr.get_field(N.FR_FIELD_PSI, pair=k).cpu().numpy(), o["phi"], f"pair {k} phi (width {width})")
+        assert_bitexact(fr.get_field(N.FR_FIELD_V, pair=k).cpu().numpy(), o["m"], f"pair {k} momentum (width {width})")
+    fr.close()
