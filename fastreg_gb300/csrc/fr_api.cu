@@ -1729,15 +1729,15 @@ int fr_interpolate_field(const float* d_field, const float* d_pos, const int dim
     static std::atomic<int> slots[64];
     const int X = dims[0], Y = dims[1], Z = dims[2];
     const long long cols = ((long long)X * Y + frg::kFieldThreads - 1) / frg::kFieldThreads;
-    // Columns of 16 slices where they make three waves of blocks or more (64.7 us on 182x218x182; 8 take
-    // 67.2 us, 24 67.6 us).  Below that the waves count: a wave of d slices takes about d + 1/2, one that
+    // Columns of 16 slices where they make two and a half waves of blocks or more (64.7 us on 182x218x182;
+    // 8 take 67.2 us, 24 67.6 us).  Below that the waves count: a wave of d slices takes about d + 1/2, one that
     // fills a share f of the GPU 0.44 + 0.56 f of it, and the depth that costs least is within 5% of the
     // best one measured on eight sizes from 45x54x45 to 160x192x160 (137x108x173: 18 slices, one
     // wave, 26.1 us; 16 slices, a second wave of 15 blocks, 31.5 us).
     const long long slots_all = std::max(resident_blocks((const void*)frg::interpolate_field_kernel, slots,
                                                          frg::kFieldThreads), 1);
     long long depth = 16;
-    if (cols * Z < 3 * 16 * slots_all) {
+    if (2 * cols * Z < 5 * 16 * slots_all) {
         double least = 1e300;
         for (int d = 1; d <= 24; ++d) {
             const long long blocks = cols * ((Z + d - 1) / d), rest = blocks % slots_all;

@@ -1,5 +1,6 @@
 // fr_smooth.cu -- the sobolev solver's separable Gaussian (x, y, z) fused with the momentum
-// update m = damping * m - step * gs, one launch over the cohort.
+// update m = damping * m - step * gs, one launch over the cohort (two for small volumes and wide
+// filters: sob_smooth_z_kernel).
 //
 // A warp owns one component of a 32-column x TY-row tile and marches z; a block is the three
 // components of a tile, and its warps never wait on one another.  Per slice the warp stages
@@ -331,8 +332,8 @@ __global__ void __launch_bounds__(kSmoothThreads) sob_smooth3_kernel(SobIterArgs
 // and y twice (a march of d slices filters d + 2 R), no z chains are held across a slice (the plane
 // kernel's 16 rows take 64 registers instead of 168), and every slice is a tile of its own, which
 // is what small volumes and wide filters lack; large volumes at small radii pay 24 bytes per voxel
-// more of traffic instead.  20 unrolled iterations: radius 3, 64^3 1.33 -> 1.14 ms, 96^3 2.46 -> 2.36,
-// 128^3 4.83 -> 4.82; radius 5, 91x109x91 3.76 -> 2.98; radius 7, 128^3 9.04 -> 6.30; radius 1, 64^3
+// more of traffic instead.  20 unrolled iterations: radius 3, 64^3 1.33 -> 1.10 ms, 96^3 2.46 -> 2.33,
+// 128^3 4.83 -> 4.85; radius 5, 91x109x91 3.76 -> 2.98; radius 7, 128^3 9.04 -> 6.30; radius 1, 64^3
 // 0.95 -> 1.03.  A thread takes kZBatch slices' loads together; bound by their latency.
 constexpr int kZBatch = 4;
 template <int R, SmoothMode MODE>
