@@ -197,7 +197,6 @@ __global__ void __launch_bounds__(256) ref_laplacian_tma_kernel(RefIterArgs a) {
     float* ring = reinterpret_cast<float*>(lap_raw);
     if (!ring_aligned(ring, a.err)) return;
     uint64_t* full = reinterpret_cast<uint64_t*>(ring + kTLS * kTSlot);
-    typedef SliceRing<kTLS> Ring;
     const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
     if (tid == 0) {
         for (int k = 0; k < kTLS; ++k) mbar_init(full + k, 1);
@@ -296,10 +295,8 @@ __global__ void __launch_bounds__(256) ref_laplacian_tma_kernel(RefIterArgs a) {
         }
     }
     if (failed && tid == 0) {
-        // the copies this block issued and nobody waited for: wait for them (bounded)
-        // before the block's shared memory goes away, then report
-        for (unsigned n = (issued > (unsigned)kTLS ? issued - kTLS : 0u); n < issued; ++n)
-            mbar_wait_bounded(full + Ring::slot(n), Ring::parity(n));
+        // the copies in flight end (bounded) before the block's shared memory goes away
+        drain_fills<kTLS>(issued, [&](int k, unsigned parity) { mbar_wait_bounded(full + k, parity); });
         atomicOr(a.err, kErrTmaTimeout);
     }
 }
@@ -590,7 +587,7 @@ __global__ void __launch_bounds__(256, 3) ref_pass_a_tma_kernel(RefIterArgs a) {
     // (thread 0) and to read, and per slot the parity of its next completion
     int fv = 0, fq = 0, rv = 0, rq = 0;
     unsigned phase = 0u;
-    int flying = 0;  // fills issued and not waited for (thread 0)
+    unsigned issued = 0;  // fills so far (thread 0)
     bool failed = false;
     for (int t = blockIdx.x; t < a.ntiles_a && !failed; t += gridDim.x) {
         Tile tl;
@@ -625,7 +622,7 @@ __global__ void __launch_bounds__(256, 3) ref_pass_a_tma_kernel(RefIterArgs a) {
                 fq = fq + 1 == kPQS ? 0 : fq + 1;
             }
             fv = fv + 1 == kPVS ? 0 : fv + 1;
-            ++flying;
+            ++issued;
         };
         __syncthreads();  // the previous tile is done with the rings
         if (tid == 0)
@@ -638,7 +635,6 @@ __global__ void __launch_bounds__(256, 3) ref_pass_a_tma_kernel(RefIterArgs a) {
         auto land = [&]() {  // waits for the next fill
             ok = mbar_wait_bounded(full + rv, (phase >> rv) & 1u) && ok;
             phase ^= 1u << rv;
-            --flying;
         };
         auto next_v = [&](int k) {
             vb[k] = vring + rv * kPVSlot + vc0;
@@ -677,12 +673,9 @@ __global__ void __launch_bounds__(256, 3) ref_pass_a_tma_kernel(RefIterArgs a) {
         }
     }
     if (failed && tid == 0) {
-        // the copies in flight end (bounded) before the block's shared memory goes
-        for (; flying > 0; --flying) {
-            mbar_wait_bounded(full + rv, (phase >> rv) & 1u);
-            phase ^= 1u << rv;
-            rv = rv + 1 == kPVS ? 0 : rv + 1;
-        }
+        // the copies in flight end (bounded) before the block's shared memory goes; every fill is one of
+        // the v ring, whose barriers the q ring's copies complete on too
+        drain_fills<kPVS>(issued, [&](int k, unsigned parity) { mbar_wait_bounded(full + k, parity); });
         atomicOr(a.err, kErrTmaTimeout);
     }
 }

@@ -106,11 +106,10 @@ __global__ void __launch_bounds__(sob_grad_threads(TMA), TMA ? 4 : 6) sob_grad_k
                     tma_load_3d(ring + k * kGSlot + kGTOff, maps + TM_LAP_T, tl.y, tl.z, z, full + k);
                 }
             }
-            if (!ok) {  // the copies in flight end (bounded) before the block's shared memory goes
-                for (unsigned m = n > (unsigned)kGS ? n - kGS : 0u; m < n; ++m)
-                    mbar_wait_bounded(full + SliceRing<kGS>::slot(m), SliceRing<kGS>::parity(m));
-                atomicOr(a.err, kErrTmaTimeout);
-            }
+            // the copies in flight end (bounded) before this thread, and with it the block's shared memory, goes:
+            // also when it saw no failure itself, as a warp that gave up on one of the last fills has left
+            drain_fills<kGS>(n, [&](int k, unsigned parity) { mbar_wait_bounded(full + k, parity); });
+            if (!ok) atomicOr(a.err, kErrTmaTimeout);
             return;
         }
     }

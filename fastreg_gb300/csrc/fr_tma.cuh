@@ -16,6 +16,8 @@
 #include <cuda.h>
 #include <cstdint>
 
+#include "fr_ring.h"
+
 namespace frg {
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -88,15 +90,6 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, i
 __device__ __forceinline__ void tma_prefetch_map(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
-
-// A ring of `S` slots filled in order by one producer thread: slice n of the block's
-// stream of slices goes to slot n % S, and the k-th fill of a slot completes phase k of its
-// barrier (parity k & 1).
-template <int S>
-struct SliceRing {
-    __device__ __forceinline__ static int slot(unsigned n) { return (int)(n % S); }
-    __device__ __forceinline__ static unsigned parity(unsigned n) { return (n / S) & 1u; }
-};
 
 // Codes of the device error word (RefIterArgs::err, SobIterArgs::err).
 constexpr unsigned kErrTmaTimeout = 1u;
