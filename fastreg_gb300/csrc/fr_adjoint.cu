@@ -65,13 +65,13 @@ __global__ void __launch_bounds__(256) adj_pack_kernel(AdjPair A, const float* _
 }
 
 // The result: the adjoint of v0 out of the interleaved accumulator.
-__global__ void __launch_bounds__(256) adj_unpack_kernel(AdjPair A, const float4* __restrict__ mbar, float* out) {
+__global__ void __launch_bounds__(256) adj_unpack_kernel(AdjPair A, const float4* mbar, float* out) {
     pdl_wait();
     const long long nu = (long long)A.X * A.Y * A.Z;
     GRID_STRIDE(i, A.N) {
         const int row = i / A.Xp, x = i - row * A.Xp;
         if (x >= A.X) continue;
-        const float4 v = __ldg(mbar + i);
+        const float4 v = chain_load(mbar + i);
         const long long u = x + (long long)A.X * row;
         out[u] = v.x;
         out[nu + u] = v.y;
@@ -121,7 +121,7 @@ __device__ __forceinline__ Pair as_pair(const AdjPair& A) {
 // J and the adjoint seeds: pbar = r dS(phi_K), mbar = 0.2 m_K (0 in the pad columns).  Every term
 // is a product of two FP32 values, exact in FP64, added by one fused multiply-add.
 __global__ void __launch_bounds__(256) adj_loss_kernel(AdjPair A, const float* __restrict__ S, const float* __restrict__ T,
-                                                       const float* __restrict__ phi, const float* __restrict__ m,
+                                                       const float* phi, const float* m,
                                                        float* pbar, float4* mbar, double* loss) {
     pdl_wait();
     __shared__ double red[32];
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(256) adj_loss_kernel(AdjPair A, const float* _
             mbar[i] = make_float4(0.f, 0.f, 0.f, 0.f);
             continue;
         }
-        const SobCell s = sob_locate(P, __ldg(phi + i), __ldg(phi + A.NT + i), __ldg(phi + 2 * A.NT + i));
+        const SobCell s = sob_locate(P, chain_load(phi + i), chain_load(phi + A.NT + i), chain_load(phi + 2 * A.NT + i));
         float f[8], d[3], W;
         load_corners(S, s.base, A.Xp, A.XYp, f);
         tri_grad(f, s, d, &W, nullptr);
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(256) adj_loss_kernel(AdjPair A, const float* _
         float mc[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            mc[c] = __ldg(m + c * A.NT + i);
+            mc[c] = chain_load(m + c * A.NT + i);
             em = fma((double)mc[c], (double)mc[c], em);
             pbar[c * A.NT + i] = r * d[c];
         }
@@ -190,8 +190,8 @@ __device__ __forceinline__ void scatter_face_warp(float4* F, int b, const float3
 // face of the next slice's cell where the cell moves up by exactly one slice, is held back and
 // added there.  The gathered corners are kept the same way, as in sob_pass_b_kernel.  On the
 // 128^3 pair 40 us; with one 4-byte reduction per corner and component, lanes merged, 144 us.
-__global__ void __launch_bounds__(256) adj_update_kernel(AdjPair A, const float* __restrict__ phi,
-                                                         const float* __restrict__ mn, float* pbar, float4* mbar) {
+__global__ void __launch_bounds__(256) adj_update_kernel(AdjPair A, const float* phi,
+                                                         const float* mn, float* pbar, float4* mbar) {
     pdl_wait();
     const Pair P = as_pair(A);
     const int nx = (A.X + kTileX - 1) / kTileX, ny = (A.Y + kTileY - 1) / kTileY;
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(256) adj_update_kernel(AdjPair A, const float*
     float np[3], nb[3];  // phi and pbar of the next slice, loaded while this one's gathers are in flight
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        np[c] = __ldg(phi + c * A.NT + i);
+        np[c] = chain_load(phi + c * A.NT + i);
         nb[c] = pbar[c * A.NT + i];
     }
     for (int z = z0; z < z1; ++z, i += act ? XY : 0) {
@@ -222,27 +222,27 @@ __global__ void __launch_bounds__(256) adj_update_kernel(AdjPair A, const float*
         float acc[3], pb[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const float* __restrict__ F = mn + c * A.NT;
+            const float* F = mn + c * A.NT;
             f[c][1] = f[c][0];
             f[c][3] = f[c][2];
             f[c][5] = f[c][4];
             f[c][7] = f[c][6];
-            f[c][0] = __ldg(F + b + 1 + Xp + XY);
-            f[c][2] = __ldg(F + b + 1 + XY);
-            f[c][4] = __ldg(F + b + Xp + XY);
-            f[c][6] = __ldg(F + b + XY);
+            f[c][0] = chain_load(F + b + 1 + Xp + XY);
+            f[c][2] = chain_load(F + b + 1 + XY);
+            f[c][4] = chain_load(F + b + Xp + XY);
+            f[c][6] = chain_load(F + b + XY);
             if (!on) {
-                f[c][1] = __ldg(F + b + 1 + Xp);
-                f[c][3] = __ldg(F + b + 1);
-                f[c][5] = __ldg(F + b + Xp);
-                f[c][7] = __ldg(F + b);
+                f[c][1] = chain_load(F + b + 1 + Xp);
+                f[c][3] = chain_load(F + b + 1);
+                f[c][5] = chain_load(F + b + Xp);
+                f[c][7] = chain_load(F + b);
             }
             acc[c] = pb[c] = nb[c];
         }
         if (act && z + 1 < z1)
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                np[c] = __ldg(phi + c * A.NT + i + XY);
+                np[c] = chain_load(phi + c * A.NT + i + XY);
                 nb[c] = pbar[c * A.NT + i + XY];
             }
 #pragma unroll
@@ -303,8 +303,8 @@ __device__ __forceinline__ void dot2(float a, float b, float& s, float& c) {
 // summed in compensated FP32 per thread and in FP64 beyond, as the FP64 pipe of this GPU takes
 // 16 cycles per warp and operation (78 us with six FP64 operations and six conversions a voxel).
 __global__ void __launch_bounds__(256) adj_grad_kernel(AdjPair A, const float* __restrict__ S, const float* __restrict__ T,
-                                                       const float* __restrict__ phi, float lambda,
-                                                       const float* __restrict__ gbar, float* pbar, double* lbar) {
+                                                       const float* phi, float lambda,
+                                                       const float* gbar, float* pbar, double* lbar) {
     pdl_wait();
     __shared__ double red[32];
     const Pair P = as_pair(A);
@@ -319,13 +319,13 @@ __global__ void __launch_bounds__(256) adj_grad_kernel(AdjPair A, const float* _
         float p[3], g[3], pz[3], gz[3];  // phi and gbar here, and their terms across the face below
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            p[c] = __ldg(phi + c * A.NT + i);
-            g[c] = __ldg(gbar + c * A.NT + i);
+            p[c] = chain_load(phi + c * A.NT + i);
+            g[c] = chain_load(gbar + c * A.NT + i);
             pz[c] = gz[c] = 0.f;
             if (z0 > 0) {
-                pz[c] = __ldg(phi + c * A.NT + i - XY) - p[c];
+                pz[c] = chain_load(phi + c * A.NT + i - XY) - p[c];
                 if (c == 2) pz[c] += 1.f;
-                gz[c] = __ldg(gbar + c * A.NT + i - XY) - g[c];
+                gz[c] = chain_load(gbar + c * A.NT + i - XY) - g[c];
             }
         }
         for (int z = z0; z < z1; ++z, i += XY) {
@@ -341,8 +341,8 @@ __global__ void __launch_bounds__(256) adj_grad_kernel(AdjPair A, const float* _
             for (int c = 0; c < 3; ++c) {
 #pragma unroll
                 for (int k = 0; k < 5; ++k) {
-                    pn[c][k] = __ldg(phi + c * A.NT + i + off[k]);
-                    gn[c][k] = __ldg(gbar + c * A.NT + i + off[k]);
+                    pn[c][k] = chain_load(phi + c * A.NT + i + off[k]);
+                    gn[c][k] = chain_load(gbar + c * A.NT + i + off[k]);
                 }
                 old[c] = pbar[c * A.NT + i];
             }
@@ -607,7 +607,7 @@ extern "C" int fr_sobolev_loss_grad(const float* d_T, const float* d_S, const in
         a.m_n = to.m;
         a.ntiles_s = cuts[1].count;
         a.depth_s = cuts[1].depth;
-        ok(launch_sob_kernel(0, a, cuts[0].count, 0, s, true));
+        ok(launch_sob_kernel(0, a, cuts[0].count, 0, s, k > 0));  // the first one behind adj_pack_kernel (pdl_wait)
         a.mid = gbar;  // free until the reverse iteration's smoothing
         ok(launch_sob_kernel(1, a, cuts[1].count, kUnrolled | (tall ? 2 : 0) | (split ? kSplit : 0), s, true));
         ok(launch_sob_kernel(2, a, cuts[2].count, kUnrolled, s, true));

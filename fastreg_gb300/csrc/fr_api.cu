@@ -991,11 +991,12 @@ int autotune(fr_handle* h, cudaStream_t s) {
     // 0), where the velocity or momentum that the update kernels gather is no longer zero
     // and the gathers leave the grid points; shapes timed at the identity state chose a
     // sobolev update 7% slower than the best
-    FR_CUDA(h, cudaMemsetAsync(h->stop, 0, sizeof(int) * h->npairs, s));
     frg::IoArgs io = io_args(h);
     io.keep_state = 0;
     frg::pack_init_kernel<<<pack_grid(h), 256, 0, s>>>(io);
     FR_LAUNCHED(h);
+    // cleared here, between the packing and the first iteration's programmatic launch (pdl_wait)
+    FR_CUDA(h, cudaMemsetAsync(h->stop, 0, sizeof(int) * h->npairs, s));
     const std::vector<float> ts = t_schedule(h->P);
     const int warm = std::min(kTuneWarmIters, (h->trace_cap - 1) / 2 * 2);  // the trace holds iteration warm + 1
     for (int it = 1; it <= warm; ++it) {

@@ -63,6 +63,15 @@ __device__ __forceinline__ long long user_lin(const Pair& P, int x, int y, int z
     return (long long)x + (long long)P.X * ((long long)y + (long long)P.Y * z);
 }
 
+// Reads a field that a kernel of the same chain of programmatic launches writes (pdl_wait): an ordinary
+// load.  __ldg and const __restrict__ kernel parameters make non-coherent loads, which are defined only
+// for memory that nothing writes as long as the kernel is resident, and which the compiler may
+// move above the wait.
+template <typename T>
+__device__ __forceinline__ T chain_load(const T* p) {
+    return *p;
+}
+
 // lerp(v0, v1, t) = fma(t, v0, fma(-t, v1, v1))
 __device__ __forceinline__ float lerpf_(float v0, float v1, float t) { return fmaf(t, v0, fmaf(-t, v1, v1)); }
 
@@ -203,9 +212,10 @@ __device__ __forceinline__ float tri_unchecked32(const float* __restrict__ F, in
 }
 
 // The three components of a vector field (planes F0, F1, F2) at one cell with
-// tri_checked32's addressing; components 0 and 1 interpolated as one packed pair.
-__device__ __forceinline__ void tri_checked32_3(const float* __restrict__ F0, const float* __restrict__ F1,
-                                                const float* __restrict__ F2, int X, int Y, int Z, int Xp, int XYp,
+// tri_checked32's addressing; components 0 and 1 interpolated as one packed pair.  The field is one that
+// the chain of launches writes (chain_load).
+__device__ __forceinline__ void tri_checked32_3(const float* F0, const float* F1,
+                                                const float* F2, int X, int Y, int Z, int Xp, int XYp,
                                                 const Cell32& cl, float out[3]) {
     const int b = cl.base;
     const bool ox = cl.gx + 1 < X, oy = cl.gy + 1 < Y, oz = cl.gz + 1 < Z;
@@ -214,27 +224,27 @@ __device__ __forceinline__ void tri_checked32_3(const float* __restrict__ F0, co
     if (ox && oy && oz) {
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            f[k][0] = __ldg(F[k] + b + 1 + Xp + XYp);
-            f[k][1] = __ldg(F[k] + b + 1 + Xp);
-            f[k][2] = __ldg(F[k] + b + 1 + XYp);
-            f[k][3] = __ldg(F[k] + b + 1);
-            f[k][4] = __ldg(F[k] + b + Xp + XYp);
-            f[k][5] = __ldg(F[k] + b + Xp);
-            f[k][6] = __ldg(F[k] + b + XYp);
-            f[k][7] = __ldg(F[k] + b);
+            f[k][0] = chain_load(F[k] + b + 1 + Xp + XYp);
+            f[k][1] = chain_load(F[k] + b + 1 + Xp);
+            f[k][2] = chain_load(F[k] + b + 1 + XYp);
+            f[k][3] = chain_load(F[k] + b + 1);
+            f[k][4] = chain_load(F[k] + b + Xp + XYp);
+            f[k][5] = chain_load(F[k] + b + Xp);
+            f[k][6] = chain_load(F[k] + b + XYp);
+            f[k][7] = chain_load(F[k] + b);
         }
     } else {
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const float f0 = __ldg(F[k]);
-            f[k][0] = (ox && oy && oz) ? __ldg(F[k] + b + 1 + Xp + XYp) : f0;
-            f[k][1] = (ox && oy) ? __ldg(F[k] + b + 1 + Xp) : f0;
-            f[k][2] = (ox && oz) ? __ldg(F[k] + b + 1 + XYp) : f0;
-            f[k][3] = ox ? __ldg(F[k] + b + 1) : f0;
-            f[k][4] = (oy && oz) ? __ldg(F[k] + b + Xp + XYp) : f0;
-            f[k][5] = oy ? __ldg(F[k] + b + Xp) : f0;
-            f[k][6] = oz ? __ldg(F[k] + b + XYp) : f0;
-            f[k][7] = __ldg(F[k] + b);
+            const float f0 = chain_load(F[k]);
+            f[k][0] = (ox && oy && oz) ? chain_load(F[k] + b + 1 + Xp + XYp) : f0;
+            f[k][1] = (ox && oy) ? chain_load(F[k] + b + 1 + Xp) : f0;
+            f[k][2] = (ox && oz) ? chain_load(F[k] + b + 1 + XYp) : f0;
+            f[k][3] = ox ? chain_load(F[k] + b + 1) : f0;
+            f[k][4] = (oy && oz) ? chain_load(F[k] + b + Xp + XYp) : f0;
+            f[k][5] = oy ? chain_load(F[k] + b + Xp) : f0;
+            f[k][6] = oz ? chain_load(F[k] + b + XYp) : f0;
+            f[k][7] = chain_load(F[k] + b);
         }
     }
     trilerp3(f, cl.a, cl.b, cl.c, out);
@@ -262,8 +272,9 @@ __device__ __forceinline__ float4 lerp4_(float4 v0, float4 v1, float t) {
     return make_float4(lerpf_(v0.x, v1.x, t), lerpf_(v0.y, v1.y, t), lerpf_(v0.z, v1.z, t), lerpf_(v0.w, v1.w, t));
 }
 
-// tri_unchecked32 on an interleaved 4-channel field (one 16-byte load per corner)
-__device__ __forceinline__ float4 tri_unchecked32_f4(const float4* __restrict__ F, int X, int XY, int N,
+// tri_unchecked32 on an interleaved 4-channel field (one 16-byte load per corner) that the
+// chain of launches writes (chain_load)
+__device__ __forceinline__ float4 tri_unchecked32_f4(const float4* F, int X, int XY, int N,
                                                      const Cell32& cl) {
     const int b = cl.base;
     int o111 = b + 1 + X + XY, o110 = b + 1 + X, o101 = b + 1 + XY, o100 = b + 1;
@@ -278,8 +289,8 @@ __device__ __forceinline__ float4 tri_unchecked32_f4(const float4* __restrict__ 
         o010 = min(o010, last);
         o001 = min(o001, last);
     }
-    const float4 f111 = __ldg(F + o111), f110 = __ldg(F + o110), f101 = __ldg(F + o101), f100 = __ldg(F + o100);
-    const float4 f011 = __ldg(F + o011), f010 = __ldg(F + o010), f001 = __ldg(F + o001), f000 = __ldg(F + b);
+    const float4 f111 = chain_load(F + o111), f110 = chain_load(F + o110), f101 = chain_load(F + o101), f100 = chain_load(F + o100);
+    const float4 f011 = chain_load(F + o011), f010 = chain_load(F + o010), f001 = chain_load(F + o001), f000 = chain_load(F + b);
     // channels (x, y) and (z, w) as packed pairs: per channel the lerp4_ arithmetic
     auto lo = [](float4 v) { return make_float2(v.x, v.y); };
     auto hi = [](float4 v) { return make_float2(v.z, v.w); };
@@ -295,6 +306,12 @@ __device__ __forceinline__ float4 tri_unchecked32_f4(const float4* __restrict__ 
 // leave the trigger to their blocks' exits: it saves part of the launch latency between two
 // kernels (64^3: 22.1 -> 21.5 us per iteration), while triggering early places blocks that hold
 // SM room and wait (27.6 us).
+//
+// A kernel launched this way may be resident before the one ahead has completed, so what the kernels of
+// a chain write is read with chain_load, by asynchronous copies or by plain loads, and every thread
+// waits before its first access.  __ldg is for what stays as it is for the whole chain: the
+// images, the labels and the pair table.  The first kernel behind the one that packs the images
+// is therefore an ordinary launch, or has a copy or a clearing between the two.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // The t-th tile of a kernel's table of 32 x rows x depth tiles and its pair; false if the pair has

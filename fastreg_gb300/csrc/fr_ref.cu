@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(256) ref_laplacian_kernel(RefIterArgs a) {
         const int zs0 = max(tl.w, 1), zs1 = min(tl.w + a.depth_l, Z - 1);
         if (zs0 >= zs1 || tl.y + kTileX <= 1 || tl.z + kTileY <= 1 || tl.y >= X - 1 || tl.z >= Y - 1) continue;
         const long long NT = a.NT;
-        const float* __restrict__ Qg[3] = {a.psi + P.off, a.psi + NT + P.off, a.psi + 2 * NT + P.off};
+        const float* Qg[3] = {a.psi + P.off, a.psi + NT + P.off, a.psi + 2 * NT + P.off};
         const float* __restrict__ Tg = a.T + P.off;
         float4* LT = a.LT + P.off;
         const int x = tl.y + tx, y = tl.z + ty;
@@ -308,8 +308,8 @@ __global__ void __launch_bounds__(256) ref_laplacian_tma_kernel(RefIterArgs a) {
 template <int VC, int QC, int QR, int QS, int RW>
 __device__ __forceinline__ void pass_a_voxel(const RefIterArgs& a, const Pair& P, int X, int Y, int Z, int N, int Xp,
                                              int XYp, int y, int z, int i, bool dv_xy, const float* const vb[5],
-                                             const float* const qb[3], const float4* __restrict__ LT,
-                                             const float* __restrict__ Tg, const float* __restrict__ const* Vg,
+                                             const float* const qb[3], const float4* LT,
+                                             const float* __restrict__ Tg, const float* const* Vg,
                                              float* rho_n,
                                              float* const* Vn, float* const* Qn) {
     auto V = [&](int k, int c) { return vb[k] + c * VC; };
@@ -390,7 +390,7 @@ __device__ __forceinline__ void pass_a_voxel(const RefIterArgs& a, const Pair& P
         for (int c = 0; c < 3; ++c) {
             const float xx = (vx < 0.f) ? (V(2, c)[2] - 2.f * vxp[c]) + vc[c]
                                         : (vc[c] - 2.f * vxm[c]) + V(2, c)[-2];
-            const float vyp2 = y_edge ? __ldg(Vg[c] + i + 2 * Xp) : V(2, c)[2 * RW];
+            const float vyp2 = y_edge ? chain_load(Vg[c] + i + 2 * Xp) : V(2, c)[2 * RW];
             const float yy = (vy < 0.f) ? (vyp2 - 2.f * vym[c]) + vc[c]
                                         : (vc[c] - 2.f * vym[c]) + V(2, c)[-2 * RW];
             const float zz = (vz < 0.f) ? (V(4, c)[0] - 2.f * vzm[c]) + vc[c]
@@ -444,12 +444,12 @@ __global__ void __launch_bounds__(256, 3) ref_pass_a_kernel(RefIterArgs a) {
         const int zs0 = max(tl.w, 1), zs1 = min(tl.w + a.depth_a, Z - 1);
         if (zs0 >= zs1 || tl.y + kTileX <= 1 || tl.z + kTileY <= 1 || tl.y >= X - 1 || tl.z >= Y - 1) continue;
         const long long NT = a.NT;
-        const float* __restrict__ Vg[3] = {a.v + P.off, a.v + NT + P.off, a.v + 2 * NT + P.off};
-        const float* __restrict__ Qg[3] = {a.pinv + P.off, a.pinv + NT + P.off, a.pinv + 2 * NT + P.off};
-        const float* __restrict__ Rg = a.rho + P.off;
+        const float* Vg[3] = {a.v + P.off, a.v + NT + P.off, a.v + 2 * NT + P.off};
+        const float* Qg[3] = {a.pinv + P.off, a.pinv + NT + P.off, a.pinv + 2 * NT + P.off};
+        const float* Rg = a.rho + P.off;
         const float* __restrict__ Sg = a.S + P.off;
         const float* __restrict__ Tg = a.T + P.off;
-        const float4* __restrict__ LT = a.LT + P.off;
+        const float4* LT = a.LT + P.off;
         float* rho_n = a.rho_n + P.off;
         float* Vn[3] = {a.v_n + P.off, a.v_n + NT + P.off, a.v_n + 2 * NT + P.off};
         float* Qn[3] = {a.pinv_n + P.off, a.pinv_n + NT + P.off, a.pinv_n + 2 * NT + P.off};
@@ -598,9 +598,9 @@ __global__ void __launch_bounds__(256, 3) ref_pass_a_tma_kernel(RefIterArgs a) {
         const int zs0 = max(tl.w, 1), zs1 = min(tl.w + a.depth_a, Z - 1);
         if (zs0 >= zs1 || tl.y + kTileX <= 1 || tl.z + kTileY <= 1 || tl.y >= X - 1 || tl.z >= Y - 1) continue;
         const long long NT = a.NT;
-        const float* __restrict__ Vg[3] = {a.v + P.off, a.v + NT + P.off, a.v + 2 * NT + P.off};
+        const float* Vg[3] = {a.v + P.off, a.v + NT + P.off, a.v + 2 * NT + P.off};
         const float* __restrict__ Tg = a.T + P.off;
-        const float4* __restrict__ LT = a.LT + P.off;
+        const float4* LT = a.LT + P.off;
         float* rho_n = a.rho_n + P.off;
         float* Vn[3] = {a.v_n + P.off, a.v_n + NT + P.off, a.v_n + 2 * NT + P.off};
         float* Qn[3] = {a.pinv_n + P.off, a.pinv_n + NT + P.off, a.pinv_n + 2 * NT + P.off};
@@ -701,7 +701,7 @@ __global__ void __launch_bounds__(kPassBThreads, 9) ref_pass_b_kernel(RefIterArg
             const int X = P.X, Y = P.Y, Z = P.Z, Xp = P.Xp, XYp = P.Xp * P.Y;
             const long long NT = a.NT;
             // the velocity pass A just wrote
-            const float* __restrict__ V[3] = {a.v_n + P.off, a.v_n + NT + P.off, a.v_n + 2 * NT + P.off};
+            const float* V[3] = {a.v_n + P.off, a.v_n + NT + P.off, a.v_n + 2 * NT + P.off};
             float* Q[3] = {a.psi + P.off, a.psi + NT + P.off, a.psi + 2 * NT + P.off};
             const int z0 = max(tl.w, 1), z1 = min(tl.w + a.depth_b, P.Z - 1);
             int i = x + Xp * y + XYp * z0;

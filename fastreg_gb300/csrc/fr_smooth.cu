@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kSmoothThreads) sob_smooth3_kernel(SobIterArgs
         const int x0 = tl.y, y0 = tl.z, zt0 = tl.w, zt1 = min(tl.w + a.depth_s, Z);
         const int nsl = (zt1 - zt0) + 2 * RZ;
         const bool edge = x0 == 0 || x0 + kTileX - 1 + R > X - 1 || y0 == 0 || y0 + TY - 1 + R > Y - 1;
-        const float* __restrict__ gc = a.g + c * a.NT + P.off;
+        const float* gc = a.g + c * a.NT + P.off;
         const CUtensorMap* mg = a.tmaps + (long long)tl.x * TM_COUNT + (TY == sob_smooth_tile_y(R, false) ? TM_SOB_G : TM_SOB_G_TALL);
 
         // cp.async: chunk f = lane + 32 j of the box is (row f / (WS / 4), chunk f % (WS / 4));
@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(256) sob_smooth_z_kernel(SobIterArgs a) {
         if (x >= X || y >= Y) continue;
         const int zt0 = tl.w, zt1 = min(zt0 + a.depth_z, Z), nsl = zt1 - zt0 + 2 * R;
         const long long at = c * a.NT + P.off + x + P.Xp * y;
-        const float* __restrict__ g = a.mid + at;
+        const float* g = a.mid + at;
         const float* m = (MODE == kOutOfPlace ? a.m : a.m_n) + at;
         float* mn = a.m_n + at;
         float part[R > 0 ? 2 * R : 1];
@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(256) sob_smooth_z_kernel(SobIterArgs a) {
             for (int u = 0; u < U; ++u) {
                 const int k = k0 + u, z = zt0 - R + k;
                 const bool in = k < nsl && (!ADJ || (z >= 0 && z < Z));
-                v[u] = in ? __ldg(g + XY * min(max(z, 0), Z - 1)) : 0.f;
+                v[u] = in ? chain_load(g + XY * min(max(z, 0), Z - 1)) : 0.f;
                 mo[u] = !ADJ && k >= 2 * R && k < nsl ? m[XY * (z - R)] : 0.f;
             }
 #pragma unroll

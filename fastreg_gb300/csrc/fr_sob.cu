@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(256, 4) sob_pass_b_kernel(SobIterArgs a) {
             const float* phi[3] = {phi_n[0], phi_n[1], phi_n[2]};
             if (UNROLLED)
                 for (int c = 0; c < 3; ++c) phi[c] = a.phi + c * NT + P.off;
-            const float* __restrict__ mc[3] = {a.m_n + P.off, a.m_n + NT + P.off, a.m_n + 2 * NT + P.off};
+            const float* mc[3] = {a.m_n + P.off, a.m_n + NT + P.off, a.m_n + 2 * NT + P.off};
             const int z1 = min(tl.w + a.depth_b, P.Z);
             int i = x + X * y + XY * tl.w;
             // phi of the next slice is loaded while this slice's gathers are in flight
@@ -309,20 +309,20 @@ __global__ void __launch_bounds__(256, 4) sob_pass_b_kernel(SobIterArgs a) {
                     f[c][3] = f[c][2];
                     f[c][5] = f[c][4];
                     f[c][7] = f[c][6];
-                    const float* __restrict__ F = mc[c];
-                    f[c][0] = __ldg(F + b + 1 + X + XY);
-                    f[c][2] = __ldg(F + b + 1 + XY);
-                    f[c][4] = __ldg(F + b + X + XY);
-                    f[c][6] = __ldg(F + b + XY);
+                    const float* F = mc[c];
+                    f[c][0] = chain_load(F + b + 1 + X + XY);
+                    f[c][2] = chain_load(F + b + 1 + XY);
+                    f[c][4] = chain_load(F + b + X + XY);
+                    f[c][6] = chain_load(F + b + XY);
                 }
                 if (b != above)
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
-                        const float* __restrict__ F = mc[c];
-                        f[c][1] = __ldg(F + b + 1 + X);
-                        f[c][3] = __ldg(F + b + 1);
-                        f[c][5] = __ldg(F + b + X);
-                        f[c][7] = __ldg(F + b);
+                        const float* F = mc[c];
+                        f[c][1] = chain_load(F + b + 1 + X);
+                        f[c][3] = chain_load(F + b + 1);
+                        f[c][5] = chain_load(F + b + X);
+                        f[c][7] = chain_load(F + b);
                     }
                 above = b + XY;
                 trilerp3(f, s.a, s.b, s.c, u);
