@@ -770,8 +770,10 @@ int launch_iter(fr_handle* h, int iter, float t, cudaStream_t s, cudaEvent_t* ev
 }
 
 // An iteration that the caller steps may have been run before: its record starts from 0 again
-// (a registration's are cleared when it begins).
+// (a registration's are cleared when it begins).  With a convergence test the record is written whole
+// by the update kernel (record_and_test), and a pair that has converged keeps the one of its last iteration.
 int clear_trace(fr_handle* h, int iter, cudaStream_t s) {
+    if (h->P.max_update_norm >= 0.f) return FR_OK;
     FR_CUDA(h, cudaMemsetAsync(h->trace + (size_t)(iter - 1) * h->npairs, 0, sizeof(unsigned long long) * h->npairs, s));
     return FR_OK;
 }
@@ -1118,10 +1120,11 @@ int begin(fr_handle* h, const fr_pair* pairs, int n, cudaStream_t s) {
         rc = autotune(h, s);  // leaves the state to the initialisation below
         if (rc != FR_OK) return rc;
     }
-    FR_CUDA(h, cudaMemsetAsync(h->stop, 0, results_bytes(h), s));
     frg::IoArgs a = io_args(h);
     frg::pack_init_kernel<<<pack_grid(h), 256, 0, s>>>(a);
     FR_LAUNCHED(h);
+    // the records; cleared here, between the packing and the first iteration's programmatic launch (pdl_wait)
+    FR_CUDA(h, cudaMemsetAsync(h->stop, 0, results_bytes(h), s));
     h->have_state = true;
     h->finished = false;
     h->stats_ready = false;

@@ -240,3 +240,29 @@ def test_smoothing_in_two_launches(cuda, dims_list, width):
         assert_bitexact(fr.get_field(N.FR_FIELD_PSI, pair=k).cpu().numpy(), o["phi"], f"pair {k} phi (width {width})")
         assert_bitexact(fr.get_field(N.FR_FIELD_V, pair=k).cpu().numpy(), o["m"], f"pair {k} momentum (width {width})")
     fr.close()
+
+
+@pytest.mark.parametrize("solver", ["reference", "sobolev"])
+def test_converged_pairs_keep_their_records(cuda, solver):
+    """With MAX_UPDATE_NORM >= 0, iterations that are stepped or timed again after a pair has converged skip the
+    pair; its trace, and the norm and voxel of its last iteration, stay as they were."""
+    import ctypes as C
+    dims_list = [(24, 20, 18), (20, 18, 16), (16, 24, 12)]
+    pairs_np = [images(d, 1300 + k) for k, d in enumerate(dims_list)]
+    fr = FastReg(Params(volume_dims=dims_list[0], no_labels=4, max_iter=40, alpha=0.02, solver=solver, step=0.5,
+                        damping=0.9, max_update_norm=1e3))  # every pair stops at its first iteration
+    fr.register_batch([tuple(_to(cuda, p[k]) for k in ("T", "labT", "S", "labS")) for p in pairs_np])
+
+    def records():
+        st = [fr.stats(pair=k) for k in range(3)]
+        return [(s.iterations, s.converged, s.last_max_update_norm, s.last_max_update_voxel,
+                 *(list(a) for a in fr.trace(pair=k))) for k, s in enumerate(st)]
+
+    before = records()
+    assert all(r[:2] == (1, True) and r[2] > 0 for r in before), before
+    fr.step(1, 0.02)
+    assert records() == before
+    ms, nk = (C.c_float * 8)(), C.c_int()
+    N.check(fr.lib.fr_time_kernels(fr.h, 3, ms, C.byref(nk), None), fr.h, "fr_time_kernels")
+    assert records() == before
+    fr.close()

@@ -67,6 +67,7 @@ def test_first_kernel_behind_a_packing_kernel():
     adj = (CSRC / "fr_adjoint.cu").read_text()
     assert re.search(r"launch_sob_kernel\(0, a, cuts\[0\]\.count, 0, s, k > 0\)", adj)
     api = (CSRC / "fr_api.cu").read_text()
-    tune = api[api.index("int autotune(fr_handle* h"):]
-    between = tune[tune.index("pack_init_kernel<<<"):tune.index("launch_iter(")]
-    assert "cudaMemsetAsync" in between
+    for fn, end in (("int autotune(fr_handle* h", "launch_iter("), ("int begin(fr_handle* h", "\n}\n")):
+        body = api[api.index(fn):]
+        between = body[body.index("pack_init_kernel<<<"):]
+        assert "cudaMemsetAsync" in between[:between.index(end)], fn
