@@ -286,12 +286,39 @@ __global__ void __launch_bounds__(256) adj_momentum_kernel(AdjPair A, float damp
 }
 
 // s + c += a * b with the product and the sum exact to about twice the FP32 precision (the
-// compensated dot product Dot2 of Ogita, Rump and Oishi, 2005)
-__device__ __forceinline__ void dot2(float a, float b, float& s, float& c) {
-    const float p = a * b, e = fmaf(a, b, -p);
+// compensated dot product Dot2 of Ogita, Rump and Oishi, 2005).  Its error terms are exact only for products
+// in kDotLeast .. kDotMost (and for a zero factor): below, the product's last bits, 47 places
+// under its first, fall under the smallest FP32 number, 2^-149; above, a few dozen sums could overflow.
+// False for any other product, and for a NaN.
+constexpr float kDotLeast = 0x1p-100f, kDotMost = 0x1p100f;
+__device__ __forceinline__ bool dot2(float a, float b, float& s, float& c) {
+    const float p = a * b, e = fmaf(a, b, -p), size = fabsf(p);
     const float t = s + p, u = t - s;
     c += e + ((s - (t - u)) + (p - u));
     s = t;
+    return ((size >= kDotLeast) & (size <= kDotMost)) | ((p == 0.f) & ((a == 0.f) | (b == 0.f)));
+}
+
+// The sum of gbar . lap(phi - x) over one column of adj_grad_kernel in FP64, terms and order as there.
+__device__ __forceinline__ double lambda_sum_f64(const AdjPair& A, const float* phi, const float* gbar, int x, int y, int z0,
+                                              int z1) {
+    const bool ok[6] = {x > 0, x < A.X - 1, y > 0, y < A.Y - 1, true, true};
+    const int off[6] = {-1, 1, -A.Xp, A.Xp, -A.XYp, A.XYp};
+    double sum = 0.0;
+    int i = x + A.Xp * y + A.XYp * z0;
+    for (int z = z0; z < z1; ++z, i += A.XYp)
+        for (int c = 0; c < 3; ++c) {
+            const float* P = phi + c * A.NT + i;
+            const float pc = chain_load(P);
+            float l = 0.f;
+            for (int k = 0; k < 6; ++k) {
+                if (k < 4 ? !ok[k] : k == 4 ? z == 0 : z == A.Z - 1) continue;
+                const float d = pc - chain_load(P + off[k]);
+                l += k / 2 == c ? d + ((k & 1) ? 1.f : -1.f) : d;
+            }
+            sum = fma((double)chain_load(gbar + c * A.NT + i), (double)l, sum);
+        }
+    return sum;
 }
 
 // g = (S(phi) - T) dS(phi) + lambda lap(phi - x): pbar += lambda lap^T(gbar) + (gbar . dS) dS + r H
@@ -302,7 +329,7 @@ __device__ __forceinline__ void dot2(float a, float b, float& s, float& c) {
 // the 128^3 pair when each neighbour was loaded where it was used, 46 us now); lambda_bar is
 // summed in compensated FP32 per thread and in FP64 beyond, as the FP64 pipe of this GPU takes
 // 16 cycles per warp and operation (78 us with six FP64 operations and six conversions a voxel).
-__global__ void __launch_bounds__(256) adj_grad_kernel(AdjPair A, const float* __restrict__ S, const float* __restrict__ T,
+__global__ void __launch_bounds__(256, 5) adj_grad_kernel(AdjPair A, const float* __restrict__ S, const float* __restrict__ T,
                                                        const float* phi, float lambda,
                                                        const float* gbar, float* pbar, double* lbar) {
     pdl_wait();
@@ -312,10 +339,12 @@ __global__ void __launch_bounds__(256) adj_grad_kernel(AdjPair A, const float* _
     const int x = (blockIdx.x % nx) * kTileX + (threadIdx.x & 31), y = (blockIdx.x / nx % ny) * kTileY + (threadIdx.x >> 5);
     const int z0 = (int)(blockIdx.x / (nx * ny)) * A.depth, z1 = min(z0 + A.depth, A.Z);
     const int Xp = A.Xp, XY = A.XYp;
-    float ls = 0.f, lc = 0.f;
+    double lsum = 0.0;
     if (x < A.X && y < A.Y) {
         const bool xl = x > 0, xr = x < A.X - 1, yl = y > 0, yr = y < A.Y - 1;
         int i = x + Xp * y + XY * z0;
+        float ls = 0.f, lc = 0.f;
+        bool held = true;  // every product of the column was in dot2's range
         float p[3], g[3], pz[3], gz[3];  // phi and gbar here, and their terms across the face below
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -364,7 +393,7 @@ __global__ void __launch_bounds__(256) adj_grad_kernel(AdjPair A, const float* _
                 gz[c] = up;
                 p[c] = pn[c][4];
                 g[c] = gn[c][4];
-                dot2(gc, l, ls, lc);
+                held &= dot2(gc, l, ls, lc);
             }
             float d[3], W, H[3];
             tri_grad(f, s, d, &W, H);
@@ -374,8 +403,9 @@ __global__ void __launch_bounds__(256) adj_grad_kernel(AdjPair A, const float* _
 #pragma unroll
             for (int k = 0; k < 3; ++k) pbar[k * A.NT + i] = old[k] + (add[k] + (gd * d[k] + r * h[k]));
         }
+        lsum = held ? (double)ls + (double)lc : lambda_sum_f64(A, phi, gbar, x, y, z0, z1);
     }
-    const double lb = block_sum_f64((double)ls + (double)lc, red);
+    const double lb = block_sum_f64(lsum, red);
     if (threadIdx.x == 0) atomicAdd(lbar, lb);
 }
 

@@ -277,3 +277,24 @@ def test_adjoint_at_128cube_50_iterations(cuda):
     assert min(rec["fd_direction_64_voxels"].values()) <= 1e-4, rec["fd_direction_64_voxels"]
     for k, v in rec["fd_voxels"].items():
         assert min(v.values()) <= 1e-4, (k, v)
+
+
+@pytest.mark.parametrize("scale,step,width,prec,tol", [(1e20, 0.5, 7, 64, 1e-5), (1e-10, 2.0 ** -118, 1, 32, 3e-4)])
+def test_lambda_gradient_outside_the_fp32_range(cuda, scale, step, width, prec, tol):
+    """dJ/dlambda sums products of two FP32 values in FP64's range: where they overflow FP32 (1e40, a
+    huge momentum) and where they vanish in it (1e-47, tiny displacements and a tiny STEP).  Within 100
+    roundings of 6e-8: of the sum in the first case, of its terms in the second, whose magnitudes add
+    up to 38 times the sum there; the displacements of the second are a few units in the last place of
+    some positions, so its oracle is the FP32 one (which sums in FP64 too)."""
+    import torch
+    dims = (20, 18, 16)
+    d = images(dims, 77)
+    P = Params(volume_dims=dims, solver="sobolev", smooth_sigma=1.5, smooth_width=width, damping=1.0, step=step)
+    v0 = (smooth_noise(rng(3), (3,) + dims[::-1], 1.0).astype(np.float64) if scale > 1 else
+          rng(3).uniform(0.5, 1.0, (3,) + dims[::-1])) * scale
+    v0 = v0.astype(np.float32)
+    T, S = (torch.from_numpy(d[k]).to(cuda) for k in ("T", "S"))
+    J, _, gl = _loss_grad(T, S, torch.from_numpy(v0).to(cuda), 0.2, 2, 2, P)
+    J_o, _, gl_o = O.sob_loss_grad(P, d["T"], d["S"], v0, 0.2, 2, True, prec=prec)
+    assert abs(J - J_o) <= 1e-5 * abs(J_o)
+    assert np.isfinite(gl) and abs(gl - gl_o) <= tol * abs(gl_o), (gl, gl_o)
