@@ -1732,19 +1732,20 @@ int fr_interpolate_field(const float* d_field, const float* d_pos, const int dim
     if (rc != FR_OK) return rc;
     static std::atomic<int> slots[64];
     const int X = dims[0], Y = dims[1], Z = dims[2];
-    const long long cols = ((long long)X * Y + frg::kFieldThreads - 1) / frg::kFieldThreads;
+    auto blocks_of = [&](long long d) { return ((long long)X * Y * ((Z + d - 1) / d) + frg::kFieldThreads - 1) / frg::kFieldThreads; };
     // Columns of 16 slices where they make two and a half waves of blocks or more (64.7 us on 182x218x182;
     // 8 take 67.2 us, 24 67.6 us).  Below that the waves count: a wave of d slices takes about d + 1/2, one that
-    // fills a share f of the GPU 0.44 + 0.56 f of it, and the depth that costs least is within 5% of the
-    // best one measured on eight sizes from 45x54x45 to 160x192x160 (137x108x173: 18 slices, one
-    // wave, 26.1 us; 16 slices, a second wave of 15 blocks, 31.5 us).
+    // fills a share f of the GPU 0.44 + 0.56 f of it (both figures fitted to the times of eight sizes).
+    // Against every depth up to 24, on 17 sizes from 33^3 to 193x229x193: within 7% of the best below
+    // two and a half waves, within 9% from there to three (176x208x176: 78.1 us, 71.7 us at 21 slices), within
+    // 2% above (137x108x173 has 18 slices and one wave; 16 and a second wave of 15 blocks are 15% slower).
     const long long slots_all = std::max(resident_blocks((const void*)frg::interpolate_field_kernel, slots,
                                                          frg::kFieldThreads), 1);
-    long long depth = 16;
-    if (2 * cols * Z < 5 * 16 * slots_all) {
+    int depth = 16;
+    if (2 * blocks_of(16) < 5 * slots_all) {
         double least = 1e300;
         for (int d = 1; d <= 24; ++d) {
-            const long long blocks = cols * ((Z + d - 1) / d), rest = blocks % slots_all;
+            const long long blocks = blocks_of(d), rest = blocks % slots_all;
             const double cost = (d + 0.5) * (blocks / slots_all + (rest ? 0.44 + 0.56 * rest / slots_all : 0.0));
             if (cost < least) {
                 least = cost;
@@ -1752,9 +1753,8 @@ int fr_interpolate_field(const float* d_field, const float* d_pos, const int dim
             }
         }
     }
-    depth = std::max(depth, (Z + 65534LL) / 65535);  // the grid's second extent is 16 bits
-    frg::interpolate_field_kernel<<<dim3((unsigned)cols, (unsigned)((Z + depth - 1) / depth)), frg::kFieldThreads, 0,
-                                    (cudaStream_t)stream>>>(d_field, d_pos, d_out, X, Y, Z, (int)depth);
+    frg::interpolate_field_kernel<<<(unsigned)blocks_of(depth), frg::kFieldThreads, 0, (cudaStream_t)stream>>>(
+        d_field, d_pos, d_out, X, Y, Z, depth);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         g_parse_error = std::string("fr_interpolate_field: ") + cudaGetErrorString(e);

@@ -123,3 +123,17 @@ def test_warp_adjoint_over_sizes(cuda, dims):
                 assert np.abs(pb.cpu().numpy() - pb64).max() <= 1e-5 * max(1.0, np.abs(pb64).max())
             if want_img:
                 assert np.abs(ib.cpu().numpy() - ib64).max() <= 1e-5 * max(1.0, np.abs(ib64).max())
+
+
+@pytest.mark.parametrize("dims", [(7, 9, 3001), (1, 3, 70001), (24, 24, 301), (601, 17, 40), (31, 33, 700)])
+def test_field_sampling_columns_of_narrow_volumes(cuda, dims):
+    """fr_interpolate_field where a block's columns run on over several slices and their last layer is
+    shorter than the others: the oracle's bits."""
+    from fastreg_gb300 import interpolate_field
+    X, Y, Z = dims
+    r = np.random.Generator(np.random.PCG64(19))
+    field = r.normal(0, 1, (3, Z, Y, X)).astype(np.float32)
+    grid = np.stack(np.meshgrid(np.arange(Z), np.arange(Y), np.arange(X), indexing="ij")[::-1]).astype(np.float32)
+    for pos in (grid + np.float32(0.25), grid + r.uniform(-2, 2, grid.shape).astype(np.float32)):
+        assert_bitexact(interpolate_field(_to(cuda, field), _to(cuda, pos)).cpu().numpy(),
+                        O.interpolate_field(field, pos), f"field {dims}")
