@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "../../include/fastreg_gb300.h"
+#include "fr_columns.h"
 #include "fr_common.cuh"
 #include "fr_kernels.h"
 #include "fr_limits.h"
@@ -41,7 +42,6 @@ struct AdjPair {
     int X, Y, Z, Xp, XYp;  // extents, row and slice pitch
     int N;                 // XYp * Z
     long long NT;          // plane stride of vector fields
-    int depth;             // slices per tile of the column kernels
 };
 
 // The caller's fields into the packed workspace: S, T, phi = identity, m = v0; pad columns zero.
@@ -183,21 +183,21 @@ __device__ __forceinline__ void scatter_face_warp(float4* F, int b, const float3
 // phi' = phi + m'(phi): pbar += (dm'/dphi)^T pbar (in place: a voxel reads only its own), mbar +=
 // scatter(w * pbar).
 //
-// A thread owns a column of a 32 x 8 x depth tile.  The reductions bound the kernel (about one lane's
+// A thread owns a column (Columns).  The reductions bound the kernel (about one lane's
 // reduction a cycle and SM whatever its width), so they are made few and wide: mbar is
 // interleaved, a 16-byte reduction per corner serves the three components; neighbouring lanes
 // share corners (scatter_face_warp); and the upper face of a voxel's cell, which is the lower
 // face of the next slice's cell where the cell moves up by exactly one slice, is held back and
 // added there.  The gathered corners are kept the same way, as in sob_pass_b_kernel.  On the
 // 128^3 pair 40 us; with one 4-byte reduction per corner and component, lanes merged, 144 us.
-__global__ void __launch_bounds__(256) adj_update_kernel(AdjPair A, const float* phi,
-                                                         const float* mn, float* pbar, float4* mbar) {
+template <bool LAYERED>
+__global__ void __launch_bounds__(256) adj_update_kernel(AdjPair A, Columns C, const float* phi, const float* mn,
+                                                         float* pbar, float4* mbar) {
     pdl_wait();
     const Pair P = as_pair(A);
-    const int nx = (A.X + kTileX - 1) / kTileX, ny = (A.Y + kTileY - 1) / kTileY;
-    const int x = (blockIdx.x % nx) * kTileX + (threadIdx.x & 31), y = (blockIdx.x / nx % ny) * kTileY + (threadIdx.x >> 5);
-    const int z0 = (int)(blockIdx.x / (nx * ny)) * A.depth, z1 = min(z0 + A.depth, A.Z);
-    const bool act = x < A.X && y < A.Y;
+    int x, y, z0, z1;
+    C.place<LAYERED>(blockIdx.x, threadIdx.x, A.Z, x, y, z0, z1);
+    const bool act = x < A.X && y < A.Y && (!LAYERED || z0 < z1);
     const int Xp = A.Xp, XY = A.XYp;
     int i = act ? x + Xp * y + XY * z0 : 0;
     float f[3][8];
@@ -322,25 +322,25 @@ __device__ __forceinline__ double lambda_sum_f64(const AdjPair& A, const float* 
 }
 
 // g = (S(phi) - T) dS(phi) + lambda lap(phi - x): pbar += lambda lap^T(gbar) + (gbar . dS) dS + r H
-// gbar; lambda_bar += gbar . lap.  A thread owns a column of a 32 x 8 x depth tile; its own
+// gbar; lambda_bar += gbar . lap.  A thread owns a column (Columns); its own
 // column of phi and gbar stays in registers from slice to slice, the neighbours along x and y
 // come through L1, and the Laplacians' terms across a z face are formed once (sob_grad_kernel).
 // The kernel waits on its loads, so all of a voxel's are issued before the arithmetic (64 us on
 // the 128^3 pair when each neighbour was loaded where it was used, 46 us now); lambda_bar is
 // summed in compensated FP32 per thread and in FP64 beyond, as the FP64 pipe of this GPU takes
 // 16 cycles per warp and operation (78 us with six FP64 operations and six conversions a voxel).
-__global__ void __launch_bounds__(256, 5) adj_grad_kernel(AdjPair A, const float* __restrict__ S, const float* __restrict__ T,
-                                                       const float* phi, float lambda,
-                                                       const float* gbar, float* pbar, double* lbar) {
+template <bool LAYERED>
+__global__ void __launch_bounds__(256, LAYERED ? 3 : 5) adj_grad_kernel(AdjPair A, Columns C, const float* __restrict__ S,
+                                                          const float* __restrict__ T, const float* phi, float lambda,
+                                                          const float* gbar, float* pbar, double* lbar) {
     pdl_wait();
     __shared__ double red[32];
     const Pair P = as_pair(A);
-    const int nx = (A.X + kTileX - 1) / kTileX, ny = (A.Y + kTileY - 1) / kTileY;
-    const int x = (blockIdx.x % nx) * kTileX + (threadIdx.x & 31), y = (blockIdx.x / nx % ny) * kTileY + (threadIdx.x >> 5);
-    const int z0 = (int)(blockIdx.x / (nx * ny)) * A.depth, z1 = min(z0 + A.depth, A.Z);
+    int x, y, z0, z1;
+    C.place<LAYERED>(blockIdx.x, threadIdx.x, A.Z, x, y, z0, z1);
     const int Xp = A.Xp, XY = A.XYp;
     double lsum = 0.0;
-    if (x < A.X && y < A.Y) {
+    if (x < A.X && y < A.Y && (!LAYERED || z0 < z1)) {
         const bool xl = x > 0, xr = x < A.X - 1, yl = y > 0, yr = y < A.Y - 1;
         int i = x + Xp * y + XY * z0;
         float ls = 0.f, lc = 0.f;
@@ -524,28 +524,33 @@ extern "C" int fr_sobolev_loss_grad(const float* d_T, const float* d_S, const in
         return FR_ERR_CUDA;
     }
     const int R = smooth_width / 2;
-    // Tiles of the gradient, the smoothing, the update and the transposed smoothing (the update's
-    // also give the reverse kernels' columns).  A tile of d slices takes d + extra steps; blocks
+    // Tiles of the gradient, the smoothing, the update and the transposed smoothing, and the reverse
+    // kernels' columns.  A tile of d slices takes d + extra steps; blocks
     // beyond `per_sm` per SM slow one another down instead of filling idle issue slots.  With the
     // blocks per SM below the depth chosen is within 4% of the best one measured at 45x54x45,
     // 64^3, 96^3 and 128^3 (20 iterations); the column kernels gain from many small tiles (128^3:
     // 6.15 ms at 6 slices, 6.48 at 13), so theirs are held to 6 slices.
+    auto best_depth = [&](auto blocks, int per_sm, int extra, int most, double* cost) {
+        int best = 1;
+        *cost = 1e300;
+        for (int d = 1; d <= std::min(A.Z, most); ++d) {
+            const double c = std::max(1.0, (double)blocks(d) / ((double)sms * per_sm)) * (d + extra);
+            if (c < *cost) {
+                *cost = c;
+                best = d;
+            }
+        }
+        return best;
+    };
     struct Cut {
         int rows, depth, count;
     };
     auto cut = [&](int per_sm, int rows, int extra, int most, double* cost) {
         const long long cols = (long long)((A.X + kTileX - 1) / kTileX) * ((A.Y + rows - 1) / rows);
-        Cut best{rows, 1, 0};
-        *cost = 1e300;
-        for (int d = 1; d <= std::min(A.Z, most); ++d) {
-            const long long tiles = cols * ((A.Z + d - 1) / d);
-            const double c = std::max(1.0, (double)tiles / ((double)sms * per_sm)) * (d + extra) * (rows + extra);
-            if (c < *cost) {
-                *cost = c;
-                best = Cut{rows, d, (int)tiles};
-            }
-        }
-        return best;
+        auto tiles = [&](int d) { return cols * ((A.Z + d - 1) / d); };
+        const int d = best_depth(tiles, per_sm, extra, most, cost);
+        *cost *= rows + extra;
+        return Cut{rows, d, (int)tiles(d)};
     };
     double cost = 0.0, cost_tall = 0.0;
     Cut cuts[4];
@@ -562,7 +567,13 @@ extern "C" int fr_sobolev_loss_grad(const float* d_T, const float* d_S, const in
     };
     const bool tall = split ? slices(true).count >= 2 * sms : cost_tall < cost;
     cuts[1] = cuts[3] = split ? slices(tall) : tall ? high : low;
-    A.depth = cuts[2].depth;
+    Columns columns(A.Xp, A.X, A.Y);
+    columns.depth = best_depth(
+        [&](int d) {
+            columns.depth = d;
+            return columns.blocks(A.Z);
+        },
+        4, 1, 6, &cost);
 
     // the workspace: checkpoints (phi, m) x nseg, the states of a segment (phi, m) x ck, two
     // working states, g, gbar, pbar, the interleaved mbar, S and T; and a small head
@@ -622,7 +633,10 @@ extern "C" int fr_sobolev_loss_grad(const float* d_T, const float* d_S, const in
     gaussian_taps(smooth_sigma, smooth_width, a.taps);
     a.radius = R;
     fold_weights(a.taps, R, a.fold);
-    const int grid = grid_for(A.N), columns = cuts[2].count;
+    const int grid = grid_for(A.N), column_blocks = (int)columns.blocks(A.Z);
+    const bool layered = columns.layers() > 1;
+    const void* update_fn = layered ? (const void*)adj_update_kernel<true> : (const void*)adj_update_kernel<false>;
+    const void* grad_fn = layered ? (const void*)adj_grad_kernel<true> : (const void*)adj_grad_kernel<false>;
     int rc = FR_OK;
     auto ok = [&](cudaError_t e) {
         if (e != cudaSuccess) rc = FR_ERR_CUDA;
@@ -691,10 +705,10 @@ extern "C" int fr_sobolev_loss_grad(const float* d_T, const float* d_S, const in
                 const float* phik = k == s0 ? ckpt[q].phi : seg[k - s0 - 1].phi;
                 // a segment's last state is the next one's checkpoint
                 const float* mn = k == s1 - 1 && q < nseg - 1 ? ckpt[q + 1].m : seg[k - s0].m;
-                reverse((const void*)adj_update_kernel, columns, A, phik, mn, pbar, mbar);
+                reverse(update_fn, column_blocks, A, columns, phik, mn, pbar, mbar);
                 reverse((const void*)adj_momentum_kernel, grid, A, damping, step, mbar, g);
                 smooth_adjoint();
-                reverse((const void*)adj_grad_kernel, columns, A, Sp, Tp, phik, lambda, gbar, pbar, dd + 1);
+                reverse(grad_fn, column_blocks, A, columns, Sp, Tp, phik, lambda, gbar, pbar, dd + 1);
             }
         }
         reverse((const void*)adj_unpack_kernel, grid, A, mbar, d_grad_v0);
@@ -737,20 +751,20 @@ __device__ __forceinline__ void scatter_face_warp(float* F, int b, const float v
 }
 
 // pos_bar = wbar * d img/d pos, img_bar += the trilinear weights times wbar, on the caller's
-// unpadded planes.  A thread owns a column of a 32 x 8 x depth tile: the corners and the upper
+// unpadded planes.  A thread owns a column (Columns): the corners and the upper
 // face of a cell that the next slice's cell stands on are kept and held back as in
 // adj_update_kernel, as the reductions bound the kernel: 57 us on 160x192x160, where eight
 // corners per voxel, lanes merged, took 83 us.
-__global__ void __launch_bounds__(256) warp_adjoint_kernel(Pair P, int depth, const float* __restrict__ pos,
+template <bool LAYERED>
+__global__ void __launch_bounds__(256) warp_adjoint_kernel(Pair P, Columns C, const float* __restrict__ pos,
                                                            const float* __restrict__ img,
                                                            const float* __restrict__ wbar, float* pos_bar,
                                                            float* img_bar) {
     const int X = P.X, XY = P.X * P.Y;
     const long long N = P.N;
-    const int nx = (P.X + kTileX - 1) / kTileX, ny = (P.Y + kTileY - 1) / kTileY;
-    const int x = (blockIdx.x % nx) * kTileX + (threadIdx.x & 31), y = (blockIdx.x / nx % ny) * kTileY + (threadIdx.x >> 5);
-    const int z0 = (int)(blockIdx.x / (nx * ny)) * depth, z1 = min(z0 + depth, P.Z);
-    const bool act = x < P.X && y < P.Y;
+    int x, y, z0, z1;
+    C.place<LAYERED>(blockIdx.x, threadIdx.x, P.Z, x, y, z0, z1);
+    const bool act = x < P.X && y < P.Y && (!LAYERED || z0 < z1);
     int i = act ? x + X * y + XY * z0 : 0;
     float f[8] = {}, held[4] = {};
     int above = -1;  // base of the cell above the previous slice's cell (-1: none)
@@ -834,13 +848,13 @@ extern "C" int fr_warp_adjoint(const float* d_pos, const float* d_img, const flo
     }
     // long columns hold more faces back, short ones fill the GPU: up to 16 slices while there are
     // eight blocks per SM
-    const long long cols = (long long)((P.X + kTileX - 1) / kTileX) * ((P.Y + kTileY - 1) / kTileY);
+    Columns C(P.X, P.X, P.Y);
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int depth = (int)std::max(1LL, std::min(16LL, cols * P.Z / (8LL * std::max(sms, 1))));
-    const long long blocks = cols * ((P.Z + depth - 1) / depth);
-    warp_adjoint_kernel<<<(unsigned)blocks, 256, 0, s>>>(P, depth, d_pos, d_img, d_wbar, d_pos_bar, d_img_bar);
+    C.depth = (int)std::max(1LL, std::min(16LL, C.blocks(P.Z) / (8LL * std::max(sms, 1))));
+    auto fn = C.layers() > 1 ? warp_adjoint_kernel<true> : warp_adjoint_kernel<false>;
+    fn<<<(unsigned)C.blocks(P.Z), 256, 0, s>>>(P, C, d_pos, d_img, d_wbar, d_pos_bar, d_img_bar);
     if (cudaGetLastError() != cudaSuccess) {
         set_global_error("fr_warp_adjoint: launch failed");
         return FR_ERR_CUDA;

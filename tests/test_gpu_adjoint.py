@@ -298,3 +298,11 @@ def test_lambda_gradient_outside_the_fp32_range(cuda, scale, step, width, prec, 
     J_o, _, gl_o = O.sob_loss_grad(P, d["T"], d["S"], v0, 0.2, 2, True, prec=prec)
     assert abs(J - J_o) <= 1e-5 * abs(J_o)
     assert np.isfinite(gl) and abs(gl - gl_o) <= tol * abs(gl_o), (gl, gl_o)
+
+
+@pytest.mark.parametrize("dims,width,K,ck", [((36, 36, 20), 5, 3, 2), ((5, 140, 33), 7, 3, 3), ((4, 61, 150), 3, 2, 2),
+                                             ((4, 4, 900), 5, 3, 2), ((7, 9, 300), 9, 3, 1)])
+def test_loss_gradient_of_narrow_volumes(cuda, dims, width, K, ck):
+    """The reverse kernels where their blocks are less than 32 columns wide or hold several layers of
+    columns: as test_loss_gradient_over_sizes_and_widths."""
+    test_loss_gradient_over_sizes_and_widths(cuda, dims, width, K, ck)

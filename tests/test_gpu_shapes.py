@@ -137,3 +137,11 @@ def test_field_sampling_columns_of_narrow_volumes(cuda, dims):
     for pos in (grid + np.float32(0.25), grid + r.uniform(-2, 2, grid.shape).astype(np.float32)):
         assert_bitexact(interpolate_field(_to(cuda, field), _to(cuda, pos)).cpu().numpy(),
                         O.interpolate_field(field, pos), f"field {dims}")
+
+
+@pytest.mark.parametrize("dims", [(5, 300, 301), (16, 31, 20), (33, 33, 100), (3, 130, 9), (4, 4, 20001), (2, 3, 5000),
+                                  (15, 9, 700)])
+def test_warp_adjoint_of_narrow_volumes(cuda, dims):
+    """fr_warp_adjoint where its blocks are less than 32 columns wide (16 x 16, 8 x 32, 4 x 64) or hold
+    several layers of columns, the last of them shorter or empty: as test_warp_adjoint_over_sizes."""
+    test_warp_adjoint_over_sizes(cuda, dims)
