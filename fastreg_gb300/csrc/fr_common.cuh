@@ -115,25 +115,6 @@ __device__ __forceinline__ float tri_unchecked(const float* __restrict__ F, cons
                   lerpf_(lerpf_(f011, f010, cl.c), lerpf_(f001, f000, cl.c), cl.b), cl.a);
 }
 
-// Trilinear sample with get_global_idx addressing (include/cuda/cuda_utils.hpp:31-37,
-// 109-136): a corner outside the grid reads element 0 of the field.
-__device__ __forceinline__ float tri_checked(const float* __restrict__ F, const Pair& P, const Cell& cl) {
-    const long long X = P.Xp, XY = (long long)P.Xp * P.Y;
-    const long long b = cl.base;
-    const bool ox = cl.gx + 1 < P.X, oy = cl.gy + 1 < P.Y, oz = cl.gz + 1 < P.Z;
-    const float f0 = __ldg(F);
-    float f000 = __ldg(F + b);
-    float f100 = ox ? __ldg(F + b + 1) : f0;
-    float f010 = oy ? __ldg(F + b + X) : f0;
-    float f001 = oz ? __ldg(F + b + XY) : f0;
-    float f110 = (ox && oy) ? __ldg(F + b + 1 + X) : f0;
-    float f101 = (ox && oz) ? __ldg(F + b + 1 + XY) : f0;
-    float f011 = (oy && oz) ? __ldg(F + b + X + XY) : f0;
-    float f111 = (ox && oy && oz) ? __ldg(F + b + 1 + X + XY) : f0;
-    return lerpf_(lerpf_(lerpf_(f111, f110, cl.c), lerpf_(f101, f100, cl.c), cl.b),
-                  lerpf_(lerpf_(f011, f010, cl.c), lerpf_(f001, f000, cl.c), cl.b), cl.a);
-}
-
 // ---- 32-bit variants used inside one pair (N < 2^31) ----
 
 struct Cell32 {
@@ -211,9 +192,10 @@ __device__ __forceinline__ float tri_unchecked32(const float* __restrict__ F, in
                    __ldg(F + min(b + X, last)), __ldg(F + min(b + XY, last)), __ldg(F + b), cl.a, cl.b, cl.c);
 }
 
-// The three components of a vector field (planes F0, F1, F2) at one cell with
-// tri_checked32's addressing; components 0 and 1 interpolated as one packed pair.  The field is one that
-// the chain of launches writes (chain_load).
+// The three components of a vector field (planes F0, F1, F2) at one cell with get_global_idx
+// addressing (include/cuda/cuda_utils.hpp:31-37, 109-136): a corner outside the grid reads element 0.
+// X, Y, Z: grid extents; Xp, XYp: strides of the array.  Components 0 and 1 are interpolated as one
+// packed pair.  The field is one that the chain of launches writes (chain_load).
 __device__ __forceinline__ void tri_checked32_3(const float* F0, const float* F1,
                                                 const float* F2, int X, int Y, int Z, int Xp, int XYp,
                                                 const Cell32& cl, float out[3]) {
@@ -250,28 +232,6 @@ __device__ __forceinline__ void tri_checked32_3(const float* F0, const float* F1
     trilerp3(f, cl.a, cl.b, cl.c, out);
 }
 
-// tri_checked with 32-bit indices: corners outside the grid read element 0.  X, Y, Z:
-// grid extents; Xp, XYp: strides of the array.
-__device__ __forceinline__ float tri_checked32(const float* __restrict__ F, int X, int Y, int Z, int Xp, int XYp,
-                                               const Cell32& cl) {
-    const int b = cl.base;
-    const bool ox = cl.gx + 1 < X, oy = cl.gy + 1 < Y, oz = cl.gz + 1 < Z;
-    if (ox && oy && oz) {
-        return trilerp(__ldg(F + b + 1 + Xp + XYp), __ldg(F + b + 1 + Xp), __ldg(F + b + 1 + XYp), __ldg(F + b + 1),
-                       __ldg(F + b + Xp + XYp), __ldg(F + b + Xp), __ldg(F + b + XYp), __ldg(F + b), cl.a, cl.b,
-                       cl.c);
-    }
-    const float f0 = __ldg(F);
-    return trilerp((ox && oy && oz) ? __ldg(F + b + 1 + Xp + XYp) : f0, (ox && oy) ? __ldg(F + b + 1 + Xp) : f0,
-                   (ox && oz) ? __ldg(F + b + 1 + XYp) : f0, ox ? __ldg(F + b + 1) : f0,
-                   (oy && oz) ? __ldg(F + b + Xp + XYp) : f0, oy ? __ldg(F + b + Xp) : f0,
-                   oz ? __ldg(F + b + XYp) : f0, __ldg(F + b), cl.a, cl.b, cl.c);
-}
-
-__device__ __forceinline__ float4 lerp4_(float4 v0, float4 v1, float t) {
-    return make_float4(lerpf_(v0.x, v1.x, t), lerpf_(v0.y, v1.y, t), lerpf_(v0.z, v1.z, t), lerpf_(v0.w, v1.w, t));
-}
-
 // tri_unchecked32 on an interleaved 4-channel field (one 16-byte load per corner) that the
 // chain of launches writes (chain_load)
 __device__ __forceinline__ float4 tri_unchecked32_f4(const float4* F, int X, int XY, int N,
@@ -291,7 +251,7 @@ __device__ __forceinline__ float4 tri_unchecked32_f4(const float4* F, int X, int
     }
     const float4 f111 = chain_load(F + o111), f110 = chain_load(F + o110), f101 = chain_load(F + o101), f100 = chain_load(F + o100);
     const float4 f011 = chain_load(F + o011), f010 = chain_load(F + o010), f001 = chain_load(F + o001), f000 = chain_load(F + b);
-    // channels (x, y) and (z, w) as packed pairs: per channel the lerp4_ arithmetic
+    // channels (x, y) and (z, w) as packed pairs: per channel exactly trilerp
     auto lo = [](float4 v) { return make_float2(v.x, v.y); };
     auto hi = [](float4 v) { return make_float2(v.z, v.w); };
     const float2 r0 = trilerp2(lo(f111), lo(f110), lo(f101), lo(f100), lo(f011), lo(f010), lo(f001), lo(f000), cl.a,

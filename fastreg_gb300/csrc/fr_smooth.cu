@@ -400,28 +400,35 @@ const void* smooth_fn(int tma, bool tall) {
                : (const void*)sob_smooth3_kernel<R, false, kShort, kInPlace>;
 }
 
+// nullptr where sob_smooth_split never asks for the form
 template <int R>
 const void* smooth_unrolled_fn(bool transposed, bool tall) {
-    constexpr int kShort = sob_smooth_tile_y(R, false), kTall = sob_smooth_tile_y(R, true);
-    if (transposed)
-        return tall ? (const void*)sob_smooth3_kernel<R, false, kTall, kTranspose>
-                    : (const void*)sob_smooth3_kernel<R, false, kShort, kTranspose>;
-    return tall ? (const void*)sob_smooth3_kernel<R, false, kTall, kOutOfPlace>
-                : (const void*)sob_smooth3_kernel<R, false, kShort, kOutOfPlace>;
+    if constexpr (sob_smooth_ever_one_unrolled(R)) {
+        constexpr int kShort = sob_smooth_tile_y(R, false), kTall = sob_smooth_tile_y(R, true);
+        if (transposed)
+            return tall ? (const void*)sob_smooth3_kernel<R, false, kTall, kTranspose>
+                        : (const void*)sob_smooth3_kernel<R, false, kShort, kTranspose>;
+        return tall ? (const void*)sob_smooth3_kernel<R, false, kTall, kOutOfPlace>
+                    : (const void*)sob_smooth3_kernel<R, false, kShort, kOutOfPlace>;
+    }
+    return nullptr;
 }
 
 template <int R>
 void smooth_split_fns(SmoothForm form, bool tall, const void** planes, const void** z) {
-    constexpr int kShort = sob_smooth_tile_y(R, false), kTall = sob_smooth_tile_y(R, true);
-    if (form == kSmoothTransposed)
-        *planes = tall ? (const void*)sob_smooth3_kernel<R, false, kTall, kPlanesTranspose>
-                       : (const void*)sob_smooth3_kernel<R, false, kShort, kPlanesTranspose>;
-    else
-        *planes = tall ? (const void*)sob_smooth3_kernel<R, false, kTall, kPlanes>
-                       : (const void*)sob_smooth3_kernel<R, false, kShort, kPlanes>;
-    *z = form == kSmoothTransposed ? (const void*)sob_smooth_z_kernel<R, kTranspose>
-         : form == kSmoothUnrolled ? (const void*)sob_smooth_z_kernel<R, kOutOfPlace>
-                                   : (const void*)sob_smooth_z_kernel<R, kInPlace>;
+    *planes = *z = nullptr;
+    if constexpr (sob_smooth_ever_split(R)) {
+        constexpr int kShort = sob_smooth_tile_y(R, false), kTall = sob_smooth_tile_y(R, true);
+        if (form == kSmoothTransposed)
+            *planes = tall ? (const void*)sob_smooth3_kernel<R, false, kTall, kPlanesTranspose>
+                           : (const void*)sob_smooth3_kernel<R, false, kShort, kPlanesTranspose>;
+        else
+            *planes = tall ? (const void*)sob_smooth3_kernel<R, false, kTall, kPlanes>
+                           : (const void*)sob_smooth3_kernel<R, false, kShort, kPlanes>;
+        *z = form == kSmoothTransposed ? (const void*)sob_smooth_z_kernel<R, kTranspose>
+             : form == kSmoothUnrolled ? (const void*)sob_smooth_z_kernel<R, kOutOfPlace>
+                                       : (const void*)sob_smooth_z_kernel<R, kInPlace>;
+    }
 }
 
 }  // namespace

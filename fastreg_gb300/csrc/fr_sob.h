@@ -100,9 +100,14 @@ cudaError_t launch_smooth_split(const SobIterArgs& a, SmoothForm form, bool tall
 // iterations), whose other kernels take more of L2, radius 2: 60x64x60 3.3 -> 3.0 ms; radius 3: 64^3 4.1 ->
 // 3.3, 112^3 the same, 128^3 13.2 -> 14.8; radius 4: 96^3 7.9 -> 6.8, 128^3 14.8 -> 15.4; radius 5: 91x109x91
 // 5.2 -> 4.6, 128^3 19.0 -> 16.5, from 160^3 on one launch (the autotuner times both).
-inline bool sob_smooth_split(int radius, long long N, bool unrolled) {
+constexpr bool sob_smooth_split(int radius, long long N, bool unrolled) {
     return radius >= (unrolled ? 4 : 5) || (radius >= 3 && N <= 3 << 19) || (radius == 2 && N <= 1 << 18);
 }
+// Whether any size is smoothed in two launches, and any unrolled one in one: the forms that fr_smooth.cu instantiates.
+constexpr bool sob_smooth_ever_split(int radius) {
+    return sob_smooth_split(radius, 1, false) || sob_smooth_split(radius, 1, true);
+}
+constexpr bool sob_smooth_ever_one_unrolled(int radius) { return !sob_smooth_split(radius, 1LL << 62, true); }
 // slices per tile of the z filter: as many, up to 32, as leave two blocks for every SM
 inline int sob_smooth_z_depth(long long columns, int Z, int sms) {  // columns: 32 x 8, of all pairs
     const long long d = 3 * columns * Z / (2LL * (sms > 0 ? sms : 1));
