@@ -1700,6 +1700,23 @@ int fr_tile_shape(const fr_handle* h, int k, int* depth, int* blocks_per_sm) {
     return FR_OK;
 }
 
+int fr_set_tile_shape(fr_handle* h, int k, int depth, int blocks_per_sm, int variant) {
+    if (!h) return FR_ERR_INVALID_ARG;
+    if (!h->have_state) return fail(h, FR_ERR_STATE, "fr_set_tile_shape before fr_begin");
+    if (k < 0 || k > 2 || depth < 1 || (blocks_per_sm < 1 && blocks_per_sm != -1))
+        return fail(h, FR_ERR_INVALID_ARG, "fr_set_tile_shape: k = %d, depth = %d, blocks_per_sm = %d", k, depth, blocks_per_sm);
+    const int r = active_roles(h)[k];
+    const std::vector<int> al = allowed_variants(h, r);
+    if (std::find(al.begin(), al.end(), variant) == al.end())
+        return fail(h, FR_ERR_INVALID_ARG, "kernel %d has no form %d with this cohort and STAGING", k, variant);
+    FR_CUDA(h, cudaStreamSynchronize(h->last_stream));  // its kernels read the tables
+    const int rc = build_role(h, r, Shape{depth, blocks_per_sm, variant}, h->last_stream);
+    if (rc != FR_OK) return rc;
+    h->graph_valid = false;  // the captured launches carry the old tables
+    h->tuned = true;
+    return FR_OK;
+}
+
 int fr_tile_staging(const fr_handle* h, int k, int* tma) {
     if (!h || !tma || k < 0 || k > 2) return FR_ERR_INVALID_ARG;
     if (!h->block) return FR_ERR_STATE;

@@ -262,6 +262,12 @@ class FastReg:
             out.append((d.value, b.value))
         return out
 
+    def set_tile_shape(self, k: int, depth: int, blocks_per_sm: int = -1, variant: int = 0) -> None:
+        """Sets the tile shape and form of one of the active solver's three kernels for the current
+        cohort (fr_set_tile_shape); results do not depend on it."""
+        N.check(self.lib.fr_set_tile_shape(self.h, int(k), int(depth), int(blocks_per_sm), int(variant)), self.h,
+                "fr_set_tile_shape")
+
     def tile_staging(self):
         """Per kernel of the active solver, in launch order: "tma" when it stages its
         operands with tensor copies, "cp.async" otherwise."""

@@ -161,6 +161,13 @@ int fr_set_pair_w_reg(fr_handle *h, const float *w_reg, int n);
  * the defaults or the autotuner's choice (AUTOTUNE). */
 int fr_tile_shape(const fr_handle *h, int k, int *depth, int *blocks_per_sm);
 
+/* Sets that shape for the current cohort (after fr_begin or a registration; the next cohort of other
+ * sizes starts from the defaults or the autotuner again) and the form of the kernel, `variant`: bit 0
+ * stages by tensor copies (TMA) instead of cp.async; the smoothing also has bit 1, tall tiles, and bit
+ * 3, two launches.  Results do not depend on any of it.  FR_ERR_INVALID_ARG if kernel k has no such
+ * form with this cohort and STAGING.  Waits for the handle's last call.  No counterpart in the reference. */
+int fr_set_tile_shape(fr_handle *h, int k, int depth, int blocks_per_sm, int variant);
+
 /* How kernel k (as in fr_tile_shape) stages its stencil operands after the last
  * fr_register / fr_begin: *tma = 1 for tensor copies (TMA, cp.async.bulk.tensor), 0 for
  * per-thread 16-byte cp.async; the default or the autotuner's choice.  No counterpart in

@@ -306,3 +306,12 @@ def test_loss_gradient_of_narrow_volumes(cuda, dims, width, K, ck):
     """The reverse kernels where their blocks are less than 32 columns wide or hold several layers of
     columns: as test_loss_gradient_over_sizes_and_widths."""
     test_loss_gradient_over_sizes_and_widths(cuda, dims, width, K, ck)
+
+
+@pytest.mark.parametrize("dims,width", [((97, 61, 50), 5), ((4, 300, 256), 5), ((256, 5, 300), 5), ((300, 256, 4), 5),
+                                        ((4, 640, 641), 7), ((641, 5, 520), 7), ((640, 643, 4), 7), ((13, 11, 9), 3)])
+def test_loss_gradient_smoothed_in_one_launch(cuda, dims, width):
+    """The transposed smoothing as one launch (radius 2 above 2^18 voxels, radius 3 above 3 2^19, radius 1), with
+    each axis in turn shorter than the filter: as test_loss_gradient_over_sizes_and_widths, whose
+    small volumes at radius 2 and 3 and whose volumes from radius 4 are smoothed in two."""
+    test_loss_gradient_over_sizes_and_widths(cuda, dims, width, 2, 2)

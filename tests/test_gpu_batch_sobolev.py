@@ -266,3 +266,38 @@ def test_converged_pairs_keep_their_records(cuda, solver):
     N.check(fr.lib.fr_time_kernels(fr.h, 3, ms, C.byref(nk), None), fr.h, "fr_time_kernels")
     assert records() == before
     fr.close()
+
+
+@pytest.mark.parametrize("width", [1, 3, 5, 7, 9, 11, 13, 15])
+@pytest.mark.parametrize("dims_list", [[(33, 17, 9)], [(70, 4, 21), (5, 34, 16)]])
+def test_every_smoothing_form(cuda, dims_list, width):
+    """Each form of the smoothing that the autotuner may choose between (staging, tile height, one launch or two),
+    set by hand, at every radius and with axes shorter than the filter: the oracle's bits."""
+    from fastreg_gb300._native import FastRegError
+    pairs_np = [images(d, 2500 + 10 * width + k) for k, d in enumerate(dims_list)]
+    kw = dict(no_labels=4, max_iter=3, solver="sobolev", smooth_sigma=0.4 + 0.3 * width, smooth_width=width,
+              damping=0.9, step=0.5, autotune=0)
+    expect = [O.sob_register(Params(volume_dims=d, **kw), p["T"], p["S"]) for d, p in zip(dims_list, pairs_np)]
+    fr = FastReg(Params(volume_dims=dims_list[0], **kw))
+    bufs = [tuple(_to(cuda, p[k]) for k in ("T", "labT", "S", "labS")) for p in pairs_np]
+    fr.begin(bufs)
+    seen = []
+    for variant in range(16):
+        try:
+            fr.set_tile_shape(1, 5, variant=variant)
+        except FastRegError as e:
+            assert e.status == N.FR_ERR_INVALID_ARG
+            continue
+        seen.append(variant)
+        fr.begin(bufs)
+        for it in (1, 2, 3):
+            fr.step(it, 1.0)
+        for k, o in enumerate(expect):
+            what = f"pair {k}, form {variant}, width {width}"
+            assert_bitexact(fr.get_field(N.FR_FIELD_PSI, pair=k).cpu().numpy(), o["phi"], "phi, " + what)
+            assert_bitexact(fr.get_field(N.FR_FIELD_V, pair=k).cpu().numpy(), o["m"], "momentum, " + what)
+    radius = width // 2
+    one = [0, 1, 2, 3] if radius <= 4 else [0, 1]
+    two = [] if radius < 2 else [8, 10] if radius <= 4 else [8]
+    assert seen == one + two, seen
+    fr.close()
