@@ -1749,15 +1749,19 @@ int fr_interpolate_field(const float* d_field, const float* d_pos, const int dim
     if (rc != FR_OK) return rc;
     static std::atomic<int> slots[64];
     const int X = dims[0], Y = dims[1], Z = dims[2];
-    auto blocks_of = [&](long long d) { return ((long long)X * Y * ((Z + d - 1) / d) + frg::kFieldThreads - 1) / frg::kFieldThreads; };
+    const long long XY = (long long)X * Y, per_slice = (XY + frg::kFieldThreads - 1) / frg::kFieldThreads;
+    const bool run_on = per_slice * frg::kFieldThreads * 32 > XY * 33;  // 3% of the threads would be idle
+    auto blocks_of = [&](long long d) {
+        const long long layers = (Z + d - 1) / d;
+        return run_on ? (XY * layers + frg::kFieldThreads - 1) / frg::kFieldThreads : per_slice * layers;
+    };
     // Columns of 16 slices where they make two and a half waves of blocks or more (64.7 us on 182x218x182;
     // 8 take 67.2 us, 24 67.6 us).  Below that the waves count: a wave of d slices takes about d + 1/2, one that
     // fills a share f of the GPU 0.44 + 0.56 f of it (both figures fitted to the times of eight sizes).
     // Against every depth up to 24, on 17 sizes from 33^3 to 193x229x193: within 7% of the best below
     // two and a half waves, within 9% from there to three (176x208x176: 78.1 us, 71.7 us at 21 slices), within
     // 2% above (137x108x173 has 18 slices and one wave; 16 and a second wave of 15 blocks are 15% slower).
-    const long long slots_all = std::max(resident_blocks((const void*)frg::interpolate_field_kernel, slots,
-                                                         frg::kFieldThreads), 1);
+    const long long slots_all = std::max(resident_blocks(frg::interpolate_field_fn(false), slots, frg::kFieldThreads), 1);  // both forms have two blocks per SM
     int depth = 16;
     if (2 * blocks_of(16) < 5 * slots_all) {
         double least = 1e300;
@@ -1770,9 +1774,10 @@ int fr_interpolate_field(const float* d_field, const float* d_pos, const int dim
             }
         }
     }
-    frg::interpolate_field_kernel<<<(unsigned)blocks_of(depth), frg::kFieldThreads, 0, (cudaStream_t)stream>>>(
-        d_field, d_pos, d_out, X, Y, Z, depth);
-    cudaError_t e = cudaGetLastError();
+    void* args[] = {&d_field, &d_pos, &d_out, (void*)&X, (void*)&Y, (void*)&Z, &depth};
+    cudaError_t e = frg::launch_kernel(frg::interpolate_field_fn(run_on), (int)blocks_of(depth), frg::kFieldThreads, 0, args,
+                                       (cudaStream_t)stream, false);
+    cudaGetLastError();
     if (e != cudaSuccess) {
         g_parse_error = std::string("fr_interpolate_field: ") + cudaGetErrorString(e);
         return FR_ERR_CUDA;

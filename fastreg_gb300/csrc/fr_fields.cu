@@ -29,27 +29,37 @@ __global__ void __launch_bounds__(256) estimate_inverse_kernel(const float* __re
     }
 }
 
-// A thread owns a column of `depth` slices; the threads are numbered along the voxels of a slice, then along
-// the columns above (rows and slices run on, so every warp but the last is full whatever the extents).
+// A thread owns a column of `depth` slices, a block kFieldThreads consecutive voxels of a slice (rows run on,
+// so every warp but the last is full and its rows start where its lanes do).  RUN_ON: blocks run on over slices
+// too, into the columns above, where the last block of every slice would be mostly idle (2x2x60000 takes 6.2 us
+// and took 45); the loop is not uniform over the block any more then (182x218x182: 65.5 us instead of 64.9).
 // The kernel is bound by the gathers' trips through L1, several cache lines per load.  Positions
 // are mostly those of a smooth map, so the cell of the next slice is often the one above this
 // slice's: its lower four corners are the upper ones already in registers, and a lane loads
 // 12 corners instead of 24; all are issued before the arithmetic.  64.7 us on 182x218x182 (36
 // bytes per voxel, 39 us at the copy bandwidth); 84 us with three component samples one after
 // the other, 80 us with 24 corners loaded together, 70 us on 32 x 8 tiles with the reuse.
-// With every block on one slice, narrow volumes left its threads idle: 2x2x60000 takes 6.2 us now and took 45.
+template <bool RUN_ON>
 __global__ void __launch_bounds__(kFieldThreads, 2) interpolate_field_kernel(const float* __restrict__ field,
                                                                              const float* __restrict__ pos,
                                                                              float* __restrict__ out, int X, int Y,
                                                                              int Z, int depth) {
     const int N = X * Y * Z, XY = X * Y, last = N - 1;
-    const int t = blockIdx.x * kFieldThreads + threadIdx.x, layer = t / XY;
-    if (layer > (Z - 1) / depth) return;
+    const int per_slice = (XY + kFieldThreads - 1) / kFieldThreads;  // blocks
+    int t = blockIdx.x * kFieldThreads + threadIdx.x, layer = t / XY;
+    if (RUN_ON) {
+        if (layer > (Z - 1) / depth) return;
+        t -= layer * XY;
+    } else {
+        layer = blockIdx.x / per_slice;
+        t -= layer * per_slice * kFieldThreads;
+        if (t >= XY) return;
+    }
     const int z0 = layer * depth, z1 = Z - z0 > depth ? z0 + depth : Z;  // no overflow near 2^31
     const float* __restrict__ p[3] = {pos, pos + N, pos + 2 * (long long)N};
     const float* __restrict__ F[3] = {field, field + N, field + 2 * (long long)N};
     float* const O[3] = {out, out + N, out + 2 * (long long)N};
-    int i = t - layer * XY + XY * z0;
+    int i = t + XY * z0;
     float n[3], f[3][8];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -86,6 +96,10 @@ __global__ void __launch_bounds__(kFieldThreads, 2) interpolate_field_kernel(con
 #pragma unroll
         for (int c = 0; c < 3; ++c) __stcs(O[c] + i, v[c]);
     }
+}
+
+const void* interpolate_field_fn(bool run_on) {
+    return run_on ? (const void*)interpolate_field_kernel<true> : (const void*)interpolate_field_kernel<false>;
 }
 
 }  // namespace frg

@@ -144,6 +144,7 @@ __global__ void warp32_kernel(const float* pos, const float* img, const int16_t*
 // the reference's unused field kernels (fr_fields.cu)
 __global__ void estimate_inverse_kernel(const float* psi, float* psi_inv, int X, int Y, int Z, int sweeps);
 constexpr int kFieldThreads = 512;  // columns per block of interpolate_field_kernel
-__global__ void interpolate_field_kernel(const float* field, const float* pos, float* out, int X, int Y, int Z, int depth);
+// interpolate_field_kernel(field, pos, out, X, Y, Z, depth); run_on: blocks run on over slices
+const void* interpolate_field_fn(bool run_on);
 
 }  // namespace frg
