@@ -18,7 +18,7 @@
 // with a separate input and output state per iteration: a checkpoint or a segment's state is
 // written where it is kept and never copied.  The reverse iteration is four kernels: the
 // update's adjoint, the momentum's, the transposed smoothing (the smoothing kernel's
-// transposed form) and the gradient's.  fr_warp_adjoint works on the caller's unpadded planes.
+// transposed form, or two) and the gradient's.  fr_warp_adjoint works on the caller's unpadded planes.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -189,7 +189,8 @@ __device__ __forceinline__ void scatter_face_warp(float4* F, int b, const float3
 // share corners (scatter_face_warp); and the upper face of a voxel's cell, which is the lower
 // face of the next slice's cell where the cell moves up by exactly one slice, is held back and
 // added there.  The gathered corners are kept the same way, as in sob_pass_b_kernel.  On the
-// 128^3 pair 40 us; with one 4-byte reduction per corner and component, lanes merged, 144 us.
+// 128^3 pair 42 us from a smooth momentum, 75 us from white noise, whose cells share little; with one 4-byte
+// reduction per corner and component, lanes merged, 144 us.
 template <bool LAYERED>
 __global__ void __launch_bounds__(256) adj_update_kernel(AdjPair A, Columns C, const float* phi, const float* mn,
                                                          float* pbar, float4* mbar) {
@@ -325,10 +326,12 @@ __device__ __forceinline__ double lambda_sum_f64(const AdjPair& A, const float* 
 // gbar; lambda_bar += gbar . lap.  A thread owns a column (Columns); its own
 // column of phi and gbar stays in registers from slice to slice, the neighbours along x and y
 // come through L1, and the Laplacians' terms across a z face are formed once (sob_grad_kernel).
-// The kernel waits on its loads, so all of a voxel's are issued before the arithmetic (64 us on
-// the 128^3 pair when each neighbour was loaded where it was used, 46 us now); lambda_bar is
+// The kernel waits on its loads, so a voxel's are issued together (64 us on
+// the 128^3 pair when each neighbour was loaded where it was used), and it is held to five blocks per SM (48
+// registers): 40 us, 46 us with four of 54.  lambda_bar is
 // summed in compensated FP32 per thread and in FP64 beyond, as the FP64 pipe of this GPU takes
-// 16 cycles per warp and operation (78 us with six FP64 operations and six conversions a voxel).
+// 16 cycles per warp and operation (78 us with six FP64 operations and six conversions a voxel); a column with a
+// product outside dot2's range is summed in FP64 (lambda_sum_f64).
 template <bool LAYERED>
 __global__ void __launch_bounds__(256, LAYERED ? 3 : 5) adj_grad_kernel(AdjPair A, Columns C, const float* __restrict__ S,
                                                           const float* __restrict__ T, const float* phi, float lambda,

@@ -39,8 +39,8 @@ enum Role { R_LAP, R_PA, R_PB, R_SG, R_SS, R_SB, R_COUNT };
 struct Shape {
     int depth = 16;  // slices per tile
     int bps = 0;     // blocks per SM (-1: one block per tile, scheduled by the hardware)
-    int variant = 0; // bit 0: staging by per-thread cp.async (0) or TMA tensor copies (1); bit 1: tall
-                     // tiles of the smoothing kernel
+    int variant = 0; // bit 0: staging by per-thread cp.async (0) or TMA tensor copies (1); of the smoothing
+                     // also bit 1: tall tiles, bit 3 (frg::kSplit): two launches
 };
 struct TileSet {
     Shape shape;
@@ -709,7 +709,7 @@ int launch_ref_iter(fr_handle* h, int iter, float t, cudaStream_t s, cudaEvent_t
     return FR_OK;
 }
 
-// kernels launched per iteration (three in either solver)
+// kernels of an iteration that are timed and shaped (three in either solver; the smoothing in two launches is one)
 int kernels_per_iter(const fr_handle*) { return 3; }
 
 frg::SobIterArgs sob_args(fr_handle* h, int iter) {
@@ -943,8 +943,8 @@ int run_registration(fr_handle* h, cudaStream_t s) {
 }
 
 // ---- autotuner ----
-// For each solver kernel, a few tile depths and blocks-per-SM counts are timed on the
-// freshly packed cohort (identity state, iteration 1), the kernel launched alone; the
+// For each solver kernel and each of its forms, a few tile depths and blocks-per-SM counts are timed on the
+// packed cohort after kTuneWarmIters iterations, the kernel launched alone; the
 // fastest shape is kept.  The choice is cached per size class (solver, SM count,
 // smoothing width and the multiset of pair sizes) for the life of the process.  A tile
 // shape changes which block computes a voxel, never how, so results do not depend on it.

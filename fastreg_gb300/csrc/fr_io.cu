@@ -106,7 +106,7 @@ __device__ __forceinline__ float det_true(const float J[3][3]) {
 
 // A thread marches a column of a 32 x 8 x io_depth tile, psi of the slice below, this one and the one
 // above in registers.  It waits on its loads and gathers, so it is held to five blocks per SM (48
-// registers): 197 us on the 182x218x182 pair with the reference solver, 237 us with four; 326 us
+// registers, which spills 22 of them): 197 us on the 182x218x182 pair with the reference solver, 237 us with four; 326 us
 // with 64-bit indices, every neighbour loaded and two blocks of 128 registers.  On the 64^3 pair
 // 21 us with tiles of two slices, 51 us with 16 (64 blocks).
 __global__ void __launch_bounds__(256, 5) finalize_kernel(IoArgs a) {

@@ -132,7 +132,9 @@ __global__ void __launch_bounds__(kSmoothThreads) sob_smooth3_kernel(SobIterArgs
 
     for (int t = blockIdx.x; t < a.ntiles_s && !failed; t += gridDim.x) {
         // The kernels of large cohorts read the table even for a single pair: with the tile and
-        // pair chosen between table and arguments the tall TMA kernel takes 75 instead of 66 us.
+        // pair chosen between table and arguments the tall TMA kernel takes 75 instead of 66 us.  Neither
+        // registers (166, 164) nor blocks per SM (4, 4) tell the two apart; the compiler orders the march differently,
+        // so another compiler may need another choice.
         constexpr bool kTable = MODE == kInPlace && (TMA || TY != sob_smooth_tile_y(R, false));
         Tile tl;
         Pair P;

@@ -200,8 +200,8 @@ int fr_interpolate_field(const float *d_field, const float *d_pos, const int dim
  * NULL, dJ/dv0 (3 planes, device) and dJ/dlambda to *grad_lambda, by hand-written
  * adjoint kernels with the forward states checkpointed every `checkpoint_every`
  * iterations.  d_T, d_S: target and source (N floats each).  Synchronises `stream`.
- * Its device workspace (checkpoints and adjoint fields, about 3 N floats x (2 (iters /
- * checkpoint_every + 1) + 2 checkpoint_every + 8)) is kept per device after the call and
+ * Its device workspace (checkpoints and adjoint fields, about 3 N floats x (2 ceil(iters /
+ * checkpoint_every) + 2 checkpoint_every + 9), N with rows padded to a multiple of 4) is kept per device after the call and
  * reused by later calls of the same or a smaller size; a call made while another host
  * thread's call holds it allocates a private one. */
 int fr_sobolev_loss_grad(const float *d_T, const float *d_S, const int dims[3], const float *d_v0, float lambda,
