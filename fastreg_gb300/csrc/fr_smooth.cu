@@ -338,8 +338,10 @@ __global__ void __launch_bounds__(kSmoothThreads) sob_smooth3_kernel(SobIterArgs
 // 128^3 4.83 -> 4.85; radius 5, 91x109x91 3.76 -> 2.98; radius 7, 128^3 9.04 -> 6.30; radius 1, 64^3
 // 0.95 -> 1.03.  A thread takes kZBatch slices' loads together; bound by their latency.
 constexpr int kZBatch = 4;
+// In place at radius 6 the compiler settles on 40 registers and a load at a time (35 us on 41x195x75); held to five
+// blocks per SM it takes 48 and the batch (31 us), as it does by itself at radius 7.
 template <int R, SmoothMode MODE>
-__global__ void __launch_bounds__(256) sob_smooth_z_kernel(SobIterArgs a) {
+__global__ void __launch_bounds__(256, R == 6 && MODE == kInPlace ? 5 : 0) sob_smooth_z_kernel(SobIterArgs a) {
     pdl_wait();
     constexpr bool ADJ = MODE == kTranspose;
     constexpr int U = kZBatch;
