@@ -191,14 +191,14 @@ __device__ __forceinline__ void scatter_face_warp(float4* F, int b, const float3
 // added there.  The gathered corners are kept the same way, as in sob_pass_b_kernel.  On the
 // 128^3 pair 42 us from a smooth momentum, 75 us from white noise, whose cells share little; with one 4-byte
 // reduction per corner and component, lanes merged, 144 us.
-template <bool LAYERED>
+template <int SHAPE>
 __global__ void __launch_bounds__(256) adj_update_kernel(AdjPair A, Columns C, const float* phi, const float* mn,
                                                          float* pbar, float4* mbar) {
     pdl_wait();
     const Pair P = as_pair(A);
     int x, y, z0, z1;
-    C.place<LAYERED>(blockIdx.x, threadIdx.x, A.Z, x, y, z0, z1);
-    const bool act = x < A.X && y < A.Y && (!LAYERED || z0 < z1);
+    C.place<SHAPE>(blockIdx.x, threadIdx.x, A.Z, x, y, z0, z1);
+    const bool act = x < A.X && y < A.Y && (SHAPE != kLayeredColumns || z0 < z1);
     const int Xp = A.Xp, XY = A.XYp;
     int i = act ? x + Xp * y + XY * z0 : 0;
     float f[3][8];
@@ -332,18 +332,18 @@ __device__ __forceinline__ double lambda_sum_f64(const AdjPair& A, const float* 
 // summed in compensated FP32 per thread and in FP64 beyond, as the FP64 pipe of this GPU takes
 // 16 cycles per warp and operation (78 us with six FP64 operations and six conversions a voxel); a column with a
 // product outside dot2's range is summed in FP64 (lambda_sum_f64).
-template <bool LAYERED>
-__global__ void __launch_bounds__(256, LAYERED ? 3 : 5) adj_grad_kernel(AdjPair A, Columns C, const float* __restrict__ S,
+template <int SHAPE>
+__global__ void __launch_bounds__(256, SHAPE == kLayeredColumns ? 3 : 5) adj_grad_kernel(AdjPair A, Columns C, const float* __restrict__ S,
                                                           const float* __restrict__ T, const float* phi, float lambda,
                                                           const float* gbar, float* pbar, double* lbar) {
     pdl_wait();
     __shared__ double red[32];
     const Pair P = as_pair(A);
     int x, y, z0, z1;
-    C.place<LAYERED>(blockIdx.x, threadIdx.x, A.Z, x, y, z0, z1);
+    C.place<SHAPE>(blockIdx.x, threadIdx.x, A.Z, x, y, z0, z1);
     const int Xp = A.Xp, XY = A.XYp;
     double lsum = 0.0;
-    if (x < A.X && y < A.Y && (!LAYERED || z0 < z1)) {
+    if (x < A.X && y < A.Y && (SHAPE != kLayeredColumns || z0 < z1)) {
         const bool xl = x > 0, xr = x < A.X - 1, yl = y > 0, yr = y < A.Y - 1;
         int i = x + Xp * y + XY * z0;
         float ls = 0.f, lc = 0.f;
@@ -637,9 +637,11 @@ extern "C" int fr_sobolev_loss_grad(const float* d_T, const float* d_S, const in
     a.radius = R;
     fold_weights(a.taps, R, a.fold);
     const int grid = grid_for(A.N), column_blocks = (int)columns.blocks(A.Z);
-    const bool layered = columns.layers() > 1;
-    const void* update_fn = layered ? (const void*)adj_update_kernel<true> : (const void*)adj_update_kernel<false>;
-    const void* grad_fn = layered ? (const void*)adj_grad_kernel<true> : (const void*)adj_grad_kernel<false>;
+    const void* const update_fns[] = {(const void*)adj_update_kernel<kTileColumns>, (const void*)adj_update_kernel<kFlatColumns>,
+                                      (const void*)adj_update_kernel<kLayeredColumns>};
+    const void* const grad_fns[] = {(const void*)adj_grad_kernel<kTileColumns>, (const void*)adj_grad_kernel<kFlatColumns>,
+                                    (const void*)adj_grad_kernel<kLayeredColumns>};
+    const void *update_fn = update_fns[columns.shape], *grad_fn = grad_fns[columns.shape];
     int rc = FR_OK;
     auto ok = [&](cudaError_t e) {
         if (e != cudaSuccess) rc = FR_ERR_CUDA;
@@ -758,7 +760,7 @@ __device__ __forceinline__ void scatter_face_warp(float* F, int b, const float v
 // face of a cell that the next slice's cell stands on are kept and held back as in
 // adj_update_kernel, as the reductions bound the kernel: 57 us on 160x192x160, where eight
 // corners per voxel, lanes merged, took 83 us.
-template <bool LAYERED>
+template <int SHAPE>
 __global__ void __launch_bounds__(256) warp_adjoint_kernel(Pair P, Columns C, const float* __restrict__ pos,
                                                            const float* __restrict__ img,
                                                            const float* __restrict__ wbar, float* pos_bar,
@@ -766,8 +768,8 @@ __global__ void __launch_bounds__(256) warp_adjoint_kernel(Pair P, Columns C, co
     const int X = P.X, XY = P.X * P.Y;
     const long long N = P.N;
     int x, y, z0, z1;
-    C.place<LAYERED>(blockIdx.x, threadIdx.x, P.Z, x, y, z0, z1);
-    const bool act = x < P.X && y < P.Y && (!LAYERED || z0 < z1);
+    C.place<SHAPE>(blockIdx.x, threadIdx.x, P.Z, x, y, z0, z1);
+    const bool act = x < P.X && y < P.Y && (SHAPE != kLayeredColumns || z0 < z1);
     int i = act ? x + X * y + XY * z0 : 0;
     float f[8] = {}, held[4] = {};
     int above = -1;  // base of the cell above the previous slice's cell (-1: none)
@@ -856,7 +858,9 @@ extern "C" int fr_warp_adjoint(const float* d_pos, const float* d_img, const flo
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     C.depth = (int)std::max(1LL, std::min(16LL, C.blocks(P.Z) / (8LL * std::max(sms, 1))));
-    auto fn = C.layers() > 1 ? warp_adjoint_kernel<true> : warp_adjoint_kernel<false>;
+    auto fn = C.shape == kTileColumns   ? warp_adjoint_kernel<kTileColumns>
+              : C.shape == kFlatColumns ? warp_adjoint_kernel<kFlatColumns>
+                                        : warp_adjoint_kernel<kLayeredColumns>;
     fn<<<(unsigned)C.blocks(P.Z), 256, 0, s>>>(P, C, d_pos, d_img, d_wbar, d_pos_bar, d_img_bar);
     if (cudaGetLastError() != cudaSuccess) {
         set_global_error("fr_warp_adjoint: launch failed");

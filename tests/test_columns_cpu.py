@@ -24,22 +24,20 @@ int main() {
                     for (int depth : {1, 2, 6, 16}) {
                         frg::Columns C(pitch, X, Y);
                         C.depth = depth;
-                        const bool layered = C.layers() > 1;
-                        seen_kind |= layered ? 4 : C.lx == 5 ? 1 : 2;
+                        seen_kind |= 1 << C.shape;
+                        auto place = [&](int b, int t, int& x, int& y, int& z0, int& z1) {
+                            if (C.shape == frg::kTileColumns) C.place<frg::kTileColumns>(b, t, Z, x, y, z0, z1);
+                            else if (C.shape == frg::kFlatColumns) C.place<frg::kFlatColumns>(b, t, Z, x, y, z0, z1);
+                            else C.place<frg::kLayeredColumns>(b, t, Z, x, y, z0, z1);
+                        };
                         std::vector<char> seen((size_t)X * Y * Z, 0);
                         for (int b = 0; b < C.blocks(Z); ++b)
                             for (int t = 0; t < 256; ++t) {
                                 int x, y, z0, z1;
-                                if (layered)
-                                    C.place<true>(b, t, Z, x, y, z0, z1);
-                                else
-                                    C.place<false>(b, t, Z, x, y, z0, z1);
+                                place(b, t, x, y, z0, z1);
                                 if (x < 0 || y < 0 || z0 < 0 || z1 > Z) return std::printf("outside\n"), 1;
                                 int x0, y0, a0, a1;  // a warp's lanes share their slices
-                                if (layered)
-                                    C.place<true>(b, t & ~31, Z, x0, y0, a0, a1);
-                                else
-                                    C.place<false>(b, t & ~31, Z, x0, y0, a0, a1);
+                                place(b, t & ~31, x0, y0, a0, a1);
                                 if (a0 != z0 || a1 != z1) return std::printf("a warp of two layers\n"), 1;
                                 if (x >= X || y >= Y) continue;
                                 for (int z = z0; z < z1; ++z)
